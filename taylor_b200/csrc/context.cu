@@ -160,13 +160,14 @@ __global__ void k_renumber_cols(int32_t n, const int32_t* __restrict__ perm, con
   for (int64_t k = lane; k < len; k += 32) col1[b0 + k] = iperm[col0[a0 + k]];
 }
 // row sums of the float-rounded packed gradients (the mixed path's sum_J g)
-__global__ void k_rowsum_pk32(int32_t n, const int64_t* __restrict__ rowptr, const float4* __restrict__ pk,
-                              double* __restrict__ out) {
+__global__ void k_rowsum_pk32(int32_t n, const int64_t* __restrict__ rowptr, const int64_t* __restrict__ rbase,
+                              const float4* __restrict__ pk, double* __restrict__ out) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   double a = 0.0, b = 0.0, c = 0.0;
-  for (int64_t p = rowptr[i]; p < rowptr[i + 1]; ++p) {
-    const float4 v = pk[p];
+  const int len = (int)(rowptr[i + 1] - rowptr[i]);
+  for (int k = 0; k < len; ++k) {
+    const float4 v = pk[rbase[i] + 32 * (k >> 2) + (k & 3)];
     a += (double)v.x; b += (double)v.y; c += (double)v.z;
   }
   out[3 * i] = a; out[3 * i + 1] = b; out[3 * i + 2] = c;
@@ -581,7 +582,7 @@ static TiledForceArgs force_args(Ctx* c, double dt, int mode, int predict) {
   TiledForceArgs f{};
   f.n = c->n; f.R = c->ct.R; f.ntiles = c->ct.ntiles; f.jmax = c->ct.jmax; f.maxcnt = c->ct.maxcnt;
   f.recmax = c->ct.recmax;
-  f.jset = c->ct.jset; f.jcnt = c->ct.jcnt; f.colptr = c->csr.colptr;
+  f.jset = c->ct.jset; f.jcnt = c->ct.jcnt; f.colptr = c->csr.colptr; f.sv = c->ct.view();
   f.pk = mixed ? c->tpk32 : c->tpk64;
   f.tshp = mixed ? c->tshp32 : c->tshp; f.tmat = c->tmat; f.has_body = c->has_body; f.predict = predict;
   f.ebc = c->ebc; f.mass = c->mass; f.matidx = c->matidx; f.mats = c->mats; f.body_id = c->body_id;
@@ -1560,11 +1561,13 @@ int mega_search_and_shapes(int64_t h, int32_t* gn, int32_t* gstart, int32_t* gst
     if (packed) {  // the row tiles first: the records carry the tile ranks
       if ((r = configure_tiled_kernels())) return r;
       r = build_tiles(c->s, n, c->csr.rowptr, c->csr.col, m, c->csr.gmaxn, c->rt, c->nbpool, nullptr);
-      if (r) return r;
+      if (r || (r = build_slices(c->s, n, c->csr.rowptr, c->rt, c->nbpool))) return r;
       float4* a = nullptr;
-      MEGA_ALLOC(c->nbpool, a, m);
+      MEGA_ALLOC(c->nbpool, a, c->rt.nrec);
       c->pk32 = a;
-      r = rk_shapes_packed(c->s, c->p, n, c->coo, c->win, c->ebc_nodes, c->csr, c->rt.lidx, c->shp, a, c->status);
+      if ((r = pad_records32(c->s, n, c->rt, c->csr.rowptr, a))) return r;
+      r = rk_shapes_packed(c->s, c->p, n, c->coo, c->win, c->ebc_nodes, c->csr, c->rt.lidx, c->rt.rbase, c->shp, a,
+                           c->status);
     } else {
       r = rk_shapes(c->s, c->p, n, c->coo, c->win, c->ebc_nodes, c->csr, c->shp, g1x, g1y, g1z, c->status);
     }
@@ -1591,21 +1594,21 @@ int mega_search_and_shapes(int64_t h, int32_t* gn, int32_t* gstart, int32_t* gst
   tr.mark("transpose");
   if (!packed) {
     r = build_tiles(c->s, n, c->csr.rowptr, c->csr.col, m, c->csr.gmaxn, c->rt, c->nbpool, nullptr);
-    if (r) return r;
+    if (r || (r = build_slices(c->s, n, c->csr.rowptr, c->rt, c->nbpool))) return r;
   }
   tr.mark("row_tiles");
   // the longest column bounds a column tile's set from below
   r = build_tiles(c->s, n, c->csr.colptr, c->csr.trow, m, c->csr.gmaxc, c->ct, c->nbpool, nullptr);
-  if (r) return r;
+  if (r || (r = build_slices(c->s, n, c->csr.colptr, c->ct, c->nbpool))) return r;
   tr.mark("column_tiles");
   if (c->prec_mask & 1) {
-    double *a = nullptr, *b = nullptr;  // 4 doubles per entry
-    MEGA_ALLOC(c->nbpool, a, 4 * m);
-    MEGA_ALLOC(c->nbpool, b, 4 * m);
+    unsigned char *a = nullptr, *b = nullptr;  // 26 bytes per record
+    MEGA_ALLOC(c->nbpool, a, 26 * c->rt.nrec);
+    MEGA_ALLOC(c->nbpool, b, 26 * c->ct.nrec);
     c->pk64 = a;
     c->tpk64 = b;
-    if ((r = pack_entries(c->s, m, c->rt.lidx, g1x, g1y, g1z, nullptr, true, c->pk64)) ||
-        (r = pack_entries(c->s, m, c->ct.lidx, g1x, g1y, g1z, c->csr.tpos, true, c->tpk64)))
+    if ((r = pack_entries(c->s, n, c->rt, c->csr.rowptr, g1x, g1y, g1z, nullptr, true, c->pk64)) ||
+        (r = pack_entries(c->s, n, c->ct, c->csr.colptr, g1x, g1y, g1z, c->csr.tpos, true, c->tpk64)))
       return r;
     MEGA_ALLOC(c->nbpool, c->sdphi, 3 * (int64_t)n);
     k_rowsum3<double><<<grid_for(n, 256), 256, 0, c->s>>>(n, c->csr.rowptr, g1x, g1y, g1z, c->sdphi);
@@ -1616,20 +1619,23 @@ int mega_search_and_shapes(int64_t h, int32_t* gn, int32_t* gstart, int32_t* gst
   // once for the gathers' shared-memory banks (bank_layout).
   if (c->prec_mask & 2) {
     float4* b = nullptr;
-    MEGA_ALLOC(c->nbpool, b, m);
+    MEGA_ALLOC(c->nbpool, b, c->ct.nrec);
     c->tpk32 = b;
     if (packed) {
-      if ((r = pack_transposed32(c->s, m, c->ct.lidx, (const float4*)c->pk32, c->csr.tpos, b))) return r;
+      if ((r = pack_transposed32(c->s, n, c->ct, c->csr.colptr, (const float4*)c->pk32, c->csr.trow, c->csr.tpos,
+                                 c->csr.rowptr, c->rt, b)))
+        return r;
     } else {
       float4* a = nullptr;
-      MEGA_ALLOC(c->nbpool, a, m);
+      MEGA_ALLOC(c->nbpool, a, c->rt.nrec);
       c->pk32 = a;
-      if ((r = pack_entries(c->s, m, c->rt.lidx, g1x, g1y, g1z, nullptr, false, c->pk32)) ||
-          (r = pack_entries(c->s, m, c->ct.lidx, g1x, g1y, g1z, c->csr.tpos, false, c->tpk32)))
+      if ((r = pack_entries(c->s, n, c->rt, c->csr.rowptr, g1x, g1y, g1z, nullptr, false, c->pk32)) ||
+          (r = pack_entries(c->s, n, c->ct, c->csr.colptr, g1x, g1y, g1z, c->csr.tpos, false, c->tpk32)))
         return r;
     }
     MEGA_ALLOC(c->nbpool, c->sdphi32, 3 * (int64_t)n);
-    k_rowsum_pk32<<<grid_for(n, 256), 256, 0, c->s>>>(n, c->csr.rowptr, (const float4*)c->pk32, c->sdphi32);
+    k_rowsum_pk32<<<grid_for(n, 256), 256, 0, c->s>>>(n, c->csr.rowptr, c->rt.rbase, (const float4*)c->pk32,
+                                                       c->sdphi32);
     MEGA_CHECK_LAUNCH();
     if (c->nsni) {  // S in both float record orders, and its row sums
       MEGA_ALLOC(c->nbpool, c->ns_srow, 6 * m);
@@ -1978,12 +1984,13 @@ static int bank_layout(Ctx* c) {
   MEGA_ALLOC(tmp, pos, m);
   int r = 0;
   // columns (the lanes per column of the force variant the context favours)
-  if ((r = record_ranks(c->s, m, (const float4*)c->tpk32, l)) || (r = iota64(c->s, m, pos)) ||
+  MEGA_TRY(cudaMemcpyAsync(l, c->ct.lidx, sizeof(uint16_t) * m, cudaMemcpyDeviceToDevice, c->s));
+  if ((r = iota64(c->s, m, pos)) ||
       (r = bank_order(c->s, n, c->ct, c->csr.colptr, l, nullptr, pos, c->nsni ? 8 : 4)))
     return r;
   float4* tp = nullptr;
-  MEGA_ALLOC(c->nbpool, tp, m);
-  if ((r = gather_records32(c->s, m, pos, (const float4*)c->tpk32, tp))) return r;
+  MEGA_ALLOC(c->nbpool, tp, c->ct.nrec);
+  if ((r = gather_records32(c->s, n, c->ct, c->csr.colptr, pos, (const float4*)c->tpk32, tp))) return r;
   double* ts = nullptr;
   if (c->tshp32) {
     MEGA_ALLOC(c->nbpool, ts, m);
@@ -1996,14 +2003,15 @@ static int bank_layout(Ctx* c) {
     if ((r = gather_f6(c->s, m, pos, c->ns_scol, sc))) return r;
   }
   // rows
-  if ((r = record_ranks(c->s, m, (const float4*)c->pk32, l)) || (r = iota64(c->s, m, pos)) ||
+  MEGA_TRY(cudaMemcpyAsync(l, c->rt.lidx, sizeof(uint16_t) * m, cudaMemcpyDeviceToDevice, c->s));
+  if ((r = iota64(c->s, m, pos)) ||
       (r = bank_order(c->s, n, c->rt, c->csr.rowptr, l, nullptr, pos, 4)))
     return r;
   float4* rp = nullptr;
   double* sh = nullptr;
-  MEGA_ALLOC(c->nbpool, rp, m);
+  MEGA_ALLOC(c->nbpool, rp, c->rt.nrec);
   MEGA_ALLOC(c->nbpool, sh, m);
-  if ((r = gather_records32(c->s, m, pos, (const float4*)c->pk32, rp))) return r;
+  if ((r = gather_records32(c->s, n, c->rt, c->csr.rowptr, pos, (const float4*)c->pk32, rp))) return r;
   k_gather_pos<<<grid_for(m, 256), 256, 0, c->s>>>(m, pos, c->shp, sh);
   MEGA_CHECK_LAUNCH();
   float* sr = nullptr;

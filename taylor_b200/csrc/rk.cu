@@ -244,7 +244,8 @@ __global__ void __launch_bounds__(128) k_rk_values(int32_t n, const double* __re
                                                    int face, const double* __restrict__ bv,
                                                    double* __restrict__ shp, double* __restrict__ gx,
                                                    double* __restrict__ gy, double* __restrict__ gz,
-                                                   float4* __restrict__ pk, const uint16_t* __restrict__ lidx) {
+                                                   float4* __restrict__ pk, const uint16_t* __restrict__ lidx,
+                                                   const int64_t* __restrict__ rbase) {
   const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kLPN;
   const int lane = threadIdx.x & (kLPN - 1);
   if (i >= n) return;
@@ -278,7 +279,9 @@ __global__ void __launch_bounds__(128) k_rk_values(int32_t n, const double* __re
     if (shp) shp[p] = C * e.phi;
     const double vx = CX * e.phi + C * e.px, vy = CY * e.phi + C * e.py, vz = CZ * e.phi + C * e.pz;
     if (pk) {  // the mixed-precision record (gradient in float, tile rank) instead of the doubles
-      pk[p] = make_float4((float)vx, (float)vy, (float)vz, __int_as_float((int)lidx[p]));
+      const int64_t k = p - p0;
+      pk[rbase[i] + 32 * (k >> 2) + (k & 3)] =
+          make_float4((float)vx, (float)vy, (float)vz, __int_as_float((int)lidx[p]));
     } else {
       gx[p] = vx;
       gy[p] = vy;
@@ -290,7 +293,7 @@ __global__ void __launch_bounds__(128) k_rk_values(int32_t n, const double* __re
 // the three kernels in order on stream s, with their per-node scratch
 int rk_run(cudaStream_t s, const mega_params& p, int32_t n, const double* coo, const double* win,
            const int32_t* ebc_nodes, const DevCSR& csr, const double* sml, int face, double* shp, double* gx,
-           double* gy, double* gz, float4* pk, const uint16_t* lidx, unsigned* status) {
+           double* gy, double* gz, float4* pk, const uint16_t* lidx, const int64_t* rbase, unsigned* status) {
   if (p.rk_degree != 1 || p.rk_cont != 3) return MEGA_ERR_UNSUPPORTED;
   DevPool scratch(s);
   double *mom = nullptr, *bv = nullptr;
@@ -304,7 +307,7 @@ int rk_run(cudaStream_t s, const mega_params& p, int32_t n, const double* coo, c
   k_rk_solve<<<gn, block, 0, s>>>(n, coo, p.ql, p.ql_coef, p.ql_len, sml, face, mom, bv, status);
   MEGA_CHECK_LAUNCH();
   k_rk_values<<<gg, block, 0, s>>>(n, coo, win, ebc_nodes, csr.rowptr, csr.col, p.ql, p.ql_coef, p.ql_len, p.shsup,
-                                   sml, face, bv, shp, gx, gy, gz, pk, lidx);
+                                   sml, face, bv, shp, gx, gy, gz, pk, lidx, rbase);
   MEGA_CHECK_LAUNCH();
   return 0;
 }
@@ -314,19 +317,20 @@ int rk_run(cudaStream_t s, const mega_params& p, int32_t n, const double* coo, c
 int rk_shapes(cudaStream_t s, const mega_params& p, int32_t n, const double* coo, const double* win,
               const int32_t* ebc_nodes, const DevCSR& csr, double* shp, double* gx, double* gy, double* gz,
               unsigned* status) {
-  return rk_run(s, p, n, coo, win, ebc_nodes, csr, nullptr, -1, shp, gx, gy, gz, nullptr, nullptr, status);
+  return rk_run(s, p, n, coo, win, ebc_nodes, csr, nullptr, -1, shp, gx, gy, gz, nullptr, nullptr, nullptr, status);
 }
 
 int rk_shapes_packed(cudaStream_t s, const mega_params& p, int32_t n, const double* coo, const double* win,
-                     const int32_t* ebc_nodes, const DevCSR& csr, const uint16_t* lidx, double* shp, float4* pk,
-                     unsigned* status) {
-  return rk_run(s, p, n, coo, win, ebc_nodes, csr, nullptr, -1, shp, nullptr, nullptr, nullptr, pk, lidx, status);
+                     const int32_t* ebc_nodes, const DevCSR& csr, const uint16_t* lidx, const int64_t* rbase,
+                     double* shp, float4* pk, unsigned* status) {
+  return rk_run(s, p, n, coo, win, ebc_nodes, csr, nullptr, -1, shp, nullptr, nullptr, nullptr, pk, lidx, rbase,
+                status);
 }
 
 int rk_grad_at_face(cudaStream_t s, const mega_params& p, int32_t n, const double* coo, const double* win,
                     const int32_t* ebc_nodes, const DevCSR& csr, const double* sml, int face, double* gx, double* gy,
                     double* gz, unsigned* status) {
-  return rk_run(s, p, n, coo, win, ebc_nodes, csr, sml, face, nullptr, gx, gy, gz, nullptr, nullptr, status);
+  return rk_run(s, p, n, coo, win, ebc_nodes, csr, sml, face, nullptr, gx, gy, gz, nullptr, nullptr, nullptr, status);
 }
 
 }  // namespace mega

@@ -6,7 +6,8 @@
 // grouped into tiles of R consecutive nodes, and each tile's neighbour set
 // (the union of its rows, "J-set") is listed once.  Every neighbour entry
 // then carries its gradient and a 16-bit tile-local index in one 16-byte
-// (float) or 32-byte (double) record, and the neighbour data the tile needs
+// (float) or 26-byte (double) record, laid out in slices of 8 rows so that a
+// warp's loads are contiguous (build_slices), and the neighbour data the tile needs
 // -- (u_tot, du) for the deformation gradient, T_i for the force -- is staged
 // in shared memory once per tile:
 //   k_defgrad_t  F = I + sum_J (u_J - u_i) (x) g + u_i (x) sum g,  G0 likewise
@@ -131,40 +132,127 @@ __global__ void __launch_bounds__(256) k_build_tiles(int32_t n, int32_t R, const
   for (int64_t p = p0 + tid; p < p1; p += blockDim.x) lidx[p] = (uint16_t)rank[slot_tmp[p]];
 }
 
-// list entries of each tile of R consecutive rows
-__global__ void k_tile_entries(int32_t n, int32_t R, int64_t ntiles, const int64_t* __restrict__ ptr,
-                               int32_t* __restrict__ ent) {
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= ntiles) return;
-  const int64_t r0 = t * R, r1 = min((int64_t)n, r0 + R);
-  ent[t] = (int32_t)(ptr[r1] - ptr[r0]);
+// Slices.  A tile's rows are ordered by length and taken 8 at a time; the
+// records of a slice are stored step by step, 4 records of each of its 8
+// rows per step: record 32 s + 4 r + q of the slice is entry 4 s + q of its
+// row r, so the 32 lanes of a warp (4 per row) read one contiguous run.  In
+// list order the same loads touched eight separate runs (29 L1 wavefronts a
+// warp for a step's FP64 records where 7 suffice), and the two gathers ran at
+// 70-83 % of the L1 data pipe.  Rows shorter than their slice are padded with
+// zero gradients at their first entry's rank: ordering the 64 rows by length
+// first keeps the pads at 5 % of the records (14 % in list order, measured on
+// the jittered bar's lists).
+//
+// Block per tile (R threads or more): the row order and the slices' steps.
+__global__ void __launch_bounds__(64) k_slice_rows(int32_t n, int32_t R, const int64_t* __restrict__ ptr,
+                                                   uint8_t* __restrict__ ord, int32_t* __restrict__ steps,
+                                                   int32_t* __restrict__ most) {
+  __shared__ int32_t len[64], sorted[64];
+  const int64_t t = blockIdx.x;
+  const int i = threadIdx.x;
+  const int64_t r = t * R + i;
+  if (i < R) len[i] = r < n ? (int32_t)(ptr[r + 1] - ptr[r]) : -1;
+  __syncthreads();
+  if (i < R) {
+    const int mine = len[i];
+    int pos = 0;  // rows longer than this one, or as long and before it
+    for (int k = 0; k < R; ++k) pos += len[k] > mine || (len[k] == mine && k < i);
+    ord[t * R + pos] = (uint8_t)i;
+    sorted[pos] = mine;
+  }
+  __syncthreads();
+  if (i < R / 8) steps[t * (R / 8) + i] = (max(sorted[8 * i], 0) + 3) / 4;
+  if (i == 0) {
+    int sum = 0;
+    for (int k = 0; k < R; k += 8) sum += (max(sorted[k], 0) + 3) / 4;
+    atomicMax(most, sum);
+  }
 }
 
-__global__ void k_pack_f32(int64_t m, const uint16_t* __restrict__ lidx, const double* __restrict__ gx,
+// rbase[row] = the record of the row's first entry (entry k: + 32 (k / 4) + k % 4)
+__global__ void k_slice_base(int32_t n, int32_t R, int64_t slots, const uint8_t* __restrict__ ord,
+                             const int64_t* __restrict__ sstep, int64_t* __restrict__ rbase) {
+  const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (k >= slots) return;
+  const int64_t row = k / R * R + ord[k];
+  if (row < n) rbase[row] = 32 * sstep[k >> 3] + 4 * (k & 7);
+}
+
+__device__ __forceinline__ int64_t rec_of(int64_t base, int64_t k) { return base + 32 * (k >> 2) + (k & 3); }
+
+// Four lanes per slot of a tile (so a warp writes a slice step by step): put
+// is called for every record of the slot's row, with the list position p of
+// its entry, or p < 0 and the row's first position for a pad.
+template <typename F>
+__device__ __forceinline__ void for_slot_records(int32_t n, int32_t R, int64_t slots, const SliceView& v,
+                                                 const int64_t* ptr, F put) {
+  const int64_t th = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t slot = th >> 2;
+  if (slot >= slots) return;
+  const int q = (int)(th & 3);
+  const int64_t row = slot / R * R + v.ord[slot];
+  const int64_t b = row < n ? ptr[row] : 0, len = row < n ? ptr[row + 1] - b : 0;
+  const int64_t s0 = v.sstep[slot >> 3], s1 = v.sstep[(slot >> 3) + 1];
+  for (int64_t s = s0; s < s1; ++s) {
+    const int64_t k = 4 * (s - s0) + q;
+    put(32 * s + 4 * (slot & 7) + q, k < len ? b + k : (int64_t)-1, len > 0 ? b : (int64_t)-1);
+  }
+}
+
+// records from gradients in list order (pos: where entry p's gradient is)
+__global__ void k_pack_f32(int32_t n, int32_t R, int64_t slots, SliceView v, const int64_t* __restrict__ ptr,
+                           const uint16_t* __restrict__ lidx, const double* __restrict__ gx,
                            const double* __restrict__ gy, const double* __restrict__ gz,
                            const int64_t* __restrict__ pos, float4* __restrict__ out) {
-  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (e >= m) return;
-  const int64_t p = pos ? pos[e] : e;
-  out[e] = make_float4((float)gx[p], (float)gy[p], (float)gz[p], __int_as_float((int)lidx[e]));
+  for_slot_records(n, R, slots, v, ptr, [&](int64_t rec, int64_t p, int64_t first) {
+    float4 o = make_float4(0.f, 0.f, 0.f, __int_as_float(first >= 0 ? (int)lidx[first] : 0));
+    if (p >= 0) {
+      const int64_t g = pos ? pos[p] : p;
+      o = make_float4((float)gx[g], (float)gy[g], (float)gz[g], __int_as_float((int)lidx[p]));
+    }
+    out[rec] = o;
+  });
 }
 
-__global__ void k_pack_t32(int64_t m, const uint16_t* __restrict__ lidx, const float4* __restrict__ in,
-                           const int64_t* __restrict__ pos, float4* __restrict__ out) {
-  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (e >= m) return;
-  const float4 v = in[pos[e]];
-  out[e] = make_float4(v.x, v.y, v.z, __int_as_float((int)lidx[e]));
-}
-
-__global__ void k_pack_f64(int64_t m, const uint16_t* __restrict__ lidx, const double* __restrict__ gx,
+__global__ void k_pack_f64(int32_t n, int32_t R, int64_t slots, SliceView v, const int64_t* __restrict__ ptr,
+                           const uint16_t* __restrict__ lidx, const double* __restrict__ gx,
                            const double* __restrict__ gy, const double* __restrict__ gz,
-                           const int64_t* __restrict__ pos, double2* __restrict__ out) {
-  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (e >= m) return;
-  const int64_t p = pos ? pos[e] : e;
-  out[2 * e] = make_double2(gx[p], gy[p]);
-  out[2 * e + 1] = make_double2(gz[p], __longlong_as_double((long long)lidx[e]));
+                           const int64_t* __restrict__ pos, void* __restrict__ out) {
+  double2* xy = (double2*)out;
+  double* z = (double*)(xy + v.nrec);
+  uint16_t* l = (uint16_t*)(z + v.nrec);
+  for_slot_records(n, R, slots, v, ptr, [&](int64_t rec, int64_t p, int64_t first) {
+    const int64_t g = p < 0 ? 0 : (pos ? pos[p] : p);
+    xy[rec] = p >= 0 ? make_double2(gx[g], gy[g]) : make_double2(0.0, 0.0);
+    z[rec] = p >= 0 ? gz[g] : 0.0;
+    l[rec] = p >= 0 ? lidx[p] : (first >= 0 ? lidx[first] : (uint16_t)0);
+  });
+}
+
+// float column records from the float row records: entry p of the columns is
+// entry pos[p] of the rows, in row trow[p]
+__global__ void k_pack_t32(int32_t n, int32_t R, int64_t slots, SliceView v, const int64_t* __restrict__ ptr,
+                           const uint16_t* __restrict__ lidx, const float4* __restrict__ in,
+                           const int32_t* __restrict__ trow, const int64_t* __restrict__ pos,
+                           const int64_t* __restrict__ rowptr, const int64_t* __restrict__ rbase,
+                           float4* __restrict__ out) {
+  for_slot_records(n, R, slots, v, ptr, [&](int64_t rec, int64_t p, int64_t first) {
+    float4 o = make_float4(0.f, 0.f, 0.f, __int_as_float(first >= 0 ? (int)lidx[first] : 0));
+    if (p >= 0) {
+      const int32_t r = trow[p];
+      const float4 x = in[rec_of(rbase[r], pos[p] - rowptr[r])];
+      o = make_float4(x.x, x.y, x.z, __int_as_float((int)lidx[p]));
+    }
+    out[rec] = o;
+  });
+}
+
+// the pads alone (the shape kernel wrote the real records)
+__global__ void k_pad_f32(int32_t n, int32_t R, int64_t slots, SliceView v, const int64_t* __restrict__ ptr,
+                          const uint16_t* __restrict__ lidx, float4* __restrict__ out) {
+  for_slot_records(n, R, slots, v, ptr, [&](int64_t rec, int64_t p, int64_t first) {
+    if (p < 0) out[rec] = make_float4(0.f, 0.f, 0.f, __int_as_float(first >= 0 ? (int)lidx[first] : 0));
+  });
 }
 
 // Entry order for conflict-free reads of the staged neighbour data.  In the
@@ -183,6 +271,7 @@ constexpr int kBankCap = 2048;  // entries of one warp's rows that its pass stag
 
 template <int KG, int NC, int GL>
 __global__ void __launch_bounds__(128) k_bank_order(int32_t n, int32_t R, int64_t nwarps,
+                                                    const uint8_t* __restrict__ ord,
                                                     const int64_t* __restrict__ ptr, uint16_t* lidx,
                                                     const int64_t* __restrict__ pos_src, int64_t* pos) {
   __shared__ int held_s[4][32];
@@ -192,7 +281,7 @@ __global__ void __launch_bounds__(128) k_bank_order(int32_t n, int32_t R, int64_
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
   int* held = held_s[wi] + (lane / GL) * NC;  // this lane's group: the rank held per class
   const int wpt = R * KG / 32;  // warps per tile
-  const int64_t c = (w / wpt) * R + (w % wpt) * (32 / KG) + lane / KG;
+  const int64_t c = (w / wpt) * R + ord[(w / wpt) * R + (w % wpt) * (32 / KG) + lane / KG];
   const int q = lane & (KG - 1);
   int64_t b = 0, e = 0;
   if (c < n) { b = ptr[c]; e = ptr[c + 1]; }
@@ -257,16 +346,19 @@ __global__ void __launch_bounds__(128) k_bank_order(int32_t n, int32_t R, int64_
     }
 }
 
-__global__ void k_gather_rec32(int64_t m, const int64_t* __restrict__ pos, const float4* __restrict__ in,
+// the records of each row in a new order: entry p takes the record of entry
+// pos[p] of the same row (pads stay)
+__global__ void k_gather_rec32(int32_t n, int32_t R, int64_t slots, SliceView v, const int64_t* __restrict__ ptr,
+                               const int64_t* __restrict__ pos, const float4* __restrict__ in,
                                float4* __restrict__ out) {
-  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (e < m) out[e] = in[pos[e]];
-}
-
-// the tile rank carried by each float record
-__global__ void k_rec_ranks(int64_t m, const float4* __restrict__ rec, uint16_t* __restrict__ out) {
-  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (e < m) out[e] = (uint16_t)__float_as_int(rec[e].w);
+  for_slot_records(n, R, slots, v, ptr, [&](int64_t rec, int64_t p, int64_t first) {
+    int64_t from = rec;
+    if (p >= 0) {
+      const int64_t k = p - first;
+      from = rec_of(rec - 32 * (k >> 2) - (k & 3), pos[p] - first);
+    }
+    out[rec] = in[from];
+  });
 }
 
 // out[6 e + k] = in[6 pos[e] + k]
@@ -283,25 +375,63 @@ __global__ void k_iota64(int64_t m, int64_t* __restrict__ out) {
   if (e < m) out[e] = e;
 }
 
+// One record as a lane holds it: the gradient in the arithmetic's type and
+// the tile rank.  FP64 records are three planes (x and y, z, rank) of nrec
+// values each, so each load of a warp is contiguous.
 template <bool F64>
-__device__ __forceinline__ void load_entry(const void* pk, int64_t p, float& g0, float& g1, float& g2, int& l);
+struct Rec;
 template <>
-__device__ __forceinline__ void load_entry<false>(const void* pk, int64_t p, float& g0, float& g1, float& g2,
-                                                  int& l) {
-  const float4 v = __ldg((const float4*)pk + p);
-  g0 = v.x; g1 = v.y; g2 = v.z; l = __float_as_int(v.w);
+struct Rec<false> {
+  float4 v;
+  __device__ __forceinline__ float x() const { return v.x; }
+  __device__ __forceinline__ float y() const { return v.y; }
+  __device__ __forceinline__ float z() const { return v.z; }
+  __device__ __forceinline__ int l() const { return __float_as_int(v.w); }
+};
+template <>
+struct Rec<true> {
+  double2 a;
+  double b;
+  uint16_t r;
+  __device__ __forceinline__ double x() const { return a.x; }
+  __device__ __forceinline__ double y() const { return a.y; }
+  __device__ __forceinline__ double z() const { return b; }
+  __device__ __forceinline__ int l() const { return (int)r; }
+};
+__device__ __forceinline__ void load_rec(const void* pk, int64_t, int64_t rec, Rec<false>& o) {
+  o.v = __ldg((const float4*)pk + rec);
 }
-__device__ __forceinline__ void load_entry64(const void* pk, int64_t p, double& g0, double& g1, double& g2, int& l) {
-  const double2 a = __ldg((const double2*)pk + 2 * p);
-  const double2 b = __ldg((const double2*)pk + 2 * p + 1);
-  g0 = a.x; g1 = a.y; g2 = b.x; l = (int)__double_as_longlong(b.y);
+__device__ __forceinline__ void load_rec(const void* pk, int64_t nrec, int64_t rec, Rec<true>& o) {
+  const double2* xy = (const double2*)pk;
+  const double* z = (const double*)(xy + nrec);
+  o.a = __ldg(xy + rec);
+  o.b = __ldg(z + rec);
+  o.r = __ldg((const uint16_t*)(z + nrec) + rec);
 }
+
+// A lane's way through its row's records: KG lanes per row (4, 8 or 16), the
+// lane's entries KG apart in list order, which is a stride of KG / 4 steps.
+// ns is uniform over a slice's lanes when KG = 4.
+template <int KG>
+struct RowWalk {
+  int64_t rec;  // the lane's first record
+  int nit;      // its records (pads among them)
+  __device__ __forceinline__ RowWalk(const SliceView& v, int64_t slot0, int slot, int lane) {
+    const int64_t sl = (slot0 + slot) >> 3;
+    const int64_t s0 = v.sstep[sl];
+    const int ns = (int)(v.sstep[sl + 1] - s0), h = lane >> 2;
+    rec = 32 * (s0 + h) + 4 * (slot & 7) + (lane & 3);
+    nit = (ns - h + KG / 4 - 1) / (KG / 4);
+  }
+  __device__ __forceinline__ int64_t at(int k) const { return rec + (int64_t)(8 * KG) * k; }
+};
 
 // The six float S values of one NSNI record (three 8-byte loads).
 struct SRec {
   float2 a, b, c;
 };
-__device__ __forceinline__ SRec load_srec(const float* base, int64_t p) {
+__device__ __forceinline__ SRec load_srec(const float* base, int64_t p, int64_t pend) {
+  if (p >= pend) return SRec{};  // a pad
   const float2* sp = reinterpret_cast<const float2*>(base) + 3 * p;
   return SRec{__ldg(sp), __ldg(sp + 1), __ldg(sp + 2)};
 }
@@ -311,7 +441,7 @@ __device__ __forceinline__ SRec load_srec(const float* base, int64_t p) {
 // sum_J S_q (du_J - du_i) + du_i,k sum_J S_q (FINT.F90:728-737 layout).
 template <typename A, bool F64, bool INTERP, int KG, int KU, bool NS = false>
 __global__ void __launch_bounds__(64 * KG, (F64 ? 12 : (NS ? 8 : 16)) / KG > 0 ? (F64 ? 12 : (NS ? 8 : 16)) / KG : 1) k_defgrad_t(int32_t n, int32_t R, int32_t jmax,
-                                                   NsniTiles ns,
+                                                   NsniTiles ns, SliceView sv,
                                                    const int64_t* __restrict__ rowptr, const void* __restrict__ pk,
                                                    const int32_t* __restrict__ jset, const int32_t* __restrict__ jcnt,
                                                    const double* __restrict__ dsp, const double* __restrict__ dsp_tot,
@@ -336,32 +466,30 @@ __global__ void __launch_bounds__(64 * KG, (F64 ? 12 : (NS ? 8 : 16)) / KG > 0 ?
   double* sd = sm + 3 * cnt;
   float* sf = reinterpret_cast<float*>(sm);
   const int64_t r0 = t * R;
-  const int64_t i = t * R + threadIdx.x / KG;
+  const int slot = threadIdx.x / KG;
+  const int64_t i = r0 + sv.ord[r0 + slot];
   const int q = threadIdx.x & (KG - 1);
   const unsigned gmask = group_mask<KG>();
-  const bool valid = threadIdx.x / KG < R && i < n;
+  const bool valid = i < n;
   // this lane's first KU packed records are requested before the staging,
   // so their latency overlaps it
-  int64_t p = 0, pend = 0;
-  bool pre = false;
-  float4 pf[KU];
-  double2 pfa[KU], pfb[KU];
-  SRec psr[NS ? KU : 1];
-  if (valid) {
-    p = rowptr[i] + q;
+  const RowWalk<KG> walk(sv, r0, slot, q);
+  const int nit = valid ? walk.nit : 0;
+  constexpr bool kPipe = !NS && (!F64 || KU <= 2);
+  constexpr bool kList = INTERP || NS;  // values that stay in list order ride along
+  int64_t p0 = 0, pend = 0;
+  if (kList && valid) {
+    p0 = rowptr[i] + q;
     pend = rowptr[i + 1];
-    pre = p + (KU - 1) * KG < pend;
-    if (pre) {
+  }
+  Rec<F64> cur[KU];
+  SRec csr[NS ? KU : 1];
+  bool have = nit >= KU;
+  if (have) {
 #pragma unroll
-      for (int u = 0; u < KU; ++u) {
-        if (F64) {
-          pfa[u] = __ldg((const double2*)pk + 2 * (p + u * KG));
-          pfb[u] = __ldg((const double2*)pk + 2 * (p + u * KG) + 1);
-        } else {
-          pf[u] = __ldg((const float4*)pk + p + u * KG);
-        }
-        if constexpr (NS) psr[u] = load_srec(ns.srow, p + u * KG);
-      }
+    for (int u = 0; u < KU; ++u) {
+      load_rec(pk, sv.nrec, walk.at(u), cur[u]);
+      if constexpr (NS) csr[u] = load_srec(ns.srow, p0 + u * KG, pend);
     }
   }
   double ur0 = 0.0, ur1 = 0.0, ur2 = 0.0, dr0 = 0.0, dr1 = 0.0, dr2 = 0.0;
@@ -396,7 +524,9 @@ __global__ void __launch_bounds__(64 * KG, (F64 ? 12 : (NS ? 8 : 16)) / KG > 0 ?
   double ph0 = 0.0, ph1 = 0.0, ph2 = 0.0;
   // One entry: F += (u_J - u_i) (x) g, L += (d_J - d_i) (x) g (+ phi d_J),
   // H(k, q) += S_q (d_J - d_i)_k.
-  auto body = [&](int64_t p, A g0, A g1, A g2, int l, const SRec& sr) {
+  auto body = [&](int it, const Rec<F64>& rec, const SRec& sr) {
+    const A g0 = (A)rec.x(), g1 = (A)rec.y(), g2 = (A)rec.z();
+    const int l = rec.l();
     A u0, u1, u2, d0, d1, d2;
     double dj0, dj1, dj2;  // du_J itself, for the per-step interpolation
     if (F64) {
@@ -425,84 +555,46 @@ __global__ void __launch_bounds__(64 * KG, (F64 ? 12 : (NS ? 8 : 16)) / KG > 0 ?
       for (int c = 0; c < 6; ++c) { H[c] += sq[c] * e0; H[6 + c] += sq[c] * e1; H[12 + c] += sq[c] * e2; }
     }
     if (INTERP) {
-      const double s = shp[p];
-      ph0 += s * dj0; ph1 += s * dj1; ph2 += s * dj2;
+      const int64_t p = p0 + (int64_t)KG * it;
+      if (p < pend) {  // (not a pad)
+        const double s = shp[p];
+        ph0 += s * dj0; ph1 += s * dj1; ph2 += s * dj2;
+      }
     }
   };
-  // KU records in flight per lane before any is used (the loop is bound by
-  // DRAM latency otherwise); each lane still sums its entries in list order.
+  // Each lane sums its entries in list order.  Where the registers allow
+  // (kPipe) the next KU records are requested before this KU's sums, so a
+  // lane keeps loads in flight while it computes.
   const SRec s0{};
-  if (pre) {
+  int it = 0;
+  while (have) {
+    const bool hn = it + 2 * KU <= nit;
+    Rec<F64> nxt[KU];
+    if constexpr (kPipe) {
+#pragma unroll
+      for (int u = 0; u < KU; ++u) {
+        if (hn) load_rec(pk, sv.nrec, walk.at(it + KU + u), nxt[u]);
+        else nxt[u] = cur[u];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < KU; ++u) body(it + u, cur[u], NS ? csr[NS ? u : 0] : s0);
 #pragma unroll
     for (int u = 0; u < KU; ++u) {
-      if (F64)
-        body(p + u * KG, (A)pfa[u].x, (A)pfa[u].y, (A)pfb[u].x, (int)__double_as_longlong(pfb[u].y), s0);
-      else
-        body(p + u * KG, (A)pf[u].x, (A)pf[u].y, (A)pf[u].z, __float_as_int(pf[u].w), NS ? psr[NS ? u : 0] : s0);
-    }
-    p += KU * KG;
-  }
-  if (F64) {
-    for (; p + (KU - 1) * KG < pend; p += KU * KG) {
-      double2 ra[KU], rb[KU];
-#pragma unroll
-      for (int u = 0; u < KU; ++u) {
-        ra[u] = __ldg((const double2*)pk + 2 * (p + u * KG));
-        rb[u] = __ldg((const double2*)pk + 2 * (p + u * KG) + 1);
+      if constexpr (kPipe) {
+        cur[u] = nxt[u];
+      } else if (hn) {
+        load_rec(pk, sv.nrec, walk.at(it + KU + u), cur[u]);
+        if constexpr (NS) csr[u] = load_srec(ns.srow, p0 + (int64_t)KG * (it + KU + u), pend);
       }
-#pragma unroll
-      for (int u = 0; u < KU; ++u)
-        body(p + u * KG, (A)ra[u].x, (A)ra[u].y, (A)rb[u].x, (int)__double_as_longlong(rb[u].y), s0);
     }
-  } else if constexpr (!NS) {
-    // software-pipelined: the next KU records are requested before this
-    // KU's sums, so a lane keeps loads in flight while it computes
-    float4 cur[KU];
-    bool have = p + (KU - 1) * KG < pend;
-    if (have) {
-#pragma unroll
-      for (int u = 0; u < KU; ++u) cur[u] = __ldg((const float4*)pk + p + u * KG);
-    }
-    while (have) {
-      const int64_t pn = p + KU * KG;
-      const bool hn = pn + (KU - 1) * KG < pend;
-      float4 nxt[KU];
-#pragma unroll
-      for (int u = 0; u < KU; ++u) nxt[u] = hn ? __ldg((const float4*)pk + pn + u * KG) : cur[u];
-#pragma unroll
-      for (int u = 0; u < KU; ++u)
-        body(p + u * KG, (A)cur[u].x, (A)cur[u].y, (A)cur[u].z, __float_as_int(cur[u].w), s0);
-#pragma unroll
-      for (int u = 0; u < KU; ++u) cur[u] = nxt[u];
-      p = pn;
-      have = hn;
-    }
-  } else {
-    for (; p + (KU - 1) * KG < pend; p += KU * KG) {
-      float4 r[KU];
-      SRec sr[NS ? KU : 1];
-#pragma unroll
-      for (int u = 0; u < KU; ++u) {
-        r[u] = __ldg((const float4*)pk + p + u * KG);
-        if constexpr (NS) sr[u] = load_srec(ns.srow, p + u * KG);
-      }
-#pragma unroll
-      for (int u = 0; u < KU; ++u)
-        body(p + u * KG, (A)r[u].x, (A)r[u].y, (A)r[u].z, __float_as_int(r[u].w), NS ? sr[NS ? u : 0] : s0);
-    }
+    it += KU;
+    have = hn;
   }
-  for (; p < pend; p += KG) {
-    if (F64) {
-      double a0, a1, a2;
-      int l;
-      load_entry64(pk, p, a0, a1, a2, l);
-      body(p, (A)a0, (A)a1, (A)a2, l, s0);
-    } else {
-      float a0, a1, a2;
-      int l;
-      load_entry<false>(pk, p, a0, a1, a2, l);
-      body(p, (A)a0, (A)a1, (A)a2, l, NS ? load_srec(ns.srow, p) : s0);
-    }
+  for (; it < nit; ++it) {
+    Rec<F64> rec;
+    load_rec(pk, sv.nrec, walk.at(it), rec);
+    body(it, rec, NS ? load_srec(ns.srow, p0 + (int64_t)KG * it, pend) : s0);
   }
 #pragma unroll
   for (int o = 1; o < KG; o <<= 1) {
@@ -634,30 +726,30 @@ __global__ void __launch_bounds__(64 * KG) k_force_t(TiledForceArgs a) {
   TS* sT = (TS*)smx;
   const int32_t* js = a.jset + t * (int64_t)a.jmax;
   const TS* tm = (const TS*)a.tmat;
-  const int64_t J = t * a.R + threadIdx.x / KG;
+  const int64_t c0 = t * a.R;
+  const int slot = threadIdx.x / KG;
+  const int64_t J = c0 + a.sv.ord[c0 + slot];
   const int q = threadIdx.x & (KG - 1);
   const unsigned gmask = group_mask<KG>();
-  const bool valid = threadIdx.x / KG < a.R && J < a.n;
+  const bool valid = J < a.n;
   // this lane's first KU packed records are requested before the staging,
-  // so their latency overlaps it (FP64 records only)
-  int64_t e = 0, c1 = 0;
-  bool pre = false;
-  float4 pf[KU];
-  double2 pfa[KU], pfb[KU];
-  if (F64 && valid) {  // measured: pays in FP64, costs occupancy in mixed
-    e = a.colptr[J] + q;
-    c1 = a.colptr[J + 1];
-    pre = e + (KU - 1) * KG < c1;
-    if (pre) {
+  // so their latency overlaps it
+  const RowWalk<KG> walk(a.sv, c0, slot, q);
+  const int nit = valid ? walk.nit : 0;
+  constexpr bool kPipe = !NS && (!F64 || KU <= 2);
+  int64_t p0 = 0, pend = 0;  // list positions, for the values that stay in list order
+  if (valid && (NS || a.has_body)) {
+    p0 = a.colptr[J] + q;
+    pend = a.colptr[J + 1];
+  }
+  Rec<F64> cur[KU];
+  SRec csr[NS ? KU : 1];
+  bool have = nit >= KU;
+  if (have) {
 #pragma unroll
-      for (int u = 0; u < KU; ++u) {
-        if (F64) {
-          pfa[u] = __ldg((const double2*)a.pk + 2 * (e + u * KG));
-          pfb[u] = __ldg((const double2*)a.pk + 2 * (e + u * KG) + 1);
-        } else {
-          pf[u] = __ldg((const float4*)a.pk + e + u * KG);
-        }
-      }
+    for (int u = 0; u < KU; ++u) {
+      load_rec(a.pk, a.sv.nrec, walk.at(u), cur[u]);
+      if constexpr (NS) csr[u] = load_srec(a.ns_scol, p0 + u * KG, pend);
     }
   }
   // thread per staged node: one index load, then its T row (12 values,
@@ -695,17 +787,14 @@ __global__ void __launch_bounds__(64 * KG) k_force_t(TiledForceArgs a) {
     }
   }
   __syncthreads();
-  if (!F64 && valid) {
-    e = a.colptr[J] + q;
-    c1 = a.colptr[J + 1];
-  }
   double ke = 0.0, ee = 0.0, tf[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   unsigned st = 0;
   if (valid) {
     A f0 = A(0), f1 = A(0), f2 = A(0);
     double e0 = 0.0, e1 = 0.0, e2 = 0.0;
-    auto body = [&](int64_t e, A g0, A g1, A g2, int l, const SRec& sr) {
-      const TS* T = sT + l;  // component k of T_l at T[k * cnt]
+    auto body = [&](int it, const Rec<F64>& rec, const SRec& sr) {
+      const A g0 = (A)rec.x(), g1 = (A)rec.y(), g2 = (A)rec.z();
+      const TS* T = sT + rec.l();  // component k of T_l at T[k * cnt]
       f0 += (A)T[0] * g0 + (A)T[cnt] * g1 + (A)T[2 * cnt] * g2;
       f1 += (A)T[3 * cnt] * g0 + (A)T[4 * cnt] * g1 + (A)T[5 * cnt] * g2;
       f2 += (A)T[6 * cnt] * g0 + (A)T[7 * cnt] * g1 + (A)T[8 * cnt] * g2;
@@ -720,82 +809,43 @@ __global__ void __launch_bounds__(64 * KG) k_force_t(TiledForceArgs a) {
         }
       }
       if (a.has_body) {
-        const double s = a.tshp[e];
-        e0 += s * (double)T[9 * cnt]; e1 += s * (double)T[10 * cnt]; e2 += s * (double)T[11 * cnt];
+        const int64_t e = p0 + (int64_t)KG * it;
+        if (e < pend) {  // (not a pad)
+          const double s = a.tshp[e];
+          e0 += s * (double)T[9 * cnt]; e1 += s * (double)T[10 * cnt]; e2 += s * (double)T[11 * cnt];
+        }
       }
     };
     const SRec s0{};
-    if (pre) {  // (FP64 only)
+    int it = 0;
+    while (have) {  // as in the row gather
+      const bool hn = it + 2 * KU <= nit;
+      Rec<F64> nxt[KU];
+      if constexpr (kPipe) {
+#pragma unroll
+        for (int u = 0; u < KU; ++u) {
+          if (hn) load_rec(a.pk, a.sv.nrec, walk.at(it + KU + u), nxt[u]);
+          else nxt[u] = cur[u];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < KU; ++u) body(it + u, cur[u], NS ? csr[NS ? u : 0] : s0);
 #pragma unroll
       for (int u = 0; u < KU; ++u) {
-        if (F64)
-          body(e + u * KG, (A)pfa[u].x, (A)pfa[u].y, (A)pfb[u].x, (int)__double_as_longlong(pfb[u].y), s0);
-        else
-          body(e + u * KG, (A)pf[u].x, (A)pf[u].y, (A)pf[u].z, __float_as_int(pf[u].w), s0);
-      }
-      e += KU * KG;
-    }
-    if (F64) {
-      for (; e + (KU - 1) * KG < c1; e += KU * KG) {
-        double2 ra[KU], rb[KU];
-#pragma unroll
-        for (int u = 0; u < KU; ++u) {
-          ra[u] = __ldg((const double2*)a.pk + 2 * (e + u * KG));
-          rb[u] = __ldg((const double2*)a.pk + 2 * (e + u * KG) + 1);
+        if constexpr (kPipe) {
+          cur[u] = nxt[u];
+        } else if (hn) {
+          load_rec(a.pk, a.sv.nrec, walk.at(it + KU + u), cur[u]);
+          if constexpr (NS) csr[u] = load_srec(a.ns_scol, p0 + (int64_t)KG * (it + KU + u), pend);
         }
-#pragma unroll
-        for (int u = 0; u < KU; ++u)
-          body(e + u * KG, (A)ra[u].x, (A)ra[u].y, (A)rb[u].x, (int)__double_as_longlong(rb[u].y), s0);
       }
-    } else if constexpr (!NS) {
-      // software-pipelined: the next KU records are requested before this
-      // KU's sums, so a lane keeps loads in flight while it computes
-      float4 cur[KU];
-      bool have = e + (KU - 1) * KG < c1;
-      if (have) {
-#pragma unroll
-        for (int u = 0; u < KU; ++u) cur[u] = __ldg((const float4*)a.pk + e + u * KG);
-      }
-      while (have) {
-        const int64_t en = e + KU * KG;
-        const bool hn = en + (KU - 1) * KG < c1;
-        float4 nxt[KU];
-#pragma unroll
-        for (int u = 0; u < KU; ++u) nxt[u] = hn ? __ldg((const float4*)a.pk + en + u * KG) : cur[u];
-#pragma unroll
-        for (int u = 0; u < KU; ++u)
-          body(e + u * KG, (A)cur[u].x, (A)cur[u].y, (A)cur[u].z, __float_as_int(cur[u].w), s0);
-#pragma unroll
-        for (int u = 0; u < KU; ++u) cur[u] = nxt[u];
-        e = en;
-        have = hn;
-      }
-    } else {
-      for (; e + (KU - 1) * KG < c1; e += KU * KG) {
-        float4 r[KU];
-        SRec sr[NS ? KU : 1];
-#pragma unroll
-        for (int u = 0; u < KU; ++u) {
-          r[u] = __ldg((const float4*)a.pk + e + u * KG);
-          if constexpr (NS) sr[u] = load_srec(a.ns_scol, e + u * KG);
-        }
-#pragma unroll
-        for (int u = 0; u < KU; ++u)
-          body(e + u * KG, (A)r[u].x, (A)r[u].y, (A)r[u].z, __float_as_int(r[u].w), NS ? sr[NS ? u : 0] : s0);
-      }
+      it += KU;
+      have = hn;
     }
-    for (; e < c1; e += KG) {
-      if (F64) {
-        double b0, b1, b2;
-        int l;
-        load_entry64(a.pk, e, b0, b1, b2, l);
-        body(e, (A)b0, (A)b1, (A)b2, l, s0);
-      } else {
-        float b0, b1, b2;
-        int l;
-        load_entry<false>(a.pk, e, b0, b1, b2, l);
-        body(e, (A)b0, (A)b1, (A)b2, l, NS ? load_srec(a.ns_scol, e) : s0);
-      }
+    for (; it < nit; ++it) {
+      Rec<F64> rec;
+      load_rec(a.pk, a.sv.nrec, walk.at(it), rec);
+      body(it, rec, NS ? load_srec(a.ns_scol, p0 + (int64_t)KG * it, pend) : s0);
     }
 #pragma unroll
     for (int o = 1; o < KG; o <<= 1) {
@@ -825,26 +875,37 @@ __global__ void __launch_bounds__(64 * KG) k_force_t(TiledForceArgs a) {
 constexpr int kChunks = 4;
 constexpr int kPollLimit = 1 << 16;
 
-// Thread 0: the barriers, then the copies of entries [0, ne) of the tile
-// (src points at its first record, RB bytes each) into rec.
-template <int RB>
-__device__ __forceinline__ void issue_records(uint64_t* bar, unsigned char* rec, const unsigned char* src,
-                                              int64_t ne) {
+// Thread 0: the barriers, then the copies of steps [0, ne) of the tile (32
+// records each) from the record planes (16-byte records, or the 16-, 8- and
+// 2-byte planes of FP64) into rec, where each plane has room for recmax
+// records.
+template <bool F64>
+__device__ __forceinline__ void issue_records(uint64_t* bar, unsigned char* rec, const void* pk, int64_t nrec,
+                                              int64_t step0, int64_t ne, int64_t recmax) {
   if (threadIdx.x != 0) return;
 #pragma unroll
   for (int c = 0; c < kChunks; ++c) mbar_init(&bar[c], 1);
   mbar_fence_init();
+  constexpr int width[3] = {16, 8, 2};
 #pragma unroll
   for (int c = 0; c < kChunks; ++c) {
     const int64_t lo = c * ne / kChunks, hi = (c + 1) * ne / kChunks;
-    const uint32_t bytes = (uint32_t)((hi - lo) * RB);
-    mbar_arrive_expect(&bar[c], bytes);
-    for (uint32_t off = 0; off < bytes; off += 32768u)
-      bulk_load(rec + lo * RB + off, src + lo * RB + off, min(32768u, bytes - off), &bar[c]);
+    mbar_arrive_expect(&bar[c], (uint32_t)((hi - lo) * 32 * (F64 ? 26 : 16)));
+    const unsigned char* src = (const unsigned char*)pk;
+    unsigned char* dst = rec;
+#pragma unroll
+    for (int k = 0; k < (F64 ? 3 : 1); ++k) {
+      const uint32_t bytes = (uint32_t)((hi - lo) * 32 * width[k]);
+      for (uint32_t off = 0; off < bytes; off += 32768u)
+        bulk_load(dst + lo * 32 * width[k] + off, src + (step0 + lo) * 32 * width[k] + off,
+                  min(32768u, bytes - off), &bar[c]);
+      src += nrec * width[k];
+      dst += recmax * width[k];
+    }
   }
 }
 
-// Wait for the chunks holding entries [a, b) of the tile.
+// Wait for the chunks holding steps [a, b) of the tile.
 __device__ __forceinline__ bool wait_records(uint64_t* bar, int64_t ne, int64_t a, int64_t b) {
   bool ok = true;
 #pragma unroll
@@ -862,15 +923,27 @@ __device__ __forceinline__ void drain_records(uint64_t* bar) {
   for (int c = 0; c < kChunks; ++c) mbar_wait_bounded(&bar[c], 0, kPollLimit);
 }
 
+// a staged record of the tile (planes of recmax records)
+__device__ __forceinline__ void staged_rec(const unsigned char* rec, int64_t, int64_t p, Rec<false>& o) {
+  o.v = reinterpret_cast<const float4*>(rec)[p];
+}
+__device__ __forceinline__ void staged_rec(const unsigned char* rec, int64_t recmax, int64_t p, Rec<true>& o) {
+  const double2* xy = reinterpret_cast<const double2*>(rec);
+  const double* z = reinterpret_cast<const double*>(xy + recmax);
+  o.a = xy[p];
+  o.b = z[p];
+  o.r = reinterpret_cast<const uint16_t*>(z + recmax)[p];
+}
+
 template <typename A, bool F64, bool INTERP, int KG>
-__global__ void __launch_bounds__(64 * KG) k_defgrad_b(int32_t n, int32_t R, int32_t jmax, int32_t recmax,
+__global__ void __launch_bounds__(64 * KG) k_defgrad_b(int32_t n, int32_t R, int32_t jmax, int32_t recmax, SliceView sv,
                                                        const int64_t* __restrict__ rowptr, const void* __restrict__ pk,
                                                        const int32_t* __restrict__ jset, const int32_t* __restrict__ jcnt,
                                                        const double* __restrict__ dsp, const double* __restrict__ dsp_tot,
                                                        const double* __restrict__ sdphi, const double* __restrict__ shp,
                                                        double* __restrict__ dsp_tot_phy, double* __restrict__ fg,
                                                        StepAccum* __restrict__ acc, unsigned* __restrict__ status) {
-  constexpr int RB = F64 ? 32 : 16;
+  constexpr int RB = F64 ? 26 : 16;
   extern __shared__ __align__(128) unsigned char smb[];
   __shared__ uint64_t bar[kChunks];
   if (acc && blockIdx.x == 0 && threadIdx.x < kSlots) {
@@ -878,19 +951,20 @@ __global__ void __launch_bounds__(64 * KG) k_defgrad_b(int32_t n, int32_t R, int
     acc->plastic[threadIdx.x] = 0ull;
   }
   const int64_t t = blockIdx.x;
-  const int64_t r0 = t * R, r1 = min((int64_t)n, r0 + R);
-  const int64_t e0 = rowptr[r0], ne = rowptr[r1] - e0;
-  issue_records<RB>(bar, smb, (const unsigned char*)pk + e0 * RB, ne);
+  const int64_t r0 = t * R;
+  const int64_t e0 = sv.sstep[r0 >> 3], ne = sv.sstep[(r0 + R) >> 3] - e0;
+  issue_records<F64>(bar, smb, pk, sv.nrec, e0, ne, recmax);
   const int cnt = jcnt[t];
   const int32_t* js = jset + t * (int64_t)jmax;
   unsigned char* stg = smb + (size_t)recmax * RB;
   double* su = reinterpret_cast<double*>(stg);
   double* sd = su + 3 * cnt;
   float* sf = reinterpret_cast<float*>(stg);  // mixed: value k of rank l at sf[k * cnt + l]
-  const int64_t i = r0 + threadIdx.x / KG;
+  const int slot = threadIdx.x / KG;
+  const int64_t i = r0 + sv.ord[r0 + slot];
   const int q = threadIdx.x & (KG - 1);
   const unsigned gmask = group_mask<KG>();
-  const bool valid = threadIdx.x / KG < R && i < n;
+  const bool valid = i < n;
   double ur0 = 0.0, ur1 = 0.0, ur2 = 0.0, dr0 = 0.0, dr1 = 0.0, dr2 = 0.0;
   if (!F64) {
     ur0 = dsp_tot[3 * r0]; ur1 = dsp_tot[3 * r0 + 1]; ur2 = dsp_tot[3 * r0 + 2];
@@ -913,8 +987,14 @@ __global__ void __launch_bounds__(64 * KG) k_defgrad_b(int32_t n, int32_t R, int
     drain_records(bar);
     return;
   }
-  const int64_t pa = rowptr[i] - e0, pb = rowptr[i + 1] - e0;
-  const bool ok = __all_sync(gmask, wait_records(bar, ne, pa, pb));
+  const int64_t sl = (r0 + slot) >> 3;
+  const bool ok = __all_sync(gmask, wait_records(bar, ne, sv.sstep[sl] - e0, sv.sstep[sl + 1] - e0));
+  const RowWalk<KG> walk(sv, r0, slot, q);
+  int64_t p0 = 0, pend = 0;
+  if (INTERP) {
+    p0 = rowptr[i] + q;
+    pend = rowptr[i + 1];
+  }
   const double ui0 = dsp_tot[3 * i], ui1 = dsp_tot[3 * i + 1], ui2 = dsp_tot[3 * i + 2];
   const double di0 = dsp[3 * i], di1 = dsp[3 * i + 1], di2 = dsp[3 * i + 2];
   const float fu0 = (float)(ui0 - ur0), fu1 = (float)(ui1 - ur1), fu2 = (float)(ui2 - ur2);
@@ -924,19 +1004,12 @@ __global__ void __launch_bounds__(64 * KG) k_defgrad_b(int32_t n, int32_t R, int
   for (int k = 0; k < 9; ++k) { F[k] = A(0); L[k] = A(0); }
   double ph0 = 0.0, ph1 = 0.0, ph2 = 0.0;
   if (ok) {
-    const float4* rec32 = reinterpret_cast<const float4*>(smb);
-    const double2* rec64 = reinterpret_cast<const double2*>(smb);
 #pragma unroll 4
-    for (int64_t p = pa + q; p < pb; p += KG) {
-      A g0, g1, g2;
-      int l;
-      if (F64) {
-        const double2 ra = rec64[2 * p], rb = rec64[2 * p + 1];
-        g0 = (A)ra.x; g1 = (A)ra.y; g2 = (A)rb.x; l = (int)__double_as_longlong(rb.y);
-      } else {
-        const float4 r = rec32[p];
-        g0 = (A)r.x; g1 = (A)r.y; g2 = (A)r.z; l = __float_as_int(r.w);
-      }
+    for (int it = 0; it < walk.nit; ++it) {
+      Rec<F64> rec;
+      staged_rec(smb, recmax, walk.at(it) - 32 * e0, rec);
+      const A g0 = (A)rec.x(), g1 = (A)rec.y(), g2 = (A)rec.z();
+      const int l = rec.l();
       A u0, u1, u2, d0, d1, d2;
       double dj0, dj1, dj2;
       if (F64) {
@@ -958,8 +1031,11 @@ __global__ void __launch_bounds__(64 * KG) k_defgrad_b(int32_t n, int32_t R, int
       L[3] += d1 * g0; L[4] += d1 * g1; L[5] += d1 * g2;
       L[6] += d2 * g0; L[7] += d2 * g1; L[8] += d2 * g2;
       if (INTERP) {
-        const double s = shp[e0 + p];
-        ph0 += s * dj0; ph1 += s * dj1; ph2 += s * dj2;
+        const int64_t p = p0 + (int64_t)KG * it;
+        if (p < pend) {
+          const double s = shp[p];
+          ph0 += s * dj0; ph1 += s * dj1; ph2 += s * dj2;
+        }
       }
     }
   }
@@ -1003,23 +1079,24 @@ __global__ void __launch_bounds__(64 * KG) k_defgrad_b(int32_t n, int32_t R, int
 
 template <typename TS, typename A, bool F64, int KG>
 __global__ void __launch_bounds__(64 * KG) k_force_b(TiledForceArgs a) {
-  constexpr int RB = F64 ? 32 : 16;
+  constexpr int RB = F64 ? 26 : 16;
   extern __shared__ __align__(128) unsigned char smb[];
   __shared__ uint64_t bar[kChunks];
   __shared__ double red[32 * 8];  // eight sums per warp, up to 32 warps (KG = 16)
   const int64_t t = blockIdx.x;
-  const int64_t c0 = t * a.R, c1 = min((int64_t)a.n, c0 + a.R);
-  const int64_t e0 = a.colptr[c0], ne = a.colptr[c1] - e0;
-  issue_records<RB>(bar, smb, (const unsigned char*)a.pk + e0 * RB, ne);
+  const int64_t c0 = t * a.R;
+  const int64_t e0 = a.sv.sstep[c0 >> 3], ne = a.sv.sstep[(c0 + a.R) >> 3] - e0;
+  issue_records<F64>(bar, smb, a.pk, a.sv.nrec, e0, ne, a.recmax);
   const int cnt = a.jcnt[t];
   const int nv = a.has_body ? 12 : 9;
   TS* sT = reinterpret_cast<TS*>(smb + (size_t)a.recmax * RB);
   const int32_t* js = a.jset + t * (int64_t)a.jmax;
   const TS* tm = (const TS*)a.tmat;
-  const int64_t J = c0 + threadIdx.x / KG;
+  const int slot = threadIdx.x / KG;
+  const int64_t J = c0 + a.sv.ord[c0 + slot];
   const int q = threadIdx.x & (KG - 1);
   const unsigned gmask = group_mask<KG>();
-  const bool valid = threadIdx.x / KG < a.R && J < a.n;
+  const bool valid = J < a.n;
   for (int l = threadIdx.x; l < cnt; l += blockDim.x) {
     const TS* src = tm + 12 * (int64_t)js[l];
     TS v[12];
@@ -1046,31 +1123,33 @@ __global__ void __launch_bounds__(64 * KG) k_force_b(TiledForceArgs a) {
   double ke = 0.0, ee = 0.0, tf[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   unsigned st = 0;
   if (valid) {
-    const int64_t pa = a.colptr[J] - e0, pb = a.colptr[J + 1] - e0;
-    const bool ok = __all_sync(gmask, wait_records(bar, ne, pa, pb));
+    const int64_t sl = (c0 + slot) >> 3;
+    const bool ok = __all_sync(gmask, wait_records(bar, ne, a.sv.sstep[sl] - e0, a.sv.sstep[sl + 1] - e0));
+    const RowWalk<KG> walk(a.sv, c0, slot, q);
+    int64_t p0 = 0, pend = 0;
+    if (a.has_body) {
+      p0 = a.colptr[J] + q;
+      pend = a.colptr[J + 1];
+    }
     A f0 = A(0), f1 = A(0), f2 = A(0);
     double b0 = 0.0, b1 = 0.0, b2 = 0.0;
     if (ok) {
-      const float4* rec32 = reinterpret_cast<const float4*>(smb);
-      const double2* rec64 = reinterpret_cast<const double2*>(smb);
 #pragma unroll 4
-      for (int64_t p = pa + q; p < pb; p += KG) {
-        A g0, g1, g2;
-        int l;
-        if (F64) {
-          const double2 ra = rec64[2 * p], rb = rec64[2 * p + 1];
-          g0 = (A)ra.x; g1 = (A)ra.y; g2 = (A)rb.x; l = (int)__double_as_longlong(rb.y);
-        } else {
-          const float4 r = rec32[p];
-          g0 = (A)r.x; g1 = (A)r.y; g2 = (A)r.z; l = __float_as_int(r.w);
-        }
+      for (int it = 0; it < walk.nit; ++it) {
+        Rec<F64> rec;
+        staged_rec(smb, a.recmax, walk.at(it) - 32 * e0, rec);
+        const A g0 = (A)rec.x(), g1 = (A)rec.y(), g2 = (A)rec.z();
+        const int l = rec.l();
         const TS* T = sT + l;  // component k of T_l at T[k * cnt]
         f0 += (A)T[0] * g0 + (A)T[cnt] * g1 + (A)T[2 * cnt] * g2;
         f1 += (A)T[3 * cnt] * g0 + (A)T[4 * cnt] * g1 + (A)T[5 * cnt] * g2;
         f2 += (A)T[6 * cnt] * g0 + (A)T[7 * cnt] * g1 + (A)T[8 * cnt] * g2;
         if (a.has_body) {
-          const double s = a.tshp[e0 + p];
-          b0 += s * (double)T[9 * cnt]; b1 += s * (double)T[10 * cnt]; b2 += s * (double)T[11 * cnt];
+          const int64_t p = p0 + (int64_t)KG * it;
+          if (p < pend) {
+            const double s = a.tshp[p];
+            b0 += s * (double)T[9 * cnt]; b1 += s * (double)T[10 * cnt]; b2 += s * (double)T[11 * cnt];
+          }
         }
       }
     }
@@ -1131,23 +1210,12 @@ int build_tiles(cudaStream_t s, int32_t n, const int64_t* ptr, const int32_t* id
     if (hovf) continue;  // too many distinct neighbours: halve the tile
     int32_t mx = 0;
     for (int32_t v : hc) mx = std::max(mx, v);
-    // the longest record range of any tile (sizes the streamed variants)
-    int32_t* ent = nullptr;
-    MEGA_ALLOC(scratch, ent, ntiles);
-    k_tile_entries<<<grid_for(ntiles, 256), 256, 0, s>>>(n, R, ntiles, ptr, ent);
-    MEGA_CHECK_LAUNCH();
-    std::vector<int32_t> he(ntiles);
-    MEGA_TRY(cudaMemcpyAsync(he.data(), ent, sizeof(int32_t) * ntiles, cudaMemcpyDeviceToHost, s));
-    MEGA_TRY(cudaStreamSynchronize(s));
-    int32_t emax = 0;
-    for (int32_t v : he) emax = std::max(emax, v);
     // keep the trial buffers: move ownership into the persistent pool
     pool.adopt(trial);
     ts.R = R;
     ts.ntiles = ntiles;
     ts.jmax = jmax;
     ts.maxcnt = mx;
-    ts.recmax = emax;
     ts.jset = jset;
     ts.jcnt = jcnt;
     ts.lidx = lidx;
@@ -1157,19 +1225,54 @@ int build_tiles(cudaStream_t s, int32_t n, const int64_t* ptr, const int32_t* id
   return MEGA_ERR_UNSUPPORTED;
 }
 
-int pack_transposed32(cudaStream_t s, int64_t m, const uint16_t* lidx, const float4* in, const int64_t* pos,
+int build_slices(cudaStream_t s, int32_t n, const int64_t* ptr, TileSet& ts, DevPool& pool) {
+  const int64_t slots = ts.ntiles * ts.R, nsl = slots / 8;
+  DevPool scratch(s);
+  int32_t *steps = nullptr, *most = nullptr;
+  MEGA_ALLOC(scratch, steps, nsl);
+  MEGA_ALLOC(scratch, most, 1);
+  MEGA_ALLOC(pool, ts.ord, slots);
+  MEGA_ALLOC(pool, ts.sstep, nsl + 1);
+  MEGA_ALLOC(pool, ts.rbase, n);
+  MEGA_TRY(cudaMemsetAsync(most, 0, sizeof(int32_t), s));
+  k_slice_rows<<<(unsigned)ts.ntiles, 64, 0, s>>>(n, ts.R, ptr, ts.ord, steps, most);
+  MEGA_CHECK_LAUNCH();
+  if (int r = scan_counts(s, steps, ts.sstep, nsl, scratch)) return r;
+  k_slice_base<<<grid_for(slots, 256), 256, 0, s>>>(n, ts.R, slots, ts.ord, ts.sstep, ts.rbase);
+  MEGA_CHECK_LAUNCH();
+  int64_t total = 0;
+  int32_t tile = 0;
+  MEGA_TRY(cudaMemcpyAsync(&total, ts.sstep + nsl, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+  MEGA_TRY(cudaMemcpyAsync(&tile, most, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+  MEGA_TRY(cudaStreamSynchronize(s));
+  ts.nrec = 32 * total;
+  ts.recmax = 32 * tile;
+  return 0;
+}
+
+int pack_transposed32(cudaStream_t s, int32_t n, const TileSet& ct, const int64_t* colptr, const float4* in,
+                      const int32_t* trow, const int64_t* pos, const int64_t* rowptr, const TileSet& rt,
                       float4* out) {
-  if (m <= 0) return 0;
-  k_pack_t32<<<grid_for(m, 256), 256, 0, s>>>(m, lidx, in, pos, out);
+  const int64_t slots = ct.ntiles * ct.R;
+  k_pack_t32<<<grid_for(4 * slots, 256), 256, 0, s>>>(n, ct.R, slots, ct.view(), colptr, ct.lidx, in, trow, pos,
+                                                      rowptr, rt.rbase, out);
   MEGA_CHECK_LAUNCH();
   return 0;
 }
 
-int pack_entries(cudaStream_t s, int64_t m, const uint16_t* lidx, const double* gx, const double* gy,
-                 const double* gz, const int64_t* pos, bool f64, void* out) {
-  if (m <= 0) return 0;
-  if (f64) k_pack_f64<<<grid_for(m, 256), 256, 0, s>>>(m, lidx, gx, gy, gz, pos, (double2*)out);
-  else k_pack_f32<<<grid_for(m, 256), 256, 0, s>>>(m, lidx, gx, gy, gz, pos, (float4*)out);
+int pack_entries(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* ptr, const double* gx,
+                 const double* gy, const double* gz, const int64_t* pos, bool f64, void* out) {
+  const int64_t slots = ts.ntiles * ts.R;
+  const unsigned grid = grid_for(4 * slots, 256);
+  if (f64) k_pack_f64<<<grid, 256, 0, s>>>(n, ts.R, slots, ts.view(), ptr, ts.lidx, gx, gy, gz, pos, out);
+  else k_pack_f32<<<grid, 256, 0, s>>>(n, ts.R, slots, ts.view(), ptr, ts.lidx, gx, gy, gz, pos, (float4*)out);
+  MEGA_CHECK_LAUNCH();
+  return 0;
+}
+
+int pad_records32(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* ptr, float4* out) {
+  const int64_t slots = ts.ntiles * ts.R;
+  k_pad_f32<<<grid_for(4 * slots, 256), 256, 0, s>>>(n, ts.R, slots, ts.view(), ptr, ts.lidx, out);
   MEGA_CHECK_LAUNCH();
   return 0;
 }
@@ -1180,8 +1283,8 @@ int bank_order(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* ptr,
   if ((lanes != 4 && lanes != 8) || ts.R * lanes < 32) return MEGA_ERR_UNSUPPORTED;
   const int64_t nwarps = ts.ntiles * (int64_t)(ts.R * lanes / 32);
   const unsigned grid = (unsigned)((nwarps * 32 + 127) / 128);
-  if (lanes == 4) k_bank_order<4, 32, 32><<<grid, 128, 0, s>>>(n, ts.R, nwarps, ptr, lidx, pos_src, pos);
-  else k_bank_order<8, 32, 32><<<grid, 128, 0, s>>>(n, ts.R, nwarps, ptr, lidx, pos_src, pos);
+  if (lanes == 4) k_bank_order<4, 32, 32><<<grid, 128, 0, s>>>(n, ts.R, nwarps, ts.ord, ptr, lidx, pos_src, pos);
+  else k_bank_order<8, 32, 32><<<grid, 128, 0, s>>>(n, ts.R, nwarps, ts.ord, ptr, lidx, pos_src, pos);
   MEGA_CHECK_LAUNCH();
   return 0;
 }
@@ -1193,13 +1296,6 @@ int iota64(cudaStream_t s, int64_t m, int64_t* out) {
   return 0;
 }
 
-int record_ranks(cudaStream_t s, int64_t m, const float4* rec, uint16_t* out) {
-  if (m <= 0) return 0;
-  k_rec_ranks<<<grid_for(m, 256), 256, 0, s>>>(m, rec, out);
-  MEGA_CHECK_LAUNCH();
-  return 0;
-}
-
 int gather_f6(cudaStream_t s, int64_t m, const int64_t* pos, const float* in, float* out) {
   if (m <= 0) return 0;
   k_gather_f6<<<grid_for(m, 256), 256, 0, s>>>(m, pos, (const float2*)in, (float2*)out);
@@ -1207,9 +1303,10 @@ int gather_f6(cudaStream_t s, int64_t m, const int64_t* pos, const float* in, fl
   return 0;
 }
 
-int gather_records32(cudaStream_t s, int64_t m, const int64_t* pos, const float4* in, float4* out) {
-  if (m <= 0) return 0;
-  k_gather_rec32<<<grid_for(m, 256), 256, 0, s>>>(m, pos, in, out);
+int gather_records32(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* ptr, const int64_t* pos,
+                     const float4* in, float4* out) {
+  const int64_t slots = ts.ntiles * ts.R;
+  k_gather_rec32<<<grid_for(4 * slots, 256), 256, 0, s>>>(n, ts.R, slots, ts.view(), ptr, pos, in, out);
   MEGA_CHECK_LAUNCH();
   return 0;
 }
@@ -1294,7 +1391,7 @@ bool tiled_variant_fits(const TileSet& ts, bool mixed, int variant, bool force, 
   if (variant < 0 || variant >= kVariants) return false;
   if (variant < 4 || variant > 5) return true;  // register variants
   const size_t stage = force ? (mixed ? sizeof(float) : sizeof(double)) * (has_body ? 12 : 9) : (mixed ? 24 : 48);
-  return (size_t)ts.recmax * (mixed ? 16 : 32) + stage * (size_t)ts.maxcnt <= (size_t)g_bulk_lim;
+  return (size_t)ts.recmax * (mixed ? 16 : 26) + stage * (size_t)ts.maxcnt <= (size_t)g_bulk_lim;
 }
 
 template <int KG>
@@ -1302,17 +1399,17 @@ static int defgrad_bulk(cudaStream_t s, bool mixed, bool interp, int32_t n, cons
                         const int64_t* rowptr, const void* pk, const double* dsp, const double* dsp_tot,
                         const double* sdphi, const double* shp, double* dsp_tot_phy, double* fg, StepAccum* acc,
                         unsigned* status) {
-  const size_t smem = (size_t)ts.recmax * (mixed ? 16 : 32) + (mixed ? 24 : 48) * (size_t)ts.maxcnt;
+  const size_t smem = (size_t)ts.recmax * (mixed ? 16 : 26) + (mixed ? 24 : 48) * (size_t)ts.maxcnt;
   if (smem > (size_t)g_bulk_lim) return MEGA_ERR_UNSUPPORTED;
   const unsigned grid = (unsigned)ts.ntiles;
   const int block = ts.R * KG;
   if (mixed) {
     auto k = interp ? k_defgrad_b<float, false, true, KG> : k_defgrad_b<float, false, false, KG>;
-    k<<<grid, block, smem, s>>>(n, ts.R, ts.jmax, ts.recmax, rowptr, pk, ts.jset, ts.jcnt, dsp, dsp_tot, sdphi, shp,
+    k<<<grid, block, smem, s>>>(n, ts.R, ts.jmax, ts.recmax, ts.view(), rowptr, pk, ts.jset, ts.jcnt, dsp, dsp_tot, sdphi, shp,
                                 dsp_tot_phy, fg, acc, status);
   } else {
     auto k = interp ? k_defgrad_b<double, true, true, KG> : k_defgrad_b<double, true, false, KG>;
-    k<<<grid, block, smem, s>>>(n, ts.R, ts.jmax, ts.recmax, rowptr, pk, ts.jset, ts.jcnt, dsp, dsp_tot, sdphi, shp,
+    k<<<grid, block, smem, s>>>(n, ts.R, ts.jmax, ts.recmax, ts.view(), rowptr, pk, ts.jset, ts.jcnt, dsp, dsp_tot, sdphi, shp,
                                 dsp_tot_phy, fg, acc, status);
   }
   return 0;
@@ -1330,11 +1427,11 @@ static void defgrad_variant(cudaStream_t s, bool mixed, bool interp, int32_t n, 
   if (mixed) {
     auto k = ns ? (interp ? k_defgrad_t<float, false, true, KG, KU, true> : k_defgrad_t<float, false, false, KG, KU, true>)
                 : (interp ? k_defgrad_t<float, false, true, KG, KU> : k_defgrad_t<float, false, false, KG, KU>);
-    k<<<grid, block, smem, s>>>(n, ts.R, ts.jmax, nz, rowptr, pk, ts.jset, ts.jcnt, dsp, dsp_tot, sdphi, shp,
+    k<<<grid, block, smem, s>>>(n, ts.R, ts.jmax, nz, ts.view(), rowptr, pk, ts.jset, ts.jcnt, dsp, dsp_tot, sdphi, shp,
                                 dsp_tot_phy, fg, acc);
   } else {
     auto k = interp ? k_defgrad_t<double, true, true, KG, KU> : k_defgrad_t<double, true, false, KG, KU>;
-    k<<<grid, block, smem, s>>>(n, ts.R, ts.jmax, nz, rowptr, pk, ts.jset, ts.jcnt, dsp, dsp_tot, sdphi, shp,
+    k<<<grid, block, smem, s>>>(n, ts.R, ts.jmax, nz, ts.view(), rowptr, pk, ts.jset, ts.jcnt, dsp, dsp_tot, sdphi, shp,
                                 dsp_tot_phy, fg, acc);
   }
 }
@@ -1375,7 +1472,7 @@ int launch_defgrad_tiled(cudaStream_t s, bool mixed, bool interp, int32_t n, con
 template <int KG>
 static int force_bulk(cudaStream_t s, bool mixed, const TiledForceArgs& a) {
   const int nv = a.has_body ? 12 : 9;
-  const size_t smem = (size_t)a.recmax * (mixed ? 16 : 32) + (mixed ? sizeof(float) : sizeof(double)) * nv *
+  const size_t smem = (size_t)a.recmax * (mixed ? 16 : 26) + (mixed ? sizeof(float) : sizeof(double)) * nv *
                       (size_t)a.maxcnt;
   if (smem > (size_t)g_bulk_lim) return MEGA_ERR_UNSUPPORTED;
   const unsigned grid = (unsigned)a.ntiles;

@@ -5,15 +5,29 @@
 
 namespace mega {
 
+// How a tile set's packed records are laid out (build_slices in tiled.cu):
+// slices of 8 rows, 32 records per step, 4 consecutive entries of each row
+struct SliceView {
+  const uint8_t* ord = nullptr;    // per slot (tile, position): the row within the tile; rows past n come last
+  const int64_t* sstep = nullptr;  // per slice of 8 slots: its first step (record 32 sstep), and the end
+  int64_t nrec = 0;                // records, pads among them
+};
+
 struct TileSet {
   int32_t R = 0;           // rows (columns) per tile; the kernels run R*4 threads per tile
   int64_t ntiles = 0;
   int32_t jmax = 0;        // stride of jset per tile
   int32_t maxcnt = 0;      // largest neighbour set of any tile
-  int32_t recmax = 0;      // most list entries of any tile (its packed-record range)
+  int32_t recmax = 0;      // most packed records of any tile (build_slices)
   int32_t* jset = nullptr; // [ntiles][jmax] sorted node ids
   int32_t* jcnt = nullptr; // [ntiles]
   uint16_t* lidx = nullptr;  // per entry: rank of its neighbour in the tile's set
+  // the slices of its records (build_slices)
+  uint8_t* ord = nullptr;
+  int64_t* sstep = nullptr;
+  int64_t* rbase = nullptr;  // per row: the record of its entry 0; entry k is 32 (k / 4) + k % 4 further
+  int64_t nrec = 0;
+  SliceView view() const { return SliceView{ord, sstep, nrec}; }
 };
 
 // NSNI terms carried by the mixed-precision tiled gathers: the smoothed
@@ -37,6 +51,7 @@ struct TiledForceArgs {
   const int32_t* jset;
   const int32_t* jcnt;
   const int64_t* colptr;
+  SliceView sv;           // the layout of pk
   const void* pk;         // packed transposed entries (gradient + local index)
   const double* tshp;     // transposed shape values (body force) or null
   const void* tmat;       // 12 values per node
@@ -68,13 +83,19 @@ struct TiledForceArgs {
 // until every tile's neighbour set fits jmax = 1024.
 int build_tiles(cudaStream_t s, int32_t n, const int64_t* ptr, const int32_t* idx, int64_t nnz, int32_t gmaxn,
                 TileSet& ts, DevPool& pool, int32_t* maxcnt_out);
-// out[e] = (g[pos[e]], lidx[e]) as float4 (f64 = false) or 2 x double2
-int pack_entries(cudaStream_t s, int64_t m, const uint16_t* lidx, const double* gx, const double* gy,
-                 const double* gz, const int64_t* pos, bool f64, void* out);
-// out[e] = (in[pos[e]] gradient, lidx[e]): mixed records of the transposed
-// view from those of the rows
-int pack_transposed32(cudaStream_t s, int64_t m, const uint16_t* lidx, const float4* in, const int64_t* pos,
+// The record layout of ts (row order, slices, record bases) into pool.
+int build_slices(cudaStream_t s, int32_t n, const int64_t* ptr, TileSet& ts, DevPool& pool);
+// records of ts.nrec entries in the slice layout: (gradient of entry pos[e],
+// rank of e) as float4, or FP64 as planes of double2 (x, y), double (z) and
+// uint16_t (rank): 16 or 26 bytes a record
+int pack_entries(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* ptr, const double* gx,
+                 const double* gy, const double* gz, const int64_t* pos, bool f64, void* out);
+// mixed records of the transposed view from those of the rows
+int pack_transposed32(cudaStream_t s, int32_t n, const TileSet& ct, const int64_t* colptr, const float4* in,
+                      const int32_t* trow, const int64_t* pos, const int64_t* rowptr, const TileSet& rt,
                       float4* out);
+// the pads of float records whose entries are written elsewhere
+int pad_records32(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* ptr, float4* out);
 // Reorder the entries within each row (column) of the tiles ts so that the
 // lanes of a warp of a gather with `lanes` (4 or 8) lanes per row read
 // distinct shared-memory banks of the staged neighbour data (one 32-bit
@@ -83,11 +104,11 @@ int pack_transposed32(cudaStream_t s, int64_t m, const uint16_t* lidx, const flo
 // position before, and must hold that same array on entry.
 int bank_order(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* ptr, uint16_t* lidx,
                const int64_t* pos_src, int64_t* pos, int lanes);
-// out[e] = e;  out[e] = in[pos[e]]
+// out[e] = e;  entry e takes the record of entry pos[e] of its row
 int iota64(cudaStream_t s, int64_t m, int64_t* out);
-int gather_records32(cudaStream_t s, int64_t m, const int64_t* pos, const float4* in, float4* out);
-// out[e] = the tile rank of float record e;  out[6 e + k] = in[6 pos[e] + k]
-int record_ranks(cudaStream_t s, int64_t m, const float4* rec, uint16_t* out);
+int gather_records32(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* ptr, const int64_t* pos,
+                     const float4* in, float4* out);
+// out[6 e + k] = in[6 pos[e] + k]
 int gather_f6(cudaStream_t s, int64_t m, const int64_t* pos, const float* in, float* out);
 int configure_tiled_kernels();
 // launch variants of the two gathers: lanes per row x records in flight
