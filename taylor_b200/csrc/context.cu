@@ -475,6 +475,7 @@ struct Ctx {
   double *f2 = nullptr, *dtime = nullptr, *vel2 = nullptr;
   double time = 0.0;
   int64_t steps = 0;
+  int64_t fsteps = 0;  // steps since F - I had to be formed afresh (0: it has to be); it is again every kGraphSteps
   int64_t launches = 0;
   // independent instances sharing the context (node ranges searched apart)
   std::vector<int32_t> inst_off;  // ninst + 1 prefix offsets, empty = one instance
@@ -644,6 +645,12 @@ static NsniStepArgs nsni_args(Ctx* c) {
   return a;
 }
 
+// Steps per captured graph; the first of them forms F afresh.  Single steps
+// follow the same count (Ctx::fsteps), so how a run is split into calls does
+// not change its bits; a run restarted from uploaded fields repeats the
+// unbroken one bit for bit where the restart falls on a multiple of it.
+constexpr int kGraphSteps = 16;
+
 // kernels one step launches (the learned start splits the stress kernel in
 // two; NSNI adds the stress-gradient kernel, and in FP64 its two gathers)
 static int kernels_per_step(const Ctx* c, int mode = 0) {
@@ -652,7 +659,9 @@ static int kernels_per_step(const Ctx* c, int mode = 0) {
          (((mode & MEGA_FLAG_LEARNED_GUESS) && c->mlp_on) ? 1 : 0);
 }
 
-static int step_once(Ctx* c, double dt, int mode, int predict, cudaEvent_t* ev) {
+// full: F is formed from the displacements; else it advances by this step's
+// increment from where the step before left it.
+static int step_once(Ctx* c, double dt, int mode, int predict, cudaEvent_t* ev, bool full) {
   const bool mixed = (mode & 0xff) == MEGA_MODE_MIXED;
   const bool interp = (mode & MEGA_FLAG_INTERP_EACH_STEP) != 0;
   if (ev) MEGA_TRY(cudaEventRecord(ev[0], c->s));
@@ -662,11 +671,13 @@ static int step_once(Ctx* c, double dt, int mode, int predict, cudaEvent_t* ev) 
   int r = launch_defgrad_tiled(c->s, mixed, interp, c->n, c->rt, nsni_tiles(c, mixed, nt), c->csr.rowptr,
                                mixed ? c->pk32 : c->pk64, c->dsp, c->dsp_tot, mixed ? c->sdphi32 : c->sdphi,
                                (mixed && c->shp32) ? c->shp32 : c->shp, c->dsp_tot_phy, c->fg, c->acc, c->status,
-                               c->var_defgrad[mixed]);
+                               c->var_defgrad[mixed], full);
   if (r) return r;
   if (c->nsni && !mixed && (r = nsni_step(c->s, nsni_args(c), c->csr, c->nsr, c->nsc, false, c->dsp, 0))) return r;
   if (ev) MEGA_TRY(cudaEventRecord(ev[1], c->s));
-  r = launch_stress(c->s, mixed, stress_args(c, dt, mode));
+  StressArgs sa = stress_args(c, dt, mode);
+  sa.add_g0 = !full;
+  r = launch_stress(c->s, mixed, sa);
   if (r) return r;
   if (c->nsni && (r = nsni_step(c->s, nsni_args(c), c->csr, c->nsr, c->nsc, mixed, c->dsp, 1))) return r;
   if (c->nsni && !mixed && (r = nsni_step(c->s, nsni_args(c), c->csr, c->nsr, c->nsc, false, c->dsp, 2))) return r;
@@ -686,7 +697,7 @@ static int graph_for(Ctx* c, double dt, int mode, int len) {
   MEGA_TRY(cudaStreamBeginCapture(c->s, cudaStreamCaptureModeThreadLocal));
   const int64_t before = c->launches;
   int r = 0;
-  for (int k = 0; k < len && !r; ++k) r = step_once(c, dt, mode, 1, nullptr);
+  for (int k = 0; k < len && !r; ++k) r = step_once(c, dt, mode, 1, nullptr, k == 0);
   cudaError_t e = cudaStreamEndCapture(c->s, &g);
   c->launches = before;
   if (r) { if (g) cudaGraphDestroy(g); return r; }
@@ -714,21 +725,23 @@ static int run_steps(Ctx* c, int32_t nsteps, double dt, int mode) {
   r = launch_predict(c->s, 3 * (int64_t)c->n, c->dsp, c->dsp_tot, c->vel, c->acl, dt, c->ndt);
   if (r) return r;
   c->launches += 1;
-  int32_t rem = nsteps - 1;
-  const int len = 16;
-  if (rem >= len) {
-    r = graph_for(c, dt, mode, len);
-    if (r) return r;
-    while (rem >= len) {
+  // whole graphs where a full step is due, single steps around them
+  for (int32_t rem = nsteps - 1; rem > 0;) {
+    if (c->fsteps % kGraphSteps == 0 && rem >= kGraphSteps) {
+      if ((r = graph_for(c, dt, mode, kGraphSteps))) return r;
       MEGA_TRY(cudaGraphLaunch(c->gexec, c->s));
-      c->launches += kernels_per_step(c, mode) * len;
-      rem -= len;
+      c->launches += kernels_per_step(c, mode) * kGraphSteps;
+      c->fsteps += kGraphSteps;
+      rem -= kGraphSteps;
+    } else {
+      if ((r = step_once(c, dt, mode, 1, nullptr, c->fsteps % kGraphSteps == 0))) return r;
+      ++c->fsteps;
+      --rem;
     }
   }
-  for (; rem > 0 && !r; --rem) r = step_once(c, dt, mode, 1, nullptr);
+  r = step_once(c, dt, mode, 0, nullptr, c->fsteps % kGraphSteps == 0);
   if (r) return r;
-  r = step_once(c, dt, mode, 0, nullptr);
-  if (r) return r;
+  ++c->fsteps;
   for (int32_t k = 0; k < nsteps; ++k) c->time = c->time + dt;  // TIME = TIME + DLT
   c->steps += nsteps;
   return 0;
@@ -1225,7 +1238,7 @@ int mega_gpu_init(const mega_params* p, int32_t n, const double* coo, const doub
   CA(c->dsp, n3); CA(c->dsp_tot, n3); CA(c->dsp_tot_phy, n3); CA(c->vel, n3); CA(c->acl, n3);
   CA(c->fint, n3); CA(c->fext, n3); CA(c->prforce, n3); CA(c->scratch3, n3);
   CA(c->stress, 6 * (int64_t)n); CA(c->strain, 6 * (int64_t)n); CA(c->eps, n); CA(c->strain_eq, n);
-  CA(c->wvel, n); CA(c->fg, 18 * (int64_t)n); CA(c->iters, n); CA(c->acc, 1); CA(c->status, 1);
+  CA(c->wvel, n); CA(c->fg, 18 * fg_ld(n)); CA(c->iters, n); CA(c->acc, 1); CA(c->status, 1);
   if (has_ebc2) {  // no windows until mega_set_fixity2: the prescribed velocity is zero (MAIN.F90:458-462)
     CA(c->dtime, 1); CA(c->vel2, 3);
     cudaMemsetAsync(c->vel2, 0, sizeof(double) * 3, c->s);
@@ -1429,6 +1442,7 @@ int mega_search_and_shapes(int64_t h, int32_t* gn, int32_t* gstart, int32_t* gst
     c->ns_ssum = nullptr;
     c->banked = false;
     c->searched = false;
+    c->fsteps = 0;
     if (c->gexec) { cudaGraphExecDestroy(c->gexec); c->gexec = nullptr; }
   }
   PhaseTrace tr(c->s, "search_and_shapes");
@@ -1691,7 +1705,7 @@ int mega_step_timed(int64_t h, int32_t nsteps, double dt, int32_t mode, float* m
   Ctx* c = get_ctx(h);
   if (!c || !ms) return c ? MEGA_ERR_ARG : MEGA_ERR_HANDLE;
   if (c->searched) { int r = ((mode & 0xff) == MEGA_MODE_MIXED) ? ensure_mixed(c) : ensure_fp64(c); if (r) return r; }
-  if (c->searched && !c->semi && nsteps > 16) { int r = graph_for(c, dt, mode, 16); if (r) return r; }
+  if (c->searched && !c->semi && nsteps > kGraphSteps) { int r = graph_for(c, dt, mode, kGraphSteps); if (r) return r; }
   cudaEvent_t e0, e1;
   MEGA_TRY(cudaEventCreate(&e0));
   MEGA_TRY(cudaEventCreate(&e1));
@@ -1721,8 +1735,9 @@ int mega_kernel_times(int64_t h, int32_t reps, double dt, int32_t mode, float* o
   double acc[3] = {0, 0, 0};
   int r = launch_predict(c->s, 3 * (int64_t)c->n, c->dsp, c->dsp_tot, c->vel, c->acl, dt, c->ndt);
   for (int32_t k = 0; k < reps && !r; ++k) {
-    r = step_once(c, dt, mode, k < reps - 1 ? 1 : 0, ev);
+    r = step_once(c, dt, mode, k < reps - 1 ? 1 : 0, ev, c->fsteps % kGraphSteps == 0);
     if (r) break;
+    ++c->fsteps;
     cudaEventSynchronize(ev[3]);
     float t;
     for (int q = 0; q < 3; ++q) {
@@ -1899,7 +1914,7 @@ int mega_upload(int64_t h, int32_t field, const double* src) {
   int w = 0;
   switch (field) {
     case MEGA_F_DSP: dst = c->dsp; w = 3; break;
-    case MEGA_F_DSP_TOT: dst = c->dsp_tot; w = 3; c->phy_valid = false; break;
+    case MEGA_F_DSP_TOT: dst = c->dsp_tot; w = 3; c->phy_valid = false; c->fsteps = 0; break;
     case MEGA_F_VEL: dst = c->vel; w = 3; break;
     case MEGA_F_ACL: dst = c->acl; w = 3; break;
     case MEGA_F_FEXT: dst = c->fext; w = 3; break;
@@ -2048,7 +2063,7 @@ int mega_autotune(int64_t h, double dt, int32_t mode, int32_t reps, int32_t* cho
   std::vector<Arr> arrs = {
       {c->dsp, 8 * n3}, {c->dsp_tot, 8 * n3}, {c->dsp_tot_phy, 8 * n3}, {c->vel, 8 * n3}, {c->acl, 8 * n3},
       {c->fint, 8 * n3}, {c->fext, 8 * n3}, {c->prforce, 8 * n3}, {c->stress, 48 * n}, {c->strain, 48 * n},
-      {c->eps, 8 * n}, {c->strain_eq, 8 * n}, {c->wvel, 8 * n}, {c->fg, 144 * n}, {c->tmat, 12 * ts * n},
+      {c->eps, 8 * n}, {c->strain_eq, 8 * n}, {c->wvel, 8 * n}, {c->fg, 144 * (size_t)fg_ld(c->n)}, {c->tmat, 12 * ts * n},
       {c->iters, 4 * n}, {c->acc, sizeof(StepAccum)}, {c->status, sizeof(unsigned)}};
   if (c->aux) arrs.push_back({c->aux, 32 * n});
   if (c->sgrad) arrs.push_back({c->sgrad, 144 * n});
@@ -2070,22 +2085,23 @@ int mega_autotune(int64_t h, double dt, int32_t mode, int32_t reps, int32_t* cho
   for (int v = 0; v < nvar && !r; ++v) {
     NsniTiles nt;
     const NsniTiles* ns = nsni_tiles(c, mixed, nt);
-    const auto def = [&]() {
+    const auto def = [&](bool full) {
       return launch_defgrad_tiled(c->s, mixed, false, c->n, c->rt, ns, c->csr.rowptr, mixed ? c->pk32 : c->pk64,
                                   c->dsp, c->dsp_tot, mixed ? c->sdphi32 : c->sdphi, c->shp, c->dsp_tot_phy, c->fg,
-                                  c->acc, c->status, v);
+                                  c->acc, c->status, v, full);
     };
-    r = def();  // warm-up (twice: the first launch of a variant may also load its code)
+    r = def(true);  // F for the stress kernel; the timed launches are the increments'
+    if (!r) r = def(false);  // warm-up (twice: the first launch of a variant may also load its code)
     if (r == MEGA_ERR_UNSUPPORTED) {  // a streamed variant whose tiles do not fit shared memory
       fits[v] = false;
       r = 0;
       continue;
     }
-    if (!r) r = def();
+    if (!r) r = def(false);
     if (r) break;
     MEGA_TRY(cudaStreamSynchronize(c->s));
     cudaEventRecord(e0, c->s);
-    for (int k = 0; k < reps && !r; ++k) r = def();
+    for (int k = 0; k < reps && !r; ++k) r = def(false);
     cudaEventRecord(e1, c->s);
     cudaEventSynchronize(e1);
     cudaEventElapsedTime(&tdef[v], e0, e1);
@@ -2590,7 +2606,7 @@ static int construct_fint_impl(const mega_params* p, const FintIO& io) {
   MEGA_ALLOC(pool, tgx, m); MEGA_ALLOC(pool, tgy, m); MEGA_ALLOC(pool, tgz, m);
   MEGA_ALLOC(pool, sd, n3); MEGA_ALLOC(pool, ddsp, n3); MEGA_ALLOC(pool, dtot, n3);
   MEGA_ALLOC(pool, dsig, 6 * (int64_t)n); MEGA_ALLOC(pool, deps6, 6 * (int64_t)n); MEGA_ALLOC(pool, dep, n);
-  MEGA_ALLOC(pool, deq, n); MEGA_ALLOC(pool, dwv, n); MEGA_ALLOC(pool, dfg, 18 * (int64_t)n);
+  MEGA_ALLOC(pool, deq, n); MEGA_ALLOC(pool, dwv, n); MEGA_ALLOC(pool, dfg, 18 * fg_ld(n));
   MEGA_ALLOC(pool, dT, 12 * (int64_t)n); MEGA_ALLOC(pool, dfi, n3); MEGA_ALLOC(pool, dfe, n3);
   MEGA_ALLOC(pool, midx, n); MEGA_ALLOC(pool, acc, 1); MEGA_ALLOC(pool, st, 1);
   bool has_body = p->gravity[0] != 0.0 || p->gravity[1] != 0.0 || p->gravity[2] != 0.0;

@@ -96,14 +96,16 @@ __global__ void __launch_bounds__(256) k_defgrad(int32_t n, const int64_t* __res
   if (q == 0) {
     const double s0 = sdphi[3 * i], s1 = sdphi[3 * i + 1], s2 = sdphi[3 * i + 2];
     const double ui[3] = {ui0, ui1, ui2}, di[3] = {di0, di1, di2}, sd[3] = {s0, s1, s2};
-    double* o = fg + 18 * i;
+    double h[9], g[9];
 #pragma unroll
     for (int k = 0; k < 3; ++k)
 #pragma unroll
       for (int l = 0; l < 3; ++l) {
-        o[3 * k + l] = (k == l ? 1.0 : 0.0) + ((double)F[3 * k + l] + ui[k] * sd[l]);
-        o[9 + 3 * k + l] = (double)L[3 * k + l] + di[k] * sd[l];
+        h[3 * k + l] = (double)F[3 * k + l] + ui[k] * sd[l];
+        g[3 * k + l] = (double)L[3 * k + l] + di[k] * sd[l];
       }
+    store_fmi(fg, fg_ld(n), i, h);
+    store_g0(fg, fg_ld(n), i, sizeof(A) == 4, g);
     if (INTERP) {
       dsp_tot_phy[3 * i] += ph0;
       dsp_tot_phy[3 * i + 1] += ph1;
@@ -151,9 +153,9 @@ struct Trial {
 // without it their branches compile out of the J2 path.
 template <typename T, bool LEAN, bool DAM>
 __device__ __forceinline__ void stress_trial(const StressArgs& a, int64_t i, Trial<T, LEAN>& w) {
-  // F, G0 (18 doubles), stress and strain (6 each) as 16-byte loads
+  // F and G0 (18 planes), stress and strain (6 each) as 16-byte loads
   double fgi[18], sv[6], ev[6];
-  load_fg(a.fg, i, sizeof(T) == 4, fgi);  // float F - I and G0 in mixed precision
+  load_fg(a.fg, fg_ld(a.n), i, sizeof(T) == 4, a.add_g0, fgi);
   {
     const double2* s2 = reinterpret_cast<const double2*>(a.stress + 6 * i);
     const double2* e2 = reinterpret_cast<const double2*>(a.strain + 6 * i);
@@ -694,18 +696,20 @@ int launch_stress(cudaStream_t s, bool mixed, const StressArgs& a) {
     const int64_t lneed = grid_for(a.n, kLearnBlock);
     const unsigned lgrid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(lneed, (int64_t)device_sm_count() * 8));
     MEGA_TRY(cudaMemsetAsync(a.qcount, 0, sizeof(unsigned), s));
+    StressArgs qa = a;
+    qa.add_g0 = 0;  // the first kernel has advanced F already
     if (a.aux) {
       if (mixed) k_stress<float, float, true, true><<<grid, block, 0, s>>>(a);
       else k_stress<double, double, true, true><<<grid, block, 0, s>>>(a);
       MEGA_CHECK_LAUNCH();
-      if (mixed) k_stress_queue<float, float, true><<<lgrid, kLearnBlock, 0, s>>>(a);
-      else k_stress_queue<double, double, true><<<lgrid, kLearnBlock, 0, s>>>(a);
+      if (mixed) k_stress_queue<float, float, true><<<lgrid, kLearnBlock, 0, s>>>(qa);
+      else k_stress_queue<double, double, true><<<lgrid, kLearnBlock, 0, s>>>(qa);
     } else {
       if (mixed) k_stress<float, float, false, true><<<grid, block, 0, s>>>(a);
       else k_stress<double, double, false, true><<<grid, block, 0, s>>>(a);
       MEGA_CHECK_LAUNCH();
-      if (mixed) k_stress_queue<float, float, false><<<lgrid, kLearnBlock, 0, s>>>(a);
-      else k_stress_queue<double, double, false><<<lgrid, kLearnBlock, 0, s>>>(a);
+      if (mixed) k_stress_queue<float, float, false><<<lgrid, kLearnBlock, 0, s>>>(qa);
+      else k_stress_queue<double, double, false><<<lgrid, kLearnBlock, 0, s>>>(qa);
     }
   } else {
     if (a.aux) {

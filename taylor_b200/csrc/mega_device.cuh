@@ -159,46 +159,53 @@ __device__ __forceinline__ T tensor_norm_strain(const T v[6]) {
   return dsqrt<T>(v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + (v[3] * v[3] + v[4] * v[4] + v[5] * v[5]));
 }
 
-// The per-node deformation gradient F and increment gradient G0 between the
-// row gather and the stress update.  FP64: 18 doubles, F with its identity.
-// Mixed precision: 18 floats holding F - I and G0 (half the bytes; the
-// identity is added back in double when read, so F keeps its FP64 unit part
-// and the float carries only the displacement gradient, itself a float sum).
-// h[0..8] = F - I, h[9..17] = G0, row-major.
-__device__ __forceinline__ void store_fg(double* fg, int64_t i, bool mixed, const double h[18]) {
+// The deformation gradient and increment gradient between the row gather and
+// the stress update: F - I as 9 planes of doubles and G0 as 9 planes of doubles
+// (FP64) or floats (mixed), fg_ld(n) values a plane, component k (row-major) of
+// node i at [k ld + i], so the thread-per-node stress kernel's loads are
+// contiguous.  F - I is a state, not scratch: u_new = u_old + du makes
+// F_new = F_old + G0, so the row gather forms F afresh only on every 16th
+// step or so (FULL) and the stress update adds G0 on the others.  Keeping it
+// without the identity leaves the sums' rounding at 1e-16 of the displacement
+// gradient, below that of F itself.
+__host__ __device__ __forceinline__ int64_t fg_ld(int64_t n) { return (n + 31) & ~(int64_t)31; }
+__device__ __forceinline__ void store_fmi(double* fg, int64_t ld, int64_t i, const double h[9]) {
+#pragma unroll
+  for (int k = 0; k < 9; ++k) fg[k * ld + i] = h[k];
+}
+__device__ __forceinline__ void store_g0(double* fg, int64_t ld, int64_t i, bool mixed, const double h[9]) {
   if (mixed) {
-    float2* o = reinterpret_cast<float2*>(reinterpret_cast<float*>(fg) + 18 * i);
+    float* o = reinterpret_cast<float*>(fg + 9 * ld) + i;
 #pragma unroll
-    for (int k = 0; k < 9; ++k) o[k] = make_float2((float)h[2 * k], (float)h[2 * k + 1]);
+    for (int k = 0; k < 9; ++k) o[k * ld] = (float)h[k];
   } else {
-    double* o = fg + 18 * i;
+    double* o = fg + 9 * ld + i;
 #pragma unroll
-    for (int k = 0; k < 9; ++k) o[k] = ((k % 4) == 0 ? 1.0 : 0.0) + h[k];
-#pragma unroll
-    for (int k = 9; k < 18; ++k) o[k] = h[k];
+    for (int k = 0; k < 9; ++k) o[k * ld] = h[k];
   }
 }
-// F (with its identity) in f[0..8], G0 in f[9..17]
-__device__ __forceinline__ void load_fg(const double* fg, int64_t i, bool mixed, double f[18]) {
+// F (with its identity) in f[0..8], G0 in f[9..17]; add: F advances by G0 first
+__device__ __forceinline__ void load_fg(double* fg, int64_t ld, int64_t i, bool mixed, bool add, double f[18]) {
   if (mixed) {
-    const float2* g = reinterpret_cast<const float2*>(reinterpret_cast<const float*>(fg) + 18 * i);
+    const float* g = reinterpret_cast<const float*>(fg + 9 * ld) + i;
 #pragma unroll
-    for (int k = 0; k < 9; ++k) {
-      const float2 v = g[k];
-      f[2 * k] = (double)v.x;
-      f[2 * k + 1] = (double)v.y;
-    }
-#pragma unroll
-    for (int k = 0; k < 9; k += 4) f[k] = 1.0 + f[k];
+    for (int k = 0; k < 9; ++k) f[9 + k] = (double)g[k * ld];
   } else {
-    const double2* g = reinterpret_cast<const double2*>(fg + 18 * i);
+    const double* g = fg + 9 * ld + i;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) f[9 + k] = g[k * ld];
+  }
+#pragma unroll
+  for (int k = 0; k < 9; ++k) f[k] = fg[k * ld + i];
+  if (add) {
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
-      const double2 v = g[k];
-      f[2 * k] = v.x;
-      f[2 * k + 1] = v.y;
+      f[k] += f[9 + k];
+      fg[k * ld + i] = f[k];
     }
   }
+#pragma unroll
+  for (int k = 0; k < 9; k += 4) f[k] = 1.0 + f[k];
 }
 
 // Per-node material constants the force kernel needs (from PROPS(30,N)).

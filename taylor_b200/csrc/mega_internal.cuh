@@ -232,7 +232,8 @@ inline unsigned long long slot_sum(const unsigned long long* v) {
 // ---------------- launchers (force.cu)
 struct StressArgs {
   int32_t n;
-  const double* fg;          // 18 per node: F (row-major 3x3), G0 (3x3)
+  double* fg;                // F - I and G0 (mega_device.cuh: planes of fg_ld(n) values)
+  int add_g0;                // F advances by G0 here (the row gather formed G0 alone)
   const uint16_t* matidx;
   const MatEntry* mats;
   const double* vol;
@@ -284,7 +285,7 @@ using NsniS = NsniArr<double>;
 using NsniSF = NsniArr<float>;
 struct NsniStepArgs {
   int32_t n;
-  const double* fg;          // F, G0 of this step
+  double* fg;                // F - I and G0 of this step
   const double* stress_old;  // the stress before this step's update
   const double* stress_new;
   const double* sml;         // SM_LEN (6, n)

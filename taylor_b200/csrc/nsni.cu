@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(128) k_nsni_stress(NsniStepArgs a) {
   double work = 0.0;
   if (i < a.n) {
     double g[18];
-    load_fg(a.fg, i, sizeof(WV) == 4, g);  // the mixed step stores F - I and G0 as floats
+    load_fg(a.fg, fg_ld(a.n), i, sizeof(WV) == 4, false, g);  // (the stress kernel has advanced F)
     double F[3][3], G0[3][3], IF[3][3], L[3][3], R[3][3], dstr[6], D[6];
 #pragma unroll
     for (int k = 0; k < 3; ++k)

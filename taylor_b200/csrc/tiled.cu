@@ -10,7 +10,8 @@
 // warp's loads are contiguous (build_slices), and the neighbour data the tile needs
 // -- (u_tot, du) for the deformation gradient, T_i for the force -- is staged
 // in shared memory once per tile:
-//   k_defgrad_t  F = I + sum_J (u_J - u_i) (x) g + u_i (x) sum g,  G0 likewise
+//   k_defgrad_t  G0 = sum_J (du_J - du_i) (x) g + du_i (x) sum g, and on FULL
+//                steps F - I likewise from u (on the others F advances by G0)
 //   k_force_t    f_J = sum_i T_i g^T_iJ, then the corrector / predictor
 // The summation order is fixed by the list order, so results are
 // deterministic, and identical in exact arithmetic to force.cu's.
@@ -436,18 +437,25 @@ __device__ __forceinline__ SRec load_srec(const float* base, int64_t p, int64_t 
   return SRec{__ldg(sp), __ldg(sp + 1), __ldg(sp + 2)};
 }
 
+// FULL: F - I is formed besides G0.  Without it the gather stages and reads
+// the increments alone, half the shared-memory traffic and sums: at 130 k nodes
+// FP64 ran at 75 % of the L1 data pipe with both, half of it staged reads.
 // NS: the NSNI gradients of the incremental displacement gradient ride
 // along, H_i(k, q) = sum_J S_q(i, J) du_J,k, formed like L as
 // sum_J S_q (du_J - du_i) + du_i,k sum_J S_q (FINT.F90:728-737 layout).
-template <typename A, bool F64, bool INTERP, int KG, int KU, bool NS = false>
-__global__ void __launch_bounds__(64 * KG, (F64 ? 12 : (NS ? 8 : 16)) / KG > 0 ? (F64 ? 12 : (NS ? 8 : 16)) / KG : 1) k_defgrad_t(int32_t n, int32_t R, int32_t jmax,
-                                                   NsniTiles ns, SliceView sv,
-                                                   const int64_t* __restrict__ rowptr, const void* __restrict__ pk,
-                                                   const int32_t* __restrict__ jset, const int32_t* __restrict__ jcnt,
-                                                   const double* __restrict__ dsp, const double* __restrict__ dsp_tot,
-                                                   const double* __restrict__ sdphi, const double* __restrict__ shp,
-                                                   double* __restrict__ dsp_tot_phy, double* __restrict__ fg,
-                                                   StepAccum* __restrict__ acc) {
+template <bool F64, int KG, bool NS, bool FULL>
+constexpr int defgrad_blocks() {  // blocks per SM the register cap asks for
+  const int w = NS ? 8 : (F64 && FULL ? 12 : 16);
+  return w / KG > 0 ? w / KG : 1;
+}
+
+template <typename A, bool F64, bool INTERP, int KG, int KU, bool NS, bool FULL>
+__global__ void __launch_bounds__(64 * KG, defgrad_blocks<F64, KG, NS, FULL>())
+    k_defgrad_t(int32_t n, int32_t R, int32_t jmax, NsniTiles ns, SliceView sv, const int64_t* __restrict__ rowptr,
+                const void* __restrict__ pk, const int32_t* __restrict__ jset, const int32_t* __restrict__ jcnt,
+                const double* __restrict__ dsp, const double* __restrict__ dsp_tot,
+                const double* __restrict__ sdphi, const double* __restrict__ shp, double* __restrict__ dsp_tot_phy,
+                double* __restrict__ fg, StepAccum* __restrict__ acc) {
   extern __shared__ double sm[];
   if (acc && blockIdx.x == 0 && threadIdx.x < kSlots) {
     acc->newton_iters[threadIdx.x] = 0ull;
@@ -456,14 +464,13 @@ __global__ void __launch_bounds__(64 * KG, (F64 ? 12 : (NS ? 8 : 16)) / KG > 0 ?
   const int64_t t = blockIdx.x;
   const int cnt = jcnt[t];
   const int32_t* js = jset + t * (int64_t)jmax;
-  // Staged neighbour displacements.  FP64: u_J and du_J as doubles.  Mixed:
-  // float offsets from the tile's first node r0 (u_J - u_r0, du_J - du_r0),
-  // half the shared-memory traffic, one array per component (value k of
-  // rank l at sf[k * cnt + l]: lanes with distinct l mod 32 read distinct
-  // banks); the differences u_J - u_i are formed between offsets, exact up
-  // to float rounding of the offsets.
-  double* su = sm;
-  double* sd = sm + 3 * cnt;
+  // Staged neighbour displacements, du_J (FULL: and u_J), one array per
+  // component (value k of rank l at [k cnt + l]: lanes with distinct ranks
+  // modulo the banks read distinct banks).  FP64 as doubles; mixed as float
+  // offsets from the tile's first node r0 (du_J - du_r0, u_J - u_r0), half
+  // the shared-memory traffic: the differences d_J - d_i are formed between
+  // offsets, exact up to float rounding of the offsets.
+  double* sd = sm;
   float* sf = reinterpret_cast<float*>(sm);
   const int64_t r0 = t * R;
   const int slot = threadIdx.x / KG;
@@ -492,65 +499,77 @@ __global__ void __launch_bounds__(64 * KG, (F64 ? 12 : (NS ? 8 : 16)) / KG > 0 ?
       if constexpr (NS) csr[u] = load_srec(ns.srow, p0 + u * KG, pend);
     }
   }
-  double ur0 = 0.0, ur1 = 0.0, ur2 = 0.0, dr0 = 0.0, dr1 = 0.0, dr2 = 0.0;
+  double ur[3] = {0.0, 0.0, 0.0}, dr[3] = {0.0, 0.0, 0.0};
   if (!F64) {
-    ur0 = dsp_tot[3 * r0]; ur1 = dsp_tot[3 * r0 + 1]; ur2 = dsp_tot[3 * r0 + 2];
-    dr0 = dsp[3 * r0]; dr1 = dsp[3 * r0 + 1]; dr2 = dsp[3 * r0 + 2];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      dr[k] = dsp[3 * r0 + k];
+      if (FULL) ur[k] = dsp_tot[3 * r0 + k];
+    }
   }
   for (int l = threadIdx.x; l < cnt; l += blockDim.x) {
     const int64_t g = js[l];
-    const double a0 = dsp_tot[3 * g], a1 = dsp_tot[3 * g + 1], a2 = dsp_tot[3 * g + 2];
-    const double b0 = dsp[3 * g], b1 = dsp[3 * g + 1], b2 = dsp[3 * g + 2];
-    if (F64) {
-      su[3 * l] = a0; su[3 * l + 1] = a1; su[3 * l + 2] = a2;
-      sd[3 * l] = b0; sd[3 * l + 1] = b1; sd[3 * l + 2] = b2;
-    } else {
-      sf[l] = (float)(a0 - ur0); sf[cnt + l] = (float)(a1 - ur1); sf[2 * cnt + l] = (float)(a2 - ur2);
-      sf[3 * cnt + l] = (float)(b0 - dr0); sf[4 * cnt + l] = (float)(b1 - dr1); sf[5 * cnt + l] = (float)(b2 - dr2);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const double b = dsp[3 * g + k];
+      const double a = FULL ? dsp_tot[3 * g + k] : 0.0;
+      if (F64) {
+        sd[k * cnt + l] = b;
+        if (FULL) sd[(3 + k) * cnt + l] = a;
+      } else {
+        sf[k * cnt + l] = (float)(b - dr[k]);
+        if (FULL) sf[(3 + k) * cnt + l] = (float)(a - ur[k]);
+      }
     }
   }
   __syncthreads();
   if (!valid) return;
-  const double ui0 = dsp_tot[3 * i], ui1 = dsp_tot[3 * i + 1], ui2 = dsp_tot[3 * i + 2];
-  const double di0 = dsp[3 * i], di1 = dsp[3 * i + 1], di2 = dsp[3 * i + 2];
-  const float fu0 = (float)(ui0 - ur0), fu1 = (float)(ui1 - ur1), fu2 = (float)(ui2 - ur2);
-  const float fd0 = (float)(di0 - dr0), fd1 = (float)(di1 - dr1), fd2 = (float)(di2 - dr2);
-  A F[9], L[9];
+  double ui[3] = {0.0, 0.0, 0.0}, di[3];
+  A fu[3], fd[3];  // this row's values as the staged ones are held
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    di[k] = dsp[3 * i + k];
+    fd[k] = F64 ? (A)di[k] : (A)(float)(di[k] - dr[k]);
+    if (FULL) {
+      ui[k] = dsp_tot[3 * i + k];
+      fu[k] = F64 ? (A)ui[k] : (A)(float)(ui[k] - ur[k]);
+    }
+  }
+  A F[FULL ? 9 : 1], L[9];
   double H[NS ? 18 : 1];  // NSNI: exact products of the float S and differences, summed in double
 #pragma unroll
-  for (int k = 0; k < 9; ++k) { F[k] = A(0); L[k] = A(0); }
+  for (int k = 0; k < 9; ++k) L[k] = A(0);
+#pragma unroll
+  for (int k = 0; k < (FULL ? 9 : 1); ++k) F[k] = A(0);
 #pragma unroll
   for (int k = 0; k < (NS ? 18 : 1); ++k) H[k] = 0.0;
-  double ph0 = 0.0, ph1 = 0.0, ph2 = 0.0;
+  double ph[3] = {0.0, 0.0, 0.0};
   // One entry: F += (u_J - u_i) (x) g, L += (d_J - d_i) (x) g (+ phi d_J),
   // H(k, q) += S_q (d_J - d_i)_k.
   auto body = [&](int it, const Rec<F64>& rec, const SRec& sr) {
-    const A g0 = (A)rec.x(), g1 = (A)rec.y(), g2 = (A)rec.z();
+    const A g[3] = {(A)rec.x(), (A)rec.y(), (A)rec.z()};
     const int l = rec.l();
-    A u0, u1, u2, d0, d1, d2;
-    double dj0, dj1, dj2;  // du_J itself, for the per-step interpolation
-    if (F64) {
-      u0 = (A)(su[3 * l] - ui0); u1 = (A)(su[3 * l + 1] - ui1); u2 = (A)(su[3 * l + 2] - ui2);
-      dj0 = sd[3 * l]; dj1 = sd[3 * l + 1]; dj2 = sd[3 * l + 2];
-      d0 = (A)(dj0 - di0); d1 = (A)(dj1 - di1); d2 = (A)(dj2 - di2);
-    } else {
-      const float* v = sf + l;
-      const float v3 = v[3 * cnt], v4 = v[4 * cnt], v5 = v[5 * cnt];
-      u0 = (A)(v[0] - fu0); u1 = (A)(v[cnt] - fu1); u2 = (A)(v[2 * cnt] - fu2);
-      d0 = (A)(v3 - fd0); d1 = (A)(v4 - fd1); d2 = (A)(v5 - fd2);
-      if (INTERP) { dj0 = dr0 + (double)v3; dj1 = dr1 + (double)v4; dj2 = dr2 + (double)v5; }
-      else { dj0 = dj1 = dj2 = 0.0; }
+    A v[3], d[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      v[k] = F64 ? (A)sd[k * cnt + l] : (A)sf[k * cnt + l];
+      d[k] = v[k] - fd[k];
     }
-    F[0] += u0 * g0; F[1] += u0 * g1; F[2] += u0 * g2;
-    F[3] += u1 * g0; F[4] += u1 * g1; F[5] += u1 * g2;
-    F[6] += u2 * g0; F[7] += u2 * g1; F[8] += u2 * g2;
-    L[0] += d0 * g0; L[1] += d0 * g1; L[2] += d0 * g2;
-    L[3] += d1 * g0; L[4] += d1 * g1; L[5] += d1 * g2;
-    L[6] += d2 * g0; L[7] += d2 * g1; L[8] += d2 * g2;
+    if constexpr (FULL) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const A u = (F64 ? (A)sd[(3 + k) * cnt + l] : (A)sf[(3 + k) * cnt + l]) - fu[k];
+        F[3 * k] += u * g[0]; F[3 * k + 1] += u * g[1]; F[3 * k + 2] += u * g[2];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      L[3 * k] += d[k] * g[0]; L[3 * k + 1] += d[k] * g[1]; L[3 * k + 2] += d[k] * g[2];
+    }
     if constexpr (NS) {
       const double sq[6] = {(double)sr.a.x, (double)sr.a.y, (double)sr.b.x, (double)sr.b.y, (double)sr.c.x,
                             (double)sr.c.y};
-      const double e0 = (double)d0, e1 = (double)d1, e2 = (double)d2;
+      const double e0 = (double)d[0], e1 = (double)d[1], e2 = (double)d[2];
 #pragma unroll
       for (int c = 0; c < 6; ++c) { H[c] += sq[c] * e0; H[6 + c] += sq[c] * e1; H[12 + c] += sq[c] * e2; }
     }
@@ -558,7 +577,8 @@ __global__ void __launch_bounds__(64 * KG, (F64 ? 12 : (NS ? 8 : 16)) / KG > 0 ?
       const int64_t p = p0 + (int64_t)KG * it;
       if (p < pend) {  // (not a pad)
         const double s = shp[p];
-        ph0 += s * dj0; ph1 += s * dj1; ph2 += s * dj2;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) ph[k] += s * (F64 ? (double)v[k] : dr[k] + (double)v[k]);
       }
     }
   };
@@ -600,7 +620,7 @@ __global__ void __launch_bounds__(64 * KG, (F64 ? 12 : (NS ? 8 : 16)) / KG > 0 ?
   for (int o = 1; o < KG; o <<= 1) {
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
-      F[k] += __shfl_xor_sync(gmask, F[k], o);
+      if constexpr (FULL) F[k] += __shfl_xor_sync(gmask, F[k], o);
       L[k] += __shfl_xor_sync(gmask, L[k], o);
     }
     if constexpr (NS) {
@@ -608,13 +628,11 @@ __global__ void __launch_bounds__(64 * KG, (F64 ? 12 : (NS ? 8 : 16)) / KG > 0 ?
       for (int k = 0; k < 18; ++k) H[k] += __shfl_xor_sync(gmask, H[k], o);
     }
     if (INTERP) {
-      ph0 += __shfl_xor_sync(gmask, ph0, o);
-      ph1 += __shfl_xor_sync(gmask, ph1, o);
-      ph2 += __shfl_xor_sync(gmask, ph2, o);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) ph[k] += __shfl_xor_sync(gmask, ph[k], o);
     }
   }
   if (q == 0) {
-    const double ui[3] = {ui0, ui1, ui2}, di[3] = {di0, di1, di2};
     if constexpr (NS) {
       double ss[6];
 #pragma unroll
@@ -625,19 +643,19 @@ __global__ void __launch_bounds__(64 * KG, (F64 ? 12 : (NS ? 8 : 16)) / KG > 0 ?
         for (int c = 0; c < 6; ++c) ns.hq[18 * i + 6 * k + c] = H[6 * k + c] + di[k] * ss[c];
     }
     const double sd3[3] = {sdphi[3 * i], sdphi[3 * i + 1], sdphi[3 * i + 2]};
-    double h[18];
+    const int64_t ld = fg_ld(n);
+    double h[9];
 #pragma unroll
-    for (int k = 0; k < 3; ++k)
+    for (int k = 0; k < 9; ++k) h[k] = (double)L[k] + di[k / 3] * sd3[k % 3];
+    store_g0(fg, ld, i, !F64, h);
+    if constexpr (FULL) {
 #pragma unroll
-      for (int l = 0; l < 3; ++l) {
-        h[3 * k + l] = (double)F[3 * k + l] + ui[k] * sd3[l];
-        h[9 + 3 * k + l] = (double)L[3 * k + l] + di[k] * sd3[l];
-      }
-    store_fg(fg, i, !F64, h);
+      for (int k = 0; k < 9; ++k) h[k] = (double)F[k] + ui[k / 3] * sd3[k % 3];
+      store_fmi(fg, ld, i, h);
+    }
     if (INTERP) {
-      dsp_tot_phy[3 * i] += ph0;
-      dsp_tot_phy[3 * i + 1] += ph1;
-      dsp_tot_phy[3 * i + 2] += ph2;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) dsp_tot_phy[3 * i + k] += ph[k];
     }
   }
 }
@@ -935,14 +953,14 @@ __device__ __forceinline__ void staged_rec(const unsigned char* rec, int64_t rec
   o.r = reinterpret_cast<const uint16_t*>(z + recmax)[p];
 }
 
+// (the increments alone: FULL steps take the register kernel)
 template <typename A, bool F64, bool INTERP, int KG>
-__global__ void __launch_bounds__(64 * KG) k_defgrad_b(int32_t n, int32_t R, int32_t jmax, int32_t recmax, SliceView sv,
-                                                       const int64_t* __restrict__ rowptr, const void* __restrict__ pk,
-                                                       const int32_t* __restrict__ jset, const int32_t* __restrict__ jcnt,
-                                                       const double* __restrict__ dsp, const double* __restrict__ dsp_tot,
-                                                       const double* __restrict__ sdphi, const double* __restrict__ shp,
-                                                       double* __restrict__ dsp_tot_phy, double* __restrict__ fg,
-                                                       StepAccum* __restrict__ acc, unsigned* __restrict__ status) {
+__global__ void __launch_bounds__(64 * KG)
+    k_defgrad_b(int32_t n, int32_t R, int32_t jmax, int32_t recmax, SliceView sv, const int64_t* __restrict__ rowptr,
+                const void* __restrict__ pk, const int32_t* __restrict__ jset, const int32_t* __restrict__ jcnt,
+                const double* __restrict__ dsp, const double* __restrict__ sdphi, const double* __restrict__ shp,
+                double* __restrict__ dsp_tot_phy, double* __restrict__ fg, StepAccum* __restrict__ acc,
+                unsigned* __restrict__ status) {
   constexpr int RB = F64 ? 26 : 16;
   extern __shared__ __align__(128) unsigned char smb[];
   __shared__ uint64_t bar[kChunks];
@@ -956,30 +974,25 @@ __global__ void __launch_bounds__(64 * KG) k_defgrad_b(int32_t n, int32_t R, int
   issue_records<F64>(bar, smb, pk, sv.nrec, e0, ne, recmax);
   const int cnt = jcnt[t];
   const int32_t* js = jset + t * (int64_t)jmax;
-  unsigned char* stg = smb + (size_t)recmax * RB;
-  double* su = reinterpret_cast<double*>(stg);
-  double* sd = su + 3 * cnt;
-  float* sf = reinterpret_cast<float*>(stg);  // mixed: value k of rank l at sf[k * cnt + l]
+  double* sd = reinterpret_cast<double*>(smb + (size_t)recmax * RB);
+  float* sf = reinterpret_cast<float*>(sd);  // value k of rank l at [k cnt + l]
   const int slot = threadIdx.x / KG;
   const int64_t i = r0 + sv.ord[r0 + slot];
   const int q = threadIdx.x & (KG - 1);
   const unsigned gmask = group_mask<KG>();
   const bool valid = i < n;
-  double ur0 = 0.0, ur1 = 0.0, ur2 = 0.0, dr0 = 0.0, dr1 = 0.0, dr2 = 0.0;
+  double dr[3] = {0.0, 0.0, 0.0};
   if (!F64) {
-    ur0 = dsp_tot[3 * r0]; ur1 = dsp_tot[3 * r0 + 1]; ur2 = dsp_tot[3 * r0 + 2];
-    dr0 = dsp[3 * r0]; dr1 = dsp[3 * r0 + 1]; dr2 = dsp[3 * r0 + 2];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) dr[k] = dsp[3 * r0 + k];
   }
   for (int l = threadIdx.x; l < cnt; l += blockDim.x) {
     const int64_t g = js[l];
-    const double a0 = dsp_tot[3 * g], a1 = dsp_tot[3 * g + 1], a2 = dsp_tot[3 * g + 2];
-    const double b0 = dsp[3 * g], b1 = dsp[3 * g + 1], b2 = dsp[3 * g + 2];
-    if (F64) {
-      su[3 * l] = a0; su[3 * l + 1] = a1; su[3 * l + 2] = a2;
-      sd[3 * l] = b0; sd[3 * l + 1] = b1; sd[3 * l + 2] = b2;
-    } else {
-      sf[l] = (float)(a0 - ur0); sf[cnt + l] = (float)(a1 - ur1); sf[2 * cnt + l] = (float)(a2 - ur2);
-      sf[3 * cnt + l] = (float)(b0 - dr0); sf[4 * cnt + l] = (float)(b1 - dr1); sf[5 * cnt + l] = (float)(b2 - dr2);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const double b = dsp[3 * g + k];
+      if (F64) sd[k * cnt + l] = b;
+      else sf[k * cnt + l] = (float)(b - dr[k]);
     }
   }
   __syncthreads();
@@ -995,46 +1008,36 @@ __global__ void __launch_bounds__(64 * KG) k_defgrad_b(int32_t n, int32_t R, int
     p0 = rowptr[i] + q;
     pend = rowptr[i + 1];
   }
-  const double ui0 = dsp_tot[3 * i], ui1 = dsp_tot[3 * i + 1], ui2 = dsp_tot[3 * i + 2];
-  const double di0 = dsp[3 * i], di1 = dsp[3 * i + 1], di2 = dsp[3 * i + 2];
-  const float fu0 = (float)(ui0 - ur0), fu1 = (float)(ui1 - ur1), fu2 = (float)(ui2 - ur2);
-  const float fd0 = (float)(di0 - dr0), fd1 = (float)(di1 - dr1), fd2 = (float)(di2 - dr2);
-  A F[9], L[9];
+  double di[3];
+  A fd[3], L[9];
 #pragma unroll
-  for (int k = 0; k < 9; ++k) { F[k] = A(0); L[k] = A(0); }
-  double ph0 = 0.0, ph1 = 0.0, ph2 = 0.0;
+  for (int k = 0; k < 3; ++k) {
+    di[k] = dsp[3 * i + k];
+    fd[k] = F64 ? (A)di[k] : (A)(float)(di[k] - dr[k]);
+  }
+#pragma unroll
+  for (int k = 0; k < 9; ++k) L[k] = A(0);
+  double ph[3] = {0.0, 0.0, 0.0};
   if (ok) {
 #pragma unroll 4
     for (int it = 0; it < walk.nit; ++it) {
       Rec<F64> rec;
       staged_rec(smb, recmax, walk.at(it) - 32 * e0, rec);
-      const A g0 = (A)rec.x(), g1 = (A)rec.y(), g2 = (A)rec.z();
+      const A g[3] = {(A)rec.x(), (A)rec.y(), (A)rec.z()};
       const int l = rec.l();
-      A u0, u1, u2, d0, d1, d2;
-      double dj0, dj1, dj2;
-      if (F64) {
-        u0 = (A)(su[3 * l] - ui0); u1 = (A)(su[3 * l + 1] - ui1); u2 = (A)(su[3 * l + 2] - ui2);
-        dj0 = sd[3 * l]; dj1 = sd[3 * l + 1]; dj2 = sd[3 * l + 2];
-        d0 = (A)(dj0 - di0); d1 = (A)(dj1 - di1); d2 = (A)(dj2 - di2);
-      } else {
-        const float* v = sf + l;
-        const float v3 = v[3 * cnt], v4 = v[4 * cnt], v5 = v[5 * cnt];
-        u0 = (A)(v[0] - fu0); u1 = (A)(v[cnt] - fu1); u2 = (A)(v[2 * cnt] - fu2);
-        d0 = (A)(v3 - fd0); d1 = (A)(v4 - fd1); d2 = (A)(v5 - fd2);
-        if (INTERP) { dj0 = dr0 + (double)v3; dj1 = dr1 + (double)v4; dj2 = dr2 + (double)v5; }
-        else { dj0 = dj1 = dj2 = 0.0; }
+      A v[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        v[k] = F64 ? (A)sd[k * cnt + l] : (A)sf[k * cnt + l];
+        const A d = v[k] - fd[k];
+        L[3 * k] += d * g[0]; L[3 * k + 1] += d * g[1]; L[3 * k + 2] += d * g[2];
       }
-      F[0] += u0 * g0; F[1] += u0 * g1; F[2] += u0 * g2;
-      F[3] += u1 * g0; F[4] += u1 * g1; F[5] += u1 * g2;
-      F[6] += u2 * g0; F[7] += u2 * g1; F[8] += u2 * g2;
-      L[0] += d0 * g0; L[1] += d0 * g1; L[2] += d0 * g2;
-      L[3] += d1 * g0; L[4] += d1 * g1; L[5] += d1 * g2;
-      L[6] += d2 * g0; L[7] += d2 * g1; L[8] += d2 * g2;
       if (INTERP) {
         const int64_t p = p0 + (int64_t)KG * it;
         if (p < pend) {
           const double s = shp[p];
-          ph0 += s * dj0; ph1 += s * dj1; ph2 += s * dj2;
+#pragma unroll
+          for (int k = 0; k < 3; ++k) ph[k] += s * (F64 ? (double)v[k] : dr[k] + (double)v[k]);
         }
       }
     }
@@ -1042,35 +1045,24 @@ __global__ void __launch_bounds__(64 * KG) k_defgrad_b(int32_t n, int32_t R, int
 #pragma unroll
   for (int o = 1; o < KG; o <<= 1) {
 #pragma unroll
-    for (int k = 0; k < 9; ++k) {
-      F[k] += __shfl_xor_sync(gmask, F[k], o);
-      L[k] += __shfl_xor_sync(gmask, L[k], o);
-    }
+    for (int k = 0; k < 9; ++k) L[k] += __shfl_xor_sync(gmask, L[k], o);
     if (INTERP) {
-      ph0 += __shfl_xor_sync(gmask, ph0, o);
-      ph1 += __shfl_xor_sync(gmask, ph1, o);
-      ph2 += __shfl_xor_sync(gmask, ph2, o);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) ph[k] += __shfl_xor_sync(gmask, ph[k], o);
     }
   }
   if (q == 0) {
     if (!ok) {
       atomicOr(status, (unsigned)MEGA_ST_WAIT_TIMEOUT);
     } else {
-      const double ui[3] = {ui0, ui1, ui2}, di[3] = {di0, di1, di2};
       const double sd3[3] = {sdphi[3 * i], sdphi[3 * i + 1], sdphi[3 * i + 2]};
-      double h[18];
+      double h[9];
 #pragma unroll
-      for (int k = 0; k < 3; ++k)
-#pragma unroll
-        for (int l = 0; l < 3; ++l) {
-          h[3 * k + l] = (double)F[3 * k + l] + ui[k] * sd3[l];
-          h[9 + 3 * k + l] = (double)L[3 * k + l] + di[k] * sd3[l];
-        }
-      store_fg(fg, i, !F64, h);
+      for (int k = 0; k < 9; ++k) h[k] = (double)L[k] + di[k / 3] * sd3[k % 3];
+      store_g0(fg, fg_ld(n), i, !F64, h);
       if (INTERP) {
-        dsp_tot_phy[3 * i] += ph0;
-        dsp_tot_phy[3 * i + 1] += ph1;
-        dsp_tot_phy[3 * i + 2] += ph2;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) dsp_tot_phy[3 * i + k] += ph[k];
       }
     }
   }
@@ -1317,6 +1309,9 @@ int gather_records32(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t
 // (16, 1), (16, 2) with register-held streams (four times the threads per
 // staged neighbour of KG = 4: the NSNI force gather stages 27 values a node).
 constexpr int kVariants = kTiledVariants;
+// records in flight per lane of the FULL gathers (one step in 16: one form
+// per lane count; the count in flight does not change a row's sum)
+constexpr int kFullKU = 2;
 // dynamic shared memory a streamed-variant block may ask for: sm_100's 227 KB
 // per block less room for the kernels' static shared memory (under 1 KB)
 constexpr int kBulkSmemMax = 227 * 1024 - 1024;
@@ -1327,15 +1322,21 @@ static int raise_smem(K k, int lim) {
   return 0;
 }
 
+template <int KG, int KU, bool FULL>
+static int configure_defgrad(int lim) {
+  int r = 0;
+  if ((r = raise_smem(k_defgrad_t<float, false, true, KG, KU, false, FULL>, lim))) return r;
+  if ((r = raise_smem(k_defgrad_t<float, false, false, KG, KU, false, FULL>, lim))) return r;
+  if ((r = raise_smem(k_defgrad_t<float, false, true, KG, KU, true, FULL>, lim))) return r;
+  if ((r = raise_smem(k_defgrad_t<float, false, false, KG, KU, true, FULL>, lim))) return r;
+  if ((r = raise_smem(k_defgrad_t<double, true, true, KG, KU, false, FULL>, lim))) return r;
+  return raise_smem(k_defgrad_t<double, true, false, KG, KU, false, FULL>, lim);
+}
+
 template <int KG, int KU>
 static int configure_variant(int lim) {
   int r = 0;
-  if ((r = raise_smem(k_defgrad_t<float, false, true, KG, KU>, lim))) return r;
-  if ((r = raise_smem(k_defgrad_t<float, false, false, KG, KU>, lim))) return r;
-  if ((r = raise_smem(k_defgrad_t<float, false, true, KG, KU, true>, lim))) return r;
-  if ((r = raise_smem(k_defgrad_t<float, false, false, KG, KU, true>, lim))) return r;
-  if ((r = raise_smem(k_defgrad_t<double, true, true, KG, KU>, lim))) return r;
-  if ((r = raise_smem(k_defgrad_t<double, true, false, KG, KU>, lim))) return r;
+  if ((r = configure_defgrad<KG, KU, false>(lim))) return r;
   if ((r = raise_smem(k_force_t<float, float, false, KG, KU>, lim))) return r;
   if ((r = raise_smem(k_force_t<float, float, false, KG, KU, true>, lim))) return r;
   return raise_smem(k_force_t<double, double, true, KG, KU>, lim);
@@ -1379,7 +1380,8 @@ int configure_tiled_kernels() {
   if ((r = configure_variant<4, 4>(lim)) || (r = configure_variant<4, 2>(lim)) ||
       (r = configure_variant<4, 1>(lim)) || (r = configure_variant<8, 2>(lim)) ||
       (r = configure_variant<16, 1>(lim)) || (r = configure_variant<16, 2>(lim)) ||
-      (r = configure_bulk<4>(kBulkSmemMax)) || (r = configure_bulk<8>(kBulkSmemMax)))
+      (r = configure_defgrad<4, kFullKU, true>(lim)) || (r = configure_defgrad<8, kFullKU, true>(lim)) ||
+      (r = configure_defgrad<16, kFullKU, true>(lim)) || (r = configure_bulk<4>(kBulkSmemMax)) || (r = configure_bulk<8>(kBulkSmemMax)))
     return r;
   done = true;
   return 0;
@@ -1390,79 +1392,74 @@ int tiled_variants() { return kVariants; }
 bool tiled_variant_fits(const TileSet& ts, bool mixed, int variant, bool force, bool has_body) {
   if (variant < 0 || variant >= kVariants) return false;
   if (variant < 4 || variant > 5) return true;  // register variants
-  const size_t stage = force ? (mixed ? sizeof(float) : sizeof(double)) * (has_body ? 12 : 9) : (mixed ? 24 : 48);
+  const size_t stage = force ? (mixed ? sizeof(float) : sizeof(double)) * (has_body ? 12 : 9) : (mixed ? 12 : 24);
   return (size_t)ts.recmax * (mixed ? 16 : 26) + stage * (size_t)ts.maxcnt <= (size_t)g_bulk_lim;
 }
 
+// one launch's arguments of the row gather
+struct DefgradArgs {
+  bool mixed, interp;
+  int32_t n;
+  const TileSet& ts;
+  const NsniTiles* ns;
+  const int64_t* rowptr;
+  const void* pk;
+  const double *dsp, *dsp_tot, *sdphi, *shp;
+  double *dsp_tot_phy, *fg;
+  StepAccum* acc;
+  unsigned* status;
+};
+
 template <int KG>
-static int defgrad_bulk(cudaStream_t s, bool mixed, bool interp, int32_t n, const TileSet& ts,
-                        const int64_t* rowptr, const void* pk, const double* dsp, const double* dsp_tot,
-                        const double* sdphi, const double* shp, double* dsp_tot_phy, double* fg, StepAccum* acc,
-                        unsigned* status) {
-  const size_t smem = (size_t)ts.recmax * (mixed ? 16 : 26) + (mixed ? 24 : 48) * (size_t)ts.maxcnt;
+static int defgrad_bulk(cudaStream_t s, const DefgradArgs& d) {
+  const TileSet& ts = d.ts;
+  const size_t smem = (size_t)ts.recmax * (d.mixed ? 16 : 26) + (d.mixed ? 12 : 24) * (size_t)ts.maxcnt;
   if (smem > (size_t)g_bulk_lim) return MEGA_ERR_UNSUPPORTED;
-  const unsigned grid = (unsigned)ts.ntiles;
-  const int block = ts.R * KG;
-  if (mixed) {
-    auto k = interp ? k_defgrad_b<float, false, true, KG> : k_defgrad_b<float, false, false, KG>;
-    k<<<grid, block, smem, s>>>(n, ts.R, ts.jmax, ts.recmax, ts.view(), rowptr, pk, ts.jset, ts.jcnt, dsp, dsp_tot, sdphi, shp,
-                                dsp_tot_phy, fg, acc, status);
-  } else {
-    auto k = interp ? k_defgrad_b<double, true, true, KG> : k_defgrad_b<double, true, false, KG>;
-    k<<<grid, block, smem, s>>>(n, ts.R, ts.jmax, ts.recmax, ts.view(), rowptr, pk, ts.jset, ts.jcnt, dsp, dsp_tot, sdphi, shp,
-                                dsp_tot_phy, fg, acc, status);
-  }
+  auto k = d.mixed ? (d.interp ? k_defgrad_b<float, false, true, KG> : k_defgrad_b<float, false, false, KG>)
+                   : (d.interp ? k_defgrad_b<double, true, true, KG> : k_defgrad_b<double, true, false, KG>);
+  k<<<(unsigned)ts.ntiles, ts.R * KG, smem, s>>>(d.n, ts.R, ts.jmax, ts.recmax, ts.view(), d.rowptr, d.pk, ts.jset,
+                                                 ts.jcnt, d.dsp, d.sdphi, d.shp, d.dsp_tot_phy, d.fg, d.acc,
+                                                 d.status);
   return 0;
 }
 
-template <int KG, int KU>
-static void defgrad_variant(cudaStream_t s, bool mixed, bool interp, int32_t n, const TileSet& ts,
-                            const NsniTiles* ns, const int64_t* rowptr, const void* pk, const double* dsp,
-                            const double* dsp_tot, const double* sdphi, const double* shp, double* dsp_tot_phy,
-                            double* fg, StepAccum* acc) {
-  const size_t smem = (mixed ? 24 : 48) * (size_t)ts.maxcnt;
-  const unsigned grid = (unsigned)ts.ntiles;
-  const int block = ts.R * KG;
-  const NsniTiles nz = ns ? *ns : NsniTiles();
-  if (mixed) {
-    auto k = ns ? (interp ? k_defgrad_t<float, false, true, KG, KU, true> : k_defgrad_t<float, false, false, KG, KU, true>)
-                : (interp ? k_defgrad_t<float, false, true, KG, KU> : k_defgrad_t<float, false, false, KG, KU>);
-    k<<<grid, block, smem, s>>>(n, ts.R, ts.jmax, nz, ts.view(), rowptr, pk, ts.jset, ts.jcnt, dsp, dsp_tot, sdphi, shp,
-                                dsp_tot_phy, fg, acc);
-  } else {
-    auto k = interp ? k_defgrad_t<double, true, true, KG, KU> : k_defgrad_t<double, true, false, KG, KU>;
-    k<<<grid, block, smem, s>>>(n, ts.R, ts.jmax, nz, ts.view(), rowptr, pk, ts.jset, ts.jcnt, dsp, dsp_tot, sdphi, shp,
-                                dsp_tot_phy, fg, acc);
-  }
+template <int KG, int KU, bool FULL = false>
+static void defgrad_variant(cudaStream_t s, const DefgradArgs& d) {
+  const TileSet& ts = d.ts;
+  const size_t smem = (size_t)((d.mixed ? 12 : 24) * (FULL ? 2 : 1)) * (size_t)ts.maxcnt;
+  const NsniTiles nz = d.ns ? *d.ns : NsniTiles();
+  auto k = !d.mixed ? (d.interp ? k_defgrad_t<double, true, true, KG, KU, false, FULL>
+                                : k_defgrad_t<double, true, false, KG, KU, false, FULL>)
+           : d.ns   ? (d.interp ? k_defgrad_t<float, false, true, KG, KU, true, FULL>
+                                : k_defgrad_t<float, false, false, KG, KU, true, FULL>)
+                    : (d.interp ? k_defgrad_t<float, false, true, KG, KU, false, FULL>
+                                : k_defgrad_t<float, false, false, KG, KU, false, FULL>);
+  k<<<(unsigned)ts.ntiles, ts.R * KG, smem, s>>>(d.n, ts.R, ts.jmax, nz, ts.view(), d.rowptr, d.pk, ts.jset, ts.jcnt,
+                                                 d.dsp, d.dsp_tot, d.sdphi, d.shp, d.dsp_tot_phy, d.fg, d.acc);
 }
 
 int launch_defgrad_tiled(cudaStream_t s, bool mixed, bool interp, int32_t n, const TileSet& ts,
                          const NsniTiles* ns, const int64_t* rowptr, const void* pk, const double* dsp,
                          const double* dsp_tot, const double* sdphi, const double* shp, double* dsp_tot_phy,
-                         double* fg, StepAccum* acc, unsigned* status, int variant) {
+                         double* fg, StepAccum* acc, unsigned* status, int variant, bool full) {
   int r = 0;
   if (ns && (!mixed || variant == 4 || variant == 5)) return MEGA_ERR_UNSUPPORTED;  // NSNI: register variants
-  switch (variant) {
-    case 4: r = defgrad_bulk<4>(s, mixed, interp, n, ts, rowptr, pk, dsp, dsp_tot, sdphi, shp, dsp_tot_phy, fg, acc,
-                                status);
-      break;
-    case 5: r = defgrad_bulk<8>(s, mixed, interp, n, ts, rowptr, pk, dsp, dsp_tot, sdphi, shp, dsp_tot_phy, fg, acc,
-                                status);
-      break;
-    case 1: defgrad_variant<4, 2>(s, mixed, interp, n, ts, ns, rowptr, pk, dsp, dsp_tot, sdphi, shp, dsp_tot_phy, fg, acc);
-      break;
-    case 2: defgrad_variant<4, 1>(s, mixed, interp, n, ts, ns, rowptr, pk, dsp, dsp_tot, sdphi, shp, dsp_tot_phy, fg, acc);
-      break;
-    case 3: defgrad_variant<8, 2>(s, mixed, interp, n, ts, ns, rowptr, pk, dsp, dsp_tot, sdphi, shp, dsp_tot_phy, fg, acc);
-      break;
-    case 6: defgrad_variant<16, 1>(s, mixed, interp, n, ts, ns, rowptr, pk, dsp, dsp_tot, sdphi, shp, dsp_tot_phy, fg,
-                                   acc);
-      break;
-    case 7: defgrad_variant<16, 2>(s, mixed, interp, n, ts, ns, rowptr, pk, dsp, dsp_tot, sdphi, shp, dsp_tot_phy, fg,
-                                   acc);
-      break;
-    default: defgrad_variant<4, 4>(s, mixed, interp, n, ts, ns, rowptr, pk, dsp, dsp_tot, sdphi, shp, dsp_tot_phy, fg,
-                                   acc);
+  const DefgradArgs d{mixed, interp, n, ts, ns, rowptr, pk, dsp, dsp_tot, sdphi, shp, dsp_tot_phy, fg, acc, status};
+  if (full) {
+    if (variant == 6 || variant == 7) defgrad_variant<16, kFullKU, true>(s, d);
+    else if (variant == 3 || variant == 5) defgrad_variant<8, kFullKU, true>(s, d);
+    else defgrad_variant<4, kFullKU, true>(s, d);
+  } else {
+    switch (variant) {
+      case 1: defgrad_variant<4, 2>(s, d); break;
+      case 2: defgrad_variant<4, 1>(s, d); break;
+      case 3: defgrad_variant<8, 2>(s, d); break;
+      case 4: r = defgrad_bulk<4>(s, d); break;
+      case 5: r = defgrad_bulk<8>(s, d); break;
+      case 6: defgrad_variant<16, 1>(s, d); break;
+      case 7: defgrad_variant<16, 2>(s, d); break;
+      default: defgrad_variant<4, 4>(s, d);
+    }
   }
   if (r) return r;
   MEGA_CHECK_LAUNCH();

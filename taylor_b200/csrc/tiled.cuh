@@ -120,12 +120,13 @@ int tiled_variants();
 // whether a variant's shared memory fits the row (defgrad) or column (force) tiles
 bool tiled_variant_fits(const TileSet& ts, bool mixed, int variant, bool force, bool has_body);
 // MEGA_ERR_UNSUPPORTED when the variant's shared memory does not fit the tiles
-// ns (mixed only, register variants 0-3): the NSNI H gather rides along
+// ns (mixed only, register variants): the NSNI H gather rides along.
+// full: F - I as well as G0 (else the stress update adds G0 to F - I)
 int launch_defgrad_tiled(cudaStream_t s, bool mixed, bool interp, int32_t n, const TileSet& ts,
                          const NsniTiles* ns, const int64_t* rowptr, const void* pk, const double* dsp,
                          const double* dsp_tot,
                          const double* sdphi, const double* shp, double* dsp_tot_phy, double* fg, StepAccum* acc,
-                         unsigned* status, int variant = 0);
+                         unsigned* status, int variant, bool full);
 int launch_force_tiled(cudaStream_t s, bool mixed, const TiledForceArgs& a, int variant = 0);
 
 }  // namespace mega
