@@ -434,8 +434,8 @@ struct Ctx {
   int32_t* iperm = nullptr;  // original node i = new node iperm[i]
   TileSet rt, ct;            // row tiles (deformation gradient), column tiles (force)
   double *shp = nullptr, *sdphi = nullptr, *sdphi32 = nullptr, *tshp = nullptr, *tshp32 = nullptr;
-  double* shp32 = nullptr;   // shp in the order of the float row records once reordered (else shp)
-  bool banked = false;       // the float records reordered for the gathers' banks (bank_layout)
+  double* shpb[2] = {nullptr, nullptr};  // [FP64, mixed]: shp in the row records' order once reordered (else shp)
+  bool banked[2] = {false, false};       // the precision's records reordered for the gathers' banks (bank_layout)
   void *pk64 = nullptr, *tpk64 = nullptr, *pk32 = nullptr, *tpk32 = nullptr;
   // state
   double *dsp = nullptr, *dsp_tot = nullptr, *dsp_tot_phy = nullptr, *vel = nullptr, *acl = nullptr;
@@ -670,13 +670,14 @@ static int step_once(Ctx* c, double dt, int mode, int predict, cudaEvent_t* ev, 
   NsniTiles nt;
   int r = launch_defgrad_tiled(c->s, mixed, interp, c->n, c->rt, nsni_tiles(c, mixed, nt), c->csr.rowptr,
                                mixed ? c->pk32 : c->pk64, c->dsp, c->dsp_tot, mixed ? c->sdphi32 : c->sdphi,
-                               (mixed && c->shp32) ? c->shp32 : c->shp, c->dsp_tot_phy, c->fg, c->acc, c->status,
+                               c->shpb[mixed] ? c->shpb[mixed] : c->shp, c->dsp_tot_phy, c->fg, c->acc, c->status,
                                c->var_defgrad[mixed], full);
   if (r) return r;
   if (c->nsni && !mixed && (r = nsni_step(c->s, nsni_args(c), c->csr, c->nsr, c->nsc, false, c->dsp, 0))) return r;
   if (ev) MEGA_TRY(cudaEventRecord(ev[1], c->s));
   StressArgs sa = stress_args(c, dt, mode);
   sa.add_g0 = !full;
+  sa.more = predict;
   r = launch_stress(c->s, mixed, sa);
   if (r) return r;
   if (c->nsni && (r = nsni_step(c->s, nsni_args(c), c->csr, c->nsr, c->nsc, mixed, c->dsp, 1))) return r;
@@ -1436,11 +1437,11 @@ int mega_search_and_shapes(int64_t h, int32_t* gn, int32_t* gstart, int32_t* gst
     c->rt = TileSet();
     c->ct = TileSet();
     c->perm = c->iperm = nullptr;
-    c->shp = c->sdphi = c->sdphi32 = c->tshp = c->tshp32 = c->shp32 = nullptr;
+    c->shp = c->sdphi = c->sdphi32 = c->tshp = c->tshp32 = c->shpb[0] = c->shpb[1] = nullptr;
     c->pk64 = c->tpk64 = c->pk32 = c->tpk32 = nullptr;
     c->ns_srow = c->ns_scol = nullptr;
     c->ns_ssum = nullptr;
-    c->banked = false;
+    c->banked[0] = c->banked[1] = false;
     c->searched = false;
     c->fsteps = 0;
     if (c->gexec) { cudaGraphExecDestroy(c->gexec); c->gexec = nullptr; }
@@ -1980,18 +1981,22 @@ int64_t mega_kernel_launches(int64_t h) {
 // Autotuner: time every launch variant of the two gathers on this context's
 // own lists (reps launches each, CUDA events), keep the fastest, and put the
 // state back as it was (the force kernel integrates when it runs).
-// One-time reordering of a context's float records (at its first mixed
-// autotune): the entries of each row and column take the order in which a
-// warp's lanes read distinct shared-memory banks of the staged data
-// (bank_order), and what travels with the records follows them (the
-// interpolation and body-force shape values, the NSNI S values).  About 6 ms
-// per gather on a 1 M-node bar; it pays back over a few hundred steps.
+// One-time reordering of a precision's records (at its first autotune): the
+// entries of each row and column take the order in which a warp's lanes read
+// distinct shared-memory banks of the staged data (bank_order), and what
+// travels with the records follows them (the interpolation and body-force
+// shape values, the float NSNI S values).  About 6 ms per gather on a 1 M-node
+// bar; it pays back over a few hundred steps.
 static void drop_graph(Ctx* c);
 
-static int bank_layout(Ctx* c) {
-  if (c->banked || !(c->prec_mask & 2) || !c->pk32 || !c->tpk32) return 0;
-  const int64_t m = c->csr.nnz;
+static int bank_layout(Ctx* c, bool mixed) {
+  void*& pk = mixed ? c->pk32 : c->pk64;
+  void*& tpk = mixed ? c->tpk32 : c->tpk64;
+  double*& tshp = mixed ? c->tshp32 : c->tshp;
+  if (c->banked[mixed] || !pk || !tpk) return 0;
+  const int64_t m = c->csr.nnz, rec = mixed ? 16 : 26;
   const int32_t n = c->n;
+  const bool ns = mixed && c->ns_scol;
   DevPool tmp(c->s);
   uint16_t* l = nullptr;
   int64_t* pos = nullptr;
@@ -2001,19 +2006,19 @@ static int bank_layout(Ctx* c) {
   // columns (the lanes per column of the force variant the context favours)
   MEGA_TRY(cudaMemcpyAsync(l, c->ct.lidx, sizeof(uint16_t) * m, cudaMemcpyDeviceToDevice, c->s));
   if ((r = iota64(c->s, m, pos)) ||
-      (r = bank_order(c->s, n, c->ct, c->csr.colptr, l, nullptr, pos, c->nsni ? 8 : 4)))
+      (r = bank_order(c->s, n, c->ct, c->csr.colptr, l, nullptr, pos, ns ? 8 : 4)))
     return r;
-  float4* tp = nullptr;
-  MEGA_ALLOC(c->nbpool, tp, c->ct.nrec);
-  if ((r = gather_records32(c->s, n, c->ct, c->csr.colptr, pos, (const float4*)c->tpk32, tp))) return r;
+  unsigned char* tp = nullptr;
+  MEGA_ALLOC(c->nbpool, tp, rec * c->ct.nrec);
+  if ((r = gather_records(c->s, n, c->ct, c->csr.colptr, pos, !mixed, tpk, tp))) return r;
   double* ts = nullptr;
-  if (c->tshp32) {
+  if (tshp) {
     MEGA_ALLOC(c->nbpool, ts, m);
-    k_gather_pos<<<grid_for(m, 256), 256, 0, c->s>>>(m, pos, c->tshp32, ts);
+    k_gather_pos<<<grid_for(m, 256), 256, 0, c->s>>>(m, pos, tshp, ts);
     MEGA_CHECK_LAUNCH();
   }
   float* sc = nullptr;
-  if (c->ns_scol) {
+  if (ns) {
     MEGA_ALLOC(c->nbpool, sc, 6 * m);
     if ((r = gather_f6(c->s, m, pos, c->ns_scol, sc))) return r;
   }
@@ -2022,27 +2027,27 @@ static int bank_layout(Ctx* c) {
   if ((r = iota64(c->s, m, pos)) ||
       (r = bank_order(c->s, n, c->rt, c->csr.rowptr, l, nullptr, pos, 4)))
     return r;
-  float4* rp = nullptr;
+  unsigned char* rp = nullptr;
   double* sh = nullptr;
-  MEGA_ALLOC(c->nbpool, rp, c->rt.nrec);
+  MEGA_ALLOC(c->nbpool, rp, rec * c->rt.nrec);
   MEGA_ALLOC(c->nbpool, sh, m);
-  if ((r = gather_records32(c->s, n, c->rt, c->csr.rowptr, pos, (const float4*)c->pk32, rp))) return r;
+  if ((r = gather_records(c->s, n, c->rt, c->csr.rowptr, pos, !mixed, pk, rp))) return r;
   k_gather_pos<<<grid_for(m, 256), 256, 0, c->s>>>(m, pos, c->shp, sh);
   MEGA_CHECK_LAUNCH();
   float* sr = nullptr;
-  if (c->ns_srow) {
+  if (ns) {
     MEGA_ALLOC(c->nbpool, sr, 6 * m);
     if ((r = gather_f6(c->s, m, pos, c->ns_srow, sr))) return r;
   }
   MEGA_TRY(cudaStreamSynchronize(c->s));
   drop_graph(c);  // captured steps hold the old arrays
-  c->nbpool.release(c->tpk32); c->tpk32 = tp;
-  if (ts) { c->nbpool.release(c->tshp32); c->tshp32 = ts; }
+  c->nbpool.release(tpk); tpk = tp;
+  if (ts) { c->nbpool.release(tshp); tshp = ts; }
   if (sc) { c->nbpool.release(c->ns_scol); c->ns_scol = sc; }
-  c->nbpool.release(c->pk32); c->pk32 = rp;
-  c->shp32 = sh;
+  c->nbpool.release(pk); pk = rp;
+  c->shpb[mixed] = sh;
   if (sr) { c->nbpool.release(c->ns_srow); c->ns_srow = sr; }
-  c->banked = true;
+  c->banked[mixed] = true;
   return 0;
 }
 
@@ -2054,7 +2059,7 @@ int mega_autotune(int64_t h, double dt, int32_t mode, int32_t reps, int32_t* cho
   if (reps <= 0) return MEGA_ERR_ARG;
   const bool mixed = (mode & 0xff) == MEGA_MODE_MIXED;
   { int r = mixed ? ensure_mixed(c) : ensure_fp64(c); if (r) return r; }
-  if (mixed) { int r = bank_layout(c); if (r) return r; }
+  if (int r = bank_layout(c, mixed)) return r;
   const int nvar = tiled_variants();
   const size_t n = (size_t)c->n, n3 = 3 * n;
   // snapshot of everything a step writes

@@ -319,7 +319,7 @@ __device__ __forceinline__ void stress_finish(const StressArgs& a, int64_t i, Tr
   if (cap) st |= MEGA_ST_NEWTON_CAP;
   nit += (unsigned long long)it;
   npl += (it > 0) ? 1ull : 0ull;
-  if (a.iters) a.iters[i] = it;
+  if (a.iters && !a.more) a.iters[i] = it;
   double sinc[6], einc[6], enew[6];
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
@@ -337,9 +337,6 @@ __device__ __forceinline__ void stress_finish(const StressArgs& a, int64_t i, Tr
     }
   }
   a.eps[i] = ep;
-  const double eq = enew[0] * enew[0] + enew[1] * enew[1] + enew[2] * enew[2] +
-                    2.0 * (enew[3] * enew[3] + enew[4] * enew[4] + enew[5] * enew[5]);
-  a.strain_eq[i] = sqrt(eq * 2.0 / 3.0);
   if (a.finite_strain) {
 #pragma unroll
     for (int k = 0; k < 6; ++k) work += 0.5 * (double)w.D[k] * (2.0 * snew[k] - sinc[k]) * vol * w.det;
@@ -347,10 +344,15 @@ __device__ __forceinline__ void stress_finish(const StressArgs& a, int64_t i, Tr
 #pragma unroll
     for (int k = 0; k < 6; ++k) work += 0.5 * einc[k] * sinc[k] * vol * w.det;
   }
-  double bulk = m.E / (3.0 * (1.0 - 2.0 * m.nu)), shear = m.E / (2.0 * (1.0 + m.nu));
-  if (m.type > 1) estimate_moduli(sinc, einc, shear, bulk);
-  const double pmod = bulk + 4.0 * shear / 3.0;
-  a.wvel[i] = sqrt(fmax(pmod, shear) / m.rho);
+  if (!a.more) {  // the last step of a call: what only a caller reads
+    const double eq = enew[0] * enew[0] + enew[1] * enew[1] + enew[2] * enew[2] +
+                      2.0 * (enew[3] * enew[3] + enew[4] * enew[4] + enew[5] * enew[5]);
+    a.strain_eq[i] = sqrt(eq * 2.0 / 3.0);
+    double bulk = m.E / (3.0 * (1.0 - 2.0 * m.nu)), shear = m.E / (2.0 * (1.0 + m.nu));
+    if (m.type > 1) estimate_moduli(sinc, einc, shear, bulk);
+    const double pmod = bulk + 4.0 * shear / 3.0;
+    a.wvel[i] = sqrt(fmax(pmod, shear) / m.rho);
+  }
   // T_i = V J sigma IF^T: f_J(k) = sum_m T(k,m) grad0 phi_iJ(m)
   const T vj = (T)(vol * w.det);
   T S[3][3];

@@ -234,6 +234,7 @@ struct StressArgs {
   int32_t n;
   double* fg;                // F - I and G0 (mega_device.cuh: planes of fg_ld(n) values)
   int add_g0;                // F advances by G0 here (the row gather formed G0 alone)
+  int more;                  // another step follows: iters, strain_eq and wvel are not written
   const uint16_t* matidx;
   const MatEntry* mats;
   const double* vol;

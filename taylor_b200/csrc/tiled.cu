@@ -258,14 +258,15 @@ __global__ void k_pad_f32(int32_t n, int32_t R, int64_t slots, SliceView v, cons
 
 // Entry order for conflict-free reads of the staged neighbour data.  In the
 // gathers the KG lanes of a row (column) take its entries KG at a time, and
-// the 32 lanes of a warp read the staged values of their current entries in
-// one instruction: lanes whose tile ranks l differ but agree modulo NC (the
-// bank period of the staged layout) are served one after another, lanes with
-// the same l by one broadcast.  This reorders the entries within each row so
-// that, at every step, the lanes of each group of GL lanes hold, per class
-// l mod NC, one rank only wherever the row's remaining entries allow (greedy,
-// lanes in order, each taking its first entry whose class is free or holds
-// the same rank); a row keeps all its entries, only their order changes.
+// the lanes of a warp read the staged 16-byte vectors of their current
+// entries in one instruction, 8 lanes at a time: lanes of such a group whose
+// tile ranks l differ but agree modulo NC = 8 (the vectors' bank period) are
+// served one after another, lanes with the same l by one broadcast.  This
+// reorders the entries within each row so that, at every step, the lanes of
+// each group of GL = 8 lanes hold, per class l mod NC, one rank only wherever
+// the row's remaining entries allow (greedy, lanes in order, each taking its
+// first entry whose class is free or holds the same rank); a row keeps all
+// its entries, only their order changes.
 // pos, when given, is permuted with lidx.  One warp per warp of the gather's
 // blocks, four warps per block.
 constexpr int kBankCap = 2048;  // entries of one warp's rows that its pass stages in shared memory
@@ -362,6 +363,27 @@ __global__ void k_gather_rec32(int32_t n, int32_t R, int64_t slots, SliceView v,
   });
 }
 
+// the same for the planes of FP64 records
+__global__ void k_gather_rec64(int32_t n, int32_t R, int64_t slots, SliceView v, const int64_t* __restrict__ ptr,
+                               const int64_t* __restrict__ pos, const void* __restrict__ in, void* __restrict__ out) {
+  const double2* xy = (const double2*)in;
+  const double* z = (const double*)(xy + v.nrec);
+  const uint16_t* l = (const uint16_t*)(z + v.nrec);
+  double2* oxy = (double2*)out;
+  double* oz = (double*)(oxy + v.nrec);
+  uint16_t* ol = (uint16_t*)(oz + v.nrec);
+  for_slot_records(n, R, slots, v, ptr, [&](int64_t rec, int64_t p, int64_t first) {
+    int64_t from = rec;
+    if (p >= 0) {
+      const int64_t k = p - first;
+      from = rec_of(rec - 32 * (k >> 2) - (k & 3), pos[p] - first);
+    }
+    oxy[rec] = xy[from];
+    oz[rec] = z[from];
+    ol[rec] = l[from];
+  });
+}
+
 // out[6 e + k] = in[6 pos[e] + k]
 __global__ void k_gather_f6(int64_t m, const int64_t* __restrict__ pos, const float2* __restrict__ in,
                             float2* __restrict__ out) {
@@ -400,15 +422,64 @@ struct Rec<true> {
   __device__ __forceinline__ int l() const { return (int)r; }
 };
 __device__ __forceinline__ void load_rec(const void* pk, int64_t, int64_t rec, Rec<false>& o) {
-  o.v = __ldg((const float4*)pk + rec);
+  asm("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(o.v.x), "=f"(o.v.y), "=f"(o.v.z), "=f"(o.v.w) : "l"((const float4*)pk + rec));
 }
 __device__ __forceinline__ void load_rec(const void* pk, int64_t nrec, int64_t rec, Rec<true>& o) {
   const double2* xy = (const double2*)pk;
   const double* z = (const double*)(xy + nrec);
-  o.a = __ldg(xy + rec);
-  o.b = __ldg(z + rec);
-  o.r = __ldg((const uint16_t*)(z + nrec) + rec);
+  asm("ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(o.a.x), "=d"(o.a.y) : "l"(xy + rec));
+  asm("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(o.b) : "l"(z + rec));
+  asm("ld.global.nc.L1::no_allocate.u16 %0, [%1];" : "=h"(o.r) : "l"((const uint16_t*)(z + nrec) + rec));
 }
+
+// N values per rank staged in shared memory: 16-byte vectors (4 floats or 2
+// doubles) of all ranks one after another, then the values left over as
+// arrays, ld ranks each.  A lane's read of 9 values is 3 (float) or 5
+// (double) instructions.  Lanes with distinct ranks modulo 8 among 8
+// neighbouring lanes read distinct banks; a warp's random ranks cost a 16-byte
+// read 8.3 wavefronts where four 4-byte reads cost 11.0 and two 8-byte reads
+// 10.3 (counted on the jittered bar's lists).  ld is a multiple of 4, so what
+// follows the values is aligned too.
+__host__ __device__ constexpr int staged_ld(int cnt) { return (cnt + 3) & ~3; }
+template <typename V, int N>
+struct Staged {
+  static constexpr int W = 16 / (int)sizeof(V), NV = N / W;
+  V* base;
+  int ld;
+  __device__ __forceinline__ V* end() const { return base + N * ld; }
+  // value k of rank l
+  __device__ __forceinline__ V& at(int l, int k) const {
+    return k < W * NV ? base[W * ((k / W) * ld + l) + k % W] : base[k * ld + l];
+  }
+  // vector k of rank l
+  __device__ __forceinline__ void put(int l, int k, const float4& x) const {
+    reinterpret_cast<float4*>(base)[k * ld + l] = x;
+  }
+  __device__ __forceinline__ void put(int l, int k, const double2& x) const {
+    reinterpret_cast<double2*>(base)[k * ld + l] = x;
+  }
+  __device__ __forceinline__ void load(int l, V* v) const {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      if constexpr (W == 4) {
+        const float4 x = reinterpret_cast<const float4*>(base)[k * ld + l];
+        v[4 * k] = x.x; v[4 * k + 1] = x.y; v[4 * k + 2] = x.z; v[4 * k + 3] = x.w;
+      } else {
+        const double2 x = reinterpret_cast<const double2*>(base)[k * ld + l];
+        v[2 * k] = x.x; v[2 * k + 1] = x.y;
+      }
+    }
+#pragma unroll
+    for (int k = W * NV; k < N; ++k) v[k] = base[k * ld + l];
+  }
+};
+
+// 32 bytes at a 32-byte boundary
+__device__ __forceinline__ void load_sector(const double* p, double v[4]) {
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p));
+}
+
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // A lane's way through its row's records: KG lanes per row (4, 8 or 16), the
 // lane's entries KG apart in list order, which is a stride of KG / 4 steps.
@@ -437,6 +508,37 @@ __device__ __forceinline__ SRec load_srec(const float* base, int64_t p, int64_t 
   return SRec{__ldg(sp), __ldg(sp + 1), __ldg(sp + 2)};
 }
 
+// the staged displacement values of a rank: three doubles, or three floats and a pad
+template <bool F64>
+struct DispStage {
+  using V = float;
+  static constexpr int N = 4;
+};
+template <>
+struct DispStage<true> {
+  using V = double;
+  static constexpr int N = 3;
+};
+
+template <bool F64>
+using StagedDisp = Staged<typename DispStage<F64>::V, DispStage<F64>::N>;
+
+// a thread per staged node
+template <bool F64>
+__device__ __forceinline__ void stage_disp(const int32_t* js, int cnt, const double* v, const double* ref,
+                                           const StagedDisp<F64>& out) {
+  for (int l = threadIdx.x; l < cnt; l += blockDim.x) {
+    const int64_t g = 3 * (int64_t)js[l];
+    const double x0 = v[g], x1 = v[g + 1], x2 = v[g + 2];
+    if constexpr (F64) {
+      out.put(l, 0, make_double2(x0, x1));
+      out.at(l, 2) = x2;
+    } else {
+      out.put(l, 0, make_float4((float)(x0 - ref[0]), (float)(x1 - ref[1]), (float)(x2 - ref[2]), 0.f));
+    }
+  }
+}
+
 // FULL: F - I is formed besides G0.  Without it the gather stages and reads
 // the increments alone, half the shared-memory traffic and sums: at 130 k nodes
 // FP64 ran at 75 % of the L1 data pipe with both, half of it staged reads.
@@ -456,7 +558,7 @@ __global__ void __launch_bounds__(64 * KG, defgrad_blocks<F64, KG, NS, FULL>())
                 const double* __restrict__ dsp, const double* __restrict__ dsp_tot,
                 const double* __restrict__ sdphi, const double* __restrict__ shp, double* __restrict__ dsp_tot_phy,
                 double* __restrict__ fg, StepAccum* __restrict__ acc) {
-  extern __shared__ double sm[];
+  extern __shared__ __align__(16) double sm[];
   if (acc && blockIdx.x == 0 && threadIdx.x < kSlots) {
     acc->newton_iters[threadIdx.x] = 0ull;
     acc->plastic[threadIdx.x] = 0ull;
@@ -464,14 +566,15 @@ __global__ void __launch_bounds__(64 * KG, defgrad_blocks<F64, KG, NS, FULL>())
   const int64_t t = blockIdx.x;
   const int cnt = jcnt[t];
   const int32_t* js = jset + t * (int64_t)jmax;
-  // Staged neighbour displacements, du_J (FULL: and u_J), one array per
-  // component (value k of rank l at [k cnt + l]: lanes with distinct ranks
-  // modulo the banks read distinct banks).  FP64 as doubles; mixed as float
-  // offsets from the tile's first node r0 (du_J - du_r0, u_J - u_r0), half
-  // the shared-memory traffic: the differences d_J - d_i are formed between
-  // offsets, exact up to float rounding of the offsets.
-  double* sd = sm;
-  float* sf = reinterpret_cast<float*>(sm);
+  // Staged neighbour displacements, du_J (FULL: and u_J).  FP64 as doubles;
+  // mixed as float offsets from the tile's first node r0 (du_J - du_r0,
+  // u_J - u_r0; one 16-byte vector with a pad), half the shared-memory
+  // traffic: the differences d_J - d_i are formed between offsets, exact up
+  // to float rounding of the offsets.
+  using SV = typename DispStage<F64>::V;
+  constexpr int SN = DispStage<F64>::N;
+  const Staged<SV, SN> sd{reinterpret_cast<SV*>(sm), staged_ld(cnt)};
+  const Staged<SV, SN> su{sd.end(), sd.ld};
   const int64_t r0 = t * R;
   const int slot = threadIdx.x / KG;
   const int64_t i = r0 + sv.ord[r0 + slot];
@@ -507,155 +610,144 @@ __global__ void __launch_bounds__(64 * KG, defgrad_blocks<F64, KG, NS, FULL>())
       if (FULL) ur[k] = dsp_tot[3 * r0 + k];
     }
   }
-  for (int l = threadIdx.x; l < cnt; l += blockDim.x) {
-    const int64_t g = js[l];
+  stage_disp<F64>(js, cnt, dsp, dr, sd);
+  if (FULL) stage_disp<F64>(js, cnt, dsp_tot, ur, su);
+  __syncthreads();
+  if (valid) {
+    double ui[3] = {0.0, 0.0, 0.0}, di[3];
+    A fu[3], fd[3];  // this row's values as the staged ones are held
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      const double b = dsp[3 * g + k];
-      const double a = FULL ? dsp_tot[3 * g + k] : 0.0;
-      if (F64) {
-        sd[k * cnt + l] = b;
-        if (FULL) sd[(3 + k) * cnt + l] = a;
-      } else {
-        sf[k * cnt + l] = (float)(b - dr[k]);
-        if (FULL) sf[(3 + k) * cnt + l] = (float)(a - ur[k]);
+      di[k] = dsp[3 * i + k];
+      fd[k] = F64 ? (A)di[k] : (A)(float)(di[k] - dr[k]);
+      if (FULL) {
+        ui[k] = dsp_tot[3 * i + k];
+        fu[k] = F64 ? (A)ui[k] : (A)(float)(ui[k] - ur[k]);
       }
     }
-  }
-  __syncthreads();
-  if (!valid) return;
-  double ui[3] = {0.0, 0.0, 0.0}, di[3];
-  A fu[3], fd[3];  // this row's values as the staged ones are held
+    A F[FULL ? 9 : 1], L[9];
+    double H[NS ? 18 : 1];  // NSNI: exact products of the float S and differences, summed in double
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    di[k] = dsp[3 * i + k];
-    fd[k] = F64 ? (A)di[k] : (A)(float)(di[k] - dr[k]);
-    if (FULL) {
-      ui[k] = dsp_tot[3 * i + k];
-      fu[k] = F64 ? (A)ui[k] : (A)(float)(ui[k] - ur[k]);
-    }
-  }
-  A F[FULL ? 9 : 1], L[9];
-  double H[NS ? 18 : 1];  // NSNI: exact products of the float S and differences, summed in double
+    for (int k = 0; k < 9; ++k) L[k] = A(0);
 #pragma unroll
-  for (int k = 0; k < 9; ++k) L[k] = A(0);
+    for (int k = 0; k < (FULL ? 9 : 1); ++k) F[k] = A(0);
 #pragma unroll
-  for (int k = 0; k < (FULL ? 9 : 1); ++k) F[k] = A(0);
+    for (int k = 0; k < (NS ? 18 : 1); ++k) H[k] = 0.0;
+    double ph[3] = {0.0, 0.0, 0.0};
+    // One entry: F += (u_J - u_i) (x) g, L += (d_J - d_i) (x) g (+ phi d_J),
+    // H(k, q) += S_q (d_J - d_i)_k.
+    auto body = [&](int it, const Rec<F64>& rec, const SRec& sr) {
+      const A g[3] = {(A)rec.x(), (A)rec.y(), (A)rec.z()};
+      const int l = rec.l();
+      SV v[SN];
+      A d[3];
+      sd.load(l, v);
 #pragma unroll
-  for (int k = 0; k < (NS ? 18 : 1); ++k) H[k] = 0.0;
-  double ph[3] = {0.0, 0.0, 0.0};
-  // One entry: F += (u_J - u_i) (x) g, L += (d_J - d_i) (x) g (+ phi d_J),
-  // H(k, q) += S_q (d_J - d_i)_k.
-  auto body = [&](int it, const Rec<F64>& rec, const SRec& sr) {
-    const A g[3] = {(A)rec.x(), (A)rec.y(), (A)rec.z()};
-    const int l = rec.l();
-    A v[3], d[3];
+      for (int k = 0; k < 3; ++k) d[k] = (A)v[k] - fd[k];
+      if constexpr (FULL) {
+        SV w[SN];
+        su.load(l, w);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      v[k] = F64 ? (A)sd[k * cnt + l] : (A)sf[k * cnt + l];
-      d[k] = v[k] - fd[k];
-    }
-    if constexpr (FULL) {
+        for (int k = 0; k < 3; ++k) {
+          const A u = (A)w[k] - fu[k];
+          F[3 * k] += u * g[0]; F[3 * k + 1] += u * g[1]; F[3 * k + 2] += u * g[2];
+        }
+      }
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
-        const A u = (F64 ? (A)sd[(3 + k) * cnt + l] : (A)sf[(3 + k) * cnt + l]) - fu[k];
-        F[3 * k] += u * g[0]; F[3 * k + 1] += u * g[1]; F[3 * k + 2] += u * g[2];
+        L[3 * k] += d[k] * g[0]; L[3 * k + 1] += d[k] * g[1]; L[3 * k + 2] += d[k] * g[2];
       }
-    }
+      if constexpr (NS) {
+        const double sq[6] = {(double)sr.a.x, (double)sr.a.y, (double)sr.b.x, (double)sr.b.y, (double)sr.c.x,
+                              (double)sr.c.y};
+        const double e0 = (double)d[0], e1 = (double)d[1], e2 = (double)d[2];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      L[3 * k] += d[k] * g[0]; L[3 * k + 1] += d[k] * g[1]; L[3 * k + 2] += d[k] * g[2];
-    }
-    if constexpr (NS) {
-      const double sq[6] = {(double)sr.a.x, (double)sr.a.y, (double)sr.b.x, (double)sr.b.y, (double)sr.c.x,
-                            (double)sr.c.y};
-      const double e0 = (double)d[0], e1 = (double)d[1], e2 = (double)d[2];
-#pragma unroll
-      for (int c = 0; c < 6; ++c) { H[c] += sq[c] * e0; H[6 + c] += sq[c] * e1; H[12 + c] += sq[c] * e2; }
-    }
-    if (INTERP) {
-      const int64_t p = p0 + (int64_t)KG * it;
-      if (p < pend) {  // (not a pad)
-        const double s = shp[p];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) ph[k] += s * (F64 ? (double)v[k] : dr[k] + (double)v[k]);
+        for (int c = 0; c < 6; ++c) { H[c] += sq[c] * e0; H[6 + c] += sq[c] * e1; H[12 + c] += sq[c] * e2; }
       }
-    }
-  };
-  // Each lane sums its entries in list order.  Where the registers allow
-  // (kPipe) the next KU records are requested before this KU's sums, so a
-  // lane keeps loads in flight while it computes.
-  const SRec s0{};
-  int it = 0;
-  while (have) {
-    const bool hn = it + 2 * KU <= nit;
-    Rec<F64> nxt[KU];
-    if constexpr (kPipe) {
+      if (INTERP) {
+        const int64_t p = p0 + (int64_t)KG * it;
+        if (p < pend) {  // (not a pad)
+          const double s = shp[p];
+#pragma unroll
+          for (int k = 0; k < 3; ++k) ph[k] += s * (F64 ? (double)v[k] : dr[k] + (double)v[k]);
+        }
+      }
+    };
+    // Each lane sums its entries in list order.  Where the registers allow
+    // (kPipe) the next KU records are requested before this KU's sums, so a
+    // lane keeps loads in flight while it computes.
+    const SRec s0{};
+    int it = 0;
+    while (have) {
+      const bool hn = it + 2 * KU <= nit;
+      Rec<F64> nxt[KU];
+      if constexpr (kPipe) {
+#pragma unroll
+        for (int u = 0; u < KU; ++u) {
+          if (hn) load_rec(pk, sv.nrec, walk.at(it + KU + u), nxt[u]);
+          else nxt[u] = cur[u];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < KU; ++u) body(it + u, cur[u], NS ? csr[NS ? u : 0] : s0);
 #pragma unroll
       for (int u = 0; u < KU; ++u) {
-        if (hn) load_rec(pk, sv.nrec, walk.at(it + KU + u), nxt[u]);
-        else nxt[u] = cur[u];
+        if constexpr (kPipe) {
+          cur[u] = nxt[u];
+        } else if (hn) {
+          load_rec(pk, sv.nrec, walk.at(it + KU + u), cur[u]);
+          if constexpr (NS) csr[u] = load_srec(ns.srow, p0 + (int64_t)KG * (it + KU + u), pend);
+        }
+      }
+      it += KU;
+      have = hn;
+    }
+    for (; it < nit; ++it) {
+      Rec<F64> rec;
+      load_rec(pk, sv.nrec, walk.at(it), rec);
+      body(it, rec, NS ? load_srec(ns.srow, p0 + (int64_t)KG * it, pend) : s0);
+    }
+#pragma unroll
+    for (int o = 1; o < KG; o <<= 1) {
+#pragma unroll
+      for (int k = 0; k < 9; ++k) {
+        if constexpr (FULL) F[k] += __shfl_xor_sync(gmask, F[k], o);
+        L[k] += __shfl_xor_sync(gmask, L[k], o);
+      }
+      if constexpr (NS) {
+#pragma unroll
+        for (int k = 0; k < 18; ++k) H[k] += __shfl_xor_sync(gmask, H[k], o);
+      }
+      if (INTERP) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) ph[k] += __shfl_xor_sync(gmask, ph[k], o);
       }
     }
+    if (q == 0) {
+      if constexpr (NS) {
+        double ss[6];
 #pragma unroll
-    for (int u = 0; u < KU; ++u) body(it + u, cur[u], NS ? csr[NS ? u : 0] : s0);
+        for (int c = 0; c < 6; ++c) ss[c] = ns.ssum[6 * i + c];
 #pragma unroll
-    for (int u = 0; u < KU; ++u) {
-      if constexpr (kPipe) {
-        cur[u] = nxt[u];
-      } else if (hn) {
-        load_rec(pk, sv.nrec, walk.at(it + KU + u), cur[u]);
-        if constexpr (NS) csr[u] = load_srec(ns.srow, p0 + (int64_t)KG * (it + KU + u), pend);
+        for (int k = 0; k < 3; ++k)
+#pragma unroll
+          for (int c = 0; c < 6; ++c) ns.hq[18 * i + 6 * k + c] = H[6 * k + c] + di[k] * ss[c];
       }
-    }
-    it += KU;
-    have = hn;
-  }
-  for (; it < nit; ++it) {
-    Rec<F64> rec;
-    load_rec(pk, sv.nrec, walk.at(it), rec);
-    body(it, rec, NS ? load_srec(ns.srow, p0 + (int64_t)KG * it, pend) : s0);
-  }
+      const double sd3[3] = {sdphi[3 * i], sdphi[3 * i + 1], sdphi[3 * i + 2]};
+      const int64_t ld = fg_ld(n);
+      double h[9];
 #pragma unroll
-  for (int o = 1; o < KG; o <<= 1) {
+      for (int k = 0; k < 9; ++k) h[k] = (double)L[k] + di[k / 3] * sd3[k % 3];
+      store_g0(fg, ld, i, !F64, h);
+      if constexpr (FULL) {
 #pragma unroll
-    for (int k = 0; k < 9; ++k) {
-      if constexpr (FULL) F[k] += __shfl_xor_sync(gmask, F[k], o);
-      L[k] += __shfl_xor_sync(gmask, L[k], o);
-    }
-    if constexpr (NS) {
+        for (int k = 0; k < 9; ++k) h[k] = (double)F[k] + ui[k / 3] * sd3[k % 3];
+        store_fmi(fg, ld, i, h);
+      }
+      if (INTERP) {
 #pragma unroll
-      for (int k = 0; k < 18; ++k) H[k] += __shfl_xor_sync(gmask, H[k], o);
-    }
-    if (INTERP) {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) ph[k] += __shfl_xor_sync(gmask, ph[k], o);
-    }
-  }
-  if (q == 0) {
-    if constexpr (NS) {
-      double ss[6];
-#pragma unroll
-      for (int c = 0; c < 6; ++c) ss[c] = ns.ssum[6 * i + c];
-#pragma unroll
-      for (int k = 0; k < 3; ++k)
-#pragma unroll
-        for (int c = 0; c < 6; ++c) ns.hq[18 * i + 6 * k + c] = H[6 * k + c] + di[k] * ss[c];
-    }
-    const double sd3[3] = {sdphi[3 * i], sdphi[3 * i + 1], sdphi[3 * i + 2]};
-    const int64_t ld = fg_ld(n);
-    double h[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) h[k] = (double)L[k] + di[k / 3] * sd3[k % 3];
-    store_g0(fg, ld, i, !F64, h);
-    if constexpr (FULL) {
-#pragma unroll
-      for (int k = 0; k < 9; ++k) h[k] = (double)F[k] + ui[k / 3] * sd3[k % 3];
-      store_fmi(fg, ld, i, h);
-    }
-    if (INTERP) {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) dsp_tot_phy[3 * i + k] += ph[k];
+        for (int k = 0; k < 3; ++k) dsp_tot_phy[3 * i + k] += ph[k];
+      }
     }
   }
 }
@@ -664,70 +756,161 @@ __global__ void __launch_bounds__(64 * KG, defgrad_blocks<F64, KG, NS, FULL>())
 // fixity, acceleration and corrector (MAIN.F90:432-488), the energy and
 // reaction sums, and the next step's predictor (MAIN.F90:353-355).
 __device__ __forceinline__ void correct_dof(const TiledForceArgs& a, int64_t J, int q, double fi, double fe,
-                                            double& ke, double& ee, double* tf, unsigned& st) {
+                                            double& ke, double& ee, double& pr, int& body, unsigned& st) {
   const int64_t m = 3 * J + q;
   const double dt = a.ndt ? a.ndt[J] : a.dt;
   if (a.fadd) fi += a.fadd[m];
   if (!isfinite(fi)) st |= MEGA_ST_NONFINITE;
   const double mass = a.mass[m];
-  const double fe_old = a.fext[m];
-  double v = a.vel[m], acc, pr;
+  const double fe_old = a.fext[m], d_old = a.dsp[m];
+  // read with the rest: behind the stores below it would cost another trip to memory
+  const double u_old = a.predict ? a.dsp_tot[m] : 0.0;
+  double v = a.vel[m], acc;
   const int code = a.ebc[m];
+  body = a.body_id ? a.body_id[J] : 1;
+  const double damp = a.mats[a.matidx[J]].damp;
   if (code == 1 || code == 2) {  // MAIN.F90:438-445 (fixed), 447-470 (prescribed velocity)
     v = code == 1 ? 0.0 : a.vel2[q];
     acc = 0.0;
     pr = -fi;
     fe = -fi;
   } else {  // MAIN.F90:472-481
-    const double mpdc = a.mats[a.matidx[J]].damp * mass;
+    const double mpdc = damp * mass;
     acc = (fe - fi - mpdc * v) / (mass + 0.5 * dt * mpdc);
     v = v + 0.5 * dt * acc;
     pr = 0.0;
   }
-  ee += 0.5 * (fe + fe_old) * a.dsp[m];
-  ke += 0.5 * mass * v * v;
-  const int b = a.body_id ? a.body_id[J] : 1;
-#pragma unroll
-  for (int k = 0; k < 3; ++k)  // constant indices: the sums stay in registers
-    if (q == k) {
-      if (b == 1) tf[k] += pr;
-      else if (b == 2) tf[3 + k] += pr;
-    }
-  a.fint[m] = fi;
+  ee = 0.5 * (fe + fe_old) * d_old;
+  ke = 0.5 * mass * v * v;
   a.fext[m] = fe;
-  a.acl[m] = acc;
-  a.prforce[m] = pr;
+  if (!a.predict) {
+    a.fint[m] = fi;
+    a.acl[m] = acc;
+    a.prforce[m] = pr;
+  }
   if (a.predict) {  // MAIN.F90:353-355 of the next step
     const double d = dt * v + dt * dt * 0.5 * acc;
     a.dsp[m] = d;
-    a.dsp_tot[m] = a.dsp_tot[m] + d;
+    a.dsp_tot[m] = u_old + d;
     v = v + dt * 0.5 * acc;
   }
   a.vel[m] = v;
 }
 
-// One block reduction of the eight step sums, then one atomic per sum into
-// this block's slot.  Every thread of the block takes part.
-__device__ __forceinline__ void step_sums(const TiledForceArgs& a, double ke, double ee, const double* tf,
-                                          double* red) {
-  double v[8] = {ke, ee, tf[0], tf[1], tf[2], tf[3], tf[4], tf[5]};
-#pragma unroll
-  for (int k = 0; k < 8; ++k)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0)
-#pragma unroll
-    for (int k = 0; k < 8; ++k) red[wid * 8 + k] = v[k];
+// The tile's columns after their sums: thread m takes DOF m of the tile
+// (component m % 3 of local column m / 3), so every array is read and written
+// in contiguous runs (the warps' own columns are in the slices' order, 8
+// scattered columns each), then one block reduction of the step sums and one
+// atomic per sum into this block's slot.  Reaction sums are formed only by
+// warps that hold a fixed DOF.  Every thread of the block takes part.
+struct ColumnSums {
+  double f[3 * 64];  // force, and body force, of DOF m
+  double e[3 * 64];
+  double red[6 * 8];
+};
+
+// the lines finish_columns will read, asked for while the sums are formed
+__device__ __forceinline__ void prefetch_columns(const TiledForceArgs& a, int64_t c0) {
+  const int64_t m = 3 * c0 + threadIdx.x;
+  if (threadIdx.x >= 3 * a.R || (threadIdx.x & 3) || m >= 3 * (int64_t)a.n) return;
+  prefetch_l2(a.mass + m);
+  prefetch_l2(a.fext + m);
+  prefetch_l2(a.vel + m);
+  prefetch_l2(a.dsp + m);
+  prefetch_l2(a.dsp_tot + m);
+}
+
+__device__ __forceinline__ void finish_columns(const TiledForceArgs& a, int64_t c0, ColumnSums& cs, unsigned st) {
   __syncthreads();
-  if (threadIdx.x < 8) {
-    const int nw = (blockDim.x + 31) >> 5;
+  const int tid = threadIdx.x, ndof = 3 * a.R, nw = (ndof + 31) >> 5, wid = tid >> 5;
+  if (wid < nw) {  // whole warps
+    double ke = 0.0, ee = 0.0, pr = 0.0;
+    int body = 0;
+    const int q = tid % 3;
+    const int64_t J = c0 + tid / 3;
+    if (tid < ndof && J < a.n) correct_dof(a, J, q, cs.f[tid], a.has_body ? cs.e[tid] : 0.0, ke, ee, pr, body, st);
+    double v[8] = {ke, ee, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+      v[1] += __shfl_xor_sync(0xffffffffu, v[1], o);
+    }
+    if (__any_sync(0xffffffffu, pr != 0.0)) {
+#pragma unroll
+      for (int k = 0; k < 6; ++k) {
+        v[2 + k] = (q == k % 3 && body == 1 + k / 3) ? pr : 0.0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v[2 + k] += __shfl_xor_sync(0xffffffffu, v[2 + k], o);
+      }
+    }
+    if ((tid & 31) == 0)
+#pragma unroll
+      for (int k = 0; k < 8; ++k) cs.red[wid * 8 + k] = v[k];
+  }
+  __syncthreads();
+  if (tid < 8) {
     double tsum = 0.0;
-    for (int w = 0; w < nw; ++w) tsum += red[w * 8 + threadIdx.x];
+    for (int w = 0; w < nw; ++w) tsum += cs.red[w * 8 + tid];
     const int sl = blockIdx.x % kSlots;
-    double* dst = threadIdx.x == 0 ? &a.acc->ke[sl] : (threadIdx.x == 1 ? &a.acc->ee[sl] : &a.acc->tf[threadIdx.x - 2][sl]);
+    double* dst = tid == 0 ? &a.acc->ke[sl] : (tid == 1 ? &a.acc->ee[sl] : &a.acc->tf[tid - 2][sl]);
     if (tsum != 0.0) atomicAdd(dst, tsum);
   }
+  if (st) atomicOr(a.status, st);
+}
+
+// The staged values of a column tile: T_i (9), the body force vectors (3, as
+// arrays) and, NS, T_i and W_i together (27 and a pad: 7 vectors, T_i's first
+// two, then T_i's last beside W_i's last two, then W_i's first 16).
+template <typename TS, bool NS>
+struct StagedT {
+  Staged<TS, NS ? 28 : 9> t;
+  TS* body;
+  int ld;
+  __device__ __forceinline__ StagedT(void* base, int cnt)
+      : t{reinterpret_cast<TS*>(base), staged_ld(cnt)}, body(t.end()), ld(t.ld) {}
+  // A thread per staged node.  FP64: the 96-byte row as three 32-byte loads,
+  // a sector each (as six 16-byte loads every line was fetched twice once the
+  // blocks' shared memory had shrunk L1).
+  __device__ __forceinline__ void fill(const TiledForceArgs& a, const int32_t* js, int cnt) const {
+    for (int l = threadIdx.x; l < cnt; l += blockDim.x) {
+      const int64_t j = js[l];
+      if constexpr (sizeof(TS) == 4) {
+        const float4* p = reinterpret_cast<const float4*>(a.tmat) + 3 * j;
+        const float4 x = __ldg(p), y = __ldg(p + 1), z = __ldg(p + 2);
+        t.put(l, 0, x);
+        t.put(l, 1, y);
+        t.at(l, 8) = z.x;
+        if (a.has_body) { body[l] = z.y; body[ld + l] = z.z; body[2 * ld + l] = z.w; }
+        if constexpr (NS) {
+          const float4* w = reinterpret_cast<const float4*>(a.ns_w) + 5 * j;
+          const float4 w0 = __ldg(w), w1 = __ldg(w + 1), w2 = __ldg(w + 2), w3 = __ldg(w + 3), w4 = __ldg(w + 4);
+          t.put(l, 3, w0);
+          t.put(l, 4, w1);
+          t.put(l, 5, w2);
+          t.put(l, 6, w3);
+          t.at(l, 9) = w4.x;
+          t.at(l, 10) = w4.y;
+        }
+      } else {
+        const double* p = reinterpret_cast<const double*>(a.tmat) + 12 * j;
+        double x[4], y[4], z[4];
+        load_sector(p, x);
+        load_sector(p + 4, y);
+        load_sector(p + 8, z);
+        t.put(l, 0, make_double2(x[0], x[1]));
+        t.put(l, 1, make_double2(x[2], x[3]));
+        t.put(l, 2, make_double2(y[0], y[1]));
+        t.put(l, 3, make_double2(y[2], y[3]));
+        t.at(l, 8) = z[0];
+        if (a.has_body) { body[l] = z[1]; body[ld + l] = z[2]; body[2 * ld + l] = z[3]; }
+      }
+    }
+  }
+};
+
+template <bool F64, int KG, int KU, bool NS>
+constexpr int force_blocks() {  // blocks per SM the register cap asks for (NS: what its staged values leave room for)
+  return KG == 4 ? (NS ? 2 : (F64 ? 3 : (KU == 4 ? 4 : 5))) : 16 / KG;
 }
 
 // TS = storage of T_i (float / double), A = accumulation, F64 = record width
@@ -735,15 +918,13 @@ __device__ __forceinline__ void step_sums(const TiledForceArgs& a, double ke, do
 // f_J += sum_i sum_q W_i(k, q) S_q(i, J) (FINT.F90:1127-1208 layout), with the
 // row weights W_i staged beside T_i.
 template <typename TS, typename A, bool F64, int KG, int KU, bool NS = false>
-__global__ void __launch_bounds__(64 * KG) k_force_t(TiledForceArgs a) {
-  extern __shared__ double smx[];
-  __shared__ double red[32 * 8];  // eight sums per warp, up to 32 warps (KG = 16)
+__global__ void __launch_bounds__(64 * KG, force_blocks<F64, KG, KU, NS>()) k_force_t(TiledForceArgs a) {
+  extern __shared__ __align__(16) double smx[];
+  __shared__ ColumnSums cs;
   const int64_t t = blockIdx.x;
   const int cnt = a.jcnt[t];
-  const int nv = a.has_body ? 12 : 9;
-  TS* sT = (TS*)smx;
+  const StagedT<TS, NS> sT(smx, cnt);
   const int32_t* js = a.jset + t * (int64_t)a.jmax;
-  const TS* tm = (const TS*)a.tmat;
   const int64_t c0 = t * a.R;
   const int slot = threadIdx.x / KG;
   const int64_t J = c0 + a.sv.ord[c0 + slot];
@@ -770,67 +951,36 @@ __global__ void __launch_bounds__(64 * KG) k_force_t(TiledForceArgs a) {
       if constexpr (NS) csr[u] = load_srec(a.ns_scol, p0 + u * KG, pend);
     }
   }
-  // thread per staged node: one index load, then its T row (12 values,
-  // 48 or 96 bytes, 16-byte aligned) as independent vector loads
-  for (int l = threadIdx.x; l < cnt; l += blockDim.x) {
-    const TS* src = tm + 12 * (int64_t)js[l];
-    TS v[12];
-    if (sizeof(TS) == 4) {
-      const float4* s4 = reinterpret_cast<const float4*>(src);
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const float4 x = __ldg(s4 + k);
-        v[4 * k] = (TS)x.x; v[4 * k + 1] = (TS)x.y; v[4 * k + 2] = (TS)x.z; v[4 * k + 3] = (TS)x.w;
-      }
-    } else {
-      const double2* s2 = reinterpret_cast<const double2*>(src);
-#pragma unroll
-      for (int k = 0; k < 6; ++k) {
-        const double2 x = __ldg(s2 + k);
-        v[2 * k] = (TS)x.x; v[2 * k + 1] = (TS)x.y;
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < 9; ++k) sT[k * cnt + l] = v[k];
-    if (nv == 12) { sT[9 * cnt + l] = v[9]; sT[10 * cnt + l] = v[10]; sT[11 * cnt + l] = v[11]; }
-    if constexpr (NS) {  // W_l: 18 of its 20 floats, as five 16-byte loads
-      const float4* w4 = reinterpret_cast<const float4*>(a.ns_w + 20 * (int64_t)js[l]);
-      TS* sW = sT + nv * cnt;
-#pragma unroll
-      for (int k = 0; k < 5; ++k) {
-        const float4 x = __ldg(w4 + k);
-        sW[(4 * k) * cnt + l] = x.x; sW[(4 * k + 1) * cnt + l] = x.y;
-        if (4 * k + 2 < 18) { sW[(4 * k + 2) * cnt + l] = x.z; sW[(4 * k + 3) * cnt + l] = x.w; }
-      }
-    }
-  }
+  sT.fill(a, js, cnt);
+  prefetch_columns(a, c0);
   __syncthreads();
-  double ke = 0.0, ee = 0.0, tf[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  unsigned st = 0;
   if (valid) {
     A f0 = A(0), f1 = A(0), f2 = A(0);
     double e0 = 0.0, e1 = 0.0, e2 = 0.0;
     auto body = [&](int it, const Rec<F64>& rec, const SRec& sr) {
       const A g0 = (A)rec.x(), g1 = (A)rec.y(), g2 = (A)rec.z();
-      const TS* T = sT + rec.l();  // component k of T_l at T[k * cnt]
-      f0 += (A)T[0] * g0 + (A)T[cnt] * g1 + (A)T[2 * cnt] * g2;
-      f1 += (A)T[3 * cnt] * g0 + (A)T[4 * cnt] * g1 + (A)T[5 * cnt] * g2;
-      f2 += (A)T[6 * cnt] * g0 + (A)T[7 * cnt] * g1 + (A)T[8 * cnt] * g2;
+      const int l = rec.l();
+      TS T[NS ? 28 : 9];
+      sT.t.load(l, T);
+      f0 += (A)T[0] * g0 + (A)T[1] * g1 + (A)T[2] * g2;
+      f1 += (A)T[3] * g0 + (A)T[4] * g1 + (A)T[5] * g2;
+      f2 += (A)T[6] * g0 + (A)T[7] * g1 + (A)T[8] * g2;
       if constexpr (NS) {
         const A sq[6] = {(A)sr.a.x, (A)sr.a.y, (A)sr.b.x, (A)sr.b.y, (A)sr.c.x, (A)sr.c.y};
-        const TS* W = T + nv * cnt;  // W_l(k, q) at W[(6 k + q) * cnt]
+        // W_l(k, q) at 6 k + q: 16 values from T[12], the last two in T[9], T[10]
 #pragma unroll
         for (int c = 0; c < 6; ++c) {
-          f0 += (A)W[c * cnt] * sq[c];
-          f1 += (A)W[(6 + c) * cnt] * sq[c];
-          f2 += (A)W[(12 + c) * cnt] * sq[c];
+          f0 += (A)T[12 + c] * sq[c];
+          f1 += (A)T[18 + c] * sq[c];
+          f2 += (A)T[c < 4 ? 24 + c : 5 + c] * sq[c];
         }
       }
       if (a.has_body) {
         const int64_t e = p0 + (int64_t)KG * it;
         if (e < pend) {  // (not a pad)
           const double s = a.tshp[e];
-          e0 += s * (double)T[9 * cnt]; e1 += s * (double)T[10 * cnt]; e2 += s * (double)T[11 * cnt];
+          const TS* b = sT.body + l;
+          e0 += s * (double)b[0]; e1 += s * (double)b[sT.ld]; e2 += s * (double)b[2 * sT.ld];
         }
       }
     };
@@ -876,10 +1026,13 @@ __global__ void __launch_bounds__(64 * KG) k_force_t(TiledForceArgs a) {
         e2 += __shfl_xor_sync(gmask, e2, o);
       }
     }
-    if (q < 3) correct_dof(a, J, q, (double)(q == 0 ? f0 : (q == 1 ? f1 : f2)), q == 0 ? e0 : (q == 1 ? e1 : e2), ke, ee, tf, st);
+    if (q < 3) {
+      const int m = 3 * (int)(J - c0) + q;
+      cs.f[m] = (double)(q == 0 ? f0 : (q == 1 ? f1 : f2));
+      if (a.has_body) cs.e[m] = q == 0 ? e0 : (q == 1 ? e1 : e2);
+    }
   }
-  step_sums(a, ke, ee, tf, red);
-  if (st) atomicOr(a.status, st);
+  finish_columns(a, c0, cs, 0u);
 }
 
 // ---- record streams through the copy engine ------------------------------
@@ -974,8 +1127,9 @@ __global__ void __launch_bounds__(64 * KG)
   issue_records<F64>(bar, smb, pk, sv.nrec, e0, ne, recmax);
   const int cnt = jcnt[t];
   const int32_t* js = jset + t * (int64_t)jmax;
-  double* sd = reinterpret_cast<double*>(smb + (size_t)recmax * RB);
-  float* sf = reinterpret_cast<float*>(sd);  // value k of rank l at [k cnt + l]
+  using SV = typename DispStage<F64>::V;
+  constexpr int SN = DispStage<F64>::N;
+  const Staged<SV, SN> sd{reinterpret_cast<SV*>(smb + (size_t)recmax * RB), staged_ld(cnt)};
   const int slot = threadIdx.x / KG;
   const int64_t i = r0 + sv.ord[r0 + slot];
   const int q = threadIdx.x & (KG - 1);
@@ -986,83 +1140,73 @@ __global__ void __launch_bounds__(64 * KG)
 #pragma unroll
     for (int k = 0; k < 3; ++k) dr[k] = dsp[3 * r0 + k];
   }
-  for (int l = threadIdx.x; l < cnt; l += blockDim.x) {
-    const int64_t g = js[l];
+  stage_disp<F64>(js, cnt, dsp, dr, sd);
+  __syncthreads();
+  if (valid) {
+    const int64_t sl = (r0 + slot) >> 3;
+    const bool ok = __all_sync(gmask, wait_records(bar, ne, sv.sstep[sl] - e0, sv.sstep[sl + 1] - e0));
+    const RowWalk<KG> walk(sv, r0, slot, q);
+    int64_t p0 = 0, pend = 0;
+    if (INTERP) {
+      p0 = rowptr[i] + q;
+      pend = rowptr[i + 1];
+    }
+    double di[3];
+    A fd[3], L[9];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      const double b = dsp[3 * g + k];
-      if (F64) sd[k * cnt + l] = b;
-      else sf[k * cnt + l] = (float)(b - dr[k]);
+      di[k] = dsp[3 * i + k];
+      fd[k] = F64 ? (A)di[k] : (A)(float)(di[k] - dr[k]);
     }
-  }
-  __syncthreads();
-  if (!valid) {
-    drain_records(bar);
-    return;
-  }
-  const int64_t sl = (r0 + slot) >> 3;
-  const bool ok = __all_sync(gmask, wait_records(bar, ne, sv.sstep[sl] - e0, sv.sstep[sl + 1] - e0));
-  const RowWalk<KG> walk(sv, r0, slot, q);
-  int64_t p0 = 0, pend = 0;
-  if (INTERP) {
-    p0 = rowptr[i] + q;
-    pend = rowptr[i + 1];
-  }
-  double di[3];
-  A fd[3], L[9];
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    di[k] = dsp[3 * i + k];
-    fd[k] = F64 ? (A)di[k] : (A)(float)(di[k] - dr[k]);
-  }
-#pragma unroll
-  for (int k = 0; k < 9; ++k) L[k] = A(0);
-  double ph[3] = {0.0, 0.0, 0.0};
-  if (ok) {
+    for (int k = 0; k < 9; ++k) L[k] = A(0);
+    double ph[3] = {0.0, 0.0, 0.0};
+    if (ok) {
 #pragma unroll 4
-    for (int it = 0; it < walk.nit; ++it) {
-      Rec<F64> rec;
-      staged_rec(smb, recmax, walk.at(it) - 32 * e0, rec);
-      const A g[3] = {(A)rec.x(), (A)rec.y(), (A)rec.z()};
-      const int l = rec.l();
-      A v[3];
+      for (int it = 0; it < walk.nit; ++it) {
+        Rec<F64> rec;
+        staged_rec(smb, recmax, walk.at(it) - 32 * e0, rec);
+        const A g[3] = {(A)rec.x(), (A)rec.y(), (A)rec.z()};
+        const int l = rec.l();
+        SV v[SN];
+        sd.load(l, v);
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        v[k] = F64 ? (A)sd[k * cnt + l] : (A)sf[k * cnt + l];
-        const A d = v[k] - fd[k];
-        L[3 * k] += d * g[0]; L[3 * k + 1] += d * g[1]; L[3 * k + 2] += d * g[2];
-      }
-      if (INTERP) {
-        const int64_t p = p0 + (int64_t)KG * it;
-        if (p < pend) {
-          const double s = shp[p];
+        for (int k = 0; k < 3; ++k) {
+          const A d = (A)v[k] - fd[k];
+          L[3 * k] += d * g[0]; L[3 * k + 1] += d * g[1]; L[3 * k + 2] += d * g[2];
+        }
+        if (INTERP) {
+          const int64_t p = p0 + (int64_t)KG * it;
+          if (p < pend) {
+            const double s = shp[p];
 #pragma unroll
-          for (int k = 0; k < 3; ++k) ph[k] += s * (F64 ? (double)v[k] : dr[k] + (double)v[k]);
+            for (int k = 0; k < 3; ++k) ph[k] += s * (F64 ? (double)v[k] : dr[k] + (double)v[k]);
+          }
         }
       }
     }
-  }
 #pragma unroll
-  for (int o = 1; o < KG; o <<= 1) {
+    for (int o = 1; o < KG; o <<= 1) {
 #pragma unroll
-    for (int k = 0; k < 9; ++k) L[k] += __shfl_xor_sync(gmask, L[k], o);
-    if (INTERP) {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) ph[k] += __shfl_xor_sync(gmask, ph[k], o);
-    }
-  }
-  if (q == 0) {
-    if (!ok) {
-      atomicOr(status, (unsigned)MEGA_ST_WAIT_TIMEOUT);
-    } else {
-      const double sd3[3] = {sdphi[3 * i], sdphi[3 * i + 1], sdphi[3 * i + 2]};
-      double h[9];
-#pragma unroll
-      for (int k = 0; k < 9; ++k) h[k] = (double)L[k] + di[k / 3] * sd3[k % 3];
-      store_g0(fg, fg_ld(n), i, !F64, h);
+      for (int k = 0; k < 9; ++k) L[k] += __shfl_xor_sync(gmask, L[k], o);
       if (INTERP) {
 #pragma unroll
-        for (int k = 0; k < 3; ++k) dsp_tot_phy[3 * i + k] += ph[k];
+        for (int k = 0; k < 3; ++k) ph[k] += __shfl_xor_sync(gmask, ph[k], o);
+      }
+    }
+    if (q == 0) {
+      if (!ok) {
+        atomicOr(status, (unsigned)MEGA_ST_WAIT_TIMEOUT);
+      } else {
+        const double sd3[3] = {sdphi[3 * i], sdphi[3 * i + 1], sdphi[3 * i + 2]};
+        double h[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) h[k] = (double)L[k] + di[k / 3] * sd3[k % 3];
+        store_g0(fg, fg_ld(n), i, !F64, h);
+        if (INTERP) {
+#pragma unroll
+          for (int k = 0; k < 3; ++k) dsp_tot_phy[3 * i + k] += ph[k];
+        }
       }
     }
   }
@@ -1074,45 +1218,22 @@ __global__ void __launch_bounds__(64 * KG) k_force_b(TiledForceArgs a) {
   constexpr int RB = F64 ? 26 : 16;
   extern __shared__ __align__(128) unsigned char smb[];
   __shared__ uint64_t bar[kChunks];
-  __shared__ double red[32 * 8];  // eight sums per warp, up to 32 warps (KG = 16)
+  __shared__ ColumnSums cs;
   const int64_t t = blockIdx.x;
   const int64_t c0 = t * a.R;
   const int64_t e0 = a.sv.sstep[c0 >> 3], ne = a.sv.sstep[(c0 + a.R) >> 3] - e0;
   issue_records<F64>(bar, smb, a.pk, a.sv.nrec, e0, ne, a.recmax);
   const int cnt = a.jcnt[t];
-  const int nv = a.has_body ? 12 : 9;
-  TS* sT = reinterpret_cast<TS*>(smb + (size_t)a.recmax * RB);
+  const StagedT<TS, false> sT(smb + (size_t)a.recmax * RB, cnt);
   const int32_t* js = a.jset + t * (int64_t)a.jmax;
-  const TS* tm = (const TS*)a.tmat;
   const int slot = threadIdx.x / KG;
   const int64_t J = c0 + a.sv.ord[c0 + slot];
   const int q = threadIdx.x & (KG - 1);
   const unsigned gmask = group_mask<KG>();
   const bool valid = J < a.n;
-  for (int l = threadIdx.x; l < cnt; l += blockDim.x) {
-    const TS* src = tm + 12 * (int64_t)js[l];
-    TS v[12];
-    if (sizeof(TS) == 4) {
-      const float4* s4 = reinterpret_cast<const float4*>(src);
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const float4 x = __ldg(s4 + k);
-        v[4 * k] = (TS)x.x; v[4 * k + 1] = (TS)x.y; v[4 * k + 2] = (TS)x.z; v[4 * k + 3] = (TS)x.w;
-      }
-    } else {
-      const double2* s2 = reinterpret_cast<const double2*>(src);
-#pragma unroll
-      for (int k = 0; k < 6; ++k) {
-        const double2 x = __ldg(s2 + k);
-        v[2 * k] = (TS)x.x; v[2 * k + 1] = (TS)x.y;
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < 9; ++k) sT[k * cnt + l] = v[k];
-    if (nv == 12) { sT[9 * cnt + l] = v[9]; sT[10 * cnt + l] = v[10]; sT[11 * cnt + l] = v[11]; }
-  }
+  sT.fill(a, js, cnt);
+  prefetch_columns(a, c0);
   __syncthreads();
-  double ke = 0.0, ee = 0.0, tf[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   unsigned st = 0;
   if (valid) {
     const int64_t sl = (c0 + slot) >> 3;
@@ -1132,15 +1253,17 @@ __global__ void __launch_bounds__(64 * KG) k_force_b(TiledForceArgs a) {
         staged_rec(smb, a.recmax, walk.at(it) - 32 * e0, rec);
         const A g0 = (A)rec.x(), g1 = (A)rec.y(), g2 = (A)rec.z();
         const int l = rec.l();
-        const TS* T = sT + l;  // component k of T_l at T[k * cnt]
-        f0 += (A)T[0] * g0 + (A)T[cnt] * g1 + (A)T[2 * cnt] * g2;
-        f1 += (A)T[3 * cnt] * g0 + (A)T[4 * cnt] * g1 + (A)T[5 * cnt] * g2;
-        f2 += (A)T[6 * cnt] * g0 + (A)T[7 * cnt] * g1 + (A)T[8 * cnt] * g2;
+        TS T[9];
+        sT.t.load(l, T);
+        f0 += (A)T[0] * g0 + (A)T[1] * g1 + (A)T[2] * g2;
+        f1 += (A)T[3] * g0 + (A)T[4] * g1 + (A)T[5] * g2;
+        f2 += (A)T[6] * g0 + (A)T[7] * g1 + (A)T[8] * g2;
         if (a.has_body) {
           const int64_t p = p0 + (int64_t)KG * it;
           if (p < pend) {
             const double s = a.tshp[p];
-            b0 += s * (double)T[9 * cnt]; b1 += s * (double)T[10 * cnt]; b2 += s * (double)T[11 * cnt];
+            const TS* b = sT.body + l;
+            b0 += s * (double)b[0]; b1 += s * (double)b[sT.ld]; b2 += s * (double)b[2 * sT.ld];
           }
         }
       }
@@ -1156,15 +1279,14 @@ __global__ void __launch_bounds__(64 * KG) k_force_b(TiledForceArgs a) {
         b2 += __shfl_xor_sync(gmask, b2, o);
       }
     }
-    if (!ok) {
-      if (q == 0) st |= MEGA_ST_WAIT_TIMEOUT;
-    } else if (q < 3) {
-      correct_dof(a, J, q, (double)(q == 0 ? f0 : (q == 1 ? f1 : f2)), q == 0 ? b0 : (q == 1 ? b1 : b2), ke, ee, tf,
-                  st);
+    if (!ok && q == 0) st |= MEGA_ST_WAIT_TIMEOUT;  // (the step's outputs are void)
+    if (q < 3) {
+      const int m = 3 * (int)(J - c0) + q;
+      cs.f[m] = (double)(q == 0 ? f0 : (q == 1 ? f1 : f2));
+      if (a.has_body) cs.e[m] = q == 0 ? b0 : (q == 1 ? b1 : b2);
     }
   }
-  step_sums(a, ke, ee, tf, red);
-  if (st) atomicOr(a.status, st);
+  finish_columns(a, c0, cs, st);
   drain_records(bar);
 }
 
@@ -1275,8 +1397,8 @@ int bank_order(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* ptr,
   if ((lanes != 4 && lanes != 8) || ts.R * lanes < 32) return MEGA_ERR_UNSUPPORTED;
   const int64_t nwarps = ts.ntiles * (int64_t)(ts.R * lanes / 32);
   const unsigned grid = (unsigned)((nwarps * 32 + 127) / 128);
-  if (lanes == 4) k_bank_order<4, 32, 32><<<grid, 128, 0, s>>>(n, ts.R, nwarps, ts.ord, ptr, lidx, pos_src, pos);
-  else k_bank_order<8, 32, 32><<<grid, 128, 0, s>>>(n, ts.R, nwarps, ts.ord, ptr, lidx, pos_src, pos);
+  if (lanes == 4) k_bank_order<4, 8, 8><<<grid, 128, 0, s>>>(n, ts.R, nwarps, ts.ord, ptr, lidx, pos_src, pos);
+  else k_bank_order<8, 8, 8><<<grid, 128, 0, s>>>(n, ts.R, nwarps, ts.ord, ptr, lidx, pos_src, pos);
   MEGA_CHECK_LAUNCH();
   return 0;
 }
@@ -1295,10 +1417,12 @@ int gather_f6(cudaStream_t s, int64_t m, const int64_t* pos, const float* in, fl
   return 0;
 }
 
-int gather_records32(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* ptr, const int64_t* pos,
-                     const float4* in, float4* out) {
+int gather_records(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* ptr, const int64_t* pos, bool f64,
+                   const void* in, void* out) {
   const int64_t slots = ts.ntiles * ts.R;
-  k_gather_rec32<<<grid_for(4 * slots, 256), 256, 0, s>>>(n, ts.R, slots, ts.view(), ptr, pos, in, out);
+  const unsigned grid = grid_for(4 * slots, 256);
+  if (f64) k_gather_rec64<<<grid, 256, 0, s>>>(n, ts.R, slots, ts.view(), ptr, pos, in, out);
+  else k_gather_rec32<<<grid, 256, 0, s>>>(n, ts.R, slots, ts.view(), ptr, pos, (const float4*)in, (float4*)out);
   MEGA_CHECK_LAUNCH();
   return 0;
 }
@@ -1375,7 +1499,7 @@ static int configure_bulk(int lim) {
 int configure_tiled_kernels() {
   static bool done = false;
   if (done) return 0;
-  const int lim = 30 * 4 * 1024 + 1024;
+  const int lim = 31 * 4 * staged_ld(1024);
   int r = 0;
   if ((r = configure_variant<4, 4>(lim)) || (r = configure_variant<4, 2>(lim)) ||
       (r = configure_variant<4, 1>(lim)) || (r = configure_variant<8, 2>(lim)) ||
@@ -1392,8 +1516,8 @@ int tiled_variants() { return kVariants; }
 bool tiled_variant_fits(const TileSet& ts, bool mixed, int variant, bool force, bool has_body) {
   if (variant < 0 || variant >= kVariants) return false;
   if (variant < 4 || variant > 5) return true;  // register variants
-  const size_t stage = force ? (mixed ? sizeof(float) : sizeof(double)) * (has_body ? 12 : 9) : (mixed ? 12 : 24);
-  return (size_t)ts.recmax * (mixed ? 16 : 26) + stage * (size_t)ts.maxcnt <= (size_t)g_bulk_lim;
+  const size_t stage = force ? (mixed ? sizeof(float) : sizeof(double)) * (has_body ? 12 : 9) : (mixed ? 16 : 24);
+  return (size_t)ts.recmax * (mixed ? 16 : 26) + stage * staged_ld(ts.maxcnt) <= (size_t)g_bulk_lim;
 }
 
 // one launch's arguments of the row gather
@@ -1413,7 +1537,7 @@ struct DefgradArgs {
 template <int KG>
 static int defgrad_bulk(cudaStream_t s, const DefgradArgs& d) {
   const TileSet& ts = d.ts;
-  const size_t smem = (size_t)ts.recmax * (d.mixed ? 16 : 26) + (d.mixed ? 12 : 24) * (size_t)ts.maxcnt;
+  const size_t smem = (size_t)ts.recmax * (d.mixed ? 16 : 26) + (size_t)(d.mixed ? 16 : 24) * staged_ld(ts.maxcnt);
   if (smem > (size_t)g_bulk_lim) return MEGA_ERR_UNSUPPORTED;
   auto k = d.mixed ? (d.interp ? k_defgrad_b<float, false, true, KG> : k_defgrad_b<float, false, false, KG>)
                    : (d.interp ? k_defgrad_b<double, true, true, KG> : k_defgrad_b<double, true, false, KG>);
@@ -1426,7 +1550,7 @@ static int defgrad_bulk(cudaStream_t s, const DefgradArgs& d) {
 template <int KG, int KU, bool FULL = false>
 static void defgrad_variant(cudaStream_t s, const DefgradArgs& d) {
   const TileSet& ts = d.ts;
-  const size_t smem = (size_t)((d.mixed ? 12 : 24) * (FULL ? 2 : 1)) * (size_t)ts.maxcnt;
+  const size_t smem = (size_t)((d.mixed ? 16 : 24) * (FULL ? 2 : 1)) * staged_ld(ts.maxcnt);
   const NsniTiles nz = d.ns ? *d.ns : NsniTiles();
   auto k = !d.mixed ? (d.interp ? k_defgrad_t<double, true, true, KG, KU, false, FULL>
                                 : k_defgrad_t<double, true, false, KG, KU, false, FULL>)
@@ -1470,7 +1594,7 @@ template <int KG>
 static int force_bulk(cudaStream_t s, bool mixed, const TiledForceArgs& a) {
   const int nv = a.has_body ? 12 : 9;
   const size_t smem = (size_t)a.recmax * (mixed ? 16 : 26) + (mixed ? sizeof(float) : sizeof(double)) * nv *
-                      (size_t)a.maxcnt;
+                      staged_ld(a.maxcnt);
   if (smem > (size_t)g_bulk_lim) return MEGA_ERR_UNSUPPORTED;
   const unsigned grid = (unsigned)a.ntiles;
   const int block = a.R * KG;
@@ -1481,8 +1605,8 @@ static int force_bulk(cudaStream_t s, bool mixed, const TiledForceArgs& a) {
 
 template <int KG, int KU>
 static void force_variant(cudaStream_t s, bool mixed, const TiledForceArgs& a) {
-  const int nv = (a.has_body ? 12 : 9) + (a.ns_scol ? 18 : 0);
-  const size_t smem = (mixed ? sizeof(float) : sizeof(double)) * nv * (size_t)a.maxcnt;
+  const int nv = (a.ns_scol ? 28 : 9) + (a.has_body ? 3 : 0);
+  const size_t smem = (mixed ? sizeof(float) : sizeof(double)) * nv * staged_ld(a.maxcnt);
   const unsigned grid = (unsigned)a.ntiles;
   const int block = a.R * KG;
   if (mixed && a.ns_scol) k_force_t<float, float, false, KG, KU, true><<<grid, block, smem, s>>>(a);

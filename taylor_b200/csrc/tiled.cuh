@@ -98,16 +98,16 @@ int pack_transposed32(cudaStream_t s, int32_t n, const TileSet& ct, const int64_
 int pad_records32(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* ptr, float4* out);
 // Reorder the entries within each row (column) of the tiles ts so that the
 // lanes of a warp of a gather with `lanes` (4 or 8) lanes per row read
-// distinct shared-memory banks of the staged neighbour data (one 32-bit
-// word per rank and value) where possible.  lidx is reordered in place;
+// distinct shared-memory banks of the staged neighbour data (16-byte vectors
+// by rank) where possible.  lidx is reordered in place;
 // pos[e] receives pos_src (or, when null, the identity) at the entry's
 // position before, and must hold that same array on entry.
 int bank_order(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* ptr, uint16_t* lidx,
                const int64_t* pos_src, int64_t* pos, int lanes);
 // out[e] = e;  entry e takes the record of entry pos[e] of its row
 int iota64(cudaStream_t s, int64_t m, int64_t* out);
-int gather_records32(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* ptr, const int64_t* pos,
-                     const float4* in, float4* out);
+int gather_records(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* ptr, const int64_t* pos, bool f64,
+                   const void* in, void* out);
 // out[6 e + k] = in[6 pos[e] + k]
 int gather_f6(cudaStream_t s, int64_t m, const int64_t* pos, const float* in, float* out);
 int configure_tiled_kernels();
