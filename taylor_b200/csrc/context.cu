@@ -665,8 +665,6 @@ static int step_once(Ctx* c, double dt, int mode, int predict, cudaEvent_t* ev, 
   const bool mixed = (mode & 0xff) == MEGA_MODE_MIXED;
   const bool interp = (mode & MEGA_FLAG_INTERP_EACH_STEP) != 0;
   if (ev) MEGA_TRY(cudaEventRecord(ev[0], c->s));
-  if (c->nsni)
-    MEGA_TRY(cudaMemcpyAsync(c->stress_prev, c->stress, sizeof(double) * 6 * c->n, cudaMemcpyDeviceToDevice, c->s));
   NsniTiles nt;
   int r = launch_defgrad_tiled(c->s, mixed, interp, c->n, c->rt, nsni_tiles(c, mixed, nt), c->csr.rowptr,
                                mixed ? c->pk32 : c->pk64, c->dsp, c->dsp_tot, mixed ? c->sdphi32 : c->sdphi,
@@ -678,6 +676,7 @@ static int step_once(Ctx* c, double dt, int mode, int predict, cudaEvent_t* ev, 
   StressArgs sa = stress_args(c, dt, mode);
   sa.add_g0 = !full;
   sa.more = predict;
+  sa.stress_prev = c->nsni ? c->stress_prev : nullptr;
   r = launch_stress(c->s, mixed, sa);
   if (r) return r;
   if (c->nsni && (r = nsni_step(c->s, nsni_args(c), c->csr, c->nsr, c->nsc, mixed, c->dsp, 1))) return r;

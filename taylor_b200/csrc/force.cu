@@ -327,6 +327,12 @@ __device__ __forceinline__ void stress_finish(const StressArgs& a, int64_t i, Tr
     sinc[k] = snew[k] - (LEAN ? a.stress[6 * i + k] : w.sold[k]);
     einc[k] = enew[k] - (LEAN ? a.strain[6 * i + k] : w.eold[k]);
   }
+  if (a.stress_prev) {
+    double2* p2 = reinterpret_cast<double2*>(a.stress_prev + 6 * i);
+    const double2* old = reinterpret_cast<const double2*>(a.stress + 6 * i);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) p2[k] = LEAN ? old[k] : make_double2(w.sold[2 * k], w.sold[2 * k + 1]);
+  }
   {
     double2* s2 = reinterpret_cast<double2*>(a.stress + 6 * i);
     double2* e2 = reinterpret_cast<double2*>(a.strain + 6 * i);
@@ -426,6 +432,7 @@ template <typename T, typename TS, bool DAM, bool QUEUE>
 __global__ void __launch_bounds__(256, 2) k_stress(StressArgs a) {
   __shared__ double smd[32];
   __shared__ unsigned long long smu[32];
+  grid_wait();
   if (blockIdx.x == 0 && threadIdx.x < kSlots) {
     a.acc->ke[threadIdx.x] = 0.0;  // the force kernel of this step accumulates it afresh
   }
@@ -469,6 +476,7 @@ __global__ void __launch_bounds__(kLearnBlock, 4) k_stress_queue(StressArgs a) {
   __shared__ __align__(16) MlpSmem net;
   __shared__ __align__(16) uint16_t sH1[kLearnBlock * kMlpLd];
   __shared__ float sOut[kLearnBlock];
+  grid_wait();
   const int64_t count = *a.qcount;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -714,13 +722,9 @@ int launch_stress(cudaStream_t s, bool mixed, const StressArgs& a) {
       else k_stress_queue<double, double, false><<<lgrid, kLearnBlock, 0, s>>>(qa);
     }
   } else {
-    if (a.aux) {
-      if (mixed) k_stress<float, float, true, false><<<grid, block, 0, s>>>(a);
-      else k_stress<double, double, true, false><<<grid, block, 0, s>>>(a);
-    } else {
-      if (mixed) k_stress<float, float, false, false><<<grid, block, 0, s>>>(a);
-      else k_stress<double, double, false, false><<<grid, block, 0, s>>>(a);
-    }
+    auto k = a.aux ? (mixed ? k_stress<float, float, true, false> : k_stress<double, double, true, false>)
+                   : (mixed ? k_stress<float, float, false, false> : k_stress<double, double, false, false>);
+    return launch_overlapped(k, grid, block, 0, s, a);
   }
   MEGA_CHECK_LAUNCH();
   return 0;

@@ -78,8 +78,9 @@ __global__ void k_nsni_combine(int32_t n, int a, const int64_t* __restrict__ row
 // hq[18 i + 6 k + q] = sum_J S_q(J) du_J,k (S double or float, sums in double)
 template <typename SV>
 __global__ void __launch_bounds__(256) k_nsni_h(int32_t n, const int64_t* __restrict__ rowptr,
-                                                const int32_t* __restrict__ col, NsniArr<SV> s,
-                                                const double* __restrict__ du, double* __restrict__ hq) {
+                                                const int32_t* __restrict__ col, NsniArr<SV> s, const double* du,
+                                                double* hq) {
+  grid_wait();
   const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kNL;
   const int q = threadIdx.x & (kNL - 1);
   const unsigned gm = 0xFFu << (threadIdx.x & 24);
@@ -167,6 +168,7 @@ __device__ __forceinline__ void estimate_moduli_nsni(const double sinc[6], const
 template <typename WV>
 __global__ void __launch_bounds__(128) k_nsni_stress(NsniStepArgs a) {
   __shared__ double red[4];
+  grid_wait();
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   double work = 0.0;
   if (i < a.n) {
@@ -282,7 +284,8 @@ __global__ void __launch_bounds__(128) k_nsni_stress(NsniStepArgs a) {
 template <typename V>
 __global__ void __launch_bounds__(256) k_nsni_force(int32_t n, const int64_t* __restrict__ colptr,
                                                     const int32_t* __restrict__ trow, NsniArr<V> st,
-                                                    const V* __restrict__ w, double* __restrict__ fstab) {
+                                                    const V* w, double* fstab) {
+  grid_wait();
   const int64_t J = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kNL;
   const int q = threadIdx.x & (kNL - 1);
   const unsigned gm = 0xFFu << (threadIdx.x & 24);
@@ -386,16 +389,10 @@ int nsni_step(cudaStream_t s, const NsniStepArgs& a, const DevCSR& csr, const Ns
   const unsigned gg = (unsigned)(((int64_t)a.n * kNL + 255) / 256);
   const unsigned gn = (unsigned)((a.n + 127) / 128);
   if (mixed && stage != 1) return MEGA_ERR_UNSUPPORTED;  // the tiled gathers carry those terms
-  if (stage == 0) {
-    k_nsni_h<double><<<gg, 256, 0, s>>>(a.n, csr.rowptr, csr.col, rows, du, a.hq);
-  } else if (stage == 1) {
-    if (mixed) k_nsni_stress<float><<<gn, 128, 0, s>>>(a);
-    else k_nsni_stress<double><<<gn, 128, 0, s>>>(a);
-  } else {
-    k_nsni_force<double><<<gg, 256, 0, s>>>(a.n, csr.colptr, csr.trow, cols, (const double*)a.w, a.fstab);
-  }
-  MEGA_CHECK_LAUNCH();
-  return 0;
+  if (stage == 0) return launch_overlapped(k_nsni_h<double>, gg, 256, 0, s, a.n, csr.rowptr, csr.col, rows, du, a.hq);
+  if (stage == 1) return launch_overlapped(mixed ? k_nsni_stress<float> : k_nsni_stress<double>, gn, 128, 0, s, a);
+  return launch_overlapped(k_nsni_force<double>, gg, 256, 0, s, a.n, csr.colptr, csr.trow, cols, (const double*)a.w,
+                           a.fstab);
 }
 
 int nsni_records(cudaStream_t s, int64_t m, const int64_t* pos, const NsniS& src, float* dst) {

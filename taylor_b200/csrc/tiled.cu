@@ -476,7 +476,7 @@ struct Staged {
 
 // 32 bytes at a 32-byte boundary
 __device__ __forceinline__ void load_sector(const double* p, double v[4]) {
-  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p));
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p));
 }
 
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
@@ -523,20 +523,46 @@ struct DispStage<true> {
 template <bool F64>
 using StagedDisp = Staged<typename DispStage<F64>::V, DispStage<F64>::N>;
 
+// The ranks a thread stages, in its order: the first ones are read before the
+// wait for the kernel before (the sets' rows have room for jmax ids, so a rank
+// past the tile's count reads stale ids that are not used).
+template <int KG>
+struct StageIds {
+  static constexpr int K = 16 / KG;
+  int32_t id[K];
+  const int32_t* js;
+  __device__ __forceinline__ StageIds(const int32_t* js_, int32_t jmax) : js(js_) {
+#pragma unroll
+    for (int u = 0; u < K; ++u) {
+      const int l = threadIdx.x + u * blockDim.x;
+      id[u] = l < jmax ? js[l] : 0;
+    }
+  }
+  // f(rank, node) for this thread's ranks below cnt
+  template <typename F>
+  __device__ __forceinline__ void each(int cnt, F f) const {
+#pragma unroll
+    for (int u = 0; u < K; ++u) {
+      const int l = threadIdx.x + u * blockDim.x;
+      if (l < cnt) f(l, (int64_t)id[u]);
+    }
+    for (int l = threadIdx.x + K * blockDim.x; l < cnt; l += blockDim.x) f(l, (int64_t)js[l]);
+  }
+};
+
 // a thread per staged node
-template <bool F64>
-__device__ __forceinline__ void stage_disp(const int32_t* js, int cnt, const double* v, const double* ref,
+template <bool F64, int KG>
+__device__ __forceinline__ void stage_disp(const StageIds<KG>& ids, int cnt, const double* v, const double* ref,
                                            const StagedDisp<F64>& out) {
-  for (int l = threadIdx.x; l < cnt; l += blockDim.x) {
-    const int64_t g = 3 * (int64_t)js[l];
-    const double x0 = v[g], x1 = v[g + 1], x2 = v[g + 2];
+  ids.each(cnt, [&](int l, int64_t j) {
+    const double x0 = v[3 * j], x1 = v[3 * j + 1], x2 = v[3 * j + 2];
     if constexpr (F64) {
       out.put(l, 0, make_double2(x0, x1));
       out.at(l, 2) = x2;
     } else {
       out.put(l, 0, make_float4((float)(x0 - ref[0]), (float)(x1 - ref[1]), (float)(x2 - ref[2]), 0.f));
     }
-  }
+  });
 }
 
 // FULL: F - I is formed besides G0.  Without it the gather stages and reads
@@ -555,17 +581,12 @@ template <typename A, bool F64, bool INTERP, int KG, int KU, bool NS, bool FULL>
 __global__ void __launch_bounds__(64 * KG, defgrad_blocks<F64, KG, NS, FULL>())
     k_defgrad_t(int32_t n, int32_t R, int32_t jmax, NsniTiles ns, SliceView sv, const int64_t* __restrict__ rowptr,
                 const void* __restrict__ pk, const int32_t* __restrict__ jset, const int32_t* __restrict__ jcnt,
-                const double* __restrict__ dsp, const double* __restrict__ dsp_tot,
-                const double* __restrict__ sdphi, const double* __restrict__ shp, double* __restrict__ dsp_tot_phy,
-                double* __restrict__ fg, StepAccum* __restrict__ acc) {
+                const double* dsp, const double* dsp_tot, const double* __restrict__ sdphi,
+                const double* __restrict__ shp, double* dsp_tot_phy, double* fg, StepAccum* acc) {
   extern __shared__ __align__(16) double sm[];
-  if (acc && blockIdx.x == 0 && threadIdx.x < kSlots) {
-    acc->newton_iters[threadIdx.x] = 0ull;
-    acc->plastic[threadIdx.x] = 0ull;
-  }
   const int64_t t = blockIdx.x;
   const int cnt = jcnt[t];
-  const int32_t* js = jset + t * (int64_t)jmax;
+  const StageIds<KG> ids(jset + t * (int64_t)jmax, jmax);
   // Staged neighbour displacements, du_J (FULL: and u_J).  FP64 as doubles;
   // mixed as float offsets from the tile's first node r0 (du_J - du_r0,
   // u_J - u_r0; one 16-byte vector with a pad), half the shared-memory
@@ -602,6 +623,11 @@ __global__ void __launch_bounds__(64 * KG, defgrad_blocks<F64, KG, NS, FULL>())
       if constexpr (NS) csr[u] = load_srec(ns.srow, p0 + u * KG, pend);
     }
   }
+  grid_wait();
+  if (acc && blockIdx.x == 0 && threadIdx.x < kSlots) {
+    acc->newton_iters[threadIdx.x] = 0ull;
+    acc->plastic[threadIdx.x] = 0ull;
+  }
   double ur[3] = {0.0, 0.0, 0.0}, dr[3] = {0.0, 0.0, 0.0};
   if (!F64) {
 #pragma unroll
@@ -610,8 +636,8 @@ __global__ void __launch_bounds__(64 * KG, defgrad_blocks<F64, KG, NS, FULL>())
       if (FULL) ur[k] = dsp_tot[3 * r0 + k];
     }
   }
-  stage_disp<F64>(js, cnt, dsp, dr, sd);
-  if (FULL) stage_disp<F64>(js, cnt, dsp_tot, ur, su);
+  stage_disp<F64, KG>(ids, cnt, dsp, dr, sd);
+  if (FULL) stage_disp<F64, KG>(ids, cnt, dsp_tot, ur, su);
   __syncthreads();
   if (valid) {
     double ui[3] = {0.0, 0.0, 0.0}, di[3];
@@ -871,19 +897,19 @@ struct StagedT {
   // A thread per staged node.  FP64: the 96-byte row as three 32-byte loads,
   // a sector each (as six 16-byte loads every line was fetched twice once the
   // blocks' shared memory had shrunk L1).
-  __device__ __forceinline__ void fill(const TiledForceArgs& a, const int32_t* js, int cnt) const {
-    for (int l = threadIdx.x; l < cnt; l += blockDim.x) {
-      const int64_t j = js[l];
+  template <int KG>
+  __device__ __forceinline__ void fill(const TiledForceArgs& a, const StageIds<KG>& ids, int cnt) const {
+    ids.each(cnt, [&](int l, int64_t j) {
       if constexpr (sizeof(TS) == 4) {
         const float4* p = reinterpret_cast<const float4*>(a.tmat) + 3 * j;
-        const float4 x = __ldg(p), y = __ldg(p + 1), z = __ldg(p + 2);
+        const float4 x = p[0], y = p[1], z = p[2];
         t.put(l, 0, x);
         t.put(l, 1, y);
         t.at(l, 8) = z.x;
         if (a.has_body) { body[l] = z.y; body[ld + l] = z.z; body[2 * ld + l] = z.w; }
         if constexpr (NS) {
           const float4* w = reinterpret_cast<const float4*>(a.ns_w) + 5 * j;
-          const float4 w0 = __ldg(w), w1 = __ldg(w + 1), w2 = __ldg(w + 2), w3 = __ldg(w + 3), w4 = __ldg(w + 4);
+          const float4 w0 = w[0], w1 = w[1], w2 = w[2], w3 = w[3], w4 = w[4];
           t.put(l, 3, w0);
           t.put(l, 4, w1);
           t.put(l, 5, w2);
@@ -904,7 +930,7 @@ struct StagedT {
         t.at(l, 8) = z[0];
         if (a.has_body) { body[l] = z[1]; body[ld + l] = z[2]; body[2 * ld + l] = z[3]; }
       }
-    }
+    });
   }
 };
 
@@ -924,7 +950,7 @@ __global__ void __launch_bounds__(64 * KG, force_blocks<F64, KG, KU, NS>()) k_fo
   const int64_t t = blockIdx.x;
   const int cnt = a.jcnt[t];
   const StagedT<TS, NS> sT(smx, cnt);
-  const int32_t* js = a.jset + t * (int64_t)a.jmax;
+  const StageIds<KG> ids(a.jset + t * (int64_t)a.jmax, a.jmax);
   const int64_t c0 = t * a.R;
   const int slot = threadIdx.x / KG;
   const int64_t J = c0 + a.sv.ord[c0 + slot];
@@ -951,7 +977,8 @@ __global__ void __launch_bounds__(64 * KG, force_blocks<F64, KG, KU, NS>()) k_fo
       if constexpr (NS) csr[u] = load_srec(a.ns_scol, p0 + u * KG, pend);
     }
   }
-  sT.fill(a, js, cnt);
+  grid_wait();
+  sT.fill(a, ids, cnt);
   prefetch_columns(a, c0);
   __syncthreads();
   if (valid) {
@@ -1111,22 +1138,17 @@ template <typename A, bool F64, bool INTERP, int KG>
 __global__ void __launch_bounds__(64 * KG)
     k_defgrad_b(int32_t n, int32_t R, int32_t jmax, int32_t recmax, SliceView sv, const int64_t* __restrict__ rowptr,
                 const void* __restrict__ pk, const int32_t* __restrict__ jset, const int32_t* __restrict__ jcnt,
-                const double* __restrict__ dsp, const double* __restrict__ sdphi, const double* __restrict__ shp,
-                double* __restrict__ dsp_tot_phy, double* __restrict__ fg, StepAccum* __restrict__ acc,
-                unsigned* __restrict__ status) {
+                const double* dsp, const double* __restrict__ sdphi, const double* __restrict__ shp,
+                double* dsp_tot_phy, double* fg, StepAccum* acc, unsigned* status) {
   constexpr int RB = F64 ? 26 : 16;
   extern __shared__ __align__(128) unsigned char smb[];
   __shared__ uint64_t bar[kChunks];
-  if (acc && blockIdx.x == 0 && threadIdx.x < kSlots) {
-    acc->newton_iters[threadIdx.x] = 0ull;
-    acc->plastic[threadIdx.x] = 0ull;
-  }
   const int64_t t = blockIdx.x;
   const int64_t r0 = t * R;
   const int64_t e0 = sv.sstep[r0 >> 3], ne = sv.sstep[(r0 + R) >> 3] - e0;
   issue_records<F64>(bar, smb, pk, sv.nrec, e0, ne, recmax);
   const int cnt = jcnt[t];
-  const int32_t* js = jset + t * (int64_t)jmax;
+  const StageIds<KG> ids(jset + t * (int64_t)jmax, jmax);
   using SV = typename DispStage<F64>::V;
   constexpr int SN = DispStage<F64>::N;
   const Staged<SV, SN> sd{reinterpret_cast<SV*>(smb + (size_t)recmax * RB), staged_ld(cnt)};
@@ -1135,12 +1157,17 @@ __global__ void __launch_bounds__(64 * KG)
   const int q = threadIdx.x & (KG - 1);
   const unsigned gmask = group_mask<KG>();
   const bool valid = i < n;
+  grid_wait();
+  if (acc && blockIdx.x == 0 && threadIdx.x < kSlots) {
+    acc->newton_iters[threadIdx.x] = 0ull;
+    acc->plastic[threadIdx.x] = 0ull;
+  }
   double dr[3] = {0.0, 0.0, 0.0};
   if (!F64) {
 #pragma unroll
     for (int k = 0; k < 3; ++k) dr[k] = dsp[3 * r0 + k];
   }
-  stage_disp<F64>(js, cnt, dsp, dr, sd);
+  stage_disp<F64, KG>(ids, cnt, dsp, dr, sd);
   __syncthreads();
   if (valid) {
     const int64_t sl = (r0 + slot) >> 3;
@@ -1225,13 +1252,14 @@ __global__ void __launch_bounds__(64 * KG) k_force_b(TiledForceArgs a) {
   issue_records<F64>(bar, smb, a.pk, a.sv.nrec, e0, ne, a.recmax);
   const int cnt = a.jcnt[t];
   const StagedT<TS, false> sT(smb + (size_t)a.recmax * RB, cnt);
-  const int32_t* js = a.jset + t * (int64_t)a.jmax;
+  const StageIds<KG> ids(a.jset + t * (int64_t)a.jmax, a.jmax);
   const int slot = threadIdx.x / KG;
   const int64_t J = c0 + a.sv.ord[c0 + slot];
   const int q = threadIdx.x & (KG - 1);
   const unsigned gmask = group_mask<KG>();
   const bool valid = J < a.n;
-  sT.fill(a, js, cnt);
+  grid_wait();
+  sT.fill(a, ids, cnt);
   prefetch_columns(a, c0);
   __syncthreads();
   unsigned st = 0;
@@ -1541,14 +1569,13 @@ static int defgrad_bulk(cudaStream_t s, const DefgradArgs& d) {
   if (smem > (size_t)g_bulk_lim) return MEGA_ERR_UNSUPPORTED;
   auto k = d.mixed ? (d.interp ? k_defgrad_b<float, false, true, KG> : k_defgrad_b<float, false, false, KG>)
                    : (d.interp ? k_defgrad_b<double, true, true, KG> : k_defgrad_b<double, true, false, KG>);
-  k<<<(unsigned)ts.ntiles, ts.R * KG, smem, s>>>(d.n, ts.R, ts.jmax, ts.recmax, ts.view(), d.rowptr, d.pk, ts.jset,
-                                                 ts.jcnt, d.dsp, d.sdphi, d.shp, d.dsp_tot_phy, d.fg, d.acc,
-                                                 d.status);
-  return 0;
+  return launch_overlapped(k, (unsigned)ts.ntiles, ts.R * KG, smem, s, d.n, ts.R, ts.jmax, ts.recmax, ts.view(),
+                           d.rowptr, d.pk, ts.jset, ts.jcnt, d.dsp, d.sdphi, d.shp, d.dsp_tot_phy, d.fg, d.acc,
+                           d.status);
 }
 
 template <int KG, int KU, bool FULL = false>
-static void defgrad_variant(cudaStream_t s, const DefgradArgs& d) {
+static int defgrad_variant(cudaStream_t s, const DefgradArgs& d) {
   const TileSet& ts = d.ts;
   const size_t smem = (size_t)((d.mixed ? 16 : 24) * (FULL ? 2 : 1)) * staged_ld(ts.maxcnt);
   const NsniTiles nz = d.ns ? *d.ns : NsniTiles();
@@ -1558,8 +1585,8 @@ static void defgrad_variant(cudaStream_t s, const DefgradArgs& d) {
                                 : k_defgrad_t<float, false, false, KG, KU, true, FULL>)
                     : (d.interp ? k_defgrad_t<float, false, true, KG, KU, false, FULL>
                                 : k_defgrad_t<float, false, false, KG, KU, false, FULL>);
-  k<<<(unsigned)ts.ntiles, ts.R * KG, smem, s>>>(d.n, ts.R, ts.jmax, nz, ts.view(), d.rowptr, d.pk, ts.jset, ts.jcnt,
-                                                 d.dsp, d.dsp_tot, d.sdphi, d.shp, d.dsp_tot_phy, d.fg, d.acc);
+  return launch_overlapped(k, (unsigned)ts.ntiles, ts.R * KG, smem, s, d.n, ts.R, ts.jmax, nz, ts.view(), d.rowptr,
+                           d.pk, ts.jset, ts.jcnt, d.dsp, d.dsp_tot, d.sdphi, d.shp, d.dsp_tot_phy, d.fg, d.acc);
 }
 
 int launch_defgrad_tiled(cudaStream_t s, bool mixed, bool interp, int32_t n, const TileSet& ts,
@@ -1570,19 +1597,19 @@ int launch_defgrad_tiled(cudaStream_t s, bool mixed, bool interp, int32_t n, con
   if (ns && (!mixed || variant == 4 || variant == 5)) return MEGA_ERR_UNSUPPORTED;  // NSNI: register variants
   const DefgradArgs d{mixed, interp, n, ts, ns, rowptr, pk, dsp, dsp_tot, sdphi, shp, dsp_tot_phy, fg, acc, status};
   if (full) {
-    if (variant == 6 || variant == 7) defgrad_variant<16, kFullKU, true>(s, d);
-    else if (variant == 3 || variant == 5) defgrad_variant<8, kFullKU, true>(s, d);
-    else defgrad_variant<4, kFullKU, true>(s, d);
+    if (variant == 6 || variant == 7) r = defgrad_variant<16, kFullKU, true>(s, d);
+    else if (variant == 3 || variant == 5) r = defgrad_variant<8, kFullKU, true>(s, d);
+    else r = defgrad_variant<4, kFullKU, true>(s, d);
   } else {
     switch (variant) {
-      case 1: defgrad_variant<4, 2>(s, d); break;
-      case 2: defgrad_variant<4, 1>(s, d); break;
-      case 3: defgrad_variant<8, 2>(s, d); break;
+      case 1: r = defgrad_variant<4, 2>(s, d); break;
+      case 2: r = defgrad_variant<4, 1>(s, d); break;
+      case 3: r = defgrad_variant<8, 2>(s, d); break;
       case 4: r = defgrad_bulk<4>(s, d); break;
       case 5: r = defgrad_bulk<8>(s, d); break;
-      case 6: defgrad_variant<16, 1>(s, d); break;
-      case 7: defgrad_variant<16, 2>(s, d); break;
-      default: defgrad_variant<4, 4>(s, d);
+      case 6: r = defgrad_variant<16, 1>(s, d); break;
+      case 7: r = defgrad_variant<16, 2>(s, d); break;
+      default: r = defgrad_variant<4, 4>(s, d);
     }
   }
   if (r) return r;
@@ -1598,34 +1625,34 @@ static int force_bulk(cudaStream_t s, bool mixed, const TiledForceArgs& a) {
   if (smem > (size_t)g_bulk_lim) return MEGA_ERR_UNSUPPORTED;
   const unsigned grid = (unsigned)a.ntiles;
   const int block = a.R * KG;
-  if (mixed) k_force_b<float, float, false, KG><<<grid, block, smem, s>>>(a);
-  else k_force_b<double, double, true, KG><<<grid, block, smem, s>>>(a);
-  return 0;
+  return launch_overlapped(mixed ? k_force_b<float, float, false, KG> : k_force_b<double, double, true, KG>, grid, block,
+                           smem, s, a);
 }
 
 template <int KG, int KU>
-static void force_variant(cudaStream_t s, bool mixed, const TiledForceArgs& a) {
+static int force_variant(cudaStream_t s, bool mixed, const TiledForceArgs& a) {
   const int nv = (a.ns_scol ? 28 : 9) + (a.has_body ? 3 : 0);
   const size_t smem = (mixed ? sizeof(float) : sizeof(double)) * nv * staged_ld(a.maxcnt);
   const unsigned grid = (unsigned)a.ntiles;
   const int block = a.R * KG;
-  if (mixed && a.ns_scol) k_force_t<float, float, false, KG, KU, true><<<grid, block, smem, s>>>(a);
-  else if (mixed) k_force_t<float, float, false, KG, KU><<<grid, block, smem, s>>>(a);
-  else k_force_t<double, double, true, KG, KU><<<grid, block, smem, s>>>(a);
+  auto k = !mixed       ? k_force_t<double, double, true, KG, KU>
+           : a.ns_scol ? k_force_t<float, float, false, KG, KU, true>
+                       : k_force_t<float, float, false, KG, KU>;
+  return launch_overlapped(k, grid, block, smem, s, a);
 }
 
 int launch_force_tiled(cudaStream_t s, bool mixed, const TiledForceArgs& a, int variant) {
   int r = 0;
   if (a.ns_scol && (!mixed || variant == 4 || variant == 5)) return MEGA_ERR_UNSUPPORTED;  // NSNI: register variants
   switch (variant) {
-    case 1: force_variant<4, 2>(s, mixed, a); break;
-    case 2: force_variant<4, 1>(s, mixed, a); break;
-    case 3: force_variant<8, 2>(s, mixed, a); break;
-    case 6: force_variant<16, 1>(s, mixed, a); break;
-    case 7: force_variant<16, 2>(s, mixed, a); break;
+    case 1: r = force_variant<4, 2>(s, mixed, a); break;
+    case 2: r = force_variant<4, 1>(s, mixed, a); break;
+    case 3: r = force_variant<8, 2>(s, mixed, a); break;
+    case 6: r = force_variant<16, 1>(s, mixed, a); break;
+    case 7: r = force_variant<16, 2>(s, mixed, a); break;
     case 4: r = force_bulk<4>(s, mixed, a); break;
     case 5: r = force_bulk<8>(s, mixed, a); break;
-    default: force_variant<4, 4>(s, mixed, a);
+    default: r = force_variant<4, 4>(s, mixed, a);
   }
   if (r) return r;
   MEGA_CHECK_LAUNCH();
