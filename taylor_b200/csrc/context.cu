@@ -444,13 +444,11 @@ struct Ctx {
   void* tmat = nullptr;
   int32_t* iters = nullptr;
   double* aux = nullptr;  // 4 per node, STATE(1, 2, 4, 5), when a damaged model is present
-  // NSNI (ITYPE_INT = 2): second derivatives per entry in CSR and CSC order,
-  // stress gradients (18 per node) and per-step scratch
+  // NSNI (ITYPE_INT = 2): per precision [FP64, mixed] the second derivatives S
+  // as planes in the row and column record layouts, the row sums of the float
+  // S, the stress gradients (18 per node) and per-step scratch
   bool nsni = false;
-  NsniS nsr{}, nsc{};
-  // mixed NSNI: S as six floats per record in the float row / column record
-  // orders, and its row sums (the tiled gathers carry the NSNI terms)
-  float *ns_srow = nullptr, *ns_scol = nullptr;
+  void *ns_srow[2] = {nullptr, nullptr}, *ns_scol[2] = {nullptr, nullptr};
   double* ns_ssum = nullptr;
   // semi-Lagrangian (LLAGRANGIAN = .FALSE.): lists and shapes rebuilt on the
   // current coordinates every step, in the caller's numbering, FP64
@@ -462,7 +460,7 @@ struct Ctx {
   double *sshp = nullptr, *sgx = nullptr, *sgy = nullptr, *sgz = nullptr, *ssd = nullptr;
   double *stgx = nullptr, *stgy = nullptr, *stgz = nullptr, *stshp = nullptr;
   double *coo_cur = nullptr, *zero3 = nullptr;
-  double *sgrad = nullptr, *hq = nullptr, *nsw = nullptr, *fstab = nullptr, *stress_prev = nullptr;
+  double *sgrad = nullptr, *hq = nullptr, *nsw = nullptr, *stress_prev = nullptr;
   StepAccum* acc = nullptr;
   unsigned* status = nullptr;
   bool phy_valid = true;
@@ -588,10 +586,10 @@ static TiledForceArgs force_args(Ctx* c, double dt, int mode, int predict) {
   f.tshp = mixed ? c->tshp32 : c->tshp; f.tmat = c->tmat; f.has_body = c->has_body; f.predict = predict;
   f.ebc = c->ebc; f.mass = c->mass; f.matidx = c->matidx; f.mats = c->mats; f.body_id = c->body_id;
   f.fint = c->fint; f.fext = c->fext; f.vel = c->vel; f.acl = c->acl; f.dsp = c->dsp; f.dsp_tot = c->dsp_tot;
-  f.prforce = c->prforce; f.fadd = (c->nsni && !mixed) ? c->fstab : nullptr; f.dt = dt; f.acc = c->acc;
+  f.prforce = c->prforce; f.dt = dt; f.acc = c->acc;
   f.status = c->status;
-  f.ns_scol = (c->nsni && mixed) ? c->ns_scol : nullptr;
-  f.ns_w = (c->nsni && mixed) ? (const float*)c->nsw : nullptr;
+  f.ns_scol = c->ns_scol[mixed];
+  f.ns_w = c->nsw;
   f.vel2 = c->vel2;
   f.ndt = c->ndt;
   return f;
@@ -627,10 +625,10 @@ static int sync_time(Ctx* c) {
   return 0;
 }
 
-// the NSNI terms of the mixed tiled row gather (null: none)
+// the NSNI terms of the tiled row gather (null: none)
 static const NsniTiles* nsni_tiles(Ctx* c, bool mixed, NsniTiles& buf) {
-  if (!c->nsni || !mixed) return nullptr;
-  buf.srow = c->ns_srow;
+  if (!c->nsni) return nullptr;
+  buf.srow = c->ns_srow[mixed];
   buf.ssum = c->ns_ssum;
   buf.hq = c->hq;
   return &buf;
@@ -640,7 +638,7 @@ static NsniStepArgs nsni_args(Ctx* c) {
   NsniStepArgs a{};
   a.n = c->n; a.fg = c->fg; a.stress_old = c->stress_prev; a.stress_new = c->stress; a.sml = c->sm_len;
   a.vol = c->vol; a.matidx = c->matidx; a.mats = c->mats; a.hq = c->hq; a.sgrad = c->sgrad; a.w = c->nsw;
-  a.fstab = c->fstab; a.finite_strain = c->p.finite_strain; a.inv3_exact = c->p.inv3_exact; a.acc = c->acc;
+  a.finite_strain = c->p.finite_strain; a.inv3_exact = c->p.inv3_exact; a.acc = c->acc;
   a.status = c->status;
   return a;
 }
@@ -652,10 +650,9 @@ static NsniStepArgs nsni_args(Ctx* c) {
 constexpr int kGraphSteps = 16;
 
 // kernels one step launches (the learned start splits the stress kernel in
-// two; NSNI adds the stress-gradient kernel, and in FP64 its two gathers)
+// two; NSNI adds the stress-gradient kernel)
 static int kernels_per_step(const Ctx* c, int mode = 0) {
-  const bool mixed = (mode & 0xff) == MEGA_MODE_MIXED;
-  return (c->nsni ? (mixed ? 4 : 6) : 3) + (c->has_ebc2 ? 1 : 0) +
+  return (c->nsni ? 4 : 3) + (c->has_ebc2 ? 1 : 0) +
          (((mode & MEGA_FLAG_LEARNED_GUESS) && c->mlp_on) ? 1 : 0);
 }
 
@@ -671,7 +668,6 @@ static int step_once(Ctx* c, double dt, int mode, int predict, cudaEvent_t* ev, 
                                c->shpb[mixed] ? c->shpb[mixed] : c->shp, c->dsp_tot_phy, c->fg, c->acc, c->status,
                                c->var_defgrad[mixed], full);
   if (r) return r;
-  if (c->nsni && !mixed && (r = nsni_step(c->s, nsni_args(c), c->csr, c->nsr, c->nsc, false, c->dsp, 0))) return r;
   if (ev) MEGA_TRY(cudaEventRecord(ev[1], c->s));
   StressArgs sa = stress_args(c, dt, mode);
   sa.add_g0 = !full;
@@ -679,8 +675,7 @@ static int step_once(Ctx* c, double dt, int mode, int predict, cudaEvent_t* ev, 
   sa.stress_prev = c->nsni ? c->stress_prev : nullptr;
   r = launch_stress(c->s, mixed, sa);
   if (r) return r;
-  if (c->nsni && (r = nsni_step(c->s, nsni_args(c), c->csr, c->nsr, c->nsc, mixed, c->dsp, 1))) return r;
-  if (c->nsni && !mixed && (r = nsni_step(c->s, nsni_args(c), c->csr, c->nsr, c->nsc, false, c->dsp, 2))) return r;
+  if (c->nsni && (r = nsni_step(c->s, nsni_args(c), c->csr, NsniS{}, NsniS{}, mixed, c->dsp, 1))) return r;
   if ((r = launch_fixity2(c, dt))) return r;
   if (ev) MEGA_TRY(cudaEventRecord(ev[2], c->s));
   r = launch_force_tiled(c->s, mixed, force_args(c, dt, mode, predict), c->var_force[mixed]);
@@ -1251,10 +1246,9 @@ int mega_gpu_init(const mega_params* p, int32_t n, const double* coo, const doub
   }
   c->nsni = p->itype_int == 2;
   if (c->nsni) {
-    CA(c->sgrad, 18 * (int64_t)n); CA(c->hq, 18 * (int64_t)n); CA(c->nsw, 18 * (int64_t)n);
-    CA(c->fstab, n3); CA(c->stress_prev, 6 * (int64_t)n);
+    CA(c->sgrad, 18 * (int64_t)n); CA(c->hq, 18 * fg_ld(n)); CA(c->nsw, 20 * (int64_t)n);
+    CA(c->stress_prev, 6 * (int64_t)n);
     cudaMemsetAsync(c->sgrad, 0, sizeof(double) * 18 * n, c->s);
-    cudaMemsetAsync(c->fstab, 0, sizeof(double) * n3, c->s);
   }
   {
     double* t = nullptr;
@@ -1438,7 +1432,7 @@ int mega_search_and_shapes(int64_t h, int32_t* gn, int32_t* gstart, int32_t* gst
     c->perm = c->iperm = nullptr;
     c->shp = c->sdphi = c->sdphi32 = c->tshp = c->tshp32 = c->shpb[0] = c->shpb[1] = nullptr;
     c->pk64 = c->tpk64 = c->pk32 = c->tpk32 = nullptr;
-    c->ns_srow = c->ns_scol = nullptr;
+    for (int k = 0; k < 2; ++k) c->ns_srow[k] = c->ns_scol[k] = nullptr;
     c->ns_ssum = nullptr;
     c->banked[0] = c->banked[1] = false;
     c->searched = false;
@@ -1551,11 +1545,9 @@ int mega_search_and_shapes(int64_t h, int32_t* gn, int32_t* gstart, int32_t* gst
   MEGA_CHECK_LAUNCH();
   r = scan_counts(c->s, len1, c->csr.rowptr, n, tmp1);
   if (r) return r;
+  NsniS nsr{};  // the second derivatives in list order
   if (c->nsni)
-    for (int k = 0; k < 6; ++k) {
-      MEGA_ALLOC(c->nbpool, c->nsr.v[k], m);
-      MEGA_ALLOC(c->nbpool, c->nsc.v[k], m);
-    }
+    for (int k = 0; k < 6; ++k) MEGA_ALLOC(tmp1, nsr.v[k], m);
   if (want) {
     k_permute_rows<<<grid_for((int64_t)n * 32, 256), 256, 0, c->s>>>(n, c->perm, c->iperm, csr0.rowptr, csr0.col,
                                                                       shp0, g0x, g0y, g0z, c->csr.rowptr, c->csr.col,
@@ -1565,7 +1557,7 @@ int mega_search_and_shapes(int64_t h, int32_t* gn, int32_t* gstart, int32_t* gst
       for (int k = 0; k < 6; k += 2)  // (the column indices are rewritten with the same values)
         k_permute_rows<<<grid_for((int64_t)n * 32, 256), 256, 0, c->s>>>(
             n, c->perm, c->iperm, csr0.rowptr, csr0.col, s0.v[k], s0.v[k + 1], s0.v[k], s0.v[k + 1], c->csr.rowptr,
-            c->csr.col, c->nsr.v[k], c->nsr.v[k + 1], c->nsr.v[k], c->nsr.v[k + 1]);
+            c->csr.col, nsr.v[k], nsr.v[k + 1], nsr.v[k], nsr.v[k + 1]);
       MEGA_CHECK_LAUNCH();
     }
   } else {
@@ -1588,7 +1580,7 @@ int mega_search_and_shapes(int64_t h, int32_t* gn, int32_t* gstart, int32_t* gst
     if (r) return r;
     tr.mark("rk_shapes");
     if (c->nsni) {
-      if ((r = second_derivatives(c->csr, c->nsr))) return r;
+      if ((r = second_derivatives(c->csr, nsr))) return r;
       tr.mark("nsni_second_derivatives");
     }
   }
@@ -1600,11 +1592,6 @@ int mega_search_and_shapes(int64_t h, int32_t* gn, int32_t* gstart, int32_t* gst
   if (r) return r;
   r = build_transpose(c->s, c->csr, c->nbpool);
   if (r) return r;
-  if (c->nsni) {
-    for (int k = 0; k < 6; ++k)
-      k_gather_pos<<<grid_for(m, 256), 256, 0, c->s>>>(m, c->csr.tpos, c->nsr.v[k], c->nsc.v[k]);
-    MEGA_CHECK_LAUNCH();
-  }
   tr.mark("transpose");
   if (!packed) {
     r = build_tiles(c->s, n, c->csr.rowptr, c->csr.col, m, c->csr.gmaxn, c->rt, c->nbpool, nullptr);
@@ -1651,15 +1638,22 @@ int mega_search_and_shapes(int64_t h, int32_t* gn, int32_t* gstart, int32_t* gst
     k_rowsum_pk32<<<grid_for(n, 256), 256, 0, c->s>>>(n, c->csr.rowptr, c->rt.rbase, (const float4*)c->pk32,
                                                        c->sdphi32);
     MEGA_CHECK_LAUNCH();
-    if (c->nsni) {  // S in both float record orders, and its row sums
-      MEGA_ALLOC(c->nbpool, c->ns_srow, 6 * m);
-      MEGA_ALLOC(c->nbpool, c->ns_scol, 6 * m);
+    if (c->nsni) {  // the row sums of the float S
       MEGA_ALLOC(c->nbpool, c->ns_ssum, 6 * (int64_t)n);
-      if ((r = nsni_records(c->s, m, nullptr, c->nsr, c->ns_srow)) ||
-          (r = nsni_records(c->s, m, c->csr.tpos, c->nsr, c->ns_scol)) ||
-          (r = nsni_rowsum(c->s, n, c->csr.rowptr, c->nsr, c->ns_ssum)))
-        return r;
+      if ((r = nsni_rowsum(c->s, n, c->csr.rowptr, nsr, c->ns_ssum))) return r;
     }
+  }
+  for (int mixed = 0; mixed < 2 && c->nsni; ++mixed) {  // S in both record layouts
+    if (!(c->prec_mask & (1 << mixed))) continue;
+    unsigned char *a = nullptr, *b = nullptr;
+    const int64_t w = mixed ? 24 : 48;
+    MEGA_ALLOC(c->nbpool, a, w * c->rt.nrec);
+    MEGA_ALLOC(c->nbpool, b, w * c->ct.nrec);
+    c->ns_srow[mixed] = a;
+    c->ns_scol[mixed] = b;
+    if ((r = pack_second(c->s, n, c->rt, c->csr.rowptr, nullptr, nsr, !mixed, a)) ||
+        (r = pack_second(c->s, n, c->ct, c->csr.colptr, c->csr.tpos, nsr, !mixed, b)))
+      return r;
   }
   if (c->has_body && (c->prec_mask & 1)) {
     MEGA_ALLOC(c->nbpool, c->tshp, m);
@@ -1672,19 +1666,21 @@ int mega_search_and_shapes(int64_t h, int32_t* gn, int32_t* gstart, int32_t* gst
     MEGA_CHECK_LAUNCH();
   }
   MEGA_TRY(cudaStreamSynchronize(c->s));
-  // the per-step kernels read neither the transposed row ids (but NSNI's
-  // column gather) nor the positions
-  if (!c->nsni) {
-    c->nbpool.release(c->csr.trow);
-    c->csr.trow = nullptr;
-  }
+  // the per-step kernels read neither the transposed row ids nor the positions
+  c->nbpool.release(c->csr.trow);
+  c->csr.trow = nullptr;
   c->nbpool.release(c->csr.tpos);
   c->csr.tpos = nullptr;
   tmp1.free_all();
   tr.mark("pack_and_release");
-  // the mixed NSNI force gather stages 27 values a node: its measured best is
-  // 8 lanes per column (variant 3); mega_autotune may pick another
-  if (c->nsni) c->var_force[1] = 3;
+  // NSNI's own starts (mega_autotune may pick others): the mixed force gather
+  // stages 27 values a node and wants 8 lanes per column; the FP64 row gather
+  // carries 18 double sums a lane and spills with 4 records in flight (130 k
+  // nodes: 213 us, 158 with 2)
+  if (c->nsni) {
+    c->var_force[1] = 3;
+    c->var_defgrad[0] = 1;
+  }
   c->searched = true;
   if (nnz) *nnz = m;
   if (gmaxn) *gmaxn = c->csr.gmaxn;
@@ -1995,7 +1991,7 @@ static int bank_layout(Ctx* c, bool mixed) {
   if (c->banked[mixed] || !pk || !tpk) return 0;
   const int64_t m = c->csr.nnz, rec = mixed ? 16 : 26;
   const int32_t n = c->n;
-  const bool ns = mixed && c->ns_scol;
+  const bool ns = c->ns_scol[mixed];
   DevPool tmp(c->s);
   uint16_t* l = nullptr;
   int64_t* pos = nullptr;
@@ -2005,7 +2001,7 @@ static int bank_layout(Ctx* c, bool mixed) {
   // columns (the lanes per column of the force variant the context favours)
   MEGA_TRY(cudaMemcpyAsync(l, c->ct.lidx, sizeof(uint16_t) * m, cudaMemcpyDeviceToDevice, c->s));
   if ((r = iota64(c->s, m, pos)) ||
-      (r = bank_order(c->s, n, c->ct, c->csr.colptr, l, nullptr, pos, ns ? 8 : 4)))
+      (r = bank_order(c->s, n, c->ct, c->csr.colptr, l, nullptr, pos, ns && mixed ? 8 : 4)))
     return r;
   unsigned char* tp = nullptr;
   MEGA_ALLOC(c->nbpool, tp, rec * c->ct.nrec);
@@ -2016,10 +2012,10 @@ static int bank_layout(Ctx* c, bool mixed) {
     k_gather_pos<<<grid_for(m, 256), 256, 0, c->s>>>(m, pos, tshp, ts);
     MEGA_CHECK_LAUNCH();
   }
-  float* sc = nullptr;
+  unsigned char* sc = nullptr;
   if (ns) {
-    MEGA_ALLOC(c->nbpool, sc, 6 * m);
-    if ((r = gather_f6(c->s, m, pos, c->ns_scol, sc))) return r;
+    MEGA_ALLOC(c->nbpool, sc, (mixed ? 24 : 48) * c->ct.nrec);
+    if ((r = gather_second(c->s, n, c->ct, c->csr.colptr, pos, !mixed, c->ns_scol[mixed], sc))) return r;
   }
   // rows
   MEGA_TRY(cudaMemcpyAsync(l, c->rt.lidx, sizeof(uint16_t) * m, cudaMemcpyDeviceToDevice, c->s));
@@ -2033,19 +2029,19 @@ static int bank_layout(Ctx* c, bool mixed) {
   if ((r = gather_records(c->s, n, c->rt, c->csr.rowptr, pos, !mixed, pk, rp))) return r;
   k_gather_pos<<<grid_for(m, 256), 256, 0, c->s>>>(m, pos, c->shp, sh);
   MEGA_CHECK_LAUNCH();
-  float* sr = nullptr;
+  unsigned char* sr = nullptr;
   if (ns) {
-    MEGA_ALLOC(c->nbpool, sr, 6 * m);
-    if ((r = gather_f6(c->s, m, pos, c->ns_srow, sr))) return r;
+    MEGA_ALLOC(c->nbpool, sr, (mixed ? 24 : 48) * c->rt.nrec);
+    if ((r = gather_second(c->s, n, c->rt, c->csr.rowptr, pos, !mixed, c->ns_srow[mixed], sr))) return r;
   }
   MEGA_TRY(cudaStreamSynchronize(c->s));
   drop_graph(c);  // captured steps hold the old arrays
   c->nbpool.release(tpk); tpk = tp;
   if (ts) { c->nbpool.release(tshp); tshp = ts; }
-  if (sc) { c->nbpool.release(c->ns_scol); c->ns_scol = sc; }
+  if (sc) { c->nbpool.release(c->ns_scol[mixed]); c->ns_scol[mixed] = sc; }
   c->nbpool.release(pk); pk = rp;
   c->shpb[mixed] = sh;
-  if (sr) { c->nbpool.release(c->ns_srow); c->ns_srow = sr; }
+  if (sr) { c->nbpool.release(c->ns_srow[mixed]); c->ns_srow[mixed] = sr; }
   c->banked[mixed] = true;
   return 0;
 }
@@ -2675,8 +2671,8 @@ static int construct_fint_impl(const mega_params* p, const FintIO& io) {
   double *sgrad = nullptr, *hq = nullptr, *nsw = nullptr, *fstab = nullptr, *sprev = nullptr;
   if (nsni) {
     for (int k = 0; k < 6; ++k) { MEGA_ALLOC(pool, nsr.v[k], m); MEGA_ALLOC(pool, nsc.v[k], m); }
-    MEGA_ALLOC(pool, sgrad, 18 * (int64_t)n); MEGA_ALLOC(pool, hq, 18 * (int64_t)n);
-    MEGA_ALLOC(pool, nsw, 18 * (int64_t)n); MEGA_ALLOC(pool, fstab, n3); MEGA_ALLOC(pool, sprev, 6 * (int64_t)n);
+    MEGA_ALLOC(pool, sgrad, 18 * (int64_t)n); MEGA_ALLOC(pool, hq, 18 * fg_ld(n));
+    MEGA_ALLOC(pool, nsw, 20 * (int64_t)n); MEGA_ALLOC(pool, fstab, n3); MEGA_ALLOC(pool, sprev, 6 * (int64_t)n);
     if (io.linit) {
       DevPool faces(s);
       double* g[6];

@@ -324,9 +324,9 @@ struct NsniStepArgs {
   const double* vol;
   const uint16_t* matidx;
   const MatEntry* mats;
-  double* hq;                // 18 per node: sum_J S_q du_J,k
+  double* hq;                // 18 planes of fg_ld(n): sum_J S_q du_J,k
   double* sgrad;             // 18 per node: sigma_,x, sigma_,y, sigma_,z (Voigt)
-  void* w;                   // 18 per node: force weights on the six S components (double, or float when mixed)
+  void* w;                   // 20 per node (18 used): force weights on the six S components (double, float when mixed)
   double* fstab;             // 3 per node: the stabilisation force
   int finite_strain;
   int inv3_exact;
@@ -338,12 +338,10 @@ int nsni_combine(cudaStream_t s, int32_t n, int axis, const int64_t* rowptr, con
 // stage 0: the row gather of H (after the displacement increment is known);
 // stage 1: stress gradients and weights (mixed: float weights);
 // stage 2: the column gather of the stabilisation force.
-// Stages 0 and 2 are the FP64 steps' own kernels: the mixed steps form H and
-// the stabilisation force in the tiled gathers (NsniTiles).
+// Stages 0 and 2 are the drop-in's: resident steps form H and the
+// stabilisation force in the tiled gathers (NsniTiles).
 int nsni_step(cudaStream_t s, const NsniStepArgs& a, const DevCSR& csr, const NsniS& rows, const NsniS& cols,
               bool mixed, const double* du, int stage);
-// dst[6 e + q] = float S_q at list position pos[e] (e when pos is null)
-int nsni_records(cudaStream_t s, int64_t m, const int64_t* pos, const NsniS& src, float* dst);
 // dst[6 i + q] = sum over row i of the float-rounded S_q, in double
 int nsni_rowsum(cudaStream_t s, int32_t n, const int64_t* rowptr, const NsniS& src, double* dst);
 

@@ -13,8 +13,8 @@
 //            mixed mode)
 //            k_nsni_h      (row gather) the gradients of the incremental
 //            displacement gradient, H_a(k,m) = sum_J S_(m a)(J) du_J,k
-//            (XLMAT/YLMAT/ZLMAT, FINT.F90:728-737); the mixed steps form H
-//            in the tiled row gather instead (tiled.cu, NS);
+//            (XLMAT/YLMAT/ZLMAT, FINT.F90:728-737); resident steps form H in
+//            the tiled row gather instead (tiled.cu, NS);
 //            k_nsni_stress (node) the strain-gradient increments of
 //            D_HUGHES_WINGET (HUGHES_WINGET.F90:84-165), stress gradients
 //            sigma_,a rotated with the step's rotation and advanced with an
@@ -24,8 +24,8 @@
 //            W_a = M_a / V * V J sigma_,a INV3(F)^T with the second moments
 //            M_a / V = (cell width_a)^2 / 12 (PRE_MODEL_SECOND_MOMENT.F90);
 //            k_nsni_force  (column gather) f_J += sum_a W_a S_(. a)(J)
-//            (FINT.F90:1127-1208), added by the force kernel before the
-//            corrector; the mixed steps sum it in the tiled column gather.
+//            (FINT.F90:1127-1208), added by the force kernel; resident steps
+//            sum it in the tiled column gather.
 #include "mega_internal.cuh"
 
 namespace mega {
@@ -33,10 +33,9 @@ namespace {
 
 constexpr int kNL = 8;  // lanes per node of the two gathers
 
-// node stride of the force weights W: 18 doubles (144 B, nine 16-byte
-// loads) or 18 floats padded to 20 (80 B, five 16-byte loads)
-template <typename V>
-constexpr int w_stride() { return sizeof(V) == 4 ? 20 : 18; }
+// node stride of the force weights W: 18 values padded to 20 (80 or 160 bytes,
+// a multiple of 16 and of a sector in double)
+constexpr int kW = 20;
 
 // index of S_(m a) in the XX, YY, ZZ, XY, YZ, XZ order
 __device__ __forceinline__ int dd_index(int m, int a) {
@@ -75,7 +74,7 @@ __global__ void k_nsni_combine(int32_t n, int a, const int64_t* __restrict__ row
   }
 }
 
-// hq[18 i + 6 k + q] = sum_J S_q(J) du_J,k (S double or float, sums in double)
+// hq[(6 k + q) ld + i] = sum_J S_q(J) du_J,k (S double or float, sums in double)
 template <typename SV>
 __global__ void __launch_bounds__(256) k_nsni_h(int32_t n, const int64_t* __restrict__ rowptr,
                                                 const int32_t* __restrict__ col, NsniArr<SV> s, const double* du,
@@ -118,7 +117,7 @@ __global__ void __launch_bounds__(256) k_nsni_h(int32_t n, const int64_t* __rest
     for (int k = 0; k < 18; ++k) h[k] += __shfl_xor_sync(gm, h[k], o);
   if (q == 0)
 #pragma unroll
-    for (int k = 0; k < 18; ++k) hq[18 * i + k] = h[k];
+    for (int k = 0; k < 18; ++k) hq[k * fg_ld(n) + i] = h[k];
 }
 
 // D_HUGHES_WINGET (HUGHES_WINGET.F90:84-165): DG = DL A^-1 - L A^-1 (DL/2)
@@ -209,8 +208,9 @@ __global__ void __launch_bounds__(128) k_nsni_stress(NsniStepArgs a) {
     }
     const double lam_s = ks - 2.0 * gs / 3.0, l2m_s = ks + 4.0 * gs / 3.0;
     const double vol = a.vol[i];
-    const double* hq = a.hq + 18 * i;
-    double* sg = a.sgrad + 18 * i;
+    const double* hq = a.hq + i;
+    const int64_t ld = fg_ld(a.n);
+    double2* sg2 = reinterpret_cast<double2*>(a.sgrad + 18 * i);
     double Wm[3][3][3];  // [a][k][m]
     unsigned st = 0;
 #pragma unroll
@@ -221,10 +221,14 @@ __global__ void __launch_bounds__(128) k_nsni_stress(NsniStepArgs a) {
 #pragma unroll
       for (int k = 0; k < 3; ++k)
 #pragma unroll
-        for (int m = 0; m < 3; ++m) Ha[k][m] = hq[6 * k + dd_index(m, ax)];
+        for (int m = 0; m < 3; ++m) Ha[k][m] = hq[(6 * k + dd_index(m, ax)) * ld];
       double de[6], sa[6];
 #pragma unroll
-      for (int k = 0; k < 6; ++k) sa[k] = sg[6 * ax + k];
+      for (int k = 0; k < 3; ++k) {
+        const double2 v = sg2[3 * ax + k];
+        sa[2 * k] = v.x;
+        sa[2 * k + 1] = v.y;
+      }
       if (a.finite_strain) {
         double La[3][3];
         mm3(Ha, IF, La);
@@ -245,9 +249,10 @@ __global__ void __launch_bounds__(128) k_nsni_stress(NsniStepArgs a) {
       for (int k = 0; k < 6; ++k) {
         sa[k] += ds[k];
         work += 0.5 * fac * de[k] * (2.0 * sa[k] - ds[k]) * vol * det;
-        sg[6 * ax + k] = sa[k];
         if (!isfinite(sa[k])) st |= MEGA_ST_NONFINITE;
       }
+#pragma unroll
+      for (int k = 0; k < 3; ++k) sg2[3 * ax + k] = make_double2(sa[2 * k], sa[2 * k + 1]);
       double S[3][3];
       v2t(sa, S);
 #pragma unroll
@@ -257,7 +262,7 @@ __global__ void __launch_bounds__(128) k_nsni_stress(NsniStepArgs a) {
           Wm[ax][k][m] = fac * vol * det * (S[k][0] * IF[m][0] + S[k][1] * IF[m][1] + S[k][2] * IF[m][2]);
     }
     // the weights folded onto the six symmetric second derivatives
-    WV* w = reinterpret_cast<WV*>(a.w) + w_stride<WV>() * i;
+    WV w[kW] = {};
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       w[6 * k + 0] = (WV)Wm[0][k][0];
@@ -266,6 +271,16 @@ __global__ void __launch_bounds__(128) k_nsni_stress(NsniStepArgs a) {
       w[6 * k + 3] = (WV)(Wm[1][k][0] + Wm[0][k][1]);  // XY
       w[6 * k + 4] = (WV)(Wm[2][k][1] + Wm[1][k][2]);  // YZ
       w[6 * k + 5] = (WV)(Wm[2][k][0] + Wm[0][k][2]);  // XZ
+    }
+    if constexpr (sizeof(WV) == 4) {
+      float4* o = reinterpret_cast<float4*>(a.w) + 5 * i;
+#pragma unroll
+      for (int k = 0; k < 5; ++k)
+        o[k] = make_float4((float)w[4 * k], (float)w[4 * k + 1], (float)w[4 * k + 2], (float)w[4 * k + 3]);
+    } else {
+      double2* o = reinterpret_cast<double2*>(a.w) + 10 * i;
+#pragma unroll
+      for (int k = 0; k < 9; ++k) o[k] = make_double2((double)w[2 * k], (double)w[2 * k + 1]);
     }
     if (st) atomicOr(a.status, st);
   }
@@ -294,14 +309,14 @@ __global__ void __launch_bounds__(256) k_nsni_force(int32_t n, const int64_t* __
   // the row's 18 weights as 16-byte loads
   auto load_w = [&](int64_t e, V* wi) {
     if constexpr (sizeof(V) == 4) {
-      const float4* src = reinterpret_cast<const float4*>(w + 20 * (int64_t)trow[e]);
+      const float4* src = reinterpret_cast<const float4*>(w + kW * (int64_t)trow[e]);
 #pragma unroll
       for (int k = 0; k < 5; ++k) {
         const float4 x = src[k];
         wi[4 * k] = x.x; wi[4 * k + 1] = x.y; wi[4 * k + 2] = x.z; wi[4 * k + 3] = x.w;
       }
     } else {
-      const double2* src = reinterpret_cast<const double2*>(w + 18 * (int64_t)trow[e]);
+      const double2* src = reinterpret_cast<const double2*>(w + kW * (int64_t)trow[e]);
 #pragma unroll
       for (int k = 0; k < 9; ++k) {
         const double2 x = src[k];
@@ -322,14 +337,14 @@ __global__ void __launch_bounds__(256) k_nsni_force(int32_t n, const int64_t* __
   int64_t e = colptr[J] + q;
   const int64_t ee = colptr[J + 1];
   for (; e + kNL < ee; e += 2 * kNL) {
-    V wa[w_stride<V>()], wb[w_stride<V>()];
+    V wa[kW], wb[kW];
     load_w(e, wa);
     load_w(e + kNL, wb);
     add(e, wa);
     add(e + kNL, wb);
   }
   if (e < ee) {
-    V wa[w_stride<V>()];
+    V wa[kW];
     load_w(e, wa);
     add(e, wa);
   }
@@ -344,21 +359,6 @@ __global__ void __launch_bounds__(256) k_nsni_force(int32_t n, const int64_t* __
     fstab[3 * J + 1] = (double)f1;
     fstab[3 * J + 2] = (double)f2;
   }
-}
-
-// dst[6 e + q] = float S_q at list position pos[e] (the record order of the
-// tiled gathers; list order without pos)
-__global__ void k_nsni_records(int64_t m, const int64_t* __restrict__ pos, NsniS src, float* __restrict__ dst) {
-  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (e >= m) return;
-  const int64_t p = pos ? pos[e] : e;
-  float v[6];
-#pragma unroll
-  for (int c = 0; c < 6; ++c) v[c] = (float)src.v[c][p];
-  float2* o = reinterpret_cast<float2*>(dst + 6 * e);
-  o[0] = make_float2(v[0], v[1]);
-  o[1] = make_float2(v[2], v[3]);
-  o[2] = make_float2(v[4], v[5]);
 }
 
 // dst[6 i + q] = sum over row i of the float-rounded S_q, in double (so that
@@ -393,13 +393,6 @@ int nsni_step(cudaStream_t s, const NsniStepArgs& a, const DevCSR& csr, const Ns
   if (stage == 1) return launch_overlapped(mixed ? k_nsni_stress<float> : k_nsni_stress<double>, gn, 128, 0, s, a);
   return launch_overlapped(k_nsni_force<double>, gg, 256, 0, s, a.n, csr.colptr, csr.trow, cols, (const double*)a.w,
                            a.fstab);
-}
-
-int nsni_records(cudaStream_t s, int64_t m, const int64_t* pos, const NsniS& src, float* dst) {
-  if (m <= 0) return 0;
-  k_nsni_records<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(m, pos, src, dst);
-  MEGA_CHECK_LAUNCH();
-  return 0;
 }
 
 int nsni_rowsum(cudaStream_t s, int32_t n, const int64_t* rowptr, const NsniS& src, double* dst) {

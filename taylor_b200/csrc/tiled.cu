@@ -384,13 +384,51 @@ __global__ void k_gather_rec64(int32_t n, int32_t R, int64_t slots, SliceView v,
   });
 }
 
-// out[6 e + k] = in[6 pos[e] + k]
-__global__ void k_gather_f6(int64_t m, const int64_t* __restrict__ pos, const float2* __restrict__ in,
-                            float2* __restrict__ out) {
-  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (e >= m) return;
-  const int64_t p = pos[e];
-  out[3 * e] = in[3 * p]; out[3 * e + 1] = in[3 * p + 1]; out[3 * e + 2] = in[3 * p + 2];
+// NSNI's second derivatives in the records' layout (planes of nrec values)
+template <bool F64>
+__device__ __forceinline__ void put_second(void* out, int64_t nrec, int64_t rec, const double v[6]) {
+  if constexpr (F64) {
+    double2* o = (double2*)out;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) o[c * nrec + rec] = make_double2(v[2 * c], v[2 * c + 1]);
+  } else {
+    ((float4*)out)[rec] = make_float4((float)v[0], (float)v[1], (float)v[2], (float)v[3]);
+    ((float2*)((float4*)out + nrec))[rec] = make_float2((float)v[4], (float)v[5]);
+  }
+}
+
+template <bool F64>
+__global__ void k_pack_second(int32_t n, int32_t R, int64_t slots, SliceView v, const int64_t* __restrict__ ptr,
+                              const int64_t* __restrict__ pos, NsniS src, void* __restrict__ out) {
+  for_slot_records(n, R, slots, v, ptr, [&](int64_t rec, int64_t p, int64_t) {
+    double x[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    if (p >= 0) {
+      const int64_t g = pos ? pos[p] : p;
+#pragma unroll
+      for (int c = 0; c < 6; ++c) x[c] = src.v[c][g];
+    }
+    put_second<F64>(out, v.nrec, rec, x);
+  });
+}
+
+template <bool F64>
+__global__ void k_gather_second(int32_t n, int32_t R, int64_t slots, SliceView v, const int64_t* __restrict__ ptr,
+                                const int64_t* __restrict__ pos, const void* __restrict__ in,
+                                void* __restrict__ out) {
+  for_slot_records(n, R, slots, v, ptr, [&](int64_t rec, int64_t p, int64_t first) {
+    int64_t from = rec;
+    if (p >= 0) {
+      const int64_t k = p - first;
+      from = rec_of(rec - 32 * (k >> 2) - (k & 3), pos[p] - first);
+    }
+    if constexpr (F64) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) ((double2*)out)[c * v.nrec + rec] = ((const double2*)in)[c * v.nrec + from];
+    } else {
+      ((float4*)out)[rec] = ((const float4*)in)[from];
+      ((float2*)((float4*)out + v.nrec))[rec] = ((const float2*)((const float4*)in + v.nrec))[from];
+    }
+  });
 }
 
 __global__ void k_iota64(int64_t m, int64_t* __restrict__ out) {
@@ -498,15 +536,42 @@ struct RowWalk {
   __device__ __forceinline__ int64_t at(int k) const { return rec + (int64_t)(8 * KG) * k; }
 };
 
-// The six float S values of one NSNI record (three 8-byte loads).
-struct SRec {
-  float2 a, b, c;
+// The six S values of one NSNI record.
+template <bool F64>
+struct SRec;
+template <>
+struct SRec<false> {
+  float4 a;
+  float2 b;
+  __device__ __forceinline__ void load(const void* base, int64_t nrec, int64_t rec) {
+    asm("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w)
+        : "l"((const float4*)base + rec));
+    asm("ld.global.nc.L1::no_allocate.v2.f32 {%0, %1}, [%2];"
+        : "=f"(b.x), "=f"(b.y)
+        : "l"((const float2*)((const float4*)base + nrec) + rec));
+  }
+  template <typename A>
+  __device__ __forceinline__ void get(A s[6]) const {
+    s[0] = (A)a.x; s[1] = (A)a.y; s[2] = (A)a.z; s[3] = (A)a.w; s[4] = (A)b.x; s[5] = (A)b.y;
+  }
 };
-__device__ __forceinline__ SRec load_srec(const float* base, int64_t p, int64_t pend) {
-  if (p >= pend) return SRec{};  // a pad
-  const float2* sp = reinterpret_cast<const float2*>(base) + 3 * p;
-  return SRec{__ldg(sp), __ldg(sp + 1), __ldg(sp + 2)};
-}
+template <>
+struct SRec<true> {
+  double2 a[3];
+  __device__ __forceinline__ void load(const void* base, int64_t nrec, int64_t rec) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+      asm("ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];"
+          : "=d"(a[c].x), "=d"(a[c].y)
+          : "l"((const double2*)base + c * nrec + rec));
+  }
+  template <typename A>
+  __device__ __forceinline__ void get(A s[6]) const {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) { s[2 * c] = (A)a[c].x; s[2 * c + 1] = (A)a[c].y; }
+  }
+};
 
 // the staged displacement values of a rank: three doubles, or three floats and a pad
 template <bool F64>
@@ -569,8 +634,8 @@ __device__ __forceinline__ void stage_disp(const StageIds<KG>& ids, int cnt, con
 // the increments alone, half the shared-memory traffic and sums: at 130 k nodes
 // FP64 ran at 75 % of the L1 data pipe with both, half of it staged reads.
 // NS: the NSNI gradients of the incremental displacement gradient ride
-// along, H_i(k, q) = sum_J S_q(i, J) du_J,k, formed like L as
-// sum_J S_q (du_J - du_i) + du_i,k sum_J S_q (FINT.F90:728-737 layout).
+// along, H_i(k, q) = sum_J S_q(i, J) du_J,k, in mixed precision formed like L
+// as sum_J S_q (du_J - du_i) + du_i,k sum_J S_q (FINT.F90:728-737 layout).
 template <bool F64, int KG, bool NS, bool FULL>
 constexpr int defgrad_blocks() {  // blocks per SM the register cap asks for
   const int w = NS ? 8 : (F64 && FULL ? 12 : 16);
@@ -607,20 +672,19 @@ __global__ void __launch_bounds__(64 * KG, defgrad_blocks<F64, KG, NS, FULL>())
   const RowWalk<KG> walk(sv, r0, slot, q);
   const int nit = valid ? walk.nit : 0;
   constexpr bool kPipe = !NS && (!F64 || KU <= 2);
-  constexpr bool kList = INTERP || NS;  // values that stay in list order ride along
-  int64_t p0 = 0, pend = 0;
-  if (kList && valid) {
+  int64_t p0 = 0, pend = 0;  // list positions, for the shape values
+  if (INTERP && valid) {
     p0 = rowptr[i] + q;
     pend = rowptr[i + 1];
   }
   Rec<F64> cur[KU];
-  SRec csr[NS ? KU : 1];
+  SRec<F64> csr[NS ? KU : 1];
   bool have = nit >= KU;
   if (have) {
 #pragma unroll
     for (int u = 0; u < KU; ++u) {
       load_rec(pk, sv.nrec, walk.at(u), cur[u]);
-      if constexpr (NS) csr[u] = load_srec(ns.srow, p0 + u * KG, pend);
+      if constexpr (NS) csr[u].load(ns.srow, sv.nrec, walk.at(u));
     }
   }
   grid_wait();
@@ -662,7 +726,7 @@ __global__ void __launch_bounds__(64 * KG, defgrad_blocks<F64, KG, NS, FULL>())
     double ph[3] = {0.0, 0.0, 0.0};
     // One entry: F += (u_J - u_i) (x) g, L += (d_J - d_i) (x) g (+ phi d_J),
     // H(k, q) += S_q (d_J - d_i)_k.
-    auto body = [&](int it, const Rec<F64>& rec, const SRec& sr) {
+    auto body = [&](int it, const Rec<F64>& rec, const SRec<F64>& sr) {
       const A g[3] = {(A)rec.x(), (A)rec.y(), (A)rec.z()};
       const int l = rec.l();
       SV v[SN];
@@ -684,9 +748,11 @@ __global__ void __launch_bounds__(64 * KG, defgrad_blocks<F64, KG, NS, FULL>())
         L[3 * k] += d[k] * g[0]; L[3 * k + 1] += d[k] * g[1]; L[3 * k + 2] += d[k] * g[2];
       }
       if constexpr (NS) {
-        const double sq[6] = {(double)sr.a.x, (double)sr.a.y, (double)sr.b.x, (double)sr.b.y, (double)sr.c.x,
-                              (double)sr.c.y};
-        const double e0 = (double)d[0], e1 = (double)d[1], e2 = (double)d[2];
+  double sq[6];
+  sr.get(sq);
+  // FP64: du_J itself
+  const double e0 = F64 ? (double)v[0] : (double)d[0], e1 = F64 ? (double)v[1] : (double)d[1],
+               e2 = F64 ? (double)v[2] : (double)d[2];
 #pragma unroll
         for (int c = 0; c < 6; ++c) { H[c] += sq[c] * e0; H[6 + c] += sq[c] * e1; H[12 + c] += sq[c] * e2; }
       }
@@ -702,8 +768,7 @@ __global__ void __launch_bounds__(64 * KG, defgrad_blocks<F64, KG, NS, FULL>())
     // Each lane sums its entries in list order.  Where the registers allow
     // (kPipe) the next KU records are requested before this KU's sums, so a
     // lane keeps loads in flight while it computes.
-    const SRec s0{};
-    int it = 0;
+      int it = 0;
     while (have) {
       const bool hn = it + 2 * KU <= nit;
       Rec<F64> nxt[KU];
@@ -715,14 +780,14 @@ __global__ void __launch_bounds__(64 * KG, defgrad_blocks<F64, KG, NS, FULL>())
         }
       }
 #pragma unroll
-      for (int u = 0; u < KU; ++u) body(it + u, cur[u], NS ? csr[NS ? u : 0] : s0);
+      for (int u = 0; u < KU; ++u) body(it + u, cur[u], csr[NS ? u : 0]);
 #pragma unroll
       for (int u = 0; u < KU; ++u) {
         if constexpr (kPipe) {
           cur[u] = nxt[u];
         } else if (hn) {
           load_rec(pk, sv.nrec, walk.at(it + KU + u), cur[u]);
-          if constexpr (NS) csr[u] = load_srec(ns.srow, p0 + (int64_t)KG * (it + KU + u), pend);
+          if constexpr (NS) csr[u].load(ns.srow, sv.nrec, walk.at(it + KU + u));
         }
       }
       it += KU;
@@ -731,7 +796,9 @@ __global__ void __launch_bounds__(64 * KG, defgrad_blocks<F64, KG, NS, FULL>())
     for (; it < nit; ++it) {
       Rec<F64> rec;
       load_rec(pk, sv.nrec, walk.at(it), rec);
-      body(it, rec, NS ? load_srec(ns.srow, p0 + (int64_t)KG * it, pend) : s0);
+      SRec<F64> sr;
+    if constexpr (NS) sr.load(ns.srow, sv.nrec, walk.at(it));
+    body(it, rec, sr);
     }
 #pragma unroll
     for (int o = 1; o < KG; o <<= 1) {
@@ -751,13 +818,14 @@ __global__ void __launch_bounds__(64 * KG, defgrad_blocks<F64, KG, NS, FULL>())
     }
     if (q == 0) {
       if constexpr (NS) {
-        double ss[6];
+        double ss[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        if (!F64)
 #pragma unroll
-        for (int c = 0; c < 6; ++c) ss[c] = ns.ssum[6 * i + c];
+          for (int c = 0; c < 6; ++c) ss[c] = ns.ssum[6 * i + c];
 #pragma unroll
         for (int k = 0; k < 3; ++k)
 #pragma unroll
-          for (int c = 0; c < 6; ++c) ns.hq[18 * i + 6 * k + c] = H[6 * k + c] + di[k] * ss[c];
+          for (int c = 0; c < 6; ++c) ns.hq[(6 * k + c) * fg_ld(n) + i] = F64 ? H[6 * k + c] : H[6 * k + c] + di[k] * ss[c];
       }
       const double sd3[3] = {sdphi[3 * i], sdphi[3 * i + 1], sdphi[3 * i + 2]};
       const int64_t ld = fg_ld(n);
@@ -785,7 +853,6 @@ __device__ __forceinline__ void correct_dof(const TiledForceArgs& a, int64_t J, 
                                             double& ke, double& ee, double& pr, int& body, unsigned& st) {
   const int64_t m = 3 * J + q;
   const double dt = a.ndt ? a.ndt[J] : a.dt;
-  if (a.fadd) fi += a.fadd[m];
   if (!isfinite(fi)) st |= MEGA_ST_NONFINITE;
   const double mass = a.mass[m];
   const double fe_old = a.fext[m], d_old = a.dsp[m];
@@ -884,19 +951,36 @@ __device__ __forceinline__ void finish_columns(const TiledForceArgs& a, int64_t 
   if (st) atomicOr(a.status, st);
 }
 
-// The staged values of a column tile: T_i (9), the body force vectors (3, as
-// arrays) and, NS, T_i and W_i together (27 and a pad: 7 vectors, T_i's first
-// two, then T_i's last beside W_i's last two, then W_i's first 16).
+// The staged values of a column tile: T_i (9), NS: with W_i (18), and the body
+// force vectors (3, as arrays).  Mixed NS: 27 values and a pad in 7 vectors,
+// T_i's first two, then T_i's last beside W_i's last two, then W_i's first
+// 16.  FP64 NS: T_i then W_i, 27 values, 216 bytes a rank, so that 1,024 ranks
+// fit; its body force is read through the node ids, which are staged instead.
 template <typename TS, bool NS>
 struct StagedT {
-  Staged<TS, NS ? 28 : 9> t;
+  static constexpr int N = NS ? (sizeof(TS) == 4 ? 28 : 27) : 9;
+  static constexpr bool kIds = NS && sizeof(TS) == 8;
+  Staged<TS, N> t;
   TS* body;
   int ld;
+  static size_t bytes(int maxcnt, bool has_body) {
+    return (size_t)staged_ld(maxcnt) * (N * sizeof(TS) + (has_body ? (kIds ? 4 : 3 * sizeof(TS)) : 0));
+  }
   __device__ __forceinline__ StagedT(void* base, int cnt)
       : t{reinterpret_cast<TS*>(base), staged_ld(cnt)}, body(t.end()), ld(t.ld) {}
-  // A thread per staged node.  FP64: the 96-byte row as three 32-byte loads,
-  // a sector each (as six 16-byte loads every line was fetched twice once the
-  // blocks' shared memory had shrunk L1).
+  // the body force vector of rank l
+  __device__ __forceinline__ void body_of(const TiledForceArgs& a, int l, double b[3]) const {
+    if constexpr (kIds) {
+      const double* p = reinterpret_cast<const double*>(a.tmat) + 12 * (int64_t)reinterpret_cast<const int32_t*>(body)[l];
+      b[0] = p[9]; b[1] = p[10]; b[2] = p[11];
+    } else {
+      b[0] = (double)body[l]; b[1] = (double)body[ld + l]; b[2] = (double)body[2 * ld + l];
+    }
+  }
+  // W_l(k, q) at 6 k + q
+  __device__ __forceinline__ static TS weight(const TS* v, int j) {
+    return sizeof(TS) == 8 ? v[9 + j] : (j < 16 ? v[12 + j] : v[j - 7]);
+  }
   template <int KG>
   __device__ __forceinline__ void fill(const TiledForceArgs& a, const StageIds<KG>& ids, int cnt) const {
     ids.each(cnt, [&](int l, int64_t j) {
@@ -927,8 +1011,20 @@ struct StagedT {
         t.put(l, 1, make_double2(x[2], x[3]));
         t.put(l, 2, make_double2(y[0], y[1]));
         t.put(l, 3, make_double2(y[2], y[3]));
-        t.at(l, 8) = z[0];
-        if (a.has_body) { body[l] = z[1]; body[ld + l] = z[2]; body[2 * ld + l] = z[3]; }
+        if constexpr (NS) {
+          const double* w = reinterpret_cast<const double*>(a.ns_w) + 20 * j;
+          double u[20];
+#pragma unroll
+          for (int k = 0; k < 5; ++k) load_sector(w + 4 * k, u + 4 * k);
+          t.put(l, 4, make_double2(z[0], u[0]));
+#pragma unroll
+          for (int k = 0; k < 8; ++k) t.put(l, 5 + k, make_double2(u[2 * k + 1], u[2 * k + 2]));
+          t.at(l, 26) = u[17];
+          if (a.has_body) reinterpret_cast<int32_t*>(body)[l] = (int32_t)j;
+        } else {
+          t.at(l, 8) = z[0];
+          if (a.has_body) { body[l] = z[1]; body[ld + l] = z[2]; body[2 * ld + l] = z[3]; }
+        }
       }
     });
   }
@@ -936,7 +1032,7 @@ struct StagedT {
 
 template <bool F64, int KG, int KU, bool NS>
 constexpr int force_blocks() {  // blocks per SM the register cap asks for (NS: what its staged values leave room for)
-  return KG == 4 ? (NS ? 2 : (F64 ? 3 : (KU == 4 ? 4 : 5))) : 16 / KG;
+  return NS && F64 ? 1 : (KG == 4 ? (NS ? 2 : (F64 ? 3 : (KU == 4 ? 4 : 5))) : 16 / KG);
 }
 
 // TS = storage of T_i (float / double), A = accumulation, F64 = record width
@@ -963,18 +1059,18 @@ __global__ void __launch_bounds__(64 * KG, force_blocks<F64, KG, KU, NS>()) k_fo
   const int nit = valid ? walk.nit : 0;
   constexpr bool kPipe = !NS && (!F64 || KU <= 2);
   int64_t p0 = 0, pend = 0;  // list positions, for the values that stay in list order
-  if (valid && (NS || a.has_body)) {
+  if (valid && a.has_body) {
     p0 = a.colptr[J] + q;
     pend = a.colptr[J + 1];
   }
   Rec<F64> cur[KU];
-  SRec csr[NS ? KU : 1];
+  SRec<F64> csr[NS ? KU : 1];
   bool have = nit >= KU;
   if (have) {
 #pragma unroll
     for (int u = 0; u < KU; ++u) {
       load_rec(a.pk, a.sv.nrec, walk.at(u), cur[u]);
-      if constexpr (NS) csr[u] = load_srec(a.ns_scol, p0 + u * KG, pend);
+      if constexpr (NS) csr[u].load(a.ns_scol, a.sv.nrec, walk.at(u));
     }
   }
   grid_wait();
@@ -984,35 +1080,35 @@ __global__ void __launch_bounds__(64 * KG, force_blocks<F64, KG, KU, NS>()) k_fo
   if (valid) {
     A f0 = A(0), f1 = A(0), f2 = A(0);
     double e0 = 0.0, e1 = 0.0, e2 = 0.0;
-    auto body = [&](int it, const Rec<F64>& rec, const SRec& sr) {
+    auto body = [&](int it, const Rec<F64>& rec, const SRec<F64>& sr) {
       const A g0 = (A)rec.x(), g1 = (A)rec.y(), g2 = (A)rec.z();
       const int l = rec.l();
-      TS T[NS ? 28 : 9];
+      TS T[StagedT<TS, NS>::N];
       sT.t.load(l, T);
       f0 += (A)T[0] * g0 + (A)T[1] * g1 + (A)T[2] * g2;
       f1 += (A)T[3] * g0 + (A)T[4] * g1 + (A)T[5] * g2;
       f2 += (A)T[6] * g0 + (A)T[7] * g1 + (A)T[8] * g2;
       if constexpr (NS) {
-        const A sq[6] = {(A)sr.a.x, (A)sr.a.y, (A)sr.b.x, (A)sr.b.y, (A)sr.c.x, (A)sr.c.y};
-        // W_l(k, q) at 6 k + q: 16 values from T[12], the last two in T[9], T[10]
+        A sq[6];
+        sr.get(sq);
 #pragma unroll
         for (int c = 0; c < 6; ++c) {
-          f0 += (A)T[12 + c] * sq[c];
-          f1 += (A)T[18 + c] * sq[c];
-          f2 += (A)T[c < 4 ? 24 + c : 5 + c] * sq[c];
+          f0 += (A)StagedT<TS, NS>::weight(T, c) * sq[c];
+          f1 += (A)StagedT<TS, NS>::weight(T, 6 + c) * sq[c];
+          f2 += (A)StagedT<TS, NS>::weight(T, 12 + c) * sq[c];
         }
       }
       if (a.has_body) {
         const int64_t e = p0 + (int64_t)KG * it;
         if (e < pend) {  // (not a pad)
           const double s = a.tshp[e];
-          const TS* b = sT.body + l;
-          e0 += s * (double)b[0]; e1 += s * (double)b[sT.ld]; e2 += s * (double)b[2 * sT.ld];
+          double b[3];
+          sT.body_of(a, l, b);
+          e0 += s * b[0]; e1 += s * b[1]; e2 += s * b[2];
         }
       }
     };
-    const SRec s0{};
-    int it = 0;
+      int it = 0;
     while (have) {  // as in the row gather
       const bool hn = it + 2 * KU <= nit;
       Rec<F64> nxt[KU];
@@ -1024,14 +1120,14 @@ __global__ void __launch_bounds__(64 * KG, force_blocks<F64, KG, KU, NS>()) k_fo
         }
       }
 #pragma unroll
-      for (int u = 0; u < KU; ++u) body(it + u, cur[u], NS ? csr[NS ? u : 0] : s0);
+      for (int u = 0; u < KU; ++u) body(it + u, cur[u], csr[NS ? u : 0]);
 #pragma unroll
       for (int u = 0; u < KU; ++u) {
         if constexpr (kPipe) {
           cur[u] = nxt[u];
         } else if (hn) {
           load_rec(a.pk, a.sv.nrec, walk.at(it + KU + u), cur[u]);
-          if constexpr (NS) csr[u] = load_srec(a.ns_scol, p0 + (int64_t)KG * (it + KU + u), pend);
+          if constexpr (NS) csr[u].load(a.ns_scol, a.sv.nrec, walk.at(it + KU + u));
         }
       }
       it += KU;
@@ -1040,7 +1136,9 @@ __global__ void __launch_bounds__(64 * KG, force_blocks<F64, KG, KU, NS>()) k_fo
     for (; it < nit; ++it) {
       Rec<F64> rec;
       load_rec(a.pk, a.sv.nrec, walk.at(it), rec);
-      body(it, rec, NS ? load_srec(a.ns_scol, p0 + (int64_t)KG * it, pend) : s0);
+      SRec<F64> sr;
+      if constexpr (NS) sr.load(a.ns_scol, a.sv.nrec, walk.at(it));
+      body(it, rec, sr);
     }
 #pragma unroll
     for (int o = 1; o < KG; o <<= 1) {
@@ -1290,8 +1388,9 @@ __global__ void __launch_bounds__(64 * KG) k_force_b(TiledForceArgs a) {
           const int64_t p = p0 + (int64_t)KG * it;
           if (p < pend) {
             const double s = a.tshp[p];
-            const TS* b = sT.body + l;
-            b0 += s * (double)b[0]; b1 += s * (double)b[sT.ld]; b2 += s * (double)b[2 * sT.ld];
+            double b[3];
+            sT.body_of(a, l, b);
+            b0 += s * b[0]; b1 += s * b[1]; b2 += s * b[2];
           }
         }
       }
@@ -1438,9 +1537,20 @@ int iota64(cudaStream_t s, int64_t m, int64_t* out) {
   return 0;
 }
 
-int gather_f6(cudaStream_t s, int64_t m, const int64_t* pos, const float* in, float* out) {
-  if (m <= 0) return 0;
-  k_gather_f6<<<grid_for(m, 256), 256, 0, s>>>(m, pos, (const float2*)in, (float2*)out);
+int pack_second(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* ptr, const int64_t* pos, const NsniS& src,
+                bool f64, void* out) {
+  const int64_t slots = ts.ntiles * ts.R;
+  auto k = f64 ? k_pack_second<true> : k_pack_second<false>;
+  k<<<grid_for(4 * slots, 256), 256, 0, s>>>(n, ts.R, slots, ts.view(), ptr, pos, src, out);
+  MEGA_CHECK_LAUNCH();
+  return 0;
+}
+
+int gather_second(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* ptr, const int64_t* pos, bool f64,
+                  const void* in, void* out) {
+  const int64_t slots = ts.ntiles * ts.R;
+  auto k = f64 ? k_gather_second<true> : k_gather_second<false>;
+  k<<<grid_for(4 * slots, 256), 256, 0, s>>>(n, ts.R, slots, ts.view(), ptr, pos, in, out);
   MEGA_CHECK_LAUNCH();
   return 0;
 }
@@ -1482,7 +1592,9 @@ static int configure_defgrad(int lim) {
   if ((r = raise_smem(k_defgrad_t<float, false, true, KG, KU, true, FULL>, lim))) return r;
   if ((r = raise_smem(k_defgrad_t<float, false, false, KG, KU, true, FULL>, lim))) return r;
   if ((r = raise_smem(k_defgrad_t<double, true, true, KG, KU, false, FULL>, lim))) return r;
-  return raise_smem(k_defgrad_t<double, true, false, KG, KU, false, FULL>, lim);
+  if ((r = raise_smem(k_defgrad_t<double, true, false, KG, KU, false, FULL>, lim))) return r;
+  if ((r = raise_smem(k_defgrad_t<double, true, true, KG, KU, true, FULL>, lim))) return r;
+  return raise_smem(k_defgrad_t<double, true, false, KG, KU, true, FULL>, lim);
 }
 
 template <int KG, int KU>
@@ -1491,6 +1603,8 @@ static int configure_variant(int lim) {
   if ((r = configure_defgrad<KG, KU, false>(lim))) return r;
   if ((r = raise_smem(k_force_t<float, float, false, KG, KU>, lim))) return r;
   if ((r = raise_smem(k_force_t<float, float, false, KG, KU, true>, lim))) return r;
+  if ((r = raise_smem(k_force_t<double, double, true, KG, KU, true>, (int)StagedT<double, true>::bytes(1024, true))))
+    return r;
   return raise_smem(k_force_t<double, double, true, KG, KU>, lim);
 }
 
@@ -1579,8 +1693,10 @@ static int defgrad_variant(cudaStream_t s, const DefgradArgs& d) {
   const TileSet& ts = d.ts;
   const size_t smem = (size_t)((d.mixed ? 16 : 24) * (FULL ? 2 : 1)) * staged_ld(ts.maxcnt);
   const NsniTiles nz = d.ns ? *d.ns : NsniTiles();
-  auto k = !d.mixed ? (d.interp ? k_defgrad_t<double, true, true, KG, KU, false, FULL>
-                                : k_defgrad_t<double, true, false, KG, KU, false, FULL>)
+  auto k = !d.mixed ? (d.ns ? (d.interp ? k_defgrad_t<double, true, true, KG, KU, true, FULL>
+                                        : k_defgrad_t<double, true, false, KG, KU, true, FULL>)
+                            : (d.interp ? k_defgrad_t<double, true, true, KG, KU, false, FULL>
+                                        : k_defgrad_t<double, true, false, KG, KU, false, FULL>))
            : d.ns   ? (d.interp ? k_defgrad_t<float, false, true, KG, KU, true, FULL>
                                 : k_defgrad_t<float, false, false, KG, KU, true, FULL>)
                     : (d.interp ? k_defgrad_t<float, false, true, KG, KU, false, FULL>
@@ -1589,12 +1705,20 @@ static int defgrad_variant(cudaStream_t s, const DefgradArgs& d) {
                            d.pk, ts.jset, ts.jcnt, d.dsp, d.dsp_tot, d.sdphi, d.shp, d.dsp_tot_phy, d.fg, d.acc);
 }
 
+// NSNI runs the register variants: mixed refuses the streamed ones, FP64 takes
+// the register variant of the same lanes per row (the same sums) for them.
+static bool ns_variant(bool mixed, int& variant) {
+  if (variant != 4 && variant != 5) return true;
+  variant = variant == 4 ? 0 : 3;
+  return !mixed;
+}
+
 int launch_defgrad_tiled(cudaStream_t s, bool mixed, bool interp, int32_t n, const TileSet& ts,
                          const NsniTiles* ns, const int64_t* rowptr, const void* pk, const double* dsp,
                          const double* dsp_tot, const double* sdphi, const double* shp, double* dsp_tot_phy,
                          double* fg, StepAccum* acc, unsigned* status, int variant, bool full) {
   int r = 0;
-  if (ns && (!mixed || variant == 4 || variant == 5)) return MEGA_ERR_UNSUPPORTED;  // NSNI: register variants
+  if (ns && !ns_variant(mixed, variant)) return MEGA_ERR_UNSUPPORTED;
   const DefgradArgs d{mixed, interp, n, ts, ns, rowptr, pk, dsp, dsp_tot, sdphi, shp, dsp_tot_phy, fg, acc, status};
   if (full) {
     if (variant == 6 || variant == 7) r = defgrad_variant<16, kFullKU, true>(s, d);
@@ -1631,11 +1755,14 @@ static int force_bulk(cudaStream_t s, bool mixed, const TiledForceArgs& a) {
 
 template <int KG, int KU>
 static int force_variant(cudaStream_t s, bool mixed, const TiledForceArgs& a) {
-  const int nv = (a.ns_scol ? 28 : 9) + (a.has_body ? 3 : 0);
-  const size_t smem = (mixed ? sizeof(float) : sizeof(double)) * nv * staged_ld(a.maxcnt);
+  const size_t smem = !mixed ? (a.ns_scol ? StagedT<double, true>::bytes(a.maxcnt, a.has_body)
+                                          : StagedT<double, false>::bytes(a.maxcnt, a.has_body))
+                             : (a.ns_scol ? StagedT<float, true>::bytes(a.maxcnt, a.has_body)
+                                          : StagedT<float, false>::bytes(a.maxcnt, a.has_body));
   const unsigned grid = (unsigned)a.ntiles;
   const int block = a.R * KG;
-  auto k = !mixed       ? k_force_t<double, double, true, KG, KU>
+  auto k = !mixed       ? (a.ns_scol ? k_force_t<double, double, true, KG, KU, true>
+                                     : k_force_t<double, double, true, KG, KU>)
            : a.ns_scol ? k_force_t<float, float, false, KG, KU, true>
                        : k_force_t<float, float, false, KG, KU>;
   return launch_overlapped(k, grid, block, smem, s, a);
@@ -1643,7 +1770,7 @@ static int force_variant(cudaStream_t s, bool mixed, const TiledForceArgs& a) {
 
 int launch_force_tiled(cudaStream_t s, bool mixed, const TiledForceArgs& a, int variant) {
   int r = 0;
-  if (a.ns_scol && (!mixed || variant == 4 || variant == 5)) return MEGA_ERR_UNSUPPORTED;  // NSNI: register variants
+  if (a.ns_scol && !ns_variant(mixed, variant)) return MEGA_ERR_UNSUPPORTED;
   switch (variant) {
     case 1: r = force_variant<4, 2>(s, mixed, a); break;
     case 2: r = force_variant<4, 1>(s, mixed, a); break;

@@ -30,15 +30,16 @@ struct TileSet {
   SliceView view() const { return SliceView{ord, sstep, nrec}; }
 };
 
-// NSNI terms carried by the mixed-precision tiled gathers: the smoothed
-// second derivatives S_q (XX, YY, ZZ, XY, YZ, XZ) of every list entry as six
-// floats in the order of the float row records (srow) and of the float
-// column records (scol), their row sums, and the per-node H output (row
-// gather) and force weights (column gather)
+// NSNI terms carried by the tiled gathers: the smoothed second derivatives
+// S_q (XX, YY, ZZ, XY, YZ, XZ) of every list entry in the layout of the row
+// records (srow) and of the column records, as planes of nrec values: float4
+// (q 0-3) and float2 (q 4, 5), or three planes of double2; their row sums
+// (mixed), and the per-node H output (row gather) and force weights (column
+// gather)
 struct NsniTiles {
-  const float* srow = nullptr;   // 6 per row record
-  const double* ssum = nullptr;  // 6 per node: sum_J S_q(i, J) in double
-  double* hq = nullptr;          // 18 per node out: sum_J S_q(i, J) du_J,k at [18 i + 6 k + q]
+  const void* srow = nullptr;
+  const double* ssum = nullptr;  // mixed: 6 per node, sum_J S_q(i, J) of the float values in double
+  double* hq = nullptr;          // out: sum_J S_q(i, J) du_J,k at [(6 k + q) fg_ld(n) + i]
 };
 
 struct TiledForceArgs {
@@ -69,9 +70,8 @@ struct TiledForceArgs {
   double* dsp;
   double* dsp_tot;
   double* prforce;
-  const double* fadd;     // 3 per node added to the internal force (NSNI), or null
-  const float* ns_scol;   // NSNI (mixed): 6 S values per column record, or null
-  const float* ns_w;      // NSNI (mixed): force weights, 20 floats per node (18 used)
+  const void* ns_scol;    // NSNI: the S planes of the column records, or null
+  const void* ns_w;       // NSNI: force weights, 20 values per node (18 used; floats when mixed)
   const double* vel2;     // prescribed velocities of fixity code 2 for this step (3), or null
   const double* ndt;      // per-node step of independent instances, or null (dt for all)
   double dt;
@@ -108,8 +108,12 @@ int bank_order(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* ptr,
 int iota64(cudaStream_t s, int64_t m, int64_t* out);
 int gather_records(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* ptr, const int64_t* pos, bool f64,
                    const void* in, void* out);
-// out[6 e + k] = in[6 pos[e] + k]
-int gather_f6(cudaStream_t s, int64_t m, const int64_t* pos, const float* in, float* out);
+// NSNI's S (list order, at pos[e] when given) as planes in the records' layout,
+// and those planes with the entries of each row reordered by pos
+int pack_second(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* ptr, const int64_t* pos, const NsniS& src,
+                bool f64, void* out);
+int gather_second(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* ptr, const int64_t* pos, bool f64,
+                  const void* in, void* out);
 int configure_tiled_kernels();
 // launch variants of the two gathers: lanes per row x records in flight
 // (register streams, variants 0-3 and 6, 7), and lanes per row with the
@@ -120,7 +124,8 @@ int tiled_variants();
 // whether a variant's shared memory fits the row (defgrad) or column (force) tiles
 bool tiled_variant_fits(const TileSet& ts, bool mixed, int variant, bool force, bool has_body);
 // MEGA_ERR_UNSUPPORTED when the variant's shared memory does not fit the tiles
-// ns (mixed only, register variants): the NSNI H gather rides along.
+// ns: the NSNI H gather rides along (register variants; FP64 takes those of
+// the same lanes per row for 4 and 5, mixed refuses them).
 // full: F - I as well as G0 (else the stress update adds G0 to F - I)
 int launch_defgrad_tiled(cudaStream_t s, bool mixed, bool interp, int32_t n, const TileSet& ts,
                          const NsniTiles* ns, const int64_t* rowptr, const void* pk, const double* dsp,
