@@ -329,8 +329,25 @@ int upload_staged(cudaStream_t s, const std::vector<HostToDevice>& items) {
   return 0;
 }
 
-// device -> host through the pinned buffer (stream s ordered, complete on return)
-int download_staged(cudaStream_t s, void* dst, const void* src, size_t bytes) {
+struct HostPart {
+  void* dst;
+  size_t bytes;
+};
+
+// One device range to host arrays, one after another, through the pinned
+// buffer (stream s ordered, complete on return)
+int download_parts(cudaStream_t s, const void* src, const std::vector<HostPart>& parts) {
+  size_t bytes = 0;
+  for (const HostPart& p : parts) bytes += p.bytes;
+  // [at, at + len) of the range into the parts it belongs to
+  auto scatter = [&](size_t at, size_t len, const unsigned char* from) {
+    size_t p0 = 0;
+    for (const HostPart& p : parts) {
+      const size_t lo = std::max(at, p0), hi = std::min(at + len, p0 + p.bytes);
+      if (lo < hi) std::memcpy((unsigned char*)p.dst + (lo - p0), from + (lo - at), hi - lo);
+      p0 += p.bytes;
+    }
+  };
   std::lock_guard<std::mutex> lk(g_stage.mu);
   if (g_stage.cap < bytes) {
     if (g_stage.p) cudaFreeHost(g_stage.p);
@@ -340,7 +357,11 @@ int download_staged(cudaStream_t s, void* dst, const void* src, size_t bytes) {
     else { g_stage.p = nullptr; cudaGetLastError(); }
   }
   if (!g_stage.p) {
-    MEGA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s));
+    size_t at = 0;
+    for (const HostPart& p : parts) {
+      MEGA_TRY(cudaMemcpyAsync(p.dst, (const unsigned char*)src + at, p.bytes, cudaMemcpyDeviceToHost, s));
+      at += p.bytes;
+    }
     MEGA_TRY(cudaStreamSynchronize(s));
     return 0;
   }
@@ -363,17 +384,43 @@ int download_staged(cudaStream_t s, void* dst, const void* src, size_t bytes) {
       for (int64_t k = lo; k < hi; ++k) {
         const size_t a = (size_t)k * kPiece, len = std::min(kPiece, bytes - a);
         if (cudaEventSynchronize(ev[k]) != cudaSuccess) { bad.store(1); continue; }
-        std::memcpy((unsigned char*)dst + a, g_stage.p + a, len);
+        scatter(a, len, g_stage.p + a);
       }
     }, 1);
   if (r || bad.load()) {
     cudaStreamSynchronize(s);  // no DMA may still write the stage
-    record_cuda_error(cudaGetLastError(), "download_staged", __FILE__, __LINE__);
+    record_cuda_error(cudaGetLastError(), "download_parts", __FILE__, __LINE__);
     r = MEGA_ERR_CUDA;
   }
   for (auto e : ev)
     if (e) cudaEventDestroy(e);
   return r;
+}
+
+int download_staged(cudaStream_t s, void* dst, const void* src, size_t bytes) {
+  return download_parts(s, src, {{dst, bytes}});
+}
+
+// upload_staged in batches of at most 128 MiB of staging (lists of a large
+// model; the staging buffer stays with the process)
+static int upload_batched(cudaStream_t s, const std::vector<HostToDevice>& items) {
+  constexpr size_t kMost = (size_t)128 << 20;
+  std::vector<HostToDevice> batch;
+  size_t held = 0;
+  for (const auto& it : items)
+    for (size_t at = 0; at < it.bytes || (at == 0 && it.fill);) {
+      const size_t len = it.fill ? it.bytes : std::min(it.bytes - at, kMost);
+      if (held + len > kMost && !batch.empty()) {
+        if (int r = upload_staged(s, batch)) return r;
+        batch.clear();
+        held = 0;
+      }
+      batch.push_back(it.fill ? it : HostToDevice{(unsigned char*)it.dst + at, (const unsigned char*)it.src + at, len});
+      held += len;
+      at += len;
+      if (it.fill) break;
+    }
+  return batch.empty() ? 0 : upload_staged(s, batch);
 }
 
 // Deduplication of PROPS(30,N) and the material type into a table of
@@ -766,6 +813,86 @@ static int upload(cudaStream_t s, T* d, const T* h, size_t count) {
 // Device CSR from the reference's 1-based (GN, GSTART, GSTACK); rows are
 // re-packed contiguously in node order.  hpos[k] = 0-based GSTACK position
 // of packed entry k (for writing per-entry values back).
+// Warp per node: a caller's row (start k0[i], raw 1-based ids from list
+// position lo on) as CSR columns and list positions; ids out of range raise bad.
+__global__ void k_caller_rows(int32_t n, const int64_t* __restrict__ rowptr, const int64_t* __restrict__ k0,
+                              const int32_t* __restrict__ raw, int32_t* __restrict__ col, int64_t* __restrict__ pos,
+                              int32_t* __restrict__ bad) {
+  const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (i >= n) return;
+  const int64_t b = rowptr[i], len = rowptr[i + 1] - b;
+  for (int64_t k = lane; k < len; k += 32) {
+    const int32_t j = raw[k0[i] + k] - 1;
+    const bool ok = j >= 0 && j < n;
+    if (!ok) *bad = 1;
+    col[b + k] = ok ? j : 0;
+    pos[b + k] = k0[i] + k;
+  }
+}
+// shapes and gradients at the entries' list positions
+__global__ void k_caller_shapes(int64_t m, const int64_t* __restrict__ pos, const double* __restrict__ shp,
+                                const double* __restrict__ dshp, double* __restrict__ osh, double* __restrict__ gx,
+                                double* __restrict__ gy, double* __restrict__ gz) {
+  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (e >= m) return;
+  const int64_t q = pos[e];
+  osh[e] = shp[q];
+  gx[e] = dshp[3 * q];
+  gy[e] = dshp[3 * q + 1];
+  gz[e] = dshp[3 * q + 2];
+}
+
+// A caller's lists as CSR on the device, checked there, with the list position
+// (from `lo` on) of every entry.  The calling thread only forms the row
+// offsets; the ids go up as they are.
+struct CallerLists {
+  int64_t lo = 0, hi = 0;    // the list positions in use
+  int64_t* pos = nullptr;    // per entry: its position less lo
+};
+static int csr_from_caller(cudaStream_t s, int32_t n, const int32_t* gn, const int32_t* gstart,
+                           const int32_t* gstack, int64_t nnz_cap, DevPool& pool, DevCSR& csr, CallerLists& cl) {
+  std::vector<int64_t> rp(n + 1, 0), k0(n, 0);
+  int64_t lo = INT64_MAX, hi = 0;
+  csr.gmaxn = 0;
+  for (int32_t i = 0; i < n; ++i) {
+    if (gn[i] < 0) return MEGA_ERR_ARG;
+    rp[i + 1] = rp[i] + gn[i];
+    csr.gmaxn = std::max(csr.gmaxn, gn[i]);
+    if (gn[i] == 0) continue;
+    k0[i] = (int64_t)gstart[i] - 1;
+    if (k0[i] < 0 || k0[i] + gn[i] > nnz_cap) return MEGA_ERR_ARG;
+    lo = std::min(lo, k0[i]);
+    hi = std::max(hi, k0[i] + gn[i]);
+  }
+  const int64_t m = rp[n];
+  csr.n = n;
+  csr.nnz = m;
+  cl.lo = m ? lo : 0;
+  cl.hi = hi;
+  for (int32_t i = 0; i < n; ++i)
+    if (gn[i] > 0) k0[i] -= cl.lo;
+  MEGA_ALLOC(pool, csr.rowptr, (int64_t)n + 1);
+  MEGA_ALLOC(pool, csr.col, m);
+  MEGA_ALLOC(pool, cl.pos, m);
+  DevPool tmp(s);
+  int64_t* dk0 = nullptr;
+  int32_t *raw = nullptr, *bad = nullptr;
+  MEGA_ALLOC(tmp, dk0, n);
+  MEGA_ALLOC(tmp, raw, cl.hi - cl.lo);
+  MEGA_ALLOC(tmp, bad, 1);
+  MEGA_TRY(cudaMemsetAsync(bad, 0, sizeof(int32_t), s));
+  int r = upload_batched(s, {{csr.rowptr, rp.data(), 8 * ((size_t)n + 1)}, {dk0, k0.data(), 8 * (size_t)n},
+                             {raw, gstack + cl.lo, 4 * (size_t)(cl.hi - cl.lo)}});
+  if (r) return r;
+  k_caller_rows<<<grid_for((int64_t)n * 32, 256), 256, 0, s>>>(n, csr.rowptr, dk0, raw, csr.col, cl.pos, bad);
+  MEGA_CHECK_LAUNCH();
+  int32_t hb = 0;
+  MEGA_TRY(cudaMemcpyAsync(&hb, bad, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+  MEGA_TRY(cudaStreamSynchronize(s));
+  return hb ? MEGA_ERR_ARG : 0;
+}
+
 static int csr_from_host(cudaStream_t s, int32_t n, const int32_t* gn, const int32_t* gstart,
                          const int32_t* gstack, int64_t nnz_cap, DevPool& pool, DevCSR& csr,
                          std::vector<int64_t>& hpos) {
@@ -2587,16 +2714,22 @@ static int construct_fint_impl(const mega_params* p, const FintIO& io) {
   int r = make_stream(&sg.s);
   if (r) return r;
   cudaStream_t s = sg.s;
-  DevPool pool;
+  DevPool pool(s);  // through the block cache: a call per step allocates nothing from the driver
   DevCSR csr;
-  std::vector<int64_t> hpos;
-  r = csr_from_host(s, n, io.gn, io.gstart, io.gstack, io.nnz, pool, csr, hpos);
+  CallerLists cl;
+  r = csr_from_caller(s, n, io.gn, io.gstart, io.gstack, io.nnz, pool, csr, cl);
   if (r) return r;
+  std::vector<int64_t> hpos;  // the entries' list positions, where the host writes or reads per entry
+  if (shapes_here || nsni) {
+    hpos.reserve(csr.nnz);
+    for (int32_t i = 0; i < n; ++i)
+      for (int32_t k = 0; k < io.gn[i]; ++k) hpos.push_back((int64_t)io.gstart[i] - 1 + k);
+  }
   r = build_transpose(s, csr, pool);
   if (r) return r;
   const int64_t n3 = 3 * (int64_t)n, m = csr.nnz;
-  double *dc, *dw, *dv, *dsh, *dgx, *dgy, *dgz, *tgx, *tgy, *tgz, *tsh = nullptr, *sd, *ddsp, *dtot, *dsig, *deps6,
-         *dep, *deq, *dwv, *dfg, *dT, *dfi, *dfe, *dbf = nullptr, *dcur = nullptr, *dsml = nullptr;
+  double *dc, *dw, *dv, *dsh, *dgx, *dgy, *dgz, *tgx, *tgy, *tgz, *tsh = nullptr, *sd, *ddsp, *dtot, *dfg, *dT, *out,
+      *dbf = nullptr, *dcur = nullptr, *dsml = nullptr;
   int32_t* den = nullptr;
   uint16_t* midx;
   StepAccum* acc;
@@ -2605,9 +2738,13 @@ static int construct_fint_impl(const mega_params* p, const FintIO& io) {
   MEGA_ALLOC(pool, dsh, m); MEGA_ALLOC(pool, dgx, m); MEGA_ALLOC(pool, dgy, m); MEGA_ALLOC(pool, dgz, m);
   MEGA_ALLOC(pool, tgx, m); MEGA_ALLOC(pool, tgy, m); MEGA_ALLOC(pool, tgz, m);
   MEGA_ALLOC(pool, sd, n3); MEGA_ALLOC(pool, ddsp, n3); MEGA_ALLOC(pool, dtot, n3);
-  MEGA_ALLOC(pool, dsig, 6 * (int64_t)n); MEGA_ALLOC(pool, deps6, 6 * (int64_t)n); MEGA_ALLOC(pool, dep, n);
-  MEGA_ALLOC(pool, deq, n); MEGA_ALLOC(pool, dwv, n); MEGA_ALLOC(pool, dfg, 18 * fg_ld(n));
-  MEGA_ALLOC(pool, dT, 12 * (int64_t)n); MEGA_ALLOC(pool, dfi, n3); MEGA_ALLOC(pool, dfe, n3);
+  MEGA_ALLOC(pool, dfg, 18 * fg_ld(n)); MEGA_ALLOC(pool, dT, 12 * (int64_t)n);
+  // what is read back, in one block: stress, strain, internal and external
+  // force (the node rows of 6 first, so they stay 16-byte aligned), plastic
+  // and equivalent strain, wave speed
+  MEGA_ALLOC(pool, out, 21 * (int64_t)n);
+  double *dsig = out, *deps6 = out + 6 * (int64_t)n, *dfi = out + 12 * (int64_t)n, *dfe = dfi + n3, *dep = dfe + n3,
+         *deq = dep + n, *dwv = deq + n;
   MEGA_ALLOC(pool, midx, n); MEGA_ALLOC(pool, acc, 1); MEGA_ALLOC(pool, st, 1);
   bool has_body = p->gravity[0] != 0.0 || p->gravity[1] != 0.0 || p->gravity[2] != 0.0;
   if (io.bodyforce)
@@ -2626,8 +2763,7 @@ static int construct_fint_impl(const mega_params* p, const FintIO& io) {
   if ((r = material_table(n, io.gprop, io.gmat_type, 65535, ents, hidx, damaged))) return r;
   MatEntry* dmat;
   MEGA_ALLOC(pool, dmat, ents.size());
-  std::vector<double> hs(n), hax;
-  for (int32_t i = 0; i < n; ++i) hs[i] = io.gstate[20 * (size_t)i + 2];
+  std::vector<double> hax;
   double* dax = nullptr;  // GSTATE(1, 2, 4, 5) when a damaged model is present
   if (damaged) {
     MEGA_ALLOC(pool, dax, 4 * (int64_t)n);
@@ -2639,31 +2775,38 @@ static int construct_fint_impl(const mega_params* p, const FintIO& io) {
     }
     if ((r = upload(s, dax, hax.data(), hax.size()))) return r;
   }
-  if ((r = upload(s, dc, io.gcoo, n3)) || (r = upload(s, dw, io.gwin, n3)) || (r = upload(s, dv, io.gvol, (size_t)n)) ||
-      (r = upload(s, ddsp, io.gdinc, n3)) || (r = upload(s, dsig, io.gstress, 6 * (size_t)n)) ||
-      (r = upload(s, deps6, io.gstrain, 6 * (size_t)n)) || (r = upload(s, dep, hs.data(), (size_t)n)) ||
-      (r = upload(s, midx, hidx.data(), (size_t)n)) || (r = upload(s, dmat, ents.data(), ents.size())))
-    return r;
+  auto fill_eps = [&](void* d) {
+    double* o = (double*)d;
+    for (int32_t i = 0; i < n; ++i) o[i] = io.gstate[20 * (size_t)i + 2];
+  };
+  const size_t n8 = 8 * (size_t)n;
+  std::vector<HostToDevice> items = {{dc, io.gcoo, 3 * n8}, {dw, io.gwin, 3 * n8}, {dv, io.gvol, n8},
+                                     {ddsp, io.gdinc, 3 * n8}, {dsig, io.gstress, 6 * n8}, {deps6, io.gstrain, 6 * n8},
+                                     {dep, nullptr, n8, fill_eps}, {midx, hidx.data(), 2 * (size_t)n},
+                                     {dmat, ents.data(), sizeof(MatEntry) * ents.size()}};
   // the total displacement pushes the gradients forward; on the
   // semi-Lagrangian path they are current already (F = I, FINT.F90:410-436)
-  if (semi) MEGA_TRY(cudaMemsetAsync(dtot, 0, sizeof(double) * n3, s));
-  else if ((r = upload(s, dtot, io.gdinc_tot, n3))) return r;
+  if (semi) MEGA_TRY(cudaMemsetAsync(dtot, 0, 3 * n8, s));
+  else items.push_back({dtot, io.gdinc_tot, 3 * n8});
+  DevPool raw(s);
+  double *rsh = nullptr, *rdsh = nullptr;
+  if (!shapes_here) {
+    const int64_t used = cl.hi - cl.lo;
+    MEGA_ALLOC(raw, rsh, used);
+    MEGA_ALLOC(raw, rdsh, 3 * used);
+    items.push_back({rsh, io.gstack_shp + cl.lo, 8 * (size_t)used});
+    items.push_back({rdsh, io.gstack_dshp + 3 * cl.lo, 24 * (size_t)used});
+  }
+  if ((r = upload_batched(s, items))) return r;
   MEGA_TRY(cudaMemsetAsync(acc, 0, sizeof(StepAccum), s));
   MEGA_TRY(cudaMemsetAsync(st, 0, sizeof(unsigned), s));
   if (shapes_here) {
     r = rk_shapes(s, *p, n, semi ? dcur : dc, dw, den, csr, dsh, dgx, dgy, dgz, st);
     if (r) return r;
   } else {
-    std::vector<double> a(m), b(m), d(m), e(m);
-    for (int64_t k = 0; k < m; ++k) {
-      const int64_t q = hpos[k];
-      a[k] = io.gstack_shp[q];
-      b[k] = io.gstack_dshp[3 * q]; d[k] = io.gstack_dshp[3 * q + 1]; e[k] = io.gstack_dshp[3 * q + 2];
-    }
-    if ((r = upload(s, dsh, a.data(), m)) || (r = upload(s, dgx, b.data(), m)) || (r = upload(s, dgy, d.data(), m)) ||
-        (r = upload(s, dgz, e.data(), m)))
-      return r;
-    MEGA_TRY(cudaStreamSynchronize(s));
+    k_caller_shapes<<<grid_for(m, 256), 256, 0, s>>>(m, cl.pos, rsh, rdsh, dsh, dgx, dgy, dgz);
+    MEGA_CHECK_LAUNCH();
+    raw.free_all();
   }
   // NSNI: second derivatives (computed at LINIT, read otherwise) in CSR and
   // CSC order, stress gradients, per-call scratch
@@ -2749,16 +2892,13 @@ static int construct_fint_impl(const mega_params* p, const FintIO& io) {
   }
   StepAccum hacc;
   unsigned hst = 0;
-  MEGA_TRY(cudaMemcpyAsync(io.fint, dfi, sizeof(double) * n3, cudaMemcpyDeviceToHost, s));
-  MEGA_TRY(cudaMemcpyAsync(io.fext, dfe, sizeof(double) * n3, cudaMemcpyDeviceToHost, s));
-  MEGA_TRY(cudaMemcpyAsync(io.gstress, dsig, sizeof(double) * 6 * n, cudaMemcpyDeviceToHost, s));
-  MEGA_TRY(cudaMemcpyAsync(io.gstrain, deps6, sizeof(double) * 6 * n, cudaMemcpyDeviceToHost, s));
-  MEGA_TRY(cudaMemcpyAsync(hs.data(), dep, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
-  if (damaged) MEGA_TRY(cudaMemcpyAsync(hax.data(), dax, sizeof(double) * 4 * n, cudaMemcpyDeviceToHost, s));
-  MEGA_TRY(cudaMemcpyAsync(io.gmax_wvel, dwv, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
-  MEGA_TRY(cudaMemcpyAsync(io.gstrain_eq, deq, sizeof(double) * n, cudaMemcpyDeviceToHost, s));
   MEGA_TRY(cudaMemcpyAsync(&hacc, acc, sizeof(hacc), cudaMemcpyDeviceToHost, s));
   MEGA_TRY(cudaMemcpyAsync(&hst, st, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+  if (damaged) MEGA_TRY(cudaMemcpyAsync(hax.data(), dax, sizeof(double) * 4 * n, cudaMemcpyDeviceToHost, s));
+  std::vector<double> hs(n);
+  if ((r = download_parts(s, out, {{io.gstress, 6 * n8}, {io.gstrain, 6 * n8}, {io.fint, 3 * n8}, {io.fext, 3 * n8},
+                                   {hs.data(), n8}, {io.gstrain_eq, n8}, {io.gmax_wvel, n8}})))
+    return r;
   if (shapes_here) {  // GSTACK_SHP / GSTACK_DSHP written where RK1 ran (FINT.F90:427-434, 580-587)
     std::vector<double> a2(m), b(m), d(m), e(m);
     MEGA_TRY(cudaMemcpyAsync(a2.data(), dsh, sizeof(double) * m, cudaMemcpyDeviceToHost, s));
