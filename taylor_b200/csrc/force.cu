@@ -30,6 +30,7 @@ namespace mega {
 namespace {
 
 constexpr int kGroup = 4;  // lanes per node in the gathers
+constexpr int kStressBlock = 64;
 
 __device__ __forceinline__ NodeMat to_nodemat(const MatEntry& e) {
   NodeMat m;
@@ -151,7 +152,7 @@ struct Trial {
 // of sigma and eps, eps += dstrain, elastic predictor.
 // DAM: the context holds damaged models (materials 3, 6) and their state;
 // without it their branches compile out of the J2 path.
-template <typename T, bool LEAN, bool DAM>
+template <typename T, bool LEAN, bool DAM, bool FAST = false>
 __device__ __forceinline__ void stress_trial(const StressArgs& a, int64_t i, Trial<T, LEAN>& w) {
   // F and G0 (18 planes), stress and strain (6 each) as 16-byte loads
   double fgi[18], sv[6], ev[6];
@@ -182,7 +183,7 @@ __device__ __forceinline__ void stress_trial(const StressArgs& a, int64_t i, Tri
     w.eps6[k] = (T)eo;
     w.D[k] = T(0);
   }
-  if (a.finite_strain) {
+  if (FAST || a.finite_strain) {
     // |det F| and INV3 in double (F carries the FP64 displacement path)
     double Fd[3][3];
 #pragma unroll
@@ -259,7 +260,7 @@ __device__ __forceinline__ double rate_features(const double spred[6], double ep
 
 // FINT.F90:797-870, 999-1116: return mapping (dg0 >= 0 starts the rate law's
 // Newton there), state write-back, strain_eq, internal work, wave speed, T_i.
-template <typename T, typename TS, bool LEAN, bool DAM>
+template <typename T, typename TS, bool LEAN, bool DAM, bool FAST = false>
 __device__ __forceinline__ void stress_finish(const StressArgs& a, int64_t i, Trial<T, LEAN>& w, double dg0, double& work,
                                               unsigned long long& nit, unsigned long long& npl, unsigned& st) {
   const MatEntry& me = LEAN ? a.mats[w.mi] : w.me;
@@ -319,7 +320,7 @@ __device__ __forceinline__ void stress_finish(const StressArgs& a, int64_t i, Tr
   if (cap) st |= MEGA_ST_NEWTON_CAP;
   nit += (unsigned long long)it;
   npl += (it > 0) ? 1ull : 0ull;
-  if (a.iters && !a.more) a.iters[i] = it;
+  if (!FAST && a.iters && !a.more) a.iters[i] = it;
   double sinc[6], einc[6], enew[6];
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
@@ -343,14 +344,14 @@ __device__ __forceinline__ void stress_finish(const StressArgs& a, int64_t i, Tr
     }
   }
   a.eps[i] = ep;
-  if (a.finite_strain) {
+  if (FAST || a.finite_strain) {
 #pragma unroll
     for (int k = 0; k < 6; ++k) work += 0.5 * (double)w.D[k] * (2.0 * snew[k] - sinc[k]) * vol * w.det;
   } else {
 #pragma unroll
     for (int k = 0; k < 6; ++k) work += 0.5 * einc[k] * sinc[k] * vol * w.det;
   }
-  if (!a.more) {  // the last step of a call: what only a caller reads
+  if (!FAST && !a.more) {  // the last step of a call: what only a caller reads
     const double eq = enew[0] * enew[0] + enew[1] * enew[1] + enew[2] * enew[2] +
                       2.0 * (enew[3] * enew[3] + enew[4] * enew[4] + enew[5] * enew[5]);
     a.strain_eq[i] = sqrt(eq * 2.0 / 3.0);
@@ -428,8 +429,16 @@ __device__ __forceinline__ double rate_overstress(const double spred[6], double 
 // QUEUE (the learned start): plastic rate-dependent nodes are not finished
 // here but listed in a.queue (one atomic per warp) for k_stress_queue, so
 // the network and its Newton polish run on full warps of plastic nodes only.
-template <typename T, typename TS, bool DAM, bool QUEUE>
-__global__ void __launch_bounds__(256, 2) k_stress(StressArgs a) {
+// FAST: finite strain on a step that another one follows (all but the last of
+// a call), compiled without the branches of the others, the old stress and
+// the material entry re-read where they are used (LEAN): 250-390 bytes of
+// spills over the 128 registers become 8-144.  What bounds it is the latency
+// of the loads and of the FP64 chain at 16 warps an SM (at 24, with 80
+// registers, it ran slower); blocks of 64 spread the coarse bars over more
+// SMs.  1.04 M nodes: mixed 108 -> 95 us (69 % of the HBM floor), FP64 123 ->
+// 113; 4,455 nodes FP64 12.2 -> 10.3 us.
+template <typename T, typename TS, bool DAM, bool QUEUE, bool FAST>
+__global__ void __launch_bounds__(kStressBlock, 512 / kStressBlock) k_stress(StressArgs a) {
   __shared__ double smd[32];
   __shared__ unsigned long long smu[32];
   grid_wait();
@@ -440,10 +449,10 @@ __global__ void __launch_bounds__(256, 2) k_stress(StressArgs a) {
   unsigned long long nit = 0, npl = 0;
   unsigned st = 0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.n; i += (int64_t)gridDim.x * blockDim.x) {
-    Trial<T, false> w;
-    stress_trial<T, false, DAM>(a, i, w);
+    Trial<T, FAST> w;
+    stress_trial<T, FAST, DAM, FAST>(a, i, w);
     if (QUEUE) {
-      const bool push = w.me.type == MEGA_MAT_VM_RATE && rate_overstress(w.spred, a.eps[i], w.me) > 0.0;
+      const bool push = a.mats[w.mi].type == MEGA_MAT_VM_RATE && rate_overstress(w.spred, a.eps[i], a.mats[w.mi]) > 0.0;
       const unsigned act = __activemask();
       const unsigned bal = __ballot_sync(act, push);
       if (bal) {
@@ -455,7 +464,7 @@ __global__ void __launch_bounds__(256, 2) k_stress(StressArgs a) {
       }
       if (push) continue;
     }
-    stress_finish<T, TS, false, DAM>(a, i, w, -1.0, work, nit, npl, st);
+    stress_finish<T, TS, FAST, DAM, FAST>(a, i, w, -1.0, work, nit, npl, st);
   }
   stress_reduce<T>(a, work, nit, npl, st, smd, smu);
 }
@@ -697,9 +706,9 @@ int launch_defgrad(cudaStream_t s, bool mixed, bool interp, int32_t n, const Dev
 }
 
 int launch_stress(cudaStream_t s, bool mixed, const StressArgs& a) {
-  const int block = 256;
+  const int block = kStressBlock;
   const int64_t need = grid_for(a.n, block);
-  const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)device_sm_count() * 8));
+  const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)device_sm_count() * (2048 / kStressBlock)));
   if (a.mlp_w2 && a.mlp_small && a.queue && a.qcount) {
     // learned start: elastic nodes finish in the first kernel, plastic
     // rate-dependent ones are queued for the network kernel
@@ -709,21 +718,24 @@ int launch_stress(cudaStream_t s, bool mixed, const StressArgs& a) {
     StressArgs qa = a;
     qa.add_g0 = 0;  // the first kernel has advanced F already
     if (a.aux) {
-      if (mixed) k_stress<float, float, true, true><<<grid, block, 0, s>>>(a);
-      else k_stress<double, double, true, true><<<grid, block, 0, s>>>(a);
+      if (mixed) k_stress<float, float, true, true, false><<<grid, block, 0, s>>>(a);
+      else k_stress<double, double, true, true, false><<<grid, block, 0, s>>>(a);
       MEGA_CHECK_LAUNCH();
       if (mixed) k_stress_queue<float, float, true><<<lgrid, kLearnBlock, 0, s>>>(qa);
       else k_stress_queue<double, double, true><<<lgrid, kLearnBlock, 0, s>>>(qa);
     } else {
-      if (mixed) k_stress<float, float, false, true><<<grid, block, 0, s>>>(a);
-      else k_stress<double, double, false, true><<<grid, block, 0, s>>>(a);
+      if (mixed) k_stress<float, float, false, true, false><<<grid, block, 0, s>>>(a);
+      else k_stress<double, double, false, true, false><<<grid, block, 0, s>>>(a);
       MEGA_CHECK_LAUNCH();
       if (mixed) k_stress_queue<float, float, false><<<lgrid, kLearnBlock, 0, s>>>(qa);
       else k_stress_queue<double, double, false><<<lgrid, kLearnBlock, 0, s>>>(qa);
     }
   } else {
-    auto k = a.aux ? (mixed ? k_stress<float, float, true, false> : k_stress<double, double, true, false>)
-                   : (mixed ? k_stress<float, float, false, false> : k_stress<double, double, false, false>);
+    const bool fast = a.finite_strain && a.more;
+    auto k = a.aux  ? (mixed ? k_stress<float, float, true, false, false> : k_stress<double, double, true, false, false>)
+             : fast ? (mixed ? k_stress<float, float, false, false, true> : k_stress<double, double, false, false, true>)
+                    : (mixed ? k_stress<float, float, false, false, false>
+                             : k_stress<double, double, false, false, false>);
     return launch_overlapped(k, grid, block, 0, s, a);
   }
   MEGA_CHECK_LAUNCH();

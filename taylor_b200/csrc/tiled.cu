@@ -913,6 +913,7 @@ __device__ __forceinline__ void prefetch_columns(const TiledForceArgs& a, int64_
   prefetch_l2(a.dsp_tot + m);
 }
 
+template <bool BODY>
 __device__ __forceinline__ void finish_columns(const TiledForceArgs& a, int64_t c0, ColumnSums& cs, unsigned st) {
   __syncthreads();
   const int tid = threadIdx.x, ndof = 3 * a.R, nw = (ndof + 31) >> 5, wid = tid >> 5;
@@ -921,7 +922,7 @@ __device__ __forceinline__ void finish_columns(const TiledForceArgs& a, int64_t 
     int body = 0;
     const int q = tid % 3;
     const int64_t J = c0 + tid / 3;
-    if (tid < ndof && J < a.n) correct_dof(a, J, q, cs.f[tid], a.has_body ? cs.e[tid] : 0.0, ke, ee, pr, body, st);
+    if (tid < ndof && J < a.n) correct_dof(a, J, q, cs.f[tid], BODY ? cs.e[tid] : 0.0, ke, ee, pr, body, st);
     double v[8] = {ke, ee, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -981,7 +982,7 @@ struct StagedT {
   __device__ __forceinline__ static TS weight(const TS* v, int j) {
     return sizeof(TS) == 8 ? v[9 + j] : (j < 16 ? v[12 + j] : v[j - 7]);
   }
-  template <int KG>
+  template <bool BODY, int KG>
   __device__ __forceinline__ void fill(const TiledForceArgs& a, const StageIds<KG>& ids, int cnt) const {
     ids.each(cnt, [&](int l, int64_t j) {
       if constexpr (sizeof(TS) == 4) {
@@ -990,7 +991,7 @@ struct StagedT {
         t.put(l, 0, x);
         t.put(l, 1, y);
         t.at(l, 8) = z.x;
-        if (a.has_body) { body[l] = z.y; body[ld + l] = z.z; body[2 * ld + l] = z.w; }
+        if (BODY) { body[l] = z.y; body[ld + l] = z.z; body[2 * ld + l] = z.w; }
         if constexpr (NS) {
           const float4* w = reinterpret_cast<const float4*>(a.ns_w) + 5 * j;
           const float4 w0 = w[0], w1 = w[1], w2 = w[2], w3 = w[3], w4 = w[4];
@@ -1020,10 +1021,10 @@ struct StagedT {
 #pragma unroll
           for (int k = 0; k < 8; ++k) t.put(l, 5 + k, make_double2(u[2 * k + 1], u[2 * k + 2]));
           t.at(l, 26) = u[17];
-          if (a.has_body) reinterpret_cast<int32_t*>(body)[l] = (int32_t)j;
+          if (BODY) reinterpret_cast<int32_t*>(body)[l] = (int32_t)j;
         } else {
           t.at(l, 8) = z[0];
-          if (a.has_body) { body[l] = z[1]; body[ld + l] = z[2]; body[2 * ld + l] = z[3]; }
+          if (BODY) { body[l] = z[1]; body[ld + l] = z[2]; body[2 * ld + l] = z[3]; }
         }
       }
     });
@@ -1039,7 +1040,9 @@ constexpr int force_blocks() {  // blocks per SM the register cap asks for (NS: 
 // NS (mixed): the NSNI stabilisation force rides along,
 // f_J += sum_i sum_q W_i(k, q) S_q(i, J) (FINT.F90:1127-1208 layout), with the
 // row weights W_i staged beside T_i.
-template <typename TS, typename A, bool F64, int KG, int KU, bool NS = false>
+// BODY: a body force (compiled apart: its sums and branches cost registers the
+// plain step has no use for).
+template <typename TS, typename A, bool F64, int KG, int KU, bool NS, bool BODY>
 __global__ void __launch_bounds__(64 * KG, force_blocks<F64, KG, KU, NS>()) k_force_t(TiledForceArgs a) {
   extern __shared__ __align__(16) double smx[];
   __shared__ ColumnSums cs;
@@ -1059,7 +1062,7 @@ __global__ void __launch_bounds__(64 * KG, force_blocks<F64, KG, KU, NS>()) k_fo
   const int nit = valid ? walk.nit : 0;
   constexpr bool kPipe = !NS && (!F64 || KU <= 2);
   int64_t p0 = 0, pend = 0;  // list positions, for the values that stay in list order
-  if (valid && a.has_body) {
+  if (valid && BODY) {
     p0 = a.colptr[J] + q;
     pend = a.colptr[J + 1];
   }
@@ -1074,7 +1077,7 @@ __global__ void __launch_bounds__(64 * KG, force_blocks<F64, KG, KU, NS>()) k_fo
     }
   }
   grid_wait();
-  sT.fill(a, ids, cnt);
+  sT.template fill<BODY>(a, ids, cnt);
   prefetch_columns(a, c0);
   __syncthreads();
   if (valid) {
@@ -1098,7 +1101,7 @@ __global__ void __launch_bounds__(64 * KG, force_blocks<F64, KG, KU, NS>()) k_fo
           f2 += (A)StagedT<TS, NS>::weight(T, 12 + c) * sq[c];
         }
       }
-      if (a.has_body) {
+      if (BODY) {
         const int64_t e = p0 + (int64_t)KG * it;
         if (e < pend) {  // (not a pad)
           const double s = a.tshp[e];
@@ -1145,7 +1148,7 @@ __global__ void __launch_bounds__(64 * KG, force_blocks<F64, KG, KU, NS>()) k_fo
       f0 += __shfl_xor_sync(gmask, f0, o);
       f1 += __shfl_xor_sync(gmask, f1, o);
       f2 += __shfl_xor_sync(gmask, f2, o);
-      if (a.has_body) {
+      if (BODY) {
         e0 += __shfl_xor_sync(gmask, e0, o);
         e1 += __shfl_xor_sync(gmask, e1, o);
         e2 += __shfl_xor_sync(gmask, e2, o);
@@ -1154,10 +1157,10 @@ __global__ void __launch_bounds__(64 * KG, force_blocks<F64, KG, KU, NS>()) k_fo
     if (q < 3) {
       const int m = 3 * (int)(J - c0) + q;
       cs.f[m] = (double)(q == 0 ? f0 : (q == 1 ? f1 : f2));
-      if (a.has_body) cs.e[m] = q == 0 ? e0 : (q == 1 ? e1 : e2);
+      if (BODY) cs.e[m] = q == 0 ? e0 : (q == 1 ? e1 : e2);
     }
   }
-  finish_columns(a, c0, cs, 0u);
+  finish_columns<BODY>(a, c0, cs, 0u);
 }
 
 // ---- record streams through the copy engine ------------------------------
@@ -1357,7 +1360,8 @@ __global__ void __launch_bounds__(64 * KG) k_force_b(TiledForceArgs a) {
   const unsigned gmask = group_mask<KG>();
   const bool valid = J < a.n;
   grid_wait();
-  sT.fill(a, ids, cnt);
+  if (a.has_body) sT.template fill<true>(a, ids, cnt);
+  else sT.template fill<false>(a, ids, cnt);
   prefetch_columns(a, c0);
   __syncthreads();
   unsigned st = 0;
@@ -1413,7 +1417,8 @@ __global__ void __launch_bounds__(64 * KG) k_force_b(TiledForceArgs a) {
       if (a.has_body) cs.e[m] = q == 0 ? b0 : (q == 1 ? b1 : b2);
     }
   }
-  finish_columns(a, c0, cs, st);
+  if (a.has_body) finish_columns<true>(a, c0, cs, st);
+  else finish_columns<false>(a, c0, cs, st);
   drain_records(bar);
 }
 
@@ -1597,15 +1602,21 @@ static int configure_defgrad(int lim) {
   return raise_smem(k_defgrad_t<double, true, false, KG, KU, true, FULL>, lim);
 }
 
+template <int KG, int KU, bool BODY>
+static int configure_force(int lim) {
+  int r = 0;
+  if ((r = raise_smem(k_force_t<float, float, false, KG, KU, false, BODY>, lim))) return r;
+  if ((r = raise_smem(k_force_t<float, float, false, KG, KU, true, BODY>, lim))) return r;
+  if ((r = raise_smem(k_force_t<double, double, true, KG, KU, false, BODY>, lim))) return r;
+  return raise_smem(k_force_t<double, double, true, KG, KU, true, BODY>, (int)StagedT<double, true>::bytes(1024, true));
+}
+
 template <int KG, int KU>
 static int configure_variant(int lim) {
   int r = 0;
   if ((r = configure_defgrad<KG, KU, false>(lim))) return r;
-  if ((r = raise_smem(k_force_t<float, float, false, KG, KU>, lim))) return r;
-  if ((r = raise_smem(k_force_t<float, float, false, KG, KU, true>, lim))) return r;
-  if ((r = raise_smem(k_force_t<double, double, true, KG, KU, true>, (int)StagedT<double, true>::bytes(1024, true))))
-    return r;
-  return raise_smem(k_force_t<double, double, true, KG, KU>, lim);
+  if ((r = configure_force<KG, KU, false>(lim))) return r;
+  return configure_force<KG, KU, true>(lim);
 }
 
 static int g_bulk_lim = kBulkSmemMax;  // what the device grants, set by configure_tiled_kernels
@@ -1753,6 +1764,12 @@ static int force_bulk(cudaStream_t s, bool mixed, const TiledForceArgs& a) {
                            smem, s, a);
 }
 
+template <int KG, int KU, bool BODY>
+static auto force_kernel(bool mixed, bool ns) {
+  return !mixed ? (ns ? k_force_t<double, double, true, KG, KU, true, BODY> : k_force_t<double, double, true, KG, KU, false, BODY>)
+                : (ns ? k_force_t<float, float, false, KG, KU, true, BODY> : k_force_t<float, float, false, KG, KU, false, BODY>);
+}
+
 template <int KG, int KU>
 static int force_variant(cudaStream_t s, bool mixed, const TiledForceArgs& a) {
   const size_t smem = !mixed ? (a.ns_scol ? StagedT<double, true>::bytes(a.maxcnt, a.has_body)
@@ -1761,10 +1778,8 @@ static int force_variant(cudaStream_t s, bool mixed, const TiledForceArgs& a) {
                                           : StagedT<float, false>::bytes(a.maxcnt, a.has_body));
   const unsigned grid = (unsigned)a.ntiles;
   const int block = a.R * KG;
-  auto k = !mixed       ? (a.ns_scol ? k_force_t<double, double, true, KG, KU, true>
-                                     : k_force_t<double, double, true, KG, KU>)
-           : a.ns_scol ? k_force_t<float, float, false, KG, KU, true>
-                       : k_force_t<float, float, false, KG, KU>;
+  auto k = force_kernel<KG, KU, false>(mixed, a.ns_scol != nullptr);
+  if (a.has_body) k = force_kernel<KG, KU, true>(mixed, a.ns_scol != nullptr);
   return launch_overlapped(k, grid, block, smem, s, a);
 }
 
