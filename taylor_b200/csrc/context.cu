@@ -107,7 +107,6 @@ __global__ void k_iperm(int32_t n, const int32_t* __restrict__ perm, int32_t* __
   const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (r < n) iperm[perm[r]] = (int32_t)r;
 }
-// dst[r*w + k] = src[perm[r]*w + k]  (gather = old -> new), element size es bytes
 __global__ void k_i32_to_f64(int64_t m, const int32_t* __restrict__ a, double* __restrict__ out) {
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (k < m) out[k] = (double)a[k];
@@ -117,14 +116,15 @@ __global__ void k_add_kernel(int64_t m, const double* __restrict__ a, const doub
   const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (k < m) out[k] = a[k] + b[k];
 }
-__global__ void k_perm_gather(int32_t n, int w, int es, const int32_t* __restrict__ perm,
-                              const unsigned char* __restrict__ src, unsigned char* __restrict__ dst) {
+// dst[r*w + k] = src[perm[r]*w + k]  (gather = old -> new).  An element moves
+// as one word of its own size, and the bound is memory.
+template <typename V>
+__global__ void k_perm_gather(int32_t n, int w, const int32_t* __restrict__ perm, const V* __restrict__ src,
+                              V* __restrict__ dst) {
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (t >= (int64_t)n * w) return;
   const int64_t r = t / w, k = t - r * w;
-  const unsigned char* a = src + ((int64_t)perm[r] * w + k) * es;
-  unsigned char* b = dst + t * es;
-  for (int q = 0; q < es; ++q) b[q] = a[q];
+  dst[t] = src[(int64_t)perm[r] * w + k];
 }
 __global__ void k_newrow_len(int32_t n, const int32_t* __restrict__ perm, const int64_t* __restrict__ rowptr0,
                              int32_t* __restrict__ len) {
@@ -174,6 +174,19 @@ __global__ void k_rowsum_pk32(int32_t n, const int64_t* __restrict__ rowptr, con
 }
 
 inline unsigned grid_for(int64_t work, int block) { return (unsigned)((work + block - 1) / block); }
+
+static int perm_gather(cudaStream_t s, int32_t n, int w, int es, const int32_t* perm, const void* src, void* dst) {
+  const unsigned grid = grid_for((int64_t)n * w, 256);
+  switch (es) {
+    case 8: k_perm_gather<<<grid, 256, 0, s>>>(n, w, perm, (const uint64_t*)src, (uint64_t*)dst); break;
+    case 4: k_perm_gather<<<grid, 256, 0, s>>>(n, w, perm, (const uint32_t*)src, (uint32_t*)dst); break;
+    case 2: k_perm_gather<<<grid, 256, 0, s>>>(n, w, perm, (const uint16_t*)src, (uint16_t*)dst); break;
+    case 1: k_perm_gather<<<grid, 256, 0, s>>>(n, w, perm, (const uint8_t*)src, (uint8_t*)dst); break;
+    default: return MEGA_ERR_ARG;
+  }
+  MEGA_CHECK_LAUNCH();
+  return 0;
+}
 
 // Worker threads for the host-side set-up loops, started once per process
 // (up to 15 besides the caller) and kept: starting threads for every loop
@@ -705,7 +718,7 @@ static int kernels_per_step(const Ctx* c, int mode = 0) {
 
 // full: F is formed from the displacements; else it advances by this step's
 // increment from where the step before left it.
-static int step_once(Ctx* c, double dt, int mode, int predict, cudaEvent_t* ev, bool full) {
+static int step_once(Ctx* c, double dt, int mode, int predict, cudaEvent_t* ev, bool full, bool load_only = false) {
   const bool mixed = (mode & 0xff) == MEGA_MODE_MIXED;
   const bool interp = (mode & MEGA_FLAG_INTERP_EACH_STEP) != 0;
   if (ev) MEGA_TRY(cudaEventRecord(ev[0], c->s));
@@ -713,8 +726,9 @@ static int step_once(Ctx* c, double dt, int mode, int predict, cudaEvent_t* ev, 
   int r = launch_defgrad_tiled(c->s, mixed, interp, c->n, c->rt, nsni_tiles(c, mixed, nt), c->csr.rowptr,
                                mixed ? c->pk32 : c->pk64, c->dsp, c->dsp_tot, mixed ? c->sdphi32 : c->sdphi,
                                c->shpb[mixed] ? c->shpb[mixed] : c->shp, c->dsp_tot_phy, c->fg, c->acc, c->status,
-                               c->var_defgrad[mixed], full);
+                               c->var_defgrad[mixed], full, load_only);
   if (r) return r;
+  if (load_only) return launch_force_tiled(c->s, mixed, force_args(c, dt, mode, predict), c->var_force[mixed], true);
   if (ev) MEGA_TRY(cudaEventRecord(ev[1], c->s));
   StressArgs sa = stress_args(c, dt, mode);
   sa.add_g0 = !full;
@@ -732,9 +746,18 @@ static int step_once(Ctx* c, double dt, int mode, int predict, cudaEvent_t* ev, 
   return 0;
 }
 
+// Rows per tile: 64, or 32 where 64 would leave more than half of the SMs
+// without a tile (one block per tile).  4,455 nodes, 70 -> 140 tiles: FP64
+// step 19.7 -> 18.9 us and 17.4 -> 15.3 tuned, with NSNI 49.2 -> 43.8 and mixed
+// NSNI 35.7 -> 33.3; 7,458 nodes, 117 tiles at 64: FP64 NSNI 53.5 -> 57.2 with
+// 32, the rest within 2 %.  16 rows gained nothing more at 957 to 3,807.
+static int32_t tile_rows(int32_t n) { return (int64_t)n <= 32 * (int64_t)device_sm_count() ? 32 : 64; }
+
 static int graph_for(Ctx* c, double dt, int mode, int len) {
   if (c->gexec && c->g_mode == mode && c->g_dt == dt && c->g_len == len) return 0;
   if (c->gexec) { cudaGraphExecDestroy(c->gexec); c->gexec = nullptr; }
+  for (int full = len > 1 ? 0 : 1; full < 2; ++full)
+    if (int r = step_once(c, dt, mode, 1, nullptr, full != 0, true)) return r;
   cudaGraph_t g = nullptr;
   MEGA_TRY(cudaStreamBeginCapture(c->s, cudaStreamCaptureModeThreadLocal));
   const int64_t before = c->launches;
@@ -1533,9 +1556,7 @@ static int permute_nodes(Ctx* c, const int32_t* map) {
   MEGA_ALLOC(tp, tmp, (int64_t)n * row_bytes);
   for (const Arr& a : list) {
     if (!a.p) continue;
-    k_perm_gather<<<grid_for((int64_t)n * a.w, 256), 256, 0, c->s>>>(n, a.w, a.es, map, (const unsigned char*)a.p,
-                                                                       tmp);
-    MEGA_CHECK_LAUNCH();
+    if (int r = perm_gather(c->s, n, a.w, a.es, map, a.p, tmp)) return r;
     MEGA_TRY(cudaMemcpyAsync(a.p, tmp, (size_t)n * a.w * a.es, cudaMemcpyDeviceToDevice, c->s));
   }
   MEGA_TRY(cudaStreamSynchronize(c->s));
@@ -1692,8 +1713,8 @@ int mega_search_and_shapes(int64_t h, int32_t* gn, int32_t* gstart, int32_t* gst
                                                                        c->csr.rowptr, c->csr.col);
     MEGA_CHECK_LAUNCH();
     if (packed) {  // the row tiles first: the records carry the tile ranks
-      if ((r = configure_tiled_kernels())) return r;
-      r = build_tiles(c->s, n, c->csr.rowptr, c->csr.col, m, c->csr.gmaxn, c->rt, c->nbpool, nullptr);
+      r = build_tiles(c->s, n, c->csr.rowptr, c->csr.col, m, c->csr.gmaxn, c->rt, c->nbpool, nullptr,
+                      tile_rows(n));
       if (r || (r = build_slices(c->s, n, c->csr.rowptr, c->rt, c->nbpool))) return r;
       float4* a = nullptr;
       MEGA_ALLOC(c->nbpool, a, c->rt.nrec);
@@ -1715,18 +1736,18 @@ int mega_search_and_shapes(int64_t h, int32_t* gn, int32_t* gstart, int32_t* gst
   tmp0.free_all();
   tr.mark("renumber");
   // 3. transposed view, tiles, packed records
-  r = configure_tiled_kernels();
-  if (r) return r;
   r = build_transpose(c->s, c->csr, c->nbpool);
   if (r) return r;
   tr.mark("transpose");
   if (!packed) {
-    r = build_tiles(c->s, n, c->csr.rowptr, c->csr.col, m, c->csr.gmaxn, c->rt, c->nbpool, nullptr);
+    r = build_tiles(c->s, n, c->csr.rowptr, c->csr.col, m, c->csr.gmaxn, c->rt, c->nbpool, nullptr,
+                      tile_rows(n));
     if (r || (r = build_slices(c->s, n, c->csr.rowptr, c->rt, c->nbpool))) return r;
   }
   tr.mark("row_tiles");
   // the longest column bounds a column tile's set from below
-  r = build_tiles(c->s, n, c->csr.colptr, c->csr.trow, m, c->csr.gmaxc, c->ct, c->nbpool, nullptr);
+  r = build_tiles(c->s, n, c->csr.colptr, c->csr.trow, m, c->csr.gmaxc, c->ct, c->nbpool, nullptr,
+                      tile_rows(n));
   if (r || (r = build_slices(c->s, n, c->csr.colptr, c->ct, c->nbpool))) return r;
   tr.mark("column_tiles");
   if (c->prec_mask & 1) {
@@ -1888,8 +1909,7 @@ static int download_nodes(Ctx* c, const void* src, int w, int es, void* dst) {
   DevPool tp(c->s);
   unsigned char* tmp = nullptr;
   MEGA_ALLOC(tp, tmp, bytes);
-  k_perm_gather<<<grid_for((int64_t)n * w, 256), 256, 0, c->s>>>(n, w, es, c->iperm, (const unsigned char*)src, tmp);
-  MEGA_CHECK_LAUNCH();
+  if (int r = perm_gather(c->s, n, w, es, c->iperm, src, tmp)) return r;
   return download_staged(c->s, dst, tmp, bytes);
 }
 
@@ -2017,12 +2037,11 @@ int mega_snapshot(int64_t h, int32_t nfields, const int32_t* fields, double* dst
         src = phy;
       }
     }
-    if (c->searched)
-      k_perm_gather<<<grid_for(n * w, 256), 256, 0, c->s>>>((int32_t)n, w, 8, c->iperm, (const unsigned char*)src,
-                                                             (unsigned char*)(out + off));
-    else
+    if (c->searched) {
+      if (int r = perm_gather(c->s, (int32_t)n, w, 8, c->iperm, src, out + off)) return r;
+    } else {
       MEGA_TRY(cudaMemcpyAsync(out + off, src, sizeof(double) * n * w, cudaMemcpyDeviceToDevice, c->s));
-    MEGA_CHECK_LAUNCH();
+    }
     off += n * w;
   }
   return download_staged(c->s, dst, out, sizeof(double) * (size_t)total);
@@ -2062,8 +2081,7 @@ int mega_upload(int64_t h, int32_t field, const double* src) {
   unsigned char* tmp = nullptr;
   MEGA_ALLOC(tp, tmp, bytes);
   MEGA_TRY(cudaMemcpyAsync(tmp, src, bytes, cudaMemcpyHostToDevice, c->s));
-  k_perm_gather<<<grid_for((int64_t)n * w, 256), 256, 0, c->s>>>(n, w, 8, c->perm, tmp, (unsigned char*)dst);
-  MEGA_CHECK_LAUNCH();
+  if (int r = perm_gather(c->s, n, w, 8, c->perm, tmp, dst)) return r;
   MEGA_TRY(cudaStreamSynchronize(c->s));
   return 0;
 }

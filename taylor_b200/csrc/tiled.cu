@@ -1427,7 +1427,7 @@ inline unsigned grid_for(int64_t work, int block) { return (unsigned)((work + bl
 }  // namespace
 
 int build_tiles(cudaStream_t s, int32_t n, const int64_t* ptr, const int32_t* idx, int64_t nnz, int32_t gmaxn,
-                TileSet& ts, DevPool& pool, int32_t* maxcnt_out) {
+                TileSet& ts, DevPool& pool, int32_t* maxcnt_out, int32_t rows) {
   constexpr int HS = 2048;
   const int32_t jmax = HS / 2;
   if (gmaxn > jmax) return MEGA_ERR_UNSUPPORTED;
@@ -1436,7 +1436,7 @@ int build_tiles(cudaStream_t s, int32_t n, const int64_t* ptr, const int32_t* id
   int32_t* ovf = nullptr;
   MEGA_ALLOC(scratch, slot_tmp, nnz);
   MEGA_ALLOC(scratch, ovf, 1);
-  for (int32_t R = 64; R >= 8; R >>= 1) {  // >= 8 keeps every block a whole warp
+  for (int32_t R = rows; R >= 8; R >>= 1) {  // >= 8 keeps every block a whole warp
     const int64_t ntiles = (n + R - 1) / R;
     int32_t *jset = nullptr, *jcnt = nullptr;
     uint16_t* lidx = nullptr;
@@ -1583,43 +1583,34 @@ constexpr int kFullKU = 2;
 // per block less room for the kernels' static shared memory (under 1 KB)
 constexpr int kBulkSmemMax = 227 * 1024 - 1024;
 
+// The dynamic shared-memory limit is raised, to the same value by every caller,
+// only for a launch that may pass 48 KB with the kernel's static part (4 KB
+// at most), and a kernel's code is loaded at its first use: raising all of them at set-up loaded all of them (20 ms of a
+// process's first search).  load_only does both ahead of a stream capture.
 template <typename K>
 static int raise_smem(K k, int lim) {
   MEGA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
   return 0;
 }
-
-template <int KG, int KU, bool FULL>
-static int configure_defgrad(int lim) {
-  int r = 0;
-  if ((r = raise_smem(k_defgrad_t<float, false, true, KG, KU, false, FULL>, lim))) return r;
-  if ((r = raise_smem(k_defgrad_t<float, false, false, KG, KU, false, FULL>, lim))) return r;
-  if ((r = raise_smem(k_defgrad_t<float, false, true, KG, KU, true, FULL>, lim))) return r;
-  if ((r = raise_smem(k_defgrad_t<float, false, false, KG, KU, true, FULL>, lim))) return r;
-  if ((r = raise_smem(k_defgrad_t<double, true, true, KG, KU, false, FULL>, lim))) return r;
-  if ((r = raise_smem(k_defgrad_t<double, true, false, KG, KU, false, FULL>, lim))) return r;
-  if ((r = raise_smem(k_defgrad_t<double, true, true, KG, KU, true, FULL>, lim))) return r;
-  return raise_smem(k_defgrad_t<double, true, false, KG, KU, true, FULL>, lim);
+template <typename... KA, typename... A>
+static int start(void (*k)(KA...), int lim, bool load_only, unsigned grid, unsigned block, size_t smem, cudaStream_t s,
+                 A&&... args) {
+  if (smem > 44 * 1024)
+    if (int r = raise_smem(k, lim)) return r;
+  if (load_only) {
+    cudaFuncAttributes fa{};
+    MEGA_TRY(cudaFuncGetAttributes(&fa, k));
+    return 0;
+  }
+  return launch_overlapped(k, grid, block, smem, s, std::forward<A>(args)...);
 }
+// A tile stages at most 1024 neighbours: 96 KB for the double-precision T_i of
+// the column gather, 120 KB for the float T_i and NSNI weights.
+static int stage_limit() { return 31 * 4 * staged_ld(1024); }
 
-template <int KG, int KU, bool BODY>
-static int configure_force(int lim) {
-  int r = 0;
-  if ((r = raise_smem(k_force_t<float, float, false, KG, KU, false, BODY>, lim))) return r;
-  if ((r = raise_smem(k_force_t<float, float, false, KG, KU, true, BODY>, lim))) return r;
-  if ((r = raise_smem(k_force_t<double, double, true, KG, KU, false, BODY>, lim))) return r;
-  return raise_smem(k_force_t<double, double, true, KG, KU, true, BODY>, (int)StagedT<double, true>::bytes(1024, true));
-}
-
-template <int KG, int KU>
-static int configure_variant(int lim) {
-  int r = 0;
-  if ((r = configure_defgrad<KG, KU, false>(lim))) return r;
-  if ((r = configure_force<KG, KU, false>(lim))) return r;
-  return configure_force<KG, KU, true>(lim);
-}
-
-static int g_bulk_lim = kBulkSmemMax;  // what the device grants, set by configure_tiled_kernels
+// what the streamed variants may ask for: the device's limit less the kernels'
+// static shared memory, raised for all of them at the first question
+static int g_bulk_lim = kBulkSmemMax;
 
 template <typename K>
 static int raise_smem_upto(K k, int lim) {
@@ -1645,23 +1636,12 @@ static int configure_bulk(int lim) {
   return raise_smem_upto(k_force_b<double, double, true, KG>, lim);
 }
 
-// Raise the dynamic shared-memory limit of the tiled kernels once (outside
-// any stream capture): a tile stages at most 1024 neighbours, 96 KB for the
-// double-precision T_i of the force kernel (120 KB for the float T_i and
-// NSNI weights); the streamed variants add the tile's records.
-int configure_tiled_kernels() {
-  static bool done = false;
-  if (done) return 0;
-  const int lim = 31 * 4 * staged_ld(1024);
-  int r = 0;
-  if ((r = configure_variant<4, 4>(lim)) || (r = configure_variant<4, 2>(lim)) ||
-      (r = configure_variant<4, 1>(lim)) || (r = configure_variant<8, 2>(lim)) ||
-      (r = configure_variant<16, 1>(lim)) || (r = configure_variant<16, 2>(lim)) ||
-      (r = configure_defgrad<4, kFullKU, true>(lim)) || (r = configure_defgrad<8, kFullKU, true>(lim)) ||
-      (r = configure_defgrad<16, kFullKU, true>(lim)) || (r = configure_bulk<4>(kBulkSmemMax)) || (r = configure_bulk<8>(kBulkSmemMax)))
-    return r;
-  done = true;
-  return 0;
+static bool bulk_fits(size_t smem) {
+  static const int r = [] {
+    const int a = configure_bulk<4>(kBulkSmemMax);
+    return a ? a : configure_bulk<8>(kBulkSmemMax);
+  }();
+  return r == 0 && smem <= (size_t)g_bulk_lim;
 }
 
 int tiled_variants() { return kVariants; }
@@ -1670,7 +1650,7 @@ bool tiled_variant_fits(const TileSet& ts, bool mixed, int variant, bool force, 
   if (variant < 0 || variant >= kVariants) return false;
   if (variant < 4 || variant > 5) return true;  // register variants
   const size_t stage = force ? (mixed ? sizeof(float) : sizeof(double)) * (has_body ? 12 : 9) : (mixed ? 16 : 24);
-  return (size_t)ts.recmax * (mixed ? 16 : 26) + stage * staged_ld(ts.maxcnt) <= (size_t)g_bulk_lim;
+  return bulk_fits((size_t)ts.recmax * (mixed ? 16 : 26) + stage * staged_ld(ts.maxcnt));
 }
 
 // one launch's arguments of the row gather
@@ -1685,18 +1665,18 @@ struct DefgradArgs {
   double *dsp_tot_phy, *fg;
   StepAccum* acc;
   unsigned* status;
+  bool load_only;
 };
 
 template <int KG>
 static int defgrad_bulk(cudaStream_t s, const DefgradArgs& d) {
   const TileSet& ts = d.ts;
   const size_t smem = (size_t)ts.recmax * (d.mixed ? 16 : 26) + (size_t)(d.mixed ? 16 : 24) * staged_ld(ts.maxcnt);
-  if (smem > (size_t)g_bulk_lim) return MEGA_ERR_UNSUPPORTED;
+  if (!bulk_fits(smem)) return MEGA_ERR_UNSUPPORTED;
   auto k = d.mixed ? (d.interp ? k_defgrad_b<float, false, true, KG> : k_defgrad_b<float, false, false, KG>)
                    : (d.interp ? k_defgrad_b<double, true, true, KG> : k_defgrad_b<double, true, false, KG>);
-  return launch_overlapped(k, (unsigned)ts.ntiles, ts.R * KG, smem, s, d.n, ts.R, ts.jmax, ts.recmax, ts.view(),
-                           d.rowptr, d.pk, ts.jset, ts.jcnt, d.dsp, d.sdphi, d.shp, d.dsp_tot_phy, d.fg, d.acc,
-                           d.status);
+  return start(k, g_bulk_lim, d.load_only, (unsigned)ts.ntiles, ts.R * KG, smem, s, d.n, ts.R, ts.jmax, ts.recmax,
+               ts.view(), d.rowptr, d.pk, ts.jset, ts.jcnt, d.dsp, d.sdphi, d.shp, d.dsp_tot_phy, d.fg, d.acc, d.status);
 }
 
 template <int KG, int KU, bool FULL = false>
@@ -1712,8 +1692,8 @@ static int defgrad_variant(cudaStream_t s, const DefgradArgs& d) {
                                 : k_defgrad_t<float, false, false, KG, KU, true, FULL>)
                     : (d.interp ? k_defgrad_t<float, false, true, KG, KU, false, FULL>
                                 : k_defgrad_t<float, false, false, KG, KU, false, FULL>);
-  return launch_overlapped(k, (unsigned)ts.ntiles, ts.R * KG, smem, s, d.n, ts.R, ts.jmax, nz, ts.view(), d.rowptr,
-                           d.pk, ts.jset, ts.jcnt, d.dsp, d.dsp_tot, d.sdphi, d.shp, d.dsp_tot_phy, d.fg, d.acc);
+  return start(k, stage_limit(), d.load_only, (unsigned)ts.ntiles, ts.R * KG, smem, s, d.n, ts.R, ts.jmax, nz, ts.view(),
+               d.rowptr, d.pk, ts.jset, ts.jcnt, d.dsp, d.dsp_tot, d.sdphi, d.shp, d.dsp_tot_phy, d.fg, d.acc);
 }
 
 // NSNI runs the register variants: mixed refuses the streamed ones, FP64 takes
@@ -1727,10 +1707,11 @@ static bool ns_variant(bool mixed, int& variant) {
 int launch_defgrad_tiled(cudaStream_t s, bool mixed, bool interp, int32_t n, const TileSet& ts,
                          const NsniTiles* ns, const int64_t* rowptr, const void* pk, const double* dsp,
                          const double* dsp_tot, const double* sdphi, const double* shp, double* dsp_tot_phy,
-                         double* fg, StepAccum* acc, unsigned* status, int variant, bool full) {
+                         double* fg, StepAccum* acc, unsigned* status, int variant, bool full, bool load_only) {
   int r = 0;
   if (ns && !ns_variant(mixed, variant)) return MEGA_ERR_UNSUPPORTED;
-  const DefgradArgs d{mixed, interp, n, ts, ns, rowptr, pk, dsp, dsp_tot, sdphi, shp, dsp_tot_phy, fg, acc, status};
+  const DefgradArgs d{mixed, interp, n, ts, ns, rowptr, pk, dsp, dsp_tot, sdphi, shp, dsp_tot_phy, fg, acc, status,
+                      load_only};
   if (full) {
     if (variant == 6 || variant == 7) r = defgrad_variant<16, kFullKU, true>(s, d);
     else if (variant == 3 || variant == 5) r = defgrad_variant<8, kFullKU, true>(s, d);
@@ -1753,15 +1734,15 @@ int launch_defgrad_tiled(cudaStream_t s, bool mixed, bool interp, int32_t n, con
 }
 
 template <int KG>
-static int force_bulk(cudaStream_t s, bool mixed, const TiledForceArgs& a) {
+static int force_bulk(cudaStream_t s, bool mixed, const TiledForceArgs& a, bool load_only) {
   const int nv = a.has_body ? 12 : 9;
   const size_t smem = (size_t)a.recmax * (mixed ? 16 : 26) + (mixed ? sizeof(float) : sizeof(double)) * nv *
                       staged_ld(a.maxcnt);
-  if (smem > (size_t)g_bulk_lim) return MEGA_ERR_UNSUPPORTED;
+  if (!bulk_fits(smem)) return MEGA_ERR_UNSUPPORTED;
   const unsigned grid = (unsigned)a.ntiles;
   const int block = a.R * KG;
-  return launch_overlapped(mixed ? k_force_b<float, float, false, KG> : k_force_b<double, double, true, KG>, grid, block,
-                           smem, s, a);
+  return start(mixed ? k_force_b<float, float, false, KG> : k_force_b<double, double, true, KG>, g_bulk_lim, load_only,
+               grid, block, smem, s, a);
 }
 
 template <int KG, int KU, bool BODY>
@@ -1771,7 +1752,7 @@ static auto force_kernel(bool mixed, bool ns) {
 }
 
 template <int KG, int KU>
-static int force_variant(cudaStream_t s, bool mixed, const TiledForceArgs& a) {
+static int force_variant(cudaStream_t s, bool mixed, const TiledForceArgs& a, bool load_only) {
   const size_t smem = !mixed ? (a.ns_scol ? StagedT<double, true>::bytes(a.maxcnt, a.has_body)
                                           : StagedT<double, false>::bytes(a.maxcnt, a.has_body))
                              : (a.ns_scol ? StagedT<float, true>::bytes(a.maxcnt, a.has_body)
@@ -1780,21 +1761,22 @@ static int force_variant(cudaStream_t s, bool mixed, const TiledForceArgs& a) {
   const int block = a.R * KG;
   auto k = force_kernel<KG, KU, false>(mixed, a.ns_scol != nullptr);
   if (a.has_body) k = force_kernel<KG, KU, true>(mixed, a.ns_scol != nullptr);
-  return launch_overlapped(k, grid, block, smem, s, a);
+  const int lim = !mixed && a.ns_scol ? (int)StagedT<double, true>::bytes(1024, true) : stage_limit();
+  return start(k, lim, load_only, grid, block, smem, s, a);
 }
 
-int launch_force_tiled(cudaStream_t s, bool mixed, const TiledForceArgs& a, int variant) {
+int launch_force_tiled(cudaStream_t s, bool mixed, const TiledForceArgs& a, int variant, bool load_only) {
   int r = 0;
   if (a.ns_scol && !ns_variant(mixed, variant)) return MEGA_ERR_UNSUPPORTED;
   switch (variant) {
-    case 1: r = force_variant<4, 2>(s, mixed, a); break;
-    case 2: r = force_variant<4, 1>(s, mixed, a); break;
-    case 3: r = force_variant<8, 2>(s, mixed, a); break;
-    case 6: r = force_variant<16, 1>(s, mixed, a); break;
-    case 7: r = force_variant<16, 2>(s, mixed, a); break;
-    case 4: r = force_bulk<4>(s, mixed, a); break;
-    case 5: r = force_bulk<8>(s, mixed, a); break;
-    default: r = force_variant<4, 4>(s, mixed, a);
+    case 1: r = force_variant<4, 2>(s, mixed, a, load_only); break;
+    case 2: r = force_variant<4, 1>(s, mixed, a, load_only); break;
+    case 3: r = force_variant<8, 2>(s, mixed, a, load_only); break;
+    case 6: r = force_variant<16, 1>(s, mixed, a, load_only); break;
+    case 7: r = force_variant<16, 2>(s, mixed, a, load_only); break;
+    case 4: r = force_bulk<4>(s, mixed, a, load_only); break;
+    case 5: r = force_bulk<8>(s, mixed, a, load_only); break;
+    default: r = force_variant<4, 4>(s, mixed, a, load_only);
   }
   if (r) return r;
   MEGA_CHECK_LAUNCH();

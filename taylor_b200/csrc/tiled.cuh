@@ -79,10 +79,10 @@ struct TiledForceArgs {
   unsigned* status;
 };
 
-// Tiles of R consecutive rows of (ptr, idx), R halved from 64 down to 8
+// Tiles of R consecutive rows of (ptr, idx), R halved from `rows` down to 8
 // until every tile's neighbour set fits jmax = 1024.
 int build_tiles(cudaStream_t s, int32_t n, const int64_t* ptr, const int32_t* idx, int64_t nnz, int32_t gmaxn,
-                TileSet& ts, DevPool& pool, int32_t* maxcnt_out);
+                TileSet& ts, DevPool& pool, int32_t* maxcnt_out, int32_t rows = 64);
 // The record layout of ts (row order, slices, record bases) into pool.
 int build_slices(cudaStream_t s, int32_t n, const int64_t* ptr, TileSet& ts, DevPool& pool);
 // records of ts.nrec entries in the slice layout: (gradient of entry pos[e],
@@ -114,7 +114,6 @@ int pack_second(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* ptr
                 bool f64, void* out);
 int gather_second(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* ptr, const int64_t* pos, bool f64,
                   const void* in, void* out);
-int configure_tiled_kernels();
 // launch variants of the two gathers: lanes per row x records in flight
 // (register streams, variants 0-3 and 6, 7), and lanes per row with the
 // tile's records streamed into shared memory by the copy engine (variants
@@ -127,11 +126,13 @@ bool tiled_variant_fits(const TileSet& ts, bool mixed, int variant, bool force, 
 // ns: the NSNI H gather rides along (register variants; FP64 takes those of
 // the same lanes per row for 4 and 5, mixed refuses them).
 // full: F - I as well as G0 (else the stress update adds G0 to F - I)
+// load_only: nothing is launched; the kernel the call would launch is loaded,
+// so that a stream capture finds it ready
 int launch_defgrad_tiled(cudaStream_t s, bool mixed, bool interp, int32_t n, const TileSet& ts,
                          const NsniTiles* ns, const int64_t* rowptr, const void* pk, const double* dsp,
                          const double* dsp_tot,
                          const double* sdphi, const double* shp, double* dsp_tot_phy, double* fg, StepAccum* acc,
-                         unsigned* status, int variant, bool full);
-int launch_force_tiled(cudaStream_t s, bool mixed, const TiledForceArgs& a, int variant = 0);
+                         unsigned* status, int variant, bool full, bool load_only = false);
+int launch_force_tiled(cudaStream_t s, bool mixed, const TiledForceArgs& a, int variant = 0, bool load_only = false);
 
 }  // namespace mega
