@@ -289,7 +289,7 @@ struct PmbArgs {
   const int64_t* rowptr;
   const int32_t* jset;    // per tile: the sorted neighbour set
   const int32_t* jcnt;
-  const uint16_t* lidx;   // per bond: rank of its neighbour in the tile's set
+  const uint16_t* lidx;   // per bond: rank of its neighbour in the tile's set (float: k_pmb_order's lt)
   uint32_t* broken;       // bit per bond
   const double* vol;
   const double* X;        // reference positions (double-precision bond geometry)
@@ -303,140 +303,27 @@ struct PmbArgs {
   double inv_rho;
   double dt;
   unsigned long long* nbroken;
+  // the float path's reference positions (k_pmb_split); lengths there are in units of 1/scale
+  const float4* hi;   // hi and lo.z
+  const float2* lo;   // lo.x, lo.y
+  const float* cvol;  // c vol
+  const double* scale;
 };
 
-// T = per-bond arithmetic: float (the mixed path: float bond geometry and
-// force, the bond vector rounded from the double difference of X and the
-// displacements from float offsets to the tile's first particle) or double
-// (the oracle's arithmetic, from X and u, for exact parity checks).
-//
-// FP64 rows are padded to multiples of 4 bonds (pads point at the particle
-// itself and start broken), so a lane reads the ranks of 4 consecutive bonds
-// as one 8-byte load and their 4 broken bits from one 32-bit word; the float
-// path, bound by its shared-memory gathers rather than by these loads, keeps
-// unpadded rows and one bond per load.
 constexpr int kGP = 8;  // lanes per particle of the bond loop
 
+// sum of the eight lanes, then one lane per component: this step's corrector
+// and the next one's predictor
 template <typename T>
-__global__ void __launch_bounds__(512) k_pmb_step(PmbArgs a) {
-  extern __shared__ double smp[];
-  const int64_t t = blockIdx.x;
-  const int cnt = a.jcnt[t];
-  const int32_t* js = a.jset + t * (int64_t)a.jmax;
-  const bool f64 = sizeof(T) == sizeof(double);
-  // staged set: FP64 7 arrays of one double per rank (X, u, vol); float: X as
-  // 3 doubles (the bond vector is rounded from the exact difference, as the
-  // FP64 path forms it: float offsets of X put 1e-6 of the bond length into
-  // the stretch and move the break of near-critical bonds), one array per
-  // axis so that the eight lanes of a particle, reading neighbours of
-  // consecutive rank, read consecutive words (fewer bank conflicts than
-  // 24-byte records), and one float4 (u - u_r0, vol)
-  double* sd = smp;
-  float4* sf = reinterpret_cast<float4*>(smp + ((3 * cnt + 1) & ~1));
-  const int64_t r0 = t * a.R;
-  const double ur0 = a.u_in[3 * r0], ur1 = a.u_in[3 * r0 + 1], ur2 = a.u_in[3 * r0 + 2];
-  for (int l = threadIdx.x; l < cnt; l += blockDim.x) {
-    const int64_t g = js[l];
-    const double x0 = a.X[3 * g], x1 = a.X[3 * g + 1], x2 = a.X[3 * g + 2];
-    const double u0 = a.u_in[3 * g], u1 = a.u_in[3 * g + 1], u2 = a.u_in[3 * g + 2];
-    const double v = a.vol[g];
-    if (f64) {  // one array per value: lanes with distinct ranks mod 16 read distinct bank pairs
-      sd[l] = x0; sd[cnt + l] = x1; sd[2 * cnt + l] = x2;
-      sd[3 * cnt + l] = u0; sd[4 * cnt + l] = u1; sd[5 * cnt + l] = u2; sd[6 * cnt + l] = v;
-    } else {
-      sd[l] = x0; sd[cnt + l] = x1; sd[2 * cnt + l] = x2;
-      sf[l] = make_float4((float)(u0 - ur0), (float)(u1 - ur1), (float)(u2 - ur2), (float)v);
-    }
-  }
-  __syncthreads();
-  const int64_t i = t * a.R + threadIdx.x / kGP;
-  const int q = threadIdx.x & (kGP - 1);
-  const unsigned gm = 0xFFu << (threadIdx.x & 24);
-  if (threadIdx.x / kGP >= a.R || i >= a.n) return;
-  const double ui0 = a.u_in[3 * i], ui1 = a.u_in[3 * i + 1], ui2 = a.u_in[3 * i + 2];
-  const double Xi0 = a.X[3 * i], Xi1 = a.X[3 * i + 1], Xi2 = a.X[3 * i + 2];
-  const float fu0 = (float)(ui0 - ur0), fu1 = (float)(ui1 - ur1), fu2 = (float)(ui2 - ur2);
-  T f0 = T(0), f1 = T(0), f2 = T(0);
-  unsigned nb = 0;
-  const T c = (T)a.c, sc = (T)a.s_c;
-  constexpr int GB = sizeof(T) == sizeof(double) ? 4 : 1;  // bonds per load group
-  constexpr int NQ = GB == 4 ? 2 : 4;                          // groups in flight per lane
-  const int64_t p1 = a.rowptr[i + 1];
-  for (int64_t pb = a.rowptr[i] + GB * q; pb < p1; pb += GB * kGP * NQ) {
-    uint32_t lw[NQ][2];
-    uint32_t wd[NQ];
-#pragma unroll
-    for (int g = 0; g < NQ; ++g) {
-      const int64_t p = pb + GB * kGP * g;
-      lw[g][0] = lw[g][1] = 0u;
-      if (p < p1) {
-        if (GB == 4) {
-          const uint2 v = *reinterpret_cast<const uint2*>(a.lidx + p);
-          lw[g][0] = v.x; lw[g][1] = v.y;
-        } else {
-          lw[g][0] = a.lidx[p];
-        }
-        wd[g] = a.broken[p >> 5] >> (p & 31);
-      } else {
-        wd[g] = 0xFu;  // past the row: skipped
-      }
-    }
-#pragma unroll
-    for (int g = 0; g < NQ; ++g)
-#pragma unroll
-      for (int u = 0; u < GB; ++u) {
-        if ((wd[g] >> u) & 1u) continue;  // broken (or a pad)
-        const int64_t p = pb + GB * kGP * g + u;
-        const int lj = (int)((lw[g][u >> 1] >> (16 * (u & 1))) & 0xFFFFu);
-        T s, e0, e1, e2, l, vj;
-        if (f64) {
-          // the oracle's arithmetic: xi from X, eta = xi + (u_j - u_i), s = (|eta| - |xi|)/|xi|
-          const double* d = sd + lj;  // value k of rank lj at d[k cnt]
-          const double x0 = d[0] - Xi0, x1 = d[cnt] - Xi1, x2 = d[2 * cnt] - Xi2;
-          const double L0d = sqrt(x0 * x0 + x1 * x1 + x2 * x2);
-          if (L0d == 0.0) continue;  // the particle itself
-          e0 = (T)(x0 + (d[3 * cnt] - ui0));
-          e1 = (T)(x1 + (d[4 * cnt] - ui1));
-          e2 = (T)(x2 + (d[5 * cnt] - ui2));
-          const T L0 = (T)L0d;
-          l = (T)sqrt((double)(e0 * e0 + e1 * e1 + e2 * e2));
-          s = (l - L0) / L0;
-          vj = (T)d[6 * cnt];
-        } else {
-          const float4 ua = sf[lj];
-          const float x0 = (float)(sd[lj] - Xi0), x1 = (float)(sd[cnt + lj] - Xi1), x2 = (float)(sd[2 * cnt + lj] - Xi2);
-          const float xx = x0 * x0 + x1 * x1 + x2 * x2;
-          if (xx == 0.f) continue;  // the particle itself
-          const float d0 = ua.x - fu0, d1 = ua.y - fu1, d2 = ua.z - fu2;
-          // stretch without cancellation: (|xi+d|^2 - |xi|^2) / (|xi| (|xi+d| + |xi|)),
-          // lengths from the hardware reciprocal square root (about 2 ulp)
-          const float f_e0 = x0 + d0, f_e1 = x1 + d1, f_e2 = x2 + d2;
-          const float ee = f_e0 * f_e0 + f_e1 * f_e1 + f_e2 * f_e2;
-          const float rL0 = rsqrtf(xx), rl = rsqrtf(ee);
-          const float fL0 = xx * rL0, fl = ee * rl;
-          const float num = 2.f * (x0 * d0 + x1 * d1 + x2 * d2) + (d0 * d0 + d1 * d1 + d2 * d2);
-          s = (T)(num * rL0 * __frcp_rn(fl + fL0));
-          // eta / |eta| directly, so the force weight needs no division
-          e0 = (T)(f_e0 * rl); e1 = (T)(f_e1 * rl); e2 = (T)(f_e2 * rl);
-          l = T(1);
-          vj = (T)ua.w;
-        }
-        if (s > sc) {
-          atomicOr(&a.broken[p >> 5], 1u << (p & 31));
-          ++nb;
-          continue;
-        }
-        const T w = f64 ? c * s * vj / l : c * s * vj;  // the float path's eta is already unit
-        f0 += w * e0; f1 += w * e1; f2 += w * e2;
-      }
-  }
+__device__ __forceinline__ void pmb_finish(const PmbArgs& a, int64_t i, int q, unsigned gm, T f0, T f1, T f2,
+                                           unsigned nb) {
 #pragma unroll
   for (int o = 1; o < kGP; o <<= 1) {
     f0 += __shfl_xor_sync(gm, f0, o);
     f1 += __shfl_xor_sync(gm, f1, o);
     f2 += __shfl_xor_sync(gm, f2, o);
-    nb += __shfl_xor_sync(gm, nb, o);
   }
+  if (nb && a.nbroken) atomicAdd(a.nbroken, (unsigned long long)nb);
   if (q < 3) {
     const int64_t m = 3 * i + q;
     const double f = (double)(q == 0 ? f0 : (q == 1 ? f1 : f2));
@@ -454,7 +341,224 @@ __global__ void __launch_bounds__(512) k_pmb_step(PmbArgs a) {
     }
     a.u_out[m] = u;
   }
-  if (q == 0 && nb && a.nbroken) atomicAdd(a.nbroken, (unsigned long long)nb);
+}
+
+// FP64 is the oracle's arithmetic, from X and u, for exact parity checks.  Its
+// rows are padded to multiples of 4 bonds (pads point at the particle itself
+// and start broken), so a lane reads the ranks of 4 consecutive bonds as one
+// 8-byte load and their 4 broken bits from one 32-bit word.
+__global__ void __launch_bounds__(512) k_pmb_step_f64(PmbArgs a) {
+  extern __shared__ double smp[];
+  const int64_t t = blockIdx.x;
+  const int cnt = a.jcnt[t];
+  const int32_t* js = a.jset + t * (int64_t)a.jmax;
+  // one array per value: lanes with distinct ranks mod 16 read distinct bank pairs
+  double* sd = smp;
+  for (int l = threadIdx.x; l < cnt; l += blockDim.x) {
+    const int64_t g = js[l];
+    sd[l] = a.X[3 * g]; sd[cnt + l] = a.X[3 * g + 1]; sd[2 * cnt + l] = a.X[3 * g + 2];
+    sd[6 * cnt + l] = a.vol[g];
+  }
+  grid_wait();
+  for (int l = threadIdx.x; l < cnt; l += blockDim.x) {
+    const int64_t g = js[l];
+    sd[3 * cnt + l] = a.u_in[3 * g]; sd[4 * cnt + l] = a.u_in[3 * g + 1]; sd[5 * cnt + l] = a.u_in[3 * g + 2];
+  }
+  __syncthreads();
+  const int64_t i = t * a.R + threadIdx.x / kGP;
+  const int q = threadIdx.x & (kGP - 1);
+  const unsigned gm = 0xFFu << (threadIdx.x & 24);
+  if (threadIdx.x / kGP >= a.R || i >= a.n) return;
+  const double ui0 = a.u_in[3 * i], ui1 = a.u_in[3 * i + 1], ui2 = a.u_in[3 * i + 2];
+  const double Xi0 = a.X[3 * i], Xi1 = a.X[3 * i + 1], Xi2 = a.X[3 * i + 2];
+  double f0 = 0.0, f1 = 0.0, f2 = 0.0;
+  unsigned nb = 0;
+  const double c = a.c, sc = a.s_c;
+  constexpr int GB = 4;  // bonds per load group
+  constexpr int NQ = 2;  // groups in flight per lane
+  const int64_t p1 = a.rowptr[i + 1];
+  for (int64_t pb = a.rowptr[i] + GB * q; pb < p1; pb += GB * kGP * NQ) {
+    uint32_t lw[NQ][2];
+    uint32_t wd[NQ];
+#pragma unroll
+    for (int g = 0; g < NQ; ++g) {
+      const int64_t p = pb + GB * kGP * g;
+      lw[g][0] = lw[g][1] = 0u;
+      if (p < p1) {
+        const uint2 v = *reinterpret_cast<const uint2*>(a.lidx + p);
+        lw[g][0] = v.x; lw[g][1] = v.y;
+        wd[g] = a.broken[p >> 5] >> (p & 31);
+      } else {
+        wd[g] = 0xFu;  // past the row: skipped
+      }
+    }
+#pragma unroll
+    for (int g = 0; g < NQ; ++g)
+#pragma unroll
+      for (int u = 0; u < GB; ++u) {
+        if ((wd[g] >> u) & 1u) continue;  // broken (or a pad)
+        const int64_t p = pb + GB * kGP * g + u;
+        // xi from X, eta = xi + (u_j - u_i), s = (|eta| - |xi|)/|xi|; value k of rank lj at d[k cnt]
+        const double* d = sd + (int)((lw[g][u >> 1] >> (16 * (u & 1))) & 0xFFFFu);
+        const double x0 = d[0] - Xi0, x1 = d[cnt] - Xi1, x2 = d[2 * cnt] - Xi2;
+        const double L0 = sqrt(x0 * x0 + x1 * x1 + x2 * x2);
+        if (L0 == 0.0) continue;  // the particle itself
+        const double e0 = x0 + (d[3 * cnt] - ui0), e1 = x1 + (d[4 * cnt] - ui1), e2 = x2 + (d[5 * cnt] - ui2);
+        const double l = sqrt(e0 * e0 + e1 * e1 + e2 * e2);
+        const double s = (l - L0) / L0;
+        if (s > sc) {
+          atomicOr(&a.broken[p >> 5], 1u << (p & 31));
+          ++nb;
+          continue;
+        }
+        const double w = c * s * d[6 * cnt] / l;
+        f0 += w * e0; f1 += w * e1; f2 += w * e2;
+      }
+  }
+  pmb_finish(a, i, q, gm, f0, f1, f2, nb);
+}
+
+// E = max |X - X of particle 0| over the finite coordinates (its bits, which
+// order like the values); then X in units of 2^k >= E as a sum of two floats:
+// hi, a multiple of 2^-22 below 2 in magnitude, so that the difference of two
+// is exact, and lo, the rest.  hi_j - hi_i + (lo_j - lo_i) is then the double
+// difference rounded to float, as long bonds as short, without a conversion.
+__global__ void k_pmb_extent(int32_t n, const double* __restrict__ X, unsigned long long* __restrict__ ext) {
+  const int64_t m = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  double e = m < 3 * (int64_t)n ? fabs(X[m] - X[m % 3]) : 0.0;
+  if (!(e < 1e300)) e = 0.0;
+  unsigned long long b = (unsigned long long)__double_as_longlong(e);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) b = max(b, __shfl_xor_sync(0xffffffffu, b, o));
+  if ((threadIdx.x & 31) == 0 && b) atomicMax(ext, b);
+}
+__global__ void k_pmb_split(int32_t n, const double* __restrict__ X, const double* __restrict__ vol, double c,
+                            const unsigned long long* __restrict__ ext, double* __restrict__ scale,
+                            float4* __restrict__ hi, float2* __restrict__ lo, float* __restrict__ cvol) {
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double E = __longlong_as_double((long long)*ext);
+  const double sg = E > 0.0 ? scalbn(1.0, -(ilogb(E) + 1)) : 1.0;  // E sg in [1/2, 1)
+  if (i == 0) *scale = sg;
+  float h[3], r[3];
+  for (int k = 0; k < 3; ++k) {
+    const double x = (X[3 * i + k] - X[k]) * sg;
+    const double d = rint(x * 4194304.0) * (1.0 / 4194304.0);
+    h[k] = (float)d;
+    r[k] = (float)(x - d);
+  }
+  hi[i] = make_float4(h[0], h[1], h[2], r[2]);
+  lo[i] = make_float2(r[0], r[1]);
+  cvol[i] = (float)(c * vol[i]);
+}
+
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float rcp_ftz(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// The mixed path: float bond geometry and force.  Per bond 2 bytes come from
+// memory; the bound is the SM itself: shared-memory gathers (L1 80 % busy) and
+// instructions (76 % of the issue slots).  So a rank's 10 values lie in two
+// 16-byte vectors and one of 8, the eight bonds read together lie in different
+// banks (k_pmb_order), a lane's four ranks of a pass come as one load ahead of
+// the pass, dead bonds are predicated off instead of branched around, and the
+// positions are sums of floats instead of doubles converted per bond.
+// 320 k particles of 96 bonds: 174 -> 114 us a step (FP64 positions, row order,
+// one 2-byte rank per load before); 19,600 particles 19.3 -> 9.6 us with the
+// launches overlapped.  40 registers for three blocks an SM: with 56 and two
+// blocks 140 us, with 32 and four (spills) 139 us.
+__global__ void __launch_bounds__(512, 3) k_pmb_step_f32(PmbArgs a) {
+  extern __shared__ __align__(16) float4 sma[];
+  const int64_t t = blockIdx.x;
+  const int cnt = a.jcnt[t];
+  const int32_t* js = a.jset + t * (int64_t)a.jmax;
+  float4* sa = sma;                                        // hi, lo.z
+  float4* sb = sma + cnt;                                  // u - u_r0, c vol
+  float2* sc2 = reinterpret_cast<float2*>(sma + 2 * cnt);  // lo.x, lo.y
+  const double sg = *a.scale;
+  for (int l = threadIdx.x; l < cnt; l += blockDim.x) {
+    const int64_t g = js[l];
+    sa[l] = a.hi[g];
+    sc2[l] = a.lo[g];
+  }
+  const int64_t i = t * a.R + threadIdx.x / kGP;
+  const int q = threadIdx.x & (kGP - 1);
+  const unsigned gm = 0xFFu << (threadIdx.x & 24);
+  const bool mine = threadIdx.x / kGP < a.R && i < a.n;
+  // rows start at multiples of 32 bonds: np passes of 32, one word of dead bits
+  // and four ranks a lane each
+  const int w0 = mine ? (int)(a.rowptr[i] >> 5) : 0;
+  const int np = mine ? (int)(a.rowptr[i + 1] >> 5) - w0 : 0;
+  const uint2* rk = reinterpret_cast<const uint2*>(a.lidx);
+  const float4 hi = mine ? a.hi[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float2 lo = mine ? a.lo[i] : make_float2(0.f, 0.f);
+  uint2 rn = np > 0 ? rk[8 * (int64_t)w0 + q] : make_uint2(0u, 0u);
+  grid_wait();
+  unsigned dn = np > 0 ? a.broken[w0] : ~0u;
+  const int64_t r0 = t * a.R;
+  const double ur0 = a.u_in[3 * r0], ur1 = a.u_in[3 * r0 + 1], ur2 = a.u_in[3 * r0 + 2];
+  for (int l = threadIdx.x; l < cnt; l += blockDim.x) {
+    const int64_t g = js[l];
+    sb[l] = make_float4((float)((a.u_in[3 * g] - ur0) * sg), (float)((a.u_in[3 * g + 1] - ur1) * sg),
+                        (float)((a.u_in[3 * g + 2] - ur2) * sg), a.cvol[g]);
+  }
+  float fu0 = 0.f, fu1 = 0.f, fu2 = 0.f;
+  if (mine) {
+    fu0 = (float)((a.u_in[3 * i] - ur0) * sg);
+    fu1 = (float)((a.u_in[3 * i + 1] - ur1) * sg);
+    fu2 = (float)((a.u_in[3 * i + 2] - ur2) * sg);
+  }
+  __syncthreads();
+  const float sc = (float)a.s_c;
+  float f0 = 0.f, f1 = 0.f, f2 = 0.f;
+  unsigned nb = 0;
+  const int nmax = __reduce_max_sync(0xffffffffu, np);  // the warp stays together
+  for (int k = 0; k < nmax; ++k) {
+    const uint2 rc = rn;
+    const unsigned live = ~dn >> q;
+    const int ng = __reduce_max_sync(0xffffffffu, (39 - __clz(~dn)) >> 3);  // groups of 8 with a live bond
+    rn = make_uint2(0u, 0u);
+    dn = ~0u;
+    if (k + 1 < np) {
+      rn = rk[8 * (int64_t)(w0 + k + 1) + q];
+      dn = a.broken[w0 + k + 1];
+    }
+    unsigned cut = 0;
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      if (g >= ng) break;
+      const int lj = (int)(((g < 2 ? rc.x : rc.y) >> (16 * (g & 1))) & 0xFFFFu);
+      const float4 A = sa[lj], B = sb[lj];
+      const float2 C = sc2[lj];
+      const float x0 = (A.x - hi.x) + (C.x - lo.x), x1 = (A.y - hi.y) + (C.y - lo.y),
+                  x2 = (A.z - hi.z) + (A.w - hi.w);
+      const float d0 = B.x - fu0, d1 = B.y - fu1, d2 = B.z - fu2;
+      const float e0 = x0 + d0, e1 = x1 + d1, e2 = x2 + d2;
+      const float xx = x0 * x0 + x1 * x1 + x2 * x2, ee = e0 * e0 + e1 * e1 + e2 * e2;
+      // stretch without cancellation: (|eta|^2 - |xi|^2) / (|xi| (|eta| + |xi|)),
+      // lengths from the hardware reciprocal square root (about 2 ulp)
+      const float num = d0 * (x0 + e0) + d1 * (x1 + e1) + d2 * (x2 + e2);
+      const float rl = rsqrt_ftz(ee);
+      const float s = num * rcp_ftz(xx + (xx * rsqrt_ftz(xx)) * (ee * rl));
+      const bool on = (live & (1u << (8 * g))) && xx != 0.f;  // else broken, a pad or the particle itself
+      const bool over = s > sc;
+      const float w = (s * B.w) * rl;
+      if (on && over) cut |= 1u << (8 * g);
+      if (on && !over) { f0 += w * e0; f1 += w * e1; f2 += w * e2; }
+    }
+    if (cut) {
+      atomicOr(&a.broken[w0 + k], cut << q);
+      nb += __popc(cut);
+    }
+  }
+  if (mine) pmb_finish(a, i, q, gm, f0, f1, f2, nb);
 }
 
 // ---- renumbering of the particles in bin-cell order
@@ -497,44 +601,106 @@ __global__ void k_pmb_padbits(int32_t n, const int32_t* __restrict__ perm, const
   const int64_t len = rowptr0[perm[r] + 1] - rowptr0[perm[r]];
   for (int64_t p = rowptr1[r] + len; p < rowptr1[r + 1]; ++p) atomicOr(&bits[p >> 5], 1u << (p & 31));
 }
-// per-bond flags between the two orders: new entry rowptr1[r] + k is old
-// entry rowptr0[perm[r]] + k.  to_new: old bytes -> new bits (OR); else new
-// bits -> old bytes.
-__global__ void k_pmb_flags(int32_t n, const int32_t* __restrict__ perm, const int64_t* __restrict__ rowptr0,
-                            const int64_t* __restrict__ rowptr1, uint32_t* __restrict__ bits,
-                            uint8_t* __restrict__ bytes, bool to_new) {
+// The mixed rows' order: the eight bonds that a particle's lanes read together
+// (slots 8 g .. 8 g + 7) have ranks of different remainders mod 8, as far as the
+// row has them, so their 16-byte vectors lie in different banks.  With the
+// bonds sorted by remainder, number t goes to group t mod G of the row's G: a
+// remainder's run is dealt round, each group at most ceil(run / G) of it.
+// col2 and kpos (the entry's place in the row before, 0xFFFF: pad) are in slot
+// order, as are the dead bits; lt holds the four ranks of each lane of a pass of
+// 32 slots side by side.  Warp per row; rows start at multiples of 32 slots.
+__global__ void k_pmb_order(int32_t n, const int32_t* __restrict__ perm, const int64_t* __restrict__ rowptr0,
+                            const int64_t* __restrict__ rowptr1, const int32_t* __restrict__ col,
+                            const uint16_t* __restrict__ lidx, int32_t* __restrict__ col2,
+                            uint16_t* __restrict__ lt, uint16_t* __restrict__ kpos, uint32_t* __restrict__ bits) {
   const int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (r >= n) return;
-  const int64_t a0 = rowptr0[perm[r]], len = rowptr0[perm[r] + 1] - a0, b0 = rowptr1[r];
-  for (int64_t k = lane; k < len; k += 32) {
-    const int64_t p = b0 + k;
+  const int64_t b0 = rowptr1[r];
+  const int len = (int)(rowptr0[perm[r] + 1] - rowptr0[perm[r]]), lp = (int)(rowptr1[r + 1] - b0);
+  const int G = (len + 7) / 8;
+  int cnt = 0;  // lane j < 8: bonds of remainder j
+  for (int k0 = 0; k0 < len; k0 += 32) {
+    const int b = k0 + lane < len ? lidx[b0 + k0 + lane] & 7 : 8;
+    for (int j = 0; j < 8; ++j) {
+      const unsigned m = __ballot_sync(0xffffffffu, b == j);
+      if (lane == j) cnt += __popc(m);
+    }
+  }
+  int next = 0;  // the number of remainder j's next bond
+  for (int j = 0; j < 7; ++j) {
+    const int c = __shfl_sync(0xffffffffu, cnt, j);
+    if (lane > j) next += c;
+  }
+  for (int k0 = 0; k0 < len; k0 += 32) {
+    const int k = k0 + lane;
+    const uint16_t rank = k < len ? lidx[b0 + k] : 0;
+    const int b = k < len ? rank & 7 : 8;
+    int t = __shfl_sync(0xffffffffu, next, b & 7);
+    for (int j = 0; j < 8; ++j) {
+      const unsigned m = __ballot_sync(0xffffffffu, b == j);
+      if (b == j) t += __popc(m & ((1u << lane) - 1u));
+      if (lane == j) next += __popc(m);
+    }
+    if (k < len) {
+      const int g = t % G, q = t / G;
+      col2[b0 + 8 * g + q] = col[b0 + k];
+      kpos[b0 + 8 * g + q] = (uint16_t)k;
+      lt[b0 + 32 * (g / 4) + 4 * q + (g & 3)] = rank;
+    }
+  }
+  for (int k0 = 0; k0 < lp; k0 += 32) {
+    const int g = (k0 + lane) / 8, q = lane & 7;
+    const bool pad = g >= G || q * G + g >= len;
+    if (pad) {
+      col2[b0 + k0 + lane] = (int32_t)r;
+      kpos[b0 + k0 + lane] = 0xFFFFu;
+      lt[b0 + k0 + 4 * q + (g & 3)] = 0;
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, pad);
+    if (lane == 0) bits[(b0 + k0) >> 5] = m;
+  }
+}
+
+// per-bond flags between the two orders: entry k of the new row is old entry
+// rowptr0[perm[r]] + k, or + kpos[k] where given.  to_new: old bytes -> new
+// bits (OR); else new bits -> old bytes.
+__global__ void k_pmb_flags(int32_t n, const int32_t* __restrict__ perm, const int64_t* __restrict__ rowptr0,
+                            const int64_t* __restrict__ rowptr1, const uint16_t* __restrict__ kpos,
+                            uint32_t* __restrict__ bits, uint8_t* __restrict__ bytes, bool to_new) {
+  const int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (r >= n) return;
+  const int64_t a0 = rowptr0[perm[r]], len = rowptr0[perm[r] + 1] - a0, b0 = rowptr1[r], lp = rowptr1[r + 1] - b0;
+  for (int64_t k = lane; k < lp; k += 32) {
+    const int64_t p = b0 + k, o = kpos ? kpos[p] : k;
+    if (o >= len) continue;  // a pad
     if (to_new) {
-      if (bytes[a0 + k]) atomicOr(&bits[p >> 5], 1u << (p & 31));
+      if (bytes[a0 + o]) atomicOr(&bits[p >> 5], 1u << (p & 31));
     } else {
-      bytes[a0 + k] = (uint8_t)((bits[p >> 5] >> (p & 31)) & 1u);
+      bytes[a0 + o] = (uint8_t)((bits[p >> 5] >> (p & 31)) & 1u);
     }
   }
 }
 
 // Local damage of each particle (Silling & Askari 2005): the fraction of its
-// bonds that are broken (the self entry excluded), written in the caller's
-// particle order.
+// bonds that are broken (the self entry excluded; the pads, all broken, are
+// taken off), written in the caller's particle order.
 __global__ void k_pmb_damage(int32_t n, const int32_t* __restrict__ perm, const int64_t* __restrict__ rowptr0,
                              const int64_t* __restrict__ rowptr1, const uint32_t* __restrict__ bits,
                              double* __restrict__ out) {
   const int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (r >= n) return;
-  const int64_t len = rowptr0[perm[r] + 1] - rowptr0[perm[r]], b0 = rowptr1[r];
+  const int64_t len = rowptr0[perm[r] + 1] - rowptr0[perm[r]], b0 = rowptr1[r], lp = rowptr1[r + 1] - b0;
   int nb = 0;
-  for (int64_t k = lane; k < len; k += 32) {
+  for (int64_t k = lane; k < lp; k += 32) {
     const int64_t p = b0 + k;
     nb += (bits[p >> 5] >> (p & 31)) & 1u;
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) nb += __shfl_xor_sync(0xffffffffu, nb, o);
-  if (lane == 0) out[perm[r]] = len > 1 ? (double)nb / (double)(len - 1) : 0.0;
+  if (lane == 0) out[perm[r]] = len > 1 ? (double)(nb - (lp - len)) / (double)(len - 1) : 0.0;
 }
 
 // Pre-crack: break every bond whose reference segment X_i -> X_j crosses the
@@ -564,6 +730,11 @@ __global__ void k_pmb_cut(int32_t n, const double* __restrict__ X, const int64_t
     }
   }
   if (cnt) atomicAdd(ncut, cnt);
+}
+
+__global__ void k_pmb_fill(int64_t m, double v, double* __restrict__ out) {
+  const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (k < m) out[k] = v;
 }
 
 // predictor of the first step: u1 = u0 + dt v0 + dt^2/2 a0
@@ -618,6 +789,11 @@ struct PmbCtx {
   int64_t* rowptr0 = nullptr;   // the caller's row offsets (bond flags map through them)
   TileSet tiles;
   double *X = nullptr, *vol = nullptr, *u[2] = {nullptr, nullptr}, *vel = nullptr, *acl = nullptr;
+  float4* hi = nullptr;  // X as sums of floats, and c vol (mixed only)
+  float2* lo = nullptr;
+  float* cvol = nullptr;
+  double* scale = nullptr;
+  uint16_t *lt = nullptr, *kpos = nullptr;  // the mixed rows' order (k_pmb_order)
   uint32_t* broken = nullptr;
   int8_t* fixed = nullptr;
   unsigned long long* nbroken = nullptr;
@@ -628,6 +804,7 @@ struct PmbCtx {
   int64_t steps = 0;
   cudaGraphExec_t g = nullptr;
   double g_dt = 0;
+  int g_cur = 0;  // the buffer the graph starts from
   ~PmbCtx() {
     if (g) cudaGraphExecDestroy(g);
     pool.free_all();  // stream-ordered frees before the stream goes
@@ -641,18 +818,18 @@ struct PmbCtx {
 static PmbArgs pmb_args(PmbCtx* c, double dt) {
   PmbArgs a{};
   a.n = c->n; a.R = c->tiles.R; a.jmax = c->tiles.jmax; a.rowptr = c->csr.rowptr; a.jset = c->tiles.jset;
-  a.jcnt = c->tiles.jcnt; a.lidx = c->tiles.lidx; a.broken = c->broken;
+  a.jcnt = c->tiles.jcnt; a.lidx = c->f64 ? c->tiles.lidx : c->lt; a.broken = c->broken;
   a.vol = c->vol; a.X = c->X; a.u_in = c->u[c->cur]; a.u_out = c->u[1 - c->cur]; a.vel = c->vel; a.acl = c->acl;
   a.fixed = c->fixed; a.c = c->c; a.s_c = c->s_c; a.inv_rho = 1.0 / c->rho; a.dt = dt; a.nbroken = c->nbroken;
+  a.hi = c->hi; a.lo = c->lo; a.cvol = c->cvol; a.scale = c->scale;
   return a;
 }
 
-static void launch_pmb(PmbCtx* c, const PmbArgs& a) {
+static int launch_pmb(PmbCtx* c, const PmbArgs& a) {
   const unsigned grid = (unsigned)c->tiles.ntiles;
   const int block = c->tiles.R * kGP;
   const size_t smem = (c->f64 ? 64 : 40) * (size_t)c->tiles.maxcnt + 16;
-  if (c->f64) k_pmb_step<double><<<grid, block, smem, c->s>>>(a);
-  else k_pmb_step<float><<<grid, block, smem, c->s>>>(a);
+  return launch_overlapped(c->f64 ? k_pmb_step_f64 : k_pmb_step_f32, grid, block, smem, c->s, a);
 }
 
 }  // namespace mega
@@ -869,7 +1046,6 @@ int mega_pmb_init(int32_t n, const double* coo, const double* vol, const double*
   PA(c->X, n3); PA(c->vol, n); PA(c->u[0], n3); PA(c->u[1], n3); PA(c->vel, n3); PA(c->acl, n3);
   PA(c->fixed, n); PA(c->nbroken, 1); PA(c->status, 1);
   if (tmp.alloc(&win, n3) || tmp.alloc(&sml, 6 * (int64_t)n)) return fail(MEGA_ERR_NOMEM);
-  std::vector<double> hw(n3, horizon);
   std::vector<int8_t> hf(n, 0);
   if (fixed)
     for (int32_t i = 0; i < n; ++i) hf[i] = (int8_t)(fixed[i] != 0);
@@ -877,7 +1053,7 @@ int mega_pmb_init(int32_t n, const double* coo, const double* vol, const double*
   cudaMemcpyAsync(c->vol, vol, sizeof(double) * n, cudaMemcpyHostToDevice, c->s);
   cudaMemcpyAsync(c->vel, vinit, sizeof(double) * n3, cudaMemcpyHostToDevice, c->s);
   cudaMemcpyAsync(c->fixed, hf.data(), n, cudaMemcpyHostToDevice, c->s);
-  cudaMemcpyAsync(win, hw.data(), sizeof(double) * n3, cudaMemcpyHostToDevice, c->s);
+  k_pmb_fill<<<(unsigned)((n3 + 255) / 256), 256, 0, c->s>>>(n3, horizon, win);
   cudaMemsetAsync(sml, 0, sizeof(double) * 6 * n, c->s);
   cudaMemsetAsync(c->u[0], 0, sizeof(double) * n3, c->s);
   cudaMemsetAsync(c->u[1], 0, sizeof(double) * n3, c->s);
@@ -909,7 +1085,7 @@ int mega_pmb_init(int32_t n, const double* coo, const double* vol, const double*
   cudaMemcpyAsync(bf8, c->fixed, n, cudaMemcpyDeviceToDevice, c->s);
   k_pmb_perm<int8_t><<<gn, 256, 0, c->s>>>(n, 1, c->perm, bf8, c->fixed, true);
   c->csr.n = n;
-  const int32_t pad = c->f64 ? 4 : 1;  // FP64 rows in groups of 4 bonds
+  const int32_t pad = c->f64 ? 4 : 32;  // FP64 rows in groups of 4 bonds, float rows in words of dead bits
   c->csr.gmaxn = (csr0.gmaxn + pad - 1) / pad * pad;
   c->nreal = m;
   PA(c->rowptr0, (int64_t)n + 1);
@@ -932,25 +1108,46 @@ int mega_pmb_init(int32_t n, const double* coo, const double* vol, const double*
   {
     static bool smem_set = false;  // FP64 stages 64 bytes per particle, float 40: up to 64 KB
     if (!smem_set) {
-      if (cudaFuncSetAttribute(k_pmb_step<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024 + 16) !=
+      if (cudaFuncSetAttribute(k_pmb_step_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024 + 16) !=
               cudaSuccess ||
-          cudaFuncSetAttribute(k_pmb_step<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 40 * 1024 + 16) !=
+          cudaFuncSetAttribute(k_pmb_step_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, 40 * 1024 + 16) !=
               cudaSuccess)
         return fail(MEGA_ERR_CUDA);
       smem_set = true;
     }
   }
-  PA(c->broken, (mp + 31) / 32);
+  const int64_t words = (mp + 31) / 32;
+  void* spent[2] = {nullptr, nullptr};
+  PA(c->broken, words);
+  if (c->f64) {
+    cudaMemsetAsync(c->broken, 0, sizeof(uint32_t) * words, c->s);
+    k_pmb_padbits<<<gn, 256, 0, c->s>>>(n, c->perm, c->rowptr0, c->csr.rowptr, c->broken);
+  } else {
+    int32_t* col2 = nullptr;
+    unsigned long long* ext = nullptr;
+    PA(c->hi, n); PA(c->lo, n); PA(c->cvol, n); PA(c->scale, 1); PA(c->lt, mp); PA(c->kpos, mp); PA(col2, mp);
+    if (tmp.alloc(&ext, 1)) return fail(MEGA_ERR_NOMEM);
+    cudaMemsetAsync(ext, 0, sizeof(*ext), c->s);
+    k_pmb_extent<<<g3, 256, 0, c->s>>>(n, c->X, ext);
+    k_pmb_split<<<gn, 256, 0, c->s>>>(n, c->X, c->vol, micromodulus, ext, c->scale, c->hi, c->lo,
+                                      c->cvol);
+    k_pmb_order<<<gw, 256, 0, c->s>>>(n, c->perm, c->rowptr0, c->csr.rowptr, c->csr.col, c->tiles.lidx, col2, c->lt,
+                                      c->kpos, c->broken);
+    spent[0] = c->csr.col;  // released below, once the kernel that reads them is done
+    spent[1] = c->tiles.lidx;
+    c->csr.col = col2;
+    c->tiles.lidx = nullptr;
+  }
 #undef PA
-  cudaMemsetAsync(c->broken, 0, sizeof(uint32_t) * ((mp + 31) / 32), c->s);
-  k_pmb_padbits<<<gn, 256, 0, c->s>>>(n, c->perm, c->rowptr0, c->csr.rowptr, c->broken);
   if (broken0) {  // the caller's order -> bits in the renumbered order
     uint8_t* b0 = nullptr;
     if (tmp.alloc(&b0, m)) return fail(MEGA_ERR_NOMEM);
     cudaMemcpyAsync(b0, broken0, (size_t)m, cudaMemcpyHostToDevice, c->s);
-    k_pmb_flags<<<gw, 256, 0, c->s>>>(n, c->perm, c->rowptr0, c->csr.rowptr, c->broken, b0, true);
+    k_pmb_flags<<<gw, 256, 0, c->s>>>(n, c->perm, c->rowptr0, c->csr.rowptr, c->kpos, c->broken, b0,
+                                         true);
   }
   if (cudaStreamSynchronize(c->s) != cudaSuccess || cudaGetLastError() != cudaSuccess) return fail(MEGA_ERR_CUDA);
+  for (void* p : spent) c->pool.release(p);
   if (nbonds) *nbonds = m;
   {
     std::lock_guard<std::mutex> lk(g_pmb_mu);
@@ -959,6 +1156,8 @@ int mega_pmb_init(int32_t n, const double* coo, const double* vol, const double*
   *handle = reinterpret_cast<int64_t>(c);
   return 0;
 }
+
+constexpr int kPmbGraph = 16;  // steps per captured graph
 
 // nsteps of velocity-Verlet: the first step starts from a = 0 like the
 // reference's STATE_INIT (the predictor of step 1 is u = dt v).
@@ -977,30 +1176,29 @@ int mega_pmb_step(int64_t h, int32_t nsteps, double dt, float* ms) {
     MEGA_CHECK_LAUNCH();
   }
   int done = 0;
-  // graph of two steps (the ping-pong buffers return to where they started)
-  if (nsteps >= 2 && (c->g == nullptr || c->g_dt != dt)) {
+  // graph of kPmbGraph steps, an even number: the ping-pong buffers return to
+  // where they started
+  if (nsteps >= kPmbGraph && (c->g == nullptr || c->g_dt != dt || c->g_cur != c->cur)) {
     if (c->g) { cudaGraphExecDestroy(c->g); c->g = nullptr; }
     cudaGraph_t gr;
     MEGA_TRY(cudaStreamBeginCapture(c->s, cudaStreamCaptureModeThreadLocal));
-    for (int k = 0; k < 2; ++k) {
-      PmbArgs a = pmb_args(c, dt);
-      launch_pmb(c, a);
+    int r = 0;
+    for (int k = 0; k < kPmbGraph; ++k) {
+      if (!r) r = launch_pmb(c, pmb_args(c, dt));
       c->cur = 1 - c->cur;
     }
     cudaError_t e = cudaStreamEndCapture(c->s, &gr);
+    if (r) { if (gr) cudaGraphDestroy(gr); return r; }
     if (e != cudaSuccess) { record_cuda_error(e, "capture", __FILE__, __LINE__); return MEGA_ERR_CUDA; }
     e = cudaGraphInstantiate(&c->g, gr, 0);
     cudaGraphDestroy(gr);
     if (e != cudaSuccess) { record_cuda_error(e, "instantiate", __FILE__, __LINE__); return MEGA_ERR_CUDA; }
     c->g_dt = dt;
+    c->g_cur = c->cur;
   }
-  while (nsteps - done >= 2) {
-    MEGA_TRY(cudaGraphLaunch(c->g, c->s));
-    done += 2;
-  }
+  for (; nsteps - done >= kPmbGraph; done += kPmbGraph) MEGA_TRY(cudaGraphLaunch(c->g, c->s));
   for (; done < nsteps; ++done) {
-    PmbArgs a = pmb_args(c, dt);
-    launch_pmb(c, a);
+    if (int r = launch_pmb(c, pmb_args(c, dt))) return r;
     MEGA_CHECK_LAUNCH();
     c->cur = 1 - c->cur;
   }
@@ -1046,7 +1244,7 @@ int mega_pmb_download(int64_t h, int32_t what, double* dst, int64_t* nbroken) {
     uint8_t* d = nullptr;
     MEGA_ALLOC(tp, d, m);
     k_pmb_flags<<<(unsigned)(((int64_t)c->n * 32 + 255) / 256), 256, 0, c->s>>>(c->n, c->perm, c->rowptr0,
-                                                                              c->csr.rowptr, c->broken, d, false);
+                                                                              c->csr.rowptr, c->kpos, c->broken, d, false);
     MEGA_CHECK_LAUNCH();
     std::vector<uint8_t> hb(m);
     MEGA_TRY(cudaMemcpyAsync(hb.data(), d, (size_t)m, cudaMemcpyDeviceToHost, c->s));
