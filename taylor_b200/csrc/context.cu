@@ -559,6 +559,7 @@ struct Ctx {
   int g_mode = -1;
   double g_dt = 0.0;
   int g_len = 0;
+  int64_t g_kernels = 0;  // kernels of one replay
   ~Ctx() {
     if (gexec) cudaGraphExecDestroy(gexec);
     // stream-ordered frees first, then the stream
@@ -716,33 +717,48 @@ static int kernels_per_step(const Ctx* c, int mode = 0) {
          (((mode & MEGA_FLAG_LEARNED_GUESS) && c->mlp_on) ? 1 : 0);
 }
 
+// whether a step's row gather goes on to the stress update
+static bool joins_stress(const Ctx* c, int mode, int predict, bool full) {
+  return predict && !full && !c->nsni && !c->aux && c->p.finite_strain && !(mode & MEGA_FLAG_INTERP_EACH_STEP) &&
+         !((mode & MEGA_FLAG_LEARNED_GUESS) && c->mlp_on) &&
+         defgrad_stress_fits(c->rt, c->var_defgrad[(mode & 0xff) == MEGA_MODE_MIXED]);
+}
+
 // full: F is formed from the displacements; else it advances by this step's
 // increment from where the step before left it.
 static int step_once(Ctx* c, double dt, int mode, int predict, cudaEvent_t* ev, bool full, bool load_only = false) {
   const bool mixed = (mode & 0xff) == MEGA_MODE_MIXED;
   const bool interp = (mode & MEGA_FLAG_INTERP_EACH_STEP) != 0;
   if (ev) MEGA_TRY(cudaEventRecord(ev[0], c->s));
-  NsniTiles nt;
-  int r = launch_defgrad_tiled(c->s, mixed, interp, c->n, c->rt, nsni_tiles(c, mixed, nt), c->csr.rowptr,
-                               mixed ? c->pk32 : c->pk64, c->dsp, c->dsp_tot, mixed ? c->sdphi32 : c->sdphi,
-                               c->shpb[mixed] ? c->shpb[mixed] : c->shp, c->dsp_tot_phy, c->fg, c->acc, c->status,
-                               c->var_defgrad[mixed], full, load_only);
-  if (r) return r;
-  if (load_only) return launch_force_tiled(c->s, mixed, force_args(c, dt, mode, predict), c->var_force[mixed], true);
-  if (ev) MEGA_TRY(cudaEventRecord(ev[1], c->s));
   StressArgs sa = stress_args(c, dt, mode);
   sa.add_g0 = !full;
   sa.more = predict;
   sa.stress_prev = c->nsni ? c->stress_prev : nullptr;
-  r = launch_stress(c->s, mixed, sa);
-  if (r) return r;
+  int r = 0;
+  if (joins_stress(c, mode, predict, full) && !ev) {
+    r = launch_defgrad_stress(c->s, mixed, c->n, c->rt, c->csr.rowptr, mixed ? c->pk32 : c->pk64, c->dsp, c->dsp_tot,
+                              mixed ? c->sdphi32 : c->sdphi, c->fg, sa, c->var_defgrad[mixed], load_only);
+    if (r) return r;
+    if (load_only) return launch_force_tiled(c->s, mixed, force_args(c, dt, mode, predict), c->var_force[mixed], true);
+  } else {
+    NsniTiles nt;
+    r = launch_defgrad_tiled(c->s, mixed, interp, c->n, c->rt, nsni_tiles(c, mixed, nt), c->csr.rowptr,
+                             mixed ? c->pk32 : c->pk64, c->dsp, c->dsp_tot, mixed ? c->sdphi32 : c->sdphi,
+                             c->shpb[mixed] ? c->shpb[mixed] : c->shp, c->dsp_tot_phy, c->fg, c->acc, c->status,
+                             c->var_defgrad[mixed], full, load_only);
+    if (r) return r;
+    if (load_only) return launch_force_tiled(c->s, mixed, force_args(c, dt, mode, predict), c->var_force[mixed], true);
+    if (ev) MEGA_TRY(cudaEventRecord(ev[1], c->s));
+    r = launch_stress(c->s, mixed, sa);
+    if (r) return r;
+  }
   if (c->nsni && (r = nsni_step(c->s, nsni_args(c), c->csr, NsniS{}, NsniS{}, mixed, c->dsp, 1))) return r;
   if ((r = launch_fixity2(c, dt))) return r;
   if (ev) MEGA_TRY(cudaEventRecord(ev[2], c->s));
   r = launch_force_tiled(c->s, mixed, force_args(c, dt, mode, predict), c->var_force[mixed]);
   if (r) return r;
   if (ev) MEGA_TRY(cudaEventRecord(ev[3], c->s));
-  c->launches += kernels_per_step(c, mode);
+  c->launches += kernels_per_step(c, mode) - (joins_stress(c, mode, predict, full) && !ev);
   return 0;
 }
 
@@ -764,6 +780,7 @@ static int graph_for(Ctx* c, double dt, int mode, int len) {
   int r = 0;
   for (int k = 0; k < len && !r; ++k) r = step_once(c, dt, mode, 1, nullptr, k == 0);
   cudaError_t e = cudaStreamEndCapture(c->s, &g);
+  c->g_kernels = c->launches - before;
   c->launches = before;
   if (r) { if (g) cudaGraphDestroy(g); return r; }
   if (e != cudaSuccess) { record_cuda_error(e, "cudaStreamEndCapture", __FILE__, __LINE__); return MEGA_ERR_CUDA; }
@@ -795,7 +812,7 @@ static int run_steps(Ctx* c, int32_t nsteps, double dt, int mode) {
     if (c->fsteps % kGraphSteps == 0 && rem >= kGraphSteps) {
       if ((r = graph_for(c, dt, mode, kGraphSteps))) return r;
       MEGA_TRY(cudaGraphLaunch(c->gexec, c->s));
-      c->launches += kernels_per_step(c, mode) * kGraphSteps;
+      c->launches += c->g_kernels;
       c->fsteps += kGraphSteps;
       rem -= kGraphSteps;
     } else {

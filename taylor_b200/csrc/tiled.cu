@@ -16,6 +16,7 @@
 // The summation order is fixed by the list order, so results are
 // deterministic, and identical in exact arithmetic to force.cu's.
 #include "mega_internal.cuh"
+#include "stress.cuh"
 #include "tiled.cuh"
 #include "bulk.cuh"
 
@@ -642,12 +643,22 @@ constexpr int defgrad_blocks() {  // blocks per SM the register cap asks for
   return w / KG > 0 ? w / KG : 1;
 }
 
-template <typename A, bool F64, bool INTERP, int KG, int KU, bool NS, bool FULL>
-__global__ void __launch_bounds__(64 * KG, defgrad_blocks<F64, KG, NS, FULL>())
+struct NoStress {};
+template <typename SA>
+constexpr bool kHasStress = !std::is_same<SA, NoStress>::value;
+
+// SA: StressArgs where the block goes on to the stress update of its rows,
+// NoStress else.  What bounds a step of a few thousand nodes is the latency of
+// its kernels, one after the other: with the rows' G0 at hand behind a block
+// barrier, the update needs no launch of its own.  It takes 128 registers, so
+// two blocks of 256 threads an SM; defgrad_stress_fits has the rule.
+template <typename A, bool F64, bool INTERP, int KG, int KU, bool NS, bool FULL, typename SA = NoStress>
+__global__ void __launch_bounds__(kHasStress<SA> && KG == 16 ? 512 : 64 * KG,
+                                  kHasStress<SA> ? (KG == 4 ? 2 : 1) : defgrad_blocks<F64, KG, NS, FULL>())
     k_defgrad_t(int32_t n, int32_t R, int32_t jmax, NsniTiles ns, SliceView sv, const int64_t* __restrict__ rowptr,
                 const void* __restrict__ pk, const int32_t* __restrict__ jset, const int32_t* __restrict__ jcnt,
                 const double* dsp, const double* dsp_tot, const double* __restrict__ sdphi,
-                const double* __restrict__ shp, double* dsp_tot_phy, double* fg, StepAccum* acc) {
+                const double* __restrict__ shp, double* dsp_tot_phy, double* fg, StepAccum* acc, SA sa) {
   extern __shared__ __align__(16) double sm[];
   const int64_t t = blockIdx.x;
   const int cnt = jcnt[t];
@@ -689,8 +700,13 @@ __global__ void __launch_bounds__(64 * KG, defgrad_blocks<F64, KG, NS, FULL>())
   }
   grid_wait();
   if (acc && blockIdx.x == 0 && threadIdx.x < kSlots) {
-    acc->newton_iters[threadIdx.x] = 0ull;
-    acc->plastic[threadIdx.x] = 0ull;
+    if constexpr (kHasStress<SA>) {
+      // (no counts of this step alone: a call's last step is not one of these)
+      acc->ke[threadIdx.x] = 0.0;
+    } else {
+      acc->newton_iters[threadIdx.x] = 0ull;
+      acc->plastic[threadIdx.x] = 0ull;
+    }
   }
   double ur[3] = {0.0, 0.0, 0.0}, dr[3] = {0.0, 0.0, 0.0};
   if (!F64) {
@@ -843,6 +859,21 @@ __global__ void __launch_bounds__(64 * KG, defgrad_blocks<F64, KG, NS, FULL>())
         for (int k = 0; k < 3; ++k) dsp_tot_phy[3 * i + k] += ph[k];
       }
     }
+  }
+  if constexpr (kHasStress<SA>) {
+    __shared__ double smd[32];
+    __shared__ unsigned long long smu[32];
+    __syncthreads();  // G0 of the tile's rows, written by other threads of this block
+    double work = 0.0;
+    unsigned long long iters = 0, npl = 0;
+    unsigned st = 0;
+    const int64_t row = r0 + threadIdx.x;
+    if ((int)threadIdx.x < R && row < n) {
+      Trial<A, true> w;
+      stress_trial<A, true, false, true>(sa, row, w);
+      stress_finish<A, A, true, false, true>(sa, row, w, -1.0, work, iters, npl, st);
+    }
+    stress_reduce<A, false>(sa, work, iters, npl, st, smd, smu);
   }
 }
 
@@ -1693,7 +1724,7 @@ static int defgrad_variant(cudaStream_t s, const DefgradArgs& d) {
                     : (d.interp ? k_defgrad_t<float, false, true, KG, KU, false, FULL>
                                 : k_defgrad_t<float, false, false, KG, KU, false, FULL>);
   return start(k, stage_limit(), d.load_only, (unsigned)ts.ntiles, ts.R * KG, smem, s, d.n, ts.R, ts.jmax, nz, ts.view(),
-               d.rowptr, d.pk, ts.jset, ts.jcnt, d.dsp, d.dsp_tot, d.sdphi, d.shp, d.dsp_tot_phy, d.fg, d.acc);
+               d.rowptr, d.pk, ts.jset, ts.jcnt, d.dsp, d.dsp_tot, d.sdphi, d.shp, d.dsp_tot_phy, d.fg, d.acc, NoStress());
 }
 
 // NSNI runs the register variants: mixed refuses the streamed ones, FP64 takes
@@ -1731,6 +1762,38 @@ int launch_defgrad_tiled(cudaStream_t s, bool mixed, bool interp, int32_t n, con
   if (r) return r;
   MEGA_CHECK_LAUNCH();
   return 0;
+}
+
+template <int KG, int KU>
+static int defgrad_stress(cudaStream_t s, const DefgradArgs& d, const StressArgs& a) {
+  const TileSet& ts = d.ts;
+  const size_t smem = (size_t)(d.mixed ? 16 : 24) * staged_ld(ts.maxcnt);
+  auto k = d.mixed ? k_defgrad_t<float, false, false, KG, KU, false, false, StressArgs>
+                   : k_defgrad_t<double, true, false, KG, KU, false, false, StressArgs>;
+  return start(k, stage_limit(), d.load_only, (unsigned)ts.ntiles, ts.R * KG, smem, s, d.n, ts.R, ts.jmax, NsniTiles(),
+               ts.view(), d.rowptr, d.pk, ts.jset, ts.jcnt, d.dsp, d.dsp_tot, d.sdphi, d.shp, d.dsp_tot_phy, d.fg, d.acc,
+               a);
+}
+
+// Joined where every block is resident at once (two of 256 threads an SM, one
+// of 512).  Steps joined and apart: 4,455 nodes FP64 16.6 and 18.3 us, mixed 12.3
+// and 14.5; 16,154 nodes FP64 24.9 and 27.3, mixed 17.5 and 19.9; past the line,
+// where the update's registers cost the gather its warps, 23,782 nodes FP64 38.8
+// and 34.4, mixed 26.8 and 23.1; 129,911 nodes mixed 109 and 90.
+bool defgrad_stress_fits(const TileSet& ts, int variant) {
+  const int lanes = variant >= 6 ? 16 : (variant == 3 || variant == 5 ? 8 : 4);
+  const int threads = ts.R * lanes;
+  return threads <= 512 && ts.ntiles <= (int64_t)device_sm_count() * (512 / threads > 2 ? 2 : 512 / threads);
+}
+
+int launch_defgrad_stress(cudaStream_t s, bool mixed, int32_t n, const TileSet& ts, const int64_t* rowptr,
+                          const void* pk, const double* dsp, const double* dsp_tot, const double* sdphi, double* fg,
+                          const StressArgs& a, int variant, bool load_only) {
+  const DefgradArgs d{mixed, false, n,      ts,   nullptr, rowptr, pk, dsp, dsp_tot, sdphi, nullptr, nullptr, fg,
+                      a.acc, a.status, load_only};
+  if (variant >= 6) return defgrad_stress<16, 2>(s, d, a);
+  if (variant == 3 || variant == 5) return defgrad_stress<8, 2>(s, d, a);
+  return defgrad_stress<4, 4>(s, d, a);
 }
 
 template <int KG>

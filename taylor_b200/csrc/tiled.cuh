@@ -133,6 +133,13 @@ int launch_defgrad_tiled(cudaStream_t s, bool mixed, bool interp, int32_t n, con
                          const double* dsp_tot,
                          const double* sdphi, const double* shp, double* dsp_tot_phy, double* fg, StepAccum* acc,
                          unsigned* status, int variant, bool full, bool load_only = false);
+// The row gather of the increments that goes on to the stress update of its
+// rows (finite strain, undamaged models, no NSNI, another step follows), and
+// whether it is the faster way: all of its blocks resident at once.
+bool defgrad_stress_fits(const TileSet& ts, int variant);
+int launch_defgrad_stress(cudaStream_t s, bool mixed, int32_t n, const TileSet& ts, const int64_t* rowptr,
+                          const void* pk, const double* dsp, const double* dsp_tot, const double* sdphi, double* fg,
+                          const StressArgs& a, int variant, bool load_only = false);
 int launch_force_tiled(cudaStream_t s, bool mixed, const TiledForceArgs& a, int variant = 0, bool load_only = false);
 
 }  // namespace mega
