@@ -642,7 +642,7 @@ static TiledForceArgs force_args(Ctx* c, double dt, int mode, int predict) {
   TiledForceArgs f{};
   f.n = c->n; f.R = c->ct.R; f.ntiles = c->ct.ntiles; f.jmax = c->ct.jmax; f.maxcnt = c->ct.maxcnt;
   f.recmax = c->ct.recmax;
-  f.jset = c->ct.jset; f.jcnt = c->ct.jcnt; f.colptr = c->csr.colptr; f.sv = c->ct.view();
+  f.jset = c->ct.jset; f.jcnt = c->ct.jcnt; f.colptr = c->csr.colptr; f.sv = c->ct.view(records_ahead(c->ct, mixed));
   f.pk = mixed ? c->tpk32 : c->tpk64;
   f.tshp = mixed ? c->tshp32 : c->tshp; f.tmat = c->tmat; f.has_body = c->has_body; f.predict = predict;
   f.ebc = c->ebc; f.mass = c->mass; f.matidx = c->matidx; f.mats = c->mats; f.body_id = c->body_id;
@@ -2205,6 +2205,7 @@ static int bank_layout(Ctx* c, bool mixed) {
   c->shpb[mixed] = sh;
   if (sr) { c->nbpool.release(c->ns_srow[mixed]); c->ns_srow[mixed] = sr; }
   c->banked[mixed] = true;
+  if (mixed) c->rt.banked32 = c->ct.banked32 = true;
   return 0;
 }
 

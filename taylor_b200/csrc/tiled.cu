@@ -537,6 +537,25 @@ struct RowWalk {
   __device__ __forceinline__ int64_t at(int k) const { return rec + (int64_t)(8 * KG) * k; }
 };
 
+// The records of a slice past its rows' first KU steps, on their way to L2 while
+// the tile's neighbours are staged (each plane 64-byte aligned: whole steps).
+template <bool F64, int KG>
+__device__ __forceinline__ void prefetch_rest(const void* pk, const SliceView& v, int64_t slot0, int slot, int ku) {
+  if ((threadIdx.x & (8 * KG - 1)) != 0) return;
+  const int64_t sl = (slot0 + slot) >> 3;
+  const int64_t s0 = v.sstep[sl] + ku * (KG / 4), n = 32 * (v.sstep[sl + 1] - s0), r = 32 * s0;
+  if (n <= 0) return;
+  const char* b = (const char*)pk;
+  const auto fetch = [](const char* p, int64_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"((unsigned)bytes) : "memory");
+  };
+  fetch(b + 16 * r, 16 * n);
+  if (F64) {
+    fetch(b + 16 * v.nrec + 8 * r, 8 * n);
+    fetch(b + 24 * v.nrec + 2 * r, 2 * n);
+  }
+}
+
 // The six S values of one NSNI record.
 template <bool F64>
 struct SRec;
@@ -680,6 +699,7 @@ __global__ void __launch_bounds__(kHasStress<SA> && KG == 16 ? 512 : 64 * KG,
   const bool valid = i < n;
   // this lane's first KU packed records are requested before the staging,
   // so their latency overlaps it
+  if (!NS && (!F64 || kHasStress<SA>) && sv.ahead) prefetch_rest<F64, KG>(pk, sv, r0, slot, KU);
   const RowWalk<KG> walk(sv, r0, slot, q);
   const int nit = valid ? walk.nit : 0;
   constexpr bool kPipe = !NS && (!F64 || KU <= 2);
@@ -1089,6 +1109,7 @@ __global__ void __launch_bounds__(64 * KG, force_blocks<F64, KG, KU, NS>()) k_fo
   const bool valid = J < a.n;
   // this lane's first KU packed records are requested before the staging,
   // so their latency overlaps it
+  if (!NS && !F64 && a.sv.ahead) prefetch_rest<F64, KG>(a.pk, a.sv, c0, slot, KU);
   const RowWalk<KG> walk(a.sv, c0, slot, q);
   const int nit = valid ? walk.nit : 0;
   constexpr bool kPipe = !NS && (!F64 || KU <= 2);
@@ -1723,7 +1744,8 @@ static int defgrad_variant(cudaStream_t s, const DefgradArgs& d) {
                                 : k_defgrad_t<float, false, false, KG, KU, true, FULL>)
                     : (d.interp ? k_defgrad_t<float, false, true, KG, KU, false, FULL>
                                 : k_defgrad_t<float, false, false, KG, KU, false, FULL>);
-  return start(k, stage_limit(), d.load_only, (unsigned)ts.ntiles, ts.R * KG, smem, s, d.n, ts.R, ts.jmax, nz, ts.view(),
+  return start(k, stage_limit(), d.load_only, (unsigned)ts.ntiles, ts.R * KG, smem, s, d.n, ts.R, ts.jmax, nz,
+               ts.view(records_ahead(ts, d.mixed)),
                d.rowptr, d.pk, ts.jset, ts.jcnt, d.dsp, d.dsp_tot, d.sdphi, d.shp, d.dsp_tot_phy, d.fg, d.acc, NoStress());
 }
 
@@ -1771,8 +1793,29 @@ static int defgrad_stress(cudaStream_t s, const DefgradArgs& d, const StressArgs
   auto k = d.mixed ? k_defgrad_t<float, false, false, KG, KU, false, false, StressArgs>
                    : k_defgrad_t<double, true, false, KG, KU, false, false, StressArgs>;
   return start(k, stage_limit(), d.load_only, (unsigned)ts.ntiles, ts.R * KG, smem, s, d.n, ts.R, ts.jmax, NsniTiles(),
-               ts.view(), d.rowptr, d.pk, ts.jset, ts.jcnt, d.dsp, d.dsp_tot, d.sdphi, d.shp, d.dsp_tot_phy, d.fg, d.acc,
+               ts.view(records_ahead(ts, d.mixed)), d.rowptr, d.pk, ts.jset, ts.jcnt, d.dsp, d.dsp_tot, d.sdphi, d.shp, d.dsp_tot_phy, d.fg, d.acc,
                a);
+}
+
+// Fetched ahead where a gather's blocks are all resident at once, so that only
+// their own latency counts (steps of 4,455 nodes, FP64 17.3 -> 16.5 us, mixed 13.3
+// -> 12.5; 16,154 nodes 25.4 -> 24.9 and 17.7 -> 17.5; FP64 in the joined row gather
+// alone: the test cost its other gathers 1 %), and mixed where bank-ordered
+// records of both gathers pass the L2 three times, so that they come from HBM
+// (1.04 M nodes: row gather 217 -> 203 us, column gather 288 -> 278, step 601 ->
+// 576; 383 k 243 -> 236; 255 k, four times the L2, 168 -> 164).  In between part of
+// the records is still in L2, and the requests only take its bandwidth: 130 k
+// nodes, twice the L2, step 88 -> 93; FP64 135 -> 148, and at 1.04 M nodes no gain.
+// In list order the gathers wait for bank conflicts instead (383 k 250 -> 253).
+bool records_ahead(const TileSet& ts, bool mixed) {
+  static const int64_t l2 = [] {
+    int dev = 0, bytes = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&bytes, cudaDevAttrL2CacheSize, dev) != cudaSuccess || bytes <= 0)
+      bytes = 126 << 20;
+    return (int64_t)bytes;
+  }();
+  return ts.ntiles <= 2 * (int64_t)device_sm_count() || (mixed && ts.banked32 && 2 * 16 * ts.nrec > 3 * l2);
 }
 
 // Joined where every block is resident at once (two of 256 threads an SM, one

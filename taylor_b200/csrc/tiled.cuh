@@ -11,6 +11,7 @@ struct SliceView {
   const uint8_t* ord = nullptr;    // per slot (tile, position): the row within the tile; rows past n come last
   const int64_t* sstep = nullptr;  // per slice of 8 slots: its first step (record 32 sstep), and the end
   int64_t nrec = 0;                // records, pads among them
+  bool ahead = false;              // fetch a slice's records to L2 as its rows begin (records_ahead)
 };
 
 struct TileSet {
@@ -27,7 +28,8 @@ struct TileSet {
   int64_t* sstep = nullptr;
   int64_t* rbase = nullptr;  // per row: the record of its entry 0; entry k is 32 (k / 4) + k % 4 further
   int64_t nrec = 0;
-  SliceView view() const { return SliceView{ord, sstep, nrec}; }
+  bool banked32 = false;     // the mixed records are in bank order
+  SliceView view(bool ahead = false) const { return SliceView{ord, sstep, nrec, ahead}; }
 };
 
 // NSNI terms carried by the tiled gathers: the smoothed second derivatives
@@ -133,6 +135,8 @@ int launch_defgrad_tiled(cudaStream_t s, bool mixed, bool interp, int32_t n, con
                          const double* dsp_tot,
                          const double* sdphi, const double* shp, double* dsp_tot_phy, double* fg, StepAccum* acc,
                          unsigned* status, int variant, bool full, bool load_only = false);
+// whether the gathers of these tiles fetch their records ahead
+bool records_ahead(const TileSet& ts, bool mixed);
 // The row gather of the increments that goes on to the stress update of its
 // rows (finite strain, undamaged models, no NSNI, another step follows), and
 // whether it is the faster way: all of its blocks resident at once.
