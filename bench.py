@@ -186,33 +186,29 @@ def workload_name(h, n):
 
 
 def kernel_bytes(n, nnz, mixed):
-    """Algorithmic bytes per launch of each per-step kernel (every array
-    touched once; neighbour data counted once per owning node)."""
-    g = 12 if mixed else 24          # three gradient components per CSR entry
+    """Algorithmic bytes per launch of each kernel of a steady step (every
+    array touched once; neighbour data counted once per owning node)."""
+    rec = 16 if mixed else 26        # a packed record: three gradient components and the neighbour's rank
     t = 36 if mixed else 72          # T_i (3x3) per node
-    fg = 72 if mixed else 144        # F (less its identity in mixed) and G0 per node
-    defgrad = nnz * (4 + g) + n * (8 + 48 + 24 + fg)            # col + grad; rowptr, u and du, sum grad, F/G0 out
-    stress = n * (fg + 192 + 16 + 8 + 8 + 8 + 2 + t)            # F/G0, sigma+eps rw, eps_p rw, eq, wvel, vol, mat, T
-    force = nnz * (4 + g) + n * (8 + t + 3 + 24 + 24 + 48 + 48 + 24 + 48 + 48 + 24)  # trow + grad^T; T, fixity,
-    return dict(defgrad=defgrad, stress=stress, force=force)     # mass, fint, fext rw, vel rw, acl, dsp rw, tot rw, pr
+    g0 = 36 if mixed else 72         # G0 per node
+    defgrad = nnz * rec + n * (1 + 24 + 24 + g0)                # row order, du, sum grad; G0 out
+    stress = n * (g0 + 2 * 72 + 192 + 16 + 8 + 2 + t)           # G0, F rw, sigma+eps rw, eps_p rw, vol, mat, T out
+    force = nnz * rec + n * (1 + t + 3 + 2 + 24 + 4 * 48)       # order, T, fixity, mat, mass; fext, vel, dsp, tot rw
+    return dict(defgrad=defgrad, stress=stress, force=force)
 
 
 def nsni_step_bytes(n, nnz, mixed):
     """Algorithmic bytes of one NSNI step (every array touched once): the
     DNI kernels on the seven-point lists (kernel_bytes), the six second
     derivatives S of every entry in both gathers (6 s bytes each, s = 4
-    mixed or 8; the FP64 NSNI gathers also read each entry's row / column
-    index, 4 bytes, and k_nsni_h gathers the increment, 24 per node, which
-    the mixed gathers have staged already), H (18 doubles written, read),
-    the stress gradients (18 doubles read and written), the force weights
-    (18 floats / doubles written, read), the stress before the step (6
-    doubles copied and read) and, in FP64, the stabilisation force (3
-    doubles written, read)."""
+    mixed or 8), H (18 doubles written, read), the stress gradients (18
+    doubles read and written), the force weights (20 floats / doubles
+    written, read) and the stress before the step (6 doubles written and
+    read)."""
     kb = kernel_bytes(n, nnz, mixed)
     s = 4 if mixed else 8
-    w = 80 if mixed else 144
-    per_entry = 2 * (6 * s) if mixed else 2 * (4 + 6 * s)
-    per_node = 2 * 144 + 2 * 144 + 2 * w + 3 * 48 + (0 if mixed else 24 + 2 * 24)
+    per_entry = 2 * (6 * s)
+    per_node = 2 * 144 + 2 * 144 + 2 * 20 * s + 2 * 48
     return kb["defgrad"] + kb["stress"] + kb["force"] + nnz * per_entry + n * per_node
 
 

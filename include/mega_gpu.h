@@ -366,11 +366,16 @@ int mega_set_instances(int64_t h, int32_t ninst, const int32_t* inst_nodes, cons
 int mega_set_instance_dt(int64_t h, const double* dt_inst);
 /* Autotuner: time each launch variant of the two per-step gathers for the
  * given precision on this context's lists, reps launches each, keep the
- * fastest, and leave the state as it was.  Variants 0..3, 6 and 7 hold the
+ * fastest, and leave the state as it was.  The first call for a precision
+ * reorders its packed records within each row and column for the gathers'
+ * shared-memory banks: from then on that precision's sums run in the new
+ * order (FP64 too, where they differ from the list order's by rounding).
+ * Variants 0..3, 6 and 7 hold the
  * packed records in registers (lanes per row x records in flight: (4, 4),
  * (4, 2), (4, 1), (8, 2), (16, 1), (16, 2)); 4 and 5 have the copy engine
  * stream each tile's records into shared memory (4 or 8 lanes per row),
- * where the tiles fit (not with NSNI in mixed precision).  choice
+ * where the tiles fit; with NSNI they are refused in mixed precision and run
+ * the register variant of the same lanes per row in FP64.  choice
  * (2) receives the deformation-gradient and force variants, times_ms
  * (2 x MEGA_TUNE_VARIANTS, may be NULL) the mean launch times, -1 for a
  * variant that does not fit. */
@@ -378,7 +383,7 @@ int mega_set_instance_dt(int64_t h, const double* dt_inst);
 /* Pin the launch variants of the two gathers for one precision (after
  * mega_search_and_shapes), e.g. to repeat a run bit for bit: variants with
  * the same lanes per row (0, 1, 2, 4; 3, 5; 6, 7) sum in the same order and
- * give identical results.  MEGA_ERR_UNSUPPORTED when a streamed variant
+ * give identical results on the same record order (see mega_autotune).  MEGA_ERR_UNSUPPORTED when a streamed variant
  * does not fit the context's tiles. */
 int mega_set_variants(int64_t h, int32_t mode, int32_t defgrad_variant, int32_t force_variant);
 int mega_autotune(int64_t h, double dt, int32_t mode, int32_t reps, int32_t* choice, float* times_ms);
@@ -394,7 +399,7 @@ int mega_autotune(int64_t h, double dt, int32_t mode, int32_t reps, int32_t* cho
 int mega_set_fixity2(int64_t h, int32_t steps, const double* ftime, const double* fdisp);
 /* Precisions the context will step: mask bit 0 FP64, bit 1 mixed (default
  * 3).  Call before mega_search_and_shapes; only the asked-for packed records
- * are built (the FP64 records are 32 B per list entry, the mixed 16 B).
+ * are built (the FP64 records are 26 B per list entry, the mixed 16 B).
  * Stepping a precision that was not built returns MEGA_ERR_STATE. */
 int mega_set_precisions(int64_t h, int32_t mask);
 

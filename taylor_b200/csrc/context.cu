@@ -2566,7 +2566,7 @@ int mega_bin_search(int32_t n, const double* coo, const double* win, const doubl
   int r = make_stream(&sg.s);
   if (r) return r;
   cudaStream_t s = sg.s;
-  DevPool pool;
+  DevPool pool(s);  // blocks from the process's cache: cudaMalloc beside it cost 10-20 ms a call
   double *dc, *dw, *ds;
   int32_t* dijk = nullptr;
   unsigned* st;
@@ -2609,7 +2609,7 @@ int mega_rk_shapes(const mega_params* p, int32_t n, const double* coo, const dou
   int r = make_stream(&sg.s);
   if (r) return r;
   cudaStream_t s = sg.s;
-  DevPool pool;
+  DevPool pool(s);  // blocks from the process's cache: cudaMalloc beside it cost 10-20 ms a call
   DevCSR csr;
   std::vector<int64_t> hpos;
   r = csr_from_host(s, n, gn, gstart, gstack, nnz, pool, csr, hpos);

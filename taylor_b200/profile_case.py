@@ -61,8 +61,11 @@ def main(argv=None):
         m.step(200, dt, mode=a.mode, allow_status=True)     # impact first: plastic nodes to learn from
         m.train_surrogate(mega.mlp_init(5), epochs=3, batch=8192, lr=2e-3, seed=9)
         m.log_rate_samples(0)
-    for _ in range(a.steps):
-        m.step(1, dt, mode=a.mode, learned=learned, allow_status=True)
+    if learned:
+        for _ in range(a.steps):
+            m.step(1, dt, mode=a.mode, learned=True, allow_status=True)
+    else:  # one call: all its steps but the last are the steady ones
+        m.step(a.steps, dt, mode=a.mode, allow_status=True)
     print(f"{a.what} bar h={case['h']*1e3:.3g}mm: {case['n']} nodes, {info['nnz']} entries, {a.mode}, "
           f"{time.perf_counter() - t0:.1f} s")
     m.close()
