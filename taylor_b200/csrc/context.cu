@@ -717,10 +717,13 @@ static int kernels_per_step(const Ctx* c, int mode = 0) {
          (((mode & MEGA_FLAG_LEARNED_GUESS) && c->mlp_on) ? 1 : 0);
 }
 
-// whether a step's row gather goes on to the stress update
+// whether a step's row gather goes on to the stress update, of any size and of this one
+static bool may_join(const Ctx* c, int mode) {
+  return !c->nsni && !c->aux && c->p.finite_strain && !(mode & MEGA_FLAG_INTERP_EACH_STEP) &&
+         !((mode & MEGA_FLAG_LEARNED_GUESS) && c->mlp_on);
+}
 static bool joins_stress(const Ctx* c, int mode, int predict, bool full) {
-  return predict && !full && !c->nsni && !c->aux && c->p.finite_strain && !(mode & MEGA_FLAG_INTERP_EACH_STEP) &&
-         !((mode & MEGA_FLAG_LEARNED_GUESS) && c->mlp_on) &&
+  return predict && !full && may_join(c, mode) &&
          defgrad_stress_fits(c->rt, c->var_defgrad[(mode & 0xff) == MEGA_MODE_MIXED]);
 }
 
@@ -2294,9 +2297,15 @@ int mega_autotune(int64_t h, double dt, int32_t mode, int32_t reps, int32_t* cho
   MEGA_TRY(cudaStreamSynchronize(c->s));
   if (r) return r;
   int bd = 0, bf = 0;
+  // a row gather that cannot go on to the stress update costs the step a launch
+  // more than one that can: 2.5 us (16,154 nodes FP64: 8 lanes 8.3 us alone and
+  // 25.0 a step, 4 lanes 8.5 and 22.4)
+  const auto cost = [&](int v) {
+    return tdef[v] + (may_join(c, mode) && !defgrad_stress_fits(c->rt, v) ? 2.5e-3f * reps : 0.f);
+  };
   for (int v = 1; v < nvar; ++v) {
     if (!fits[v]) { tdef[v] = tfor[v] = -1.f; continue; }  // reported as -1: not launchable on these tiles
-    if (tdef[v] < tdef[bd]) bd = v;
+    if (cost(v) < cost(bd)) bd = v;
     if (tfor[v] < tfor[bf]) bf = v;
   }
   c->var_defgrad[mixed] = bd;
