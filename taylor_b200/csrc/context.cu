@@ -2145,7 +2145,7 @@ int64_t mega_kernel_launches(int64_t h) {
 // entries of each row and column take the order in which a warp's lanes read
 // distinct shared-memory banks of the staged data (bank_order), and what
 // travels with the records follows them (the interpolation and body-force
-// shape values, the float NSNI S values).  About 6 ms per gather on a 1 M-node
+// shape values, the float NSNI S values).  About 7 ms per gather on a 1 M-node
 // bar; it pays back over a few hundred steps.
 static void drop_graph(Ctx* c);
 
