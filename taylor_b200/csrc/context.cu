@@ -534,6 +534,7 @@ struct Ctx {
   double time = 0.0;
   int64_t steps = 0;
   int64_t fsteps = 0;  // steps since F - I had to be formed afresh (0: it has to be); it is again every kGraphSteps
+  int fprec = -1;      // the precision those steps were in (set_fprec)
   int64_t launches = 0;
   // independent instances sharing the context (node ranges searched apart)
   std::vector<int32_t> inst_off;  // ninst + 1 prefix offsets, empty = one instance
@@ -611,6 +612,13 @@ static int read_status(Ctx* c, bool reset) {
   MEGA_TRY(cudaStreamSynchronize(c->s));
   if (reset && st) MEGA_TRY(cudaMemsetAsync(c->status, 0, sizeof(unsigned), c->s));
   return (int)st;
+}
+
+// F - I of the other precision's sums (float ones before an FP64 step) does not
+// go on: the first step after a change forms it afresh.
+static void set_fprec(Ctx* c, int prec) {
+  if (c->fprec != prec) c->fsteps = 0;
+  c->fprec = prec;
 }
 
 // The records of a precision are packed at search time only when the
@@ -807,6 +815,7 @@ static int run_steps(Ctx* c, int32_t nsteps, double dt, int mode) {
   if (!(mode & MEGA_FLAG_INTERP_EACH_STEP)) c->phy_valid = false;
   int r = sync_time(c);
   if (r) return r;
+  set_fprec(c, prec);
   r = launch_predict(c->s, 3 * (int64_t)c->n, c->dsp, c->dsp_tot, c->vel, c->acl, dt, c->ndt);
   if (r) return r;
   c->launches += 1;
@@ -1897,6 +1906,7 @@ int mega_kernel_times(int64_t h, int32_t reps, double dt, int32_t mode, float* o
   cudaEvent_t ev[4];
   for (auto& e : ev) MEGA_TRY(cudaEventCreate(&e));
   double acc[3] = {0, 0, 0};
+  set_fprec(c, mode & 0xff);
   int r = launch_predict(c->s, 3 * (int64_t)c->n, c->dsp, c->dsp_tot, c->vel, c->acl, dt, c->ndt);
   for (int32_t k = 0; k < reps && !r; ++k) {
     r = step_once(c, dt, mode, k < reps - 1 ? 1 : 0, ev, c->fsteps % kGraphSteps == 0);
