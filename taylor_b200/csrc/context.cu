@@ -534,7 +534,7 @@ struct Ctx {
   double time = 0.0;
   int64_t steps = 0;
   int64_t fsteps = 0;  // steps since F - I had to be formed afresh (0: it has to be); it is again every kGraphSteps
-  int fprec = -1;      // the precision those steps were in (set_fprec)
+  int fprec = -1;      // the precision those steps were in (take_fsteps)
   int64_t launches = 0;
   // independent instances sharing the context (node ranges searched apart)
   std::vector<int32_t> inst_off;  // ninst + 1 prefix offsets, empty = one instance
@@ -611,14 +611,19 @@ static int read_status(Ctx* c, bool reset) {
   MEGA_TRY(cudaMemcpyAsync(&st, c->status, sizeof(unsigned), cudaMemcpyDeviceToHost, c->s));
   MEGA_TRY(cudaStreamSynchronize(c->s));
   if (reset && st) MEGA_TRY(cudaMemsetAsync(c->status, 0, sizeof(unsigned), c->s));
+  if (st & (MEGA_ST_WAIT_TIMEOUT | MEGA_ST_NONFINITE)) c->fsteps = 0;  // increments void or lost: F afresh
   return (int)st;
 }
 
-// F - I of the other precision's sums (float ones before an FP64 step) does not
-// go on: the first step after a change forms it afresh.
-static void set_fprec(Ctx* c, int prec) {
-  if (c->fprec != prec) c->fsteps = 0;
+// The steps F - I has been advanced by for a call in precision prec: none, so
+// that its first step forms F afresh, where the other precision's sums formed
+// it.  The context's own count stays 0 until the call hands it back: one that
+// fails on the way may have moved the displacements without F.
+static int64_t take_fsteps(Ctx* c, int prec) {
+  const int64_t f = c->fprec == prec ? c->fsteps : 0;
   c->fprec = prec;
+  c->fsteps = 0;
+  return f;
 }
 
 // The records of a precision are packed at search time only when the
@@ -815,27 +820,27 @@ static int run_steps(Ctx* c, int32_t nsteps, double dt, int mode) {
   if (!(mode & MEGA_FLAG_INTERP_EACH_STEP)) c->phy_valid = false;
   int r = sync_time(c);
   if (r) return r;
-  set_fprec(c, prec);
+  int64_t fsteps = take_fsteps(c, prec);
   r = launch_predict(c->s, 3 * (int64_t)c->n, c->dsp, c->dsp_tot, c->vel, c->acl, dt, c->ndt);
   if (r) return r;
   c->launches += 1;
   // whole graphs where a full step is due, single steps around them
   for (int32_t rem = nsteps - 1; rem > 0;) {
-    if (c->fsteps % kGraphSteps == 0 && rem >= kGraphSteps) {
+    if (fsteps % kGraphSteps == 0 && rem >= kGraphSteps) {
       if ((r = graph_for(c, dt, mode, kGraphSteps))) return r;
       MEGA_TRY(cudaGraphLaunch(c->gexec, c->s));
       c->launches += c->g_kernels;
-      c->fsteps += kGraphSteps;
+      fsteps += kGraphSteps;
       rem -= kGraphSteps;
     } else {
-      if ((r = step_once(c, dt, mode, 1, nullptr, c->fsteps % kGraphSteps == 0))) return r;
-      ++c->fsteps;
+      if ((r = step_once(c, dt, mode, 1, nullptr, fsteps % kGraphSteps == 0))) return r;
+      ++fsteps;
       --rem;
     }
   }
-  r = step_once(c, dt, mode, 0, nullptr, c->fsteps % kGraphSteps == 0);
+  r = step_once(c, dt, mode, 0, nullptr, fsteps % kGraphSteps == 0);
   if (r) return r;
-  ++c->fsteps;
+  c->fsteps = fsteps + 1;
   for (int32_t k = 0; k < nsteps; ++k) c->time = c->time + dt;  // TIME = TIME + DLT
   c->steps += nsteps;
   return 0;
@@ -1906,12 +1911,12 @@ int mega_kernel_times(int64_t h, int32_t reps, double dt, int32_t mode, float* o
   cudaEvent_t ev[4];
   for (auto& e : ev) MEGA_TRY(cudaEventCreate(&e));
   double acc[3] = {0, 0, 0};
-  set_fprec(c, mode & 0xff);
+  int64_t fsteps = take_fsteps(c, mode & 0xff);
   int r = launch_predict(c->s, 3 * (int64_t)c->n, c->dsp, c->dsp_tot, c->vel, c->acl, dt, c->ndt);
   for (int32_t k = 0; k < reps && !r; ++k) {
-    r = step_once(c, dt, mode, k < reps - 1 ? 1 : 0, ev, c->fsteps % kGraphSteps == 0);
+    r = step_once(c, dt, mode, k < reps - 1 ? 1 : 0, ev, fsteps % kGraphSteps == 0);
     if (r) break;
-    ++c->fsteps;
+    ++fsteps;
     cudaEventSynchronize(ev[3]);
     float t;
     for (int q = 0; q < 3; ++q) {
@@ -1923,6 +1928,7 @@ int mega_kernel_times(int64_t h, int32_t reps, double dt, int32_t mode, float* o
   }
   for (auto& e : ev) cudaEventDestroy(e);
   if (r) return r;
+  c->fsteps = fsteps;
   for (int q = 0; q < 3; ++q) out_ms[q] = (float)(acc[q] / reps);
   return read_status(c, true);
 }

@@ -44,3 +44,24 @@ def test_precision_changed_on_a_live_context(first, second, timed):
         else:
             m.step(10, dt, mode=second)
     _assert_equal(a, b)
+
+
+@pytest.mark.parametrize("mode", ["fp64", "mixed"])
+def test_step_that_was_not_finite(mode):
+    """After a call that ended with a status of lost sums F is formed afresh: the
+    caller puts the fields right that were not finite, the displacements (which
+    were) stay."""
+    a, b, dt = _pair()
+    a.step(21, dt, mode=mode)
+    good = {f: a.download(f) for f in FIELDS}
+    bad = good[_lib.F_STRESS].copy()
+    bad[len(bad) // 2] = np.nan
+    a.upload(_lib.F_STRESS, bad)
+    assert a.step(1, dt, mode=mode, allow_status=True) & _lib.ST_NONFINITE
+    assert np.isfinite(a.download(_lib.F_DSP_TOT)).all()
+    for f in FIELDS[1:]:
+        a.upload(f, good[f])
+    _copy(a, b)
+    for m in (a, b):
+        m.step(10, dt, mode=mode)
+    _assert_equal(a, b)
