@@ -719,13 +719,15 @@ __global__ void __launch_bounds__(kHasStress<SA> && KG == 16 ? 512 : 64 * KG,
     }
   }
   grid_wait();
-  if (acc && blockIdx.x == 0 && threadIdx.x < kSlots) {
-    if constexpr (kHasStress<SA>) {
-      // (no counts of this step alone: a call's last step is not one of these)
-      acc->ke[threadIdx.x] = 0.0;
-    } else {
-      acc->newton_iters[threadIdx.x] = 0ull;
-      acc->plastic[threadIdx.x] = 0ull;
+  if (acc && blockIdx.x == 0) {
+    for (int k = threadIdx.x; k < kSlots; k += blockDim.x) {  // (a tile of 8 rows has 32 threads)
+      if constexpr (kHasStress<SA>) {
+        // (no counts of this step alone: a call's last step is not one of these)
+        acc->ke[k] = 0.0;
+      } else {
+        acc->newton_iters[k] = 0ull;
+        acc->plastic[k] = 0ull;
+      }
     }
   }
   double ur[3] = {0.0, 0.0, 0.0}, dr[3] = {0.0, 0.0, 0.0};
@@ -1311,9 +1313,11 @@ __global__ void __launch_bounds__(64 * KG)
   const unsigned gmask = group_mask<KG>();
   const bool valid = i < n;
   grid_wait();
-  if (acc && blockIdx.x == 0 && threadIdx.x < kSlots) {
-    acc->newton_iters[threadIdx.x] = 0ull;
-    acc->plastic[threadIdx.x] = 0ull;
+  if (acc && blockIdx.x == 0) {
+    for (int k = threadIdx.x; k < kSlots; k += blockDim.x) {
+      acc->newton_iters[k] = 0ull;
+      acc->plastic[k] = 0ull;
+    }
   }
   double dr[3] = {0.0, 0.0, 0.0};
   if (!F64) {
