@@ -418,27 +418,49 @@ __global__ void __launch_bounds__(512) k_pmb_step_f64(PmbArgs a) {
   pmb_finish(a, i, q, gm, f0, f1, f2, nb);
 }
 
-// E = max |X - X of particle 0| over the finite coordinates (its bits, which
-// order like the values); then X in units of 2^k >= E as a sum of two floats:
-// hi, a multiple of 2^-22 below 2 in magnitude, so that the difference of two
-// is exact, and lo, the rest.  hi_j - hi_i + (lo_j - lo_i) is then the double
-// difference rounded to float, as long bonds as short, without a conversion.
+// E = max |X - X of particle 0|, infinite with a coordinate that is not finite
+// (its bits, which order like the values), and the shortest bond; then X in
+// units of 2^k >= E as a sum of two floats: hi, a multiple of 2^-22 below 2 in
+// magnitude, so that the difference of two is exact, and lo, the rest.  hi_j -
+// hi_i + (lo_j - lo_i) is the double difference to 2^-46 E, and then rounded to
+// float, without a conversion; below a quarter of that rounding while no bond is
+// shorter than 2^-20 E.  Other particles (one far from the rest, two that almost
+// coincide) take the step that holds X in double (split_holds).
 __global__ void k_pmb_extent(int32_t n, const double* __restrict__ X, unsigned long long* __restrict__ ext) {
   const int64_t m = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   double e = m < 3 * (int64_t)n ? fabs(X[m] - X[m % 3]) : 0.0;
-  if (!(e < 1e300)) e = 0.0;
+  if (!(e < 1e300)) e = INFINITY;
   unsigned long long b = (unsigned long long)__double_as_longlong(e);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) b = max(b, __shfl_xor_sync(0xffffffffu, b, o));
   if ((threadIdx.x & 31) == 0 && b) atomicMax(ext, b);
 }
+// warp per row; *shortest starts at infinity
+__global__ void k_pmb_shortest(int32_t n, const double* __restrict__ X, const int64_t* __restrict__ rowptr,
+                               const int32_t* __restrict__ col, unsigned long long* shortest) {
+  const int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  if (r >= n) return;
+  double least = INFINITY;
+  for (int64_t p = rowptr[r] + (threadIdx.x & 31); p < rowptr[r + 1]; p += 32) {
+    const int64_t j = col[p];
+    const double x = X[3 * j] - X[3 * r], y = X[3 * j + 1] - X[3 * r + 1], z = X[3 * j + 2] - X[3 * r + 2];
+    const double d = sqrt(x * x + y * y + z * z);
+    if (d > 0.0) least = fmin(least, d);
+  }
+  unsigned long long b = (unsigned long long)__double_as_longlong(least);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) b = min(b, __shfl_xor_sync(0xffffffffu, b, o));
+  if ((threadIdx.x & 31) == 0 && b < *(volatile unsigned long long*)shortest) atomicMin(shortest, b);
+}
+inline bool split_holds(double extent, double shortest) { return extent <= 0x1p20 * shortest && extent < 1e300; }
+
 __global__ void k_pmb_split(int32_t n, const double* __restrict__ X, const double* __restrict__ vol, double c,
                             const unsigned long long* __restrict__ ext, double* __restrict__ scale,
                             float4* __restrict__ hi, float2* __restrict__ lo, float* __restrict__ cvol) {
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double E = __longlong_as_double((long long)*ext);
-  const double sg = E > 0.0 ? scalbn(1.0, -(ilogb(E) + 1)) : 1.0;  // E sg in [1/2, 1)
+  const double sg = E > 0.0 && E < 1e300 ? scalbn(1.0, -(ilogb(E) + 1)) : 1.0;  // E sg in [1/2, 1)
   if (i == 0) *scale = sg;
   float h[3], r[3];
   for (int k = 0; k < 3; ++k) {
@@ -474,7 +496,10 @@ __device__ __forceinline__ float rcp_ftz(float x) {
 // one 2-byte rank per load before); 19,600 particles 19.3 -> 9.6 us with the
 // launches overlapped.  40 registers for three blocks an SM: with 56 and two
 // blocks 140 us, with 32 and four (spills) 139 us.
-__global__ void __launch_bounds__(512, 3) k_pmb_step_f32(PmbArgs a) {
+// WIDE: positions in double, the bond vector rounded from their difference,
+// lengths as they are given (split_holds has the rule).
+template <bool WIDE>
+__global__ void __launch_bounds__(512, WIDE ? 2 : 3) k_pmb_step_f32(PmbArgs a) {
   extern __shared__ __align__(16) float4 sma[];
   const int64_t t = blockIdx.x;
   const int cnt = a.jcnt[t];
@@ -482,11 +507,19 @@ __global__ void __launch_bounds__(512, 3) k_pmb_step_f32(PmbArgs a) {
   float4* sa = sma;                                        // hi, lo.z
   float4* sb = sma + cnt;                                  // u - u_r0, c vol
   float2* sc2 = reinterpret_cast<float2*>(sma + 2 * cnt);  // lo.x, lo.y
-  const double sg = *a.scale;
+  double* sx = reinterpret_cast<double*>(sma);             // WIDE: X.x, X.y in sa's place, X.z in sc2's
+  double* sz = reinterpret_cast<double*>(sma + 2 * cnt);
+  const double sg = WIDE ? 1.0 : *a.scale;
   for (int l = threadIdx.x; l < cnt; l += blockDim.x) {
     const int64_t g = js[l];
-    sa[l] = a.hi[g];
-    sc2[l] = a.lo[g];
+    if constexpr (WIDE) {
+      sx[l] = a.X[3 * g];
+      sx[cnt + l] = a.X[3 * g + 1];
+      sz[l] = a.X[3 * g + 2];
+    } else {
+      sa[l] = a.hi[g];
+      sc2[l] = a.lo[g];
+    }
   }
   const int64_t i = t * a.R + threadIdx.x / kGP;
   const int q = threadIdx.x & (kGP - 1);
@@ -497,8 +530,10 @@ __global__ void __launch_bounds__(512, 3) k_pmb_step_f32(PmbArgs a) {
   const int w0 = mine ? (int)(a.rowptr[i] >> 5) : 0;
   const int np = mine ? (int)(a.rowptr[i + 1] >> 5) - w0 : 0;
   const uint2* rk = reinterpret_cast<const uint2*>(a.lidx);
-  const float4 hi = mine ? a.hi[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-  const float2 lo = mine ? a.lo[i] : make_float2(0.f, 0.f);
+  const float4 hi = !WIDE && mine ? a.hi[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float2 lo = !WIDE && mine ? a.lo[i] : make_float2(0.f, 0.f);
+  const double Xi0 = WIDE && mine ? a.X[3 * i] : 0.0, Xi1 = WIDE && mine ? a.X[3 * i + 1] : 0.0,
+               Xi2 = WIDE && mine ? a.X[3 * i + 2] : 0.0;
   uint2 rn = np > 0 ? rk[8 * (int64_t)w0 + q] : make_uint2(0u, 0u);
   grid_wait();
   unsigned dn = np > 0 ? a.broken[w0] : ~0u;
@@ -535,18 +570,28 @@ __global__ void __launch_bounds__(512, 3) k_pmb_step_f32(PmbArgs a) {
     for (int g = 0; g < 4; ++g) {
       if (g >= ng) break;
       const int lj = (int)(((g < 2 ? rc.x : rc.y) >> (16 * (g & 1))) & 0xFFFFu);
-      const float4 A = sa[lj], B = sb[lj];
-      const float2 C = sc2[lj];
-      const float x0 = (A.x - hi.x) + (C.x - lo.x), x1 = (A.y - hi.y) + (C.y - lo.y),
-                  x2 = (A.z - hi.z) + (A.w - hi.w);
+      const float4 B = sb[lj];
+      float x0, x1, x2;
+      if constexpr (WIDE) {
+        x0 = (float)(sx[lj] - Xi0);
+        x1 = (float)(sx[cnt + lj] - Xi1);
+        x2 = (float)(sz[lj] - Xi2);
+      } else {
+        const float4 A = sa[lj];
+        const float2 C = sc2[lj];
+        x0 = (A.x - hi.x) + (C.x - lo.x);
+        x1 = (A.y - hi.y) + (C.y - lo.y);
+        x2 = (A.z - hi.z) + (A.w - hi.w);
+      }
       const float d0 = B.x - fu0, d1 = B.y - fu1, d2 = B.z - fu2;
       const float e0 = x0 + d0, e1 = x1 + d1, e2 = x2 + d2;
       const float xx = x0 * x0 + x1 * x1 + x2 * x2, ee = e0 * e0 + e1 * e1 + e2 * e2;
       // stretch without cancellation: (|eta|^2 - |xi|^2) / (|xi| (|eta| + |xi|)),
       // lengths from the hardware reciprocal square root (about 2 ulp)
       const float num = d0 * (x0 + e0) + d1 * (x1 + e1) + d2 * (x2 + e2);
-      const float rl = rsqrt_ftz(ee);
-      const float s = num * rcp_ftz(xx + (xx * rsqrt_ftz(xx)) * (ee * rl));
+      const float rl = WIDE ? rsqrtf(ee) : rsqrt_ftz(ee);
+      const float sum = xx + (xx * (WIDE ? rsqrtf(xx) : rsqrt_ftz(xx))) * (ee * rl);
+      const float s = num * (WIDE ? __frcp_rn(sum) : rcp_ftz(sum));
       const bool on = (live & (1u << (8 * g))) && xx != 0.f;  // else broken, a pad or the particle itself
       const bool over = s > sc;
       const float w = (s * B.w) * rl;
@@ -793,6 +838,7 @@ struct PmbCtx {
   float2* lo = nullptr;
   float* cvol = nullptr;
   double* scale = nullptr;
+  bool wide = false;  // mixed: X in double instead (split_holds)
   uint16_t *lt = nullptr, *kpos = nullptr;  // the mixed rows' order (k_pmb_order)
   uint32_t* broken = nullptr;
   int8_t* fixed = nullptr;
@@ -829,7 +875,8 @@ static int launch_pmb(PmbCtx* c, const PmbArgs& a) {
   const unsigned grid = (unsigned)c->tiles.ntiles;
   const int block = c->tiles.R * kGP;
   const size_t smem = (c->f64 ? 64 : 40) * (size_t)c->tiles.maxcnt + 16;
-  return launch_overlapped(c->f64 ? k_pmb_step_f64 : k_pmb_step_f32, grid, block, smem, c->s, a);
+  auto k = c->f64 ? k_pmb_step_f64 : (c->wide ? k_pmb_step_f32<true> : k_pmb_step_f32<false>);
+  return launch_overlapped(k, grid, block, smem, c->s, a);
 }
 
 }  // namespace mega
@@ -1110,7 +1157,9 @@ int mega_pmb_init(int32_t n, const double* coo, const double* vol, const double*
     if (!smem_set) {
       if (cudaFuncSetAttribute(k_pmb_step_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024 + 16) !=
               cudaSuccess ||
-          cudaFuncSetAttribute(k_pmb_step_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, 40 * 1024 + 16) !=
+          cudaFuncSetAttribute(k_pmb_step_f32<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 40 * 1024 + 16) !=
+              cudaSuccess ||
+          cudaFuncSetAttribute(k_pmb_step_f32<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 40 * 1024 + 16) !=
               cudaSuccess)
         return fail(MEGA_ERR_CUDA);
       smem_set = true;
@@ -1118,19 +1167,23 @@ int mega_pmb_init(int32_t n, const double* coo, const double* vol, const double*
   }
   const int64_t words = (mp + 31) / 32;
   void* spent[2] = {nullptr, nullptr};
+  double range[2] = {0.0, INFINITY};  // extent and shortest bond
   PA(c->broken, words);
   if (c->f64) {
     cudaMemsetAsync(c->broken, 0, sizeof(uint32_t) * words, c->s);
     k_pmb_padbits<<<gn, 256, 0, c->s>>>(n, c->perm, c->rowptr0, c->csr.rowptr, c->broken);
   } else {
     int32_t* col2 = nullptr;
-    unsigned long long* ext = nullptr;
+    double* ext = nullptr;
     PA(c->hi, n); PA(c->lo, n); PA(c->cvol, n); PA(c->scale, 1); PA(c->lt, mp); PA(c->kpos, mp); PA(col2, mp);
-    if (tmp.alloc(&ext, 1)) return fail(MEGA_ERR_NOMEM);
-    cudaMemsetAsync(ext, 0, sizeof(*ext), c->s);
-    k_pmb_extent<<<g3, 256, 0, c->s>>>(n, c->X, ext);
-    k_pmb_split<<<gn, 256, 0, c->s>>>(n, c->X, c->vol, micromodulus, ext, c->scale, c->hi, c->lo,
+    if (tmp.alloc(&ext, 2)) return fail(MEGA_ERR_NOMEM);
+    cudaMemcpyAsync(ext, range, sizeof(range), cudaMemcpyHostToDevice, c->s);
+    unsigned long long* bits = reinterpret_cast<unsigned long long*>(ext);
+    k_pmb_extent<<<g3, 256, 0, c->s>>>(n, c->X, bits);
+    k_pmb_shortest<<<gw, 256, 0, c->s>>>(n, c->X, c->csr.rowptr, c->csr.col, bits + 1);
+    k_pmb_split<<<gn, 256, 0, c->s>>>(n, c->X, c->vol, micromodulus, bits, c->scale, c->hi, c->lo,
                                       c->cvol);
+    cudaMemcpyAsync(range, ext, sizeof(range), cudaMemcpyDeviceToHost, c->s);
     k_pmb_order<<<gw, 256, 0, c->s>>>(n, c->perm, c->rowptr0, c->csr.rowptr, c->csr.col, c->tiles.lidx, col2, c->lt,
                                       c->kpos, c->broken);
     spent[0] = c->csr.col;  // released below, once the kernel that reads them is done
@@ -1147,6 +1200,7 @@ int mega_pmb_init(int32_t n, const double* coo, const double* vol, const double*
                                          true);
   }
   if (cudaStreamSynchronize(c->s) != cudaSuccess || cudaGetLastError() != cudaSuccess) return fail(MEGA_ERR_CUDA);
+  c->wide = !c->f64 && !split_holds(range[0], range[1]);
   for (void* p : spent) c->pool.release(p);
   if (nbonds) *nbonds = m;
   {
