@@ -848,11 +848,17 @@ struct PmbCtx {
   int f64 = 0;
   int cur = 0;
   int64_t steps = 0;
-  cudaGraphExec_t g = nullptr;
+  cudaGraphExec_t g[2][2] = {};  // kPmbGraph, and two, steps captured from either buffer, at dt g_dt
   double g_dt = 0;
-  int g_cur = 0;  // the buffer the graph starts from
+  void drop_graphs() {
+    for (auto& of : g)
+      for (auto& e : of) {
+        if (e) cudaGraphExecDestroy(e);
+        e = nullptr;
+      }
+  }
   ~PmbCtx() {
-    if (g) cudaGraphExecDestroy(g);
+    drop_graphs();
     pool.free_all();  // stream-ordered frees before the stream goes
     if (s) {
       cudaStreamSynchronize(s);
@@ -1213,6 +1219,31 @@ int mega_pmb_init(int32_t n, const double* coo, const double* vol, const double*
 
 constexpr int kPmbGraph = 16;  // steps per captured graph
 
+// A graph of len steps, an even number: the ping-pong buffers return to where
+// they started.  A context holds one for either buffer, as calls of an odd
+// number of steps start from each in turn (17 a call, 1,600 particles in FP64:
+// captured in each call 14.7 us a step, held 5.4), and one of two steps for calls
+// of two or three, which single launches serve worse (calls of two 11.3 and 10.3
+// us a step; from five on single launches are ahead).
+static int capture_steps(PmbCtx* c, double dt, int len, cudaGraphExec_t& out) {
+  cudaGraph_t gr = nullptr;
+  MEGA_TRY(cudaStreamBeginCapture(c->s, cudaStreamCaptureModeThreadLocal));
+  int r = 0;
+  for (int k = 0; k < len; ++k) {
+    if (!r) r = launch_pmb(c, pmb_args(c, dt));
+    c->cur = 1 - c->cur;
+  }
+  cudaError_t e = cudaStreamEndCapture(c->s, &gr);
+  if (r) { if (gr) cudaGraphDestroy(gr); return r; }
+  if (e != cudaSuccess) { record_cuda_error(e, "capture", __FILE__, __LINE__); return MEGA_ERR_CUDA; }
+  e = cudaGraphInstantiate(&out, gr, 0);
+  cudaGraphDestroy(gr);
+  if (e == cudaSuccess) return 0;
+  out = nullptr;
+  record_cuda_error(e, "instantiate", __FILE__, __LINE__);
+  return MEGA_ERR_CUDA;
+}
+
 // nsteps of velocity-Verlet: the first step starts from a = 0 like the
 // reference's STATE_INIT (the predictor of step 1 is u = dt v).
 int mega_pmb_step(int64_t h, int32_t nsteps, double dt, float* ms) {
@@ -1230,27 +1261,16 @@ int mega_pmb_step(int64_t h, int32_t nsteps, double dt, float* ms) {
     MEGA_CHECK_LAUNCH();
   }
   int done = 0;
-  // graph of kPmbGraph steps, an even number: the ping-pong buffers return to
-  // where they started
-  if (nsteps >= kPmbGraph && (c->g == nullptr || c->g_dt != dt || c->g_cur != c->cur)) {
-    if (c->g) { cudaGraphExecDestroy(c->g); c->g = nullptr; }
-    cudaGraph_t gr;
-    MEGA_TRY(cudaStreamBeginCapture(c->s, cudaStreamCaptureModeThreadLocal));
-    int r = 0;
-    for (int k = 0; k < kPmbGraph; ++k) {
-      if (!r) r = launch_pmb(c, pmb_args(c, dt));
-      c->cur = 1 - c->cur;
-    }
-    cudaError_t e = cudaStreamEndCapture(c->s, &gr);
-    if (r) { if (gr) cudaGraphDestroy(gr); return r; }
-    if (e != cudaSuccess) { record_cuda_error(e, "capture", __FILE__, __LINE__); return MEGA_ERR_CUDA; }
-    e = cudaGraphInstantiate(&c->g, gr, 0);
-    cudaGraphDestroy(gr);
-    if (e != cudaSuccess) { record_cuda_error(e, "instantiate", __FILE__, __LINE__); return MEGA_ERR_CUDA; }
+  const bool pair = nsteps == 2 || nsteps == 3;
+  if (nsteps >= kPmbGraph || pair) {
+    const int len = pair ? 2 : kPmbGraph;
+    if (c->g_dt != dt) c->drop_graphs();
+    cudaGraphExec_t& g = c->g[pair][c->cur];
+    if (!g)
+      if (int r = capture_steps(c, dt, len, g)) return r;
     c->g_dt = dt;
-    c->g_cur = c->cur;
+    for (; nsteps - done >= len; done += len) MEGA_TRY(cudaGraphLaunch(g, c->s));
   }
-  for (; nsteps - done >= kPmbGraph; done += kPmbGraph) MEGA_TRY(cudaGraphLaunch(c->g, c->s));
   for (; done < nsteps; ++done) {
     if (int r = launch_pmb(c, pmb_args(c, dt))) return r;
     MEGA_CHECK_LAUNCH();
