@@ -867,82 +867,92 @@ static int upload(cudaStream_t s, T* d, const T* h, size_t count) {
   return 0;
 }
 
-// Device CSR from the reference's 1-based (GN, GSTART, GSTACK); rows are
-// re-packed contiguously in node order.  hpos[k] = 0-based GSTACK position
-// of packed entry k (for writing per-entry values back).
-// Warp per node: a caller's row (start k0[i], raw 1-based ids from list
-// position lo on) as CSR columns and list positions; ids out of range raise bad.
-__global__ void k_caller_rows(int32_t n, const int64_t* __restrict__ rowptr, const int64_t* __restrict__ k0,
-                              const int32_t* __restrict__ raw, int32_t* __restrict__ col, int64_t* __restrict__ pos,
-                              int32_t* __restrict__ bad) {
-  const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (i >= n) return;
-  const int64_t b = rowptr[i], len = rowptr[i + 1] - b;
-  for (int64_t k = lane; k < len; k += 32) {
-    const int32_t j = raw[k0[i] + k] - 1;
-    const bool ok = j >= 0 && j < n;
-    if (!ok) *bad = 1;
-    col[b + k] = ok ? j : 0;
-    pos[b + k] = k0[i] + k;
-  }
-}
-// shapes and gradients at the entries' list positions
-__global__ void k_caller_shapes(int64_t m, const int64_t* __restrict__ pos, const double* __restrict__ shp,
-                                const double* __restrict__ dshp, double* __restrict__ osh, double* __restrict__ gx,
-                                double* __restrict__ gy, double* __restrict__ gz) {
+// raw 1-based ids as CSR columns, in place; ids out of range raise bad
+__global__ void k_caller_ids(int64_t m, int32_t n, int32_t* __restrict__ col, int32_t* __restrict__ bad) {
   const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (e >= m) return;
-  const int64_t q = pos[e];
-  osh[e] = shp[q];
-  gx[e] = dshp[3 * q];
-  gy[e] = dshp[3 * q + 1];
-  gz[e] = dshp[3 * q + 2];
+  const int32_t j = col[e] - 1;
+  const bool ok = j >= 0 && j < n;
+  if (!ok) *bad = 1;
+  col[e] = ok ? j : 0;
+}
+// a caller's gradients (3, m) as three arrays
+__global__ void k_caller_gradients(int64_t m, const double* __restrict__ dshp, double* __restrict__ gx,
+                                   double* __restrict__ gy, double* __restrict__ gz) {
+  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (e >= m) return;
+  gx[e] = dshp[3 * e];
+  gy[e] = dshp[3 * e + 1];
+  gz[e] = dshp[3 * e + 2];
 }
 
-// A caller's lists as CSR on the device, checked there, with the list position
-// (from `lo` on) of every entry.  The calling thread only forms the row
-// offsets; the ids go up as they are.
+// A caller's lists: the row offsets of the packed entries and where in the
+// caller's stacks each row starts.
 struct CallerLists {
-  int64_t lo = 0, hi = 0;    // the list positions in use
-  int64_t* pos = nullptr;    // per entry: its position less lo
+  std::vector<int64_t> rp, k0;
+  int64_t first = 0;  // the place of entry 0
+  bool tight = true;  // the rows lie one after another in node order
 };
+
+// `width` values of T per list place, the rows' places packed in node order, as
+// arrays to upload to dst: lists without gaps as they lie, others row by row on
+// the way through the stage (so the device holds what the rows use, not the
+// places between them), in pieces of 4 MiB.
+template <typename T>
+static void upload_rows(std::vector<HostToDevice>& items, T* dst, const T* src, int width, const CallerLists& cl) {
+  const int64_t m = cl.rp.back(), per = sizeof(T) * width;
+  if (m == 0) return;
+  if (cl.tight) {
+    items.push_back({dst, src + width * cl.first, (size_t)(m * per)});
+    return;
+  }
+  const int64_t piece = ((int64_t)4 << 20) / per;
+  for (int64_t e0 = 0; e0 < m; e0 += piece) {
+    const int64_t e1 = std::min(m, e0 + piece);
+    items.push_back({dst + width * e0, nullptr, (size_t)((e1 - e0) * per), [=, &cl](void* to) {
+      size_t i = std::upper_bound(cl.rp.begin(), cl.rp.end(), e0) - cl.rp.begin() - 1;  // the row of entry e0
+      T* o = (T*)to;
+      for (int64_t e = e0; e < e1; ++i) {
+        const int64_t k = std::min(e1, cl.rp[i + 1]) - e;
+        std::memcpy(o, src + width * (cl.k0[i] + e - cl.rp[i]), (size_t)(k * per));
+        o += width * k;
+        e += k;
+      }
+    }});
+  }
+}
+
+// A caller's lists as CSR on the device, checked there.
 static int csr_from_caller(cudaStream_t s, int32_t n, const int32_t* gn, const int32_t* gstart,
                            const int32_t* gstack, int64_t nnz_cap, DevPool& pool, DevCSR& csr, CallerLists& cl) {
-  std::vector<int64_t> rp(n + 1, 0), k0(n, 0);
-  int64_t lo = INT64_MAX, hi = 0;
+  cl.rp.assign((size_t)n + 1, 0);
+  cl.k0.assign(n, 0);
   csr.gmaxn = 0;
+  int64_t next = -1;
   for (int32_t i = 0; i < n; ++i) {
     if (gn[i] < 0) return MEGA_ERR_ARG;
-    rp[i + 1] = rp[i] + gn[i];
+    cl.rp[i + 1] = cl.rp[i] + gn[i];
     csr.gmaxn = std::max(csr.gmaxn, gn[i]);
     if (gn[i] == 0) continue;
-    k0[i] = (int64_t)gstart[i] - 1;
-    if (k0[i] < 0 || k0[i] + gn[i] > nnz_cap) return MEGA_ERR_ARG;
-    lo = std::min(lo, k0[i]);
-    hi = std::max(hi, k0[i] + gn[i]);
+    cl.k0[i] = (int64_t)gstart[i] - 1;
+    if (cl.k0[i] < 0 || cl.k0[i] + gn[i] > nnz_cap) return MEGA_ERR_ARG;
+    if (next < 0) cl.first = cl.k0[i];
+    else cl.tight = cl.tight && cl.k0[i] == next;
+    next = cl.k0[i] + gn[i];
   }
-  const int64_t m = rp[n];
+  const int64_t m = cl.rp[n];
   csr.n = n;
   csr.nnz = m;
-  cl.lo = m ? lo : 0;
-  cl.hi = hi;
-  for (int32_t i = 0; i < n; ++i)
-    if (gn[i] > 0) k0[i] -= cl.lo;
   MEGA_ALLOC(pool, csr.rowptr, (int64_t)n + 1);
   MEGA_ALLOC(pool, csr.col, m);
-  MEGA_ALLOC(pool, cl.pos, m);
   DevPool tmp(s);
-  int64_t* dk0 = nullptr;
-  int32_t *raw = nullptr, *bad = nullptr;
-  MEGA_ALLOC(tmp, dk0, n);
-  MEGA_ALLOC(tmp, raw, cl.hi - cl.lo);
+  int32_t* bad = nullptr;
   MEGA_ALLOC(tmp, bad, 1);
   MEGA_TRY(cudaMemsetAsync(bad, 0, sizeof(int32_t), s));
-  int r = upload_batched(s, {{csr.rowptr, rp.data(), 8 * ((size_t)n + 1)}, {dk0, k0.data(), 8 * (size_t)n},
-                             {raw, gstack + cl.lo, 4 * (size_t)(cl.hi - cl.lo)}});
-  if (r) return r;
-  k_caller_rows<<<grid_for((int64_t)n * 32, 256), 256, 0, s>>>(n, csr.rowptr, dk0, raw, csr.col, cl.pos, bad);
+  std::vector<HostToDevice> items = {{csr.rowptr, cl.rp.data(), 8 * ((size_t)n + 1)}};
+  upload_rows(items, csr.col, gstack, 1, cl);
+  if (int r = upload_batched(s, items)) return r;
+  k_caller_ids<<<grid_for(m, 256), 256, 0, s>>>(m, n, csr.col, bad);
   MEGA_CHECK_LAUNCH();
   int32_t hb = 0;
   MEGA_TRY(cudaMemcpyAsync(&hb, bad, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
@@ -950,6 +960,9 @@ static int csr_from_caller(cudaStream_t s, int32_t n, const int32_t* gn, const i
   return hb ? MEGA_ERR_ARG : 0;
 }
 
+// Device CSR from the reference's 1-based (GN, GSTART, GSTACK); rows are
+// re-packed contiguously in node order.  hpos[k] = 0-based GSTACK position
+// of packed entry k (for writing per-entry values back).
 static int csr_from_host(cudaStream_t s, int32_t n, const int32_t* gn, const int32_t* gstart,
                          const int32_t* gstack, int64_t nnz_cap, DevPool& pool, DevCSR& csr,
                          std::vector<int64_t>& hpos) {
@@ -2850,13 +2863,11 @@ static int construct_fint_impl(const mega_params* p, const FintIO& io) {
   if (semi) MEGA_TRY(cudaMemsetAsync(dtot, 0, 3 * n8, s));
   else items.push_back({dtot, io.gdinc_tot, 3 * n8});
   DevPool raw(s);
-  double *rsh = nullptr, *rdsh = nullptr;
+  double* rdsh = nullptr;
   if (!shapes_here) {
-    const int64_t used = cl.hi - cl.lo;
-    MEGA_ALLOC(raw, rsh, used);
-    MEGA_ALLOC(raw, rdsh, 3 * used);
-    items.push_back({rsh, io.gstack_shp + cl.lo, 8 * (size_t)used});
-    items.push_back({rdsh, io.gstack_dshp + 3 * cl.lo, 24 * (size_t)used});
+    MEGA_ALLOC(raw, rdsh, 3 * m);
+    upload_rows(items, dsh, (const double*)io.gstack_shp, 1, cl);
+    upload_rows(items, rdsh, (const double*)io.gstack_dshp, 3, cl);
   }
   if ((r = upload_batched(s, items))) return r;
   MEGA_TRY(cudaMemsetAsync(acc, 0, sizeof(StepAccum), s));
@@ -2865,7 +2876,7 @@ static int construct_fint_impl(const mega_params* p, const FintIO& io) {
     r = rk_shapes(s, *p, n, semi ? dcur : dc, dw, den, csr, dsh, dgx, dgy, dgz, st);
     if (r) return r;
   } else {
-    k_caller_shapes<<<grid_for(m, 256), 256, 0, s>>>(m, cl.pos, rsh, rdsh, dsh, dgx, dgy, dgz);
+    k_caller_gradients<<<grid_for(m, 256), 256, 0, s>>>(m, rdsh, dgx, dgy, dgz);
     MEGA_CHECK_LAUNCH();
     raw.free_all();
   }
