@@ -369,7 +369,8 @@ int mega_set_instance_dt(int64_t h, const double* dt_inst);
  * fastest, and leave the state as it was.  The first call for a precision
  * reorders its packed records within each row and column for the gathers'
  * shared-memory banks: from then on that precision's sums run in the new
- * order (FP64 too, where they differ from the list order's by rounding).
+ * order (FP64 too, where they differ from the list order's by rounding);
+ * without the device memory for a second set of them they stay as they are.
  * Variants 0..3, 6 and 7 hold the
  * packed records in registers (lanes per row x records in flight: (4, 4),
  * (4, 2), (4, 1), (8, 2), (16, 1), (16, 2)); 4 and 5 have the copy engine

@@ -1148,6 +1148,7 @@ int cached_alloc(void** p, size_t bytes, cudaStream_t s, size_t* got) {
     e = cudaMallocAsync(p, want, s);
   }
   if (e != cudaSuccess) {
+    cudaGetLastError();  // not for the next launch's check to find
     record_cuda_error(e, "cudaMallocAsync", __FILE__, __LINE__);
     *p = nullptr;
     return MEGA_ERR_NOMEM;
@@ -2186,7 +2187,7 @@ static int bank_layout(Ctx* c, bool mixed) {
   const int64_t m = c->csr.nnz, rec = mixed ? 16 : 26;
   const int32_t n = c->n;
   const bool ns = c->ns_scol[mixed];
-  DevPool tmp(c->s);
+  DevPool tmp(c->s), fresh(c->s);  // (the new arrays, the context's once they are all there)
   uint16_t* l = nullptr;
   int64_t* pos = nullptr;
   MEGA_ALLOC(tmp, l, m);
@@ -2198,17 +2199,17 @@ static int bank_layout(Ctx* c, bool mixed) {
       (r = bank_order(c->s, n, c->ct, c->csr.colptr, l, nullptr, pos, ns && mixed ? 8 : 4)))
     return r;
   unsigned char* tp = nullptr;
-  MEGA_ALLOC(c->nbpool, tp, rec * c->ct.nrec);
+  MEGA_ALLOC(fresh, tp, rec * c->ct.nrec);
   if ((r = gather_records(c->s, n, c->ct, c->csr.colptr, pos, !mixed, tpk, tp))) return r;
   double* ts = nullptr;
   if (tshp) {
-    MEGA_ALLOC(c->nbpool, ts, m);
+    MEGA_ALLOC(fresh, ts, m);
     k_gather_pos<<<grid_for(m, 256), 256, 0, c->s>>>(m, pos, tshp, ts);
     MEGA_CHECK_LAUNCH();
   }
   unsigned char* sc = nullptr;
   if (ns) {
-    MEGA_ALLOC(c->nbpool, sc, (mixed ? 24 : 48) * c->ct.nrec);
+    MEGA_ALLOC(fresh, sc, (mixed ? 24 : 48) * c->ct.nrec);
     if ((r = gather_second(c->s, n, c->ct, c->csr.colptr, pos, !mixed, c->ns_scol[mixed], sc))) return r;
   }
   // rows
@@ -2218,18 +2219,19 @@ static int bank_layout(Ctx* c, bool mixed) {
     return r;
   unsigned char* rp = nullptr;
   double* sh = nullptr;
-  MEGA_ALLOC(c->nbpool, rp, rec * c->rt.nrec);
-  MEGA_ALLOC(c->nbpool, sh, m);
+  MEGA_ALLOC(fresh, rp, rec * c->rt.nrec);
+  MEGA_ALLOC(fresh, sh, m);
   if ((r = gather_records(c->s, n, c->rt, c->csr.rowptr, pos, !mixed, pk, rp))) return r;
   k_gather_pos<<<grid_for(m, 256), 256, 0, c->s>>>(m, pos, c->shp, sh);
   MEGA_CHECK_LAUNCH();
   unsigned char* sr = nullptr;
   if (ns) {
-    MEGA_ALLOC(c->nbpool, sr, (mixed ? 24 : 48) * c->rt.nrec);
+    MEGA_ALLOC(fresh, sr, (mixed ? 24 : 48) * c->rt.nrec);
     if ((r = gather_second(c->s, n, c->rt, c->csr.rowptr, pos, !mixed, c->ns_srow[mixed], sr))) return r;
   }
   MEGA_TRY(cudaStreamSynchronize(c->s));
   drop_graph(c);  // captured steps hold the old arrays
+  c->nbpool.adopt(fresh);
   c->nbpool.release(tpk); tpk = tp;
   if (ts) { c->nbpool.release(tshp); tshp = ts; }
   if (sc) { c->nbpool.release(c->ns_scol[mixed]); c->ns_scol[mixed] = sc; }
@@ -2249,7 +2251,8 @@ int mega_autotune(int64_t h, double dt, int32_t mode, int32_t reps, int32_t* cho
   if (reps <= 0) return MEGA_ERR_ARG;
   const bool mixed = (mode & 0xff) == MEGA_MODE_MIXED;
   { int r = mixed ? ensure_mixed(c) : ensure_fp64(c); if (r) return r; }
-  if (int r = bank_layout(c, mixed)) return r;
+  // without the device memory for a second set of records they stay as they are
+  if (int r = bank_layout(c, mixed); r && r != MEGA_ERR_NOMEM) return r;
   const int nvar = tiled_variants();
   const size_t n = (size_t)c->n, n3 = 3 * n;
   // snapshot of everything a step writes
