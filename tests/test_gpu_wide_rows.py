@@ -38,3 +38,33 @@ def test_counts_of_the_last_step(mode, variant):
     assert s["plastic_nodes"] > 0.9 * c["n"]
     assert s["plastic_nodes"] == s["plastic_nodes_total"] - before["plastic_nodes_total"]
     assert s["newton_iters"] == s["newton_iters_total"] - before["newton_iters_total"]
+
+
+@pytest.mark.parametrize("wide", [False, True])
+@pytest.mark.parametrize("variant", [0, 3])
+@pytest.mark.parametrize("mode", ["fp64", "mixed"])
+def test_bank_ordered_records_match_list_order(mode, variant, wide):
+    """Records reordered by the tuner, in tiles of 64 rows (7,458 nodes) and in rows
+    too long for the pass's shared memory (8 of up to 441 entries a warp), with the
+    interpolation's and the body force's shape values following them.  20 steps of
+    sums of up to 441 terms: 20 * 441 * 1.1e-16 = 1e-12 of the largest value, taken
+    as 1e-10; mixed the same with 6e-8, 5.3e-4."""
+    c = _wide_bar() if wide else cases.taylor_bar(h=0.5e-3, seed=6)
+    c["bodyforce"] = np.random.default_rng(7).normal(scale=1.0e5, size=(c["n"], 3))
+    p = _lib.params(**cases.param_kwargs(c, gravity=(0.0, 1.0e5, -2.0e5)))
+    dt = cases.lattice_dt(c, 0.25)
+    out = []
+    for tuned in (False, True):
+        m = mega.Mega(c, p)
+        m.search_and_shapes()
+        if tuned:
+            m.autotune(dt, mode=mode, reps=1)
+        m.set_variants(variant, variant, mode=mode)
+        m.step(20, dt, mode=mode, interp_each_step=True)
+        out.append([m.download(_lib.F_COO_CURRENT) - c["coo"]] +
+                   [m.download(f) for f in (_lib.F_VEL, _lib.F_STRESS, _lib.F_FEXT)])
+        m.close()
+    tol = 1e-10 if mode == "fp64" else 5.3e-4
+    assert any((a != b).any() for a, b in zip(*out))  # (the sums did run in another order)
+    for want, got in zip(*out):
+        assert np.abs(got - want).max() <= tol * np.abs(want).max()
