@@ -2196,7 +2196,7 @@ static int bank_layout(Ctx* c, bool mixed) {
   // columns (the lanes per column of the force variant the context favours)
   MEGA_TRY(cudaMemcpyAsync(l, c->ct.lidx, sizeof(uint16_t) * m, cudaMemcpyDeviceToDevice, c->s));
   if ((r = iota64(c->s, m, pos)) ||
-      (r = bank_order(c->s, n, c->ct, c->csr.colptr, l, nullptr, pos, ns && mixed ? 8 : 4)))
+      (r = bank_order(c->s, n, c->ct, c->csr.colptr, l, pos, ns && mixed ? 8 : 4)))
     return r;
   unsigned char* tp = nullptr;
   MEGA_ALLOC(fresh, tp, rec * c->ct.nrec);
@@ -2215,7 +2215,7 @@ static int bank_layout(Ctx* c, bool mixed) {
   // rows
   MEGA_TRY(cudaMemcpyAsync(l, c->rt.lidx, sizeof(uint16_t) * m, cudaMemcpyDeviceToDevice, c->s));
   if ((r = iota64(c->s, m, pos)) ||
-      (r = bank_order(c->s, n, c->rt, c->csr.rowptr, l, nullptr, pos, 4)))
+      (r = bank_order(c->s, n, c->rt, c->csr.rowptr, l, pos, 4)))
     return r;
   unsigned char* rp = nullptr;
   double* sh = nullptr;

@@ -307,14 +307,10 @@ int launch_stress(cudaStream_t s, bool mixed, const StressArgs& a);
 
 // ---------------- NSNI (nsni.cu)
 // smoothed second derivatives per list entry, one array per component:
-// XX, YY, ZZ, XY, YZ, XZ (double for the set-up and FP64 steps, float for
-// the mixed steps)
-template <typename V>
-struct NsniArr {
-  V* v[6];
+// XX, YY, ZZ, XY, YZ, XZ
+struct NsniS {
+  double* v[6];
 };
-using NsniS = NsniArr<double>;
-using NsniSF = NsniArr<float>;
 struct NsniStepArgs {
   int32_t n;
   double* fg;                // F - I and G0 of this step

@@ -74,10 +74,9 @@ __global__ void k_nsni_combine(int32_t n, int a, const int64_t* __restrict__ row
   }
 }
 
-// hq[(6 k + q) ld + i] = sum_J S_q(J) du_J,k (S double or float, sums in double)
-template <typename SV>
+// hq[(6 k + q) ld + i] = sum_J S_q(J) du_J,k
 __global__ void __launch_bounds__(256) k_nsni_h(int32_t n, const int64_t* __restrict__ rowptr,
-                                                const int32_t* __restrict__ col, NsniArr<SV> s, const double* du,
+                                                const int32_t* __restrict__ col, NsniS s, const double* du,
                                                 double* hq) {
   grid_wait();
   const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kNL;
@@ -92,7 +91,7 @@ __global__ void __launch_bounds__(256) k_nsni_h(int32_t n, const int64_t* __rest
   auto add = [&](int64_t p, double u0, double u1, double u2) {
 #pragma unroll
     for (int c = 0; c < 6; ++c) {
-      const double sv = (double)s.v[c][p];
+      const double sv = s.v[c][p];
       h[c] += sv * u0;
       h[6 + c] += sv * u1;
       h[12 + c] += sv * u2;
@@ -294,40 +293,29 @@ __global__ void __launch_bounds__(128) k_nsni_stress(NsniStepArgs a) {
   }
 }
 
-// fstab[3 J + k] = sum over the rows i holding J of sum_q W_i(k, q) S_q(i, J);
-// V = the arithmetic and storage type of S and W (double or float)
-template <typename V>
+// fstab[3 J + k] = sum over the rows i holding J of sum_q W_i(k, q) S_q(i, J)
 __global__ void __launch_bounds__(256) k_nsni_force(int32_t n, const int64_t* __restrict__ colptr,
-                                                    const int32_t* __restrict__ trow, NsniArr<V> st,
-                                                    const V* w, double* fstab) {
+                                                    const int32_t* __restrict__ trow, NsniS st,
+                                                    const double* w, double* fstab) {
   grid_wait();
   const int64_t J = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / kNL;
   const int q = threadIdx.x & (kNL - 1);
   const unsigned gm = 0xFFu << (threadIdx.x & 24);
   if (J >= n) return;
-  V f0 = V(0), f1 = V(0), f2 = V(0);
+  double f0 = 0.0, f1 = 0.0, f2 = 0.0;
   // the row's 18 weights as 16-byte loads
-  auto load_w = [&](int64_t e, V* wi) {
-    if constexpr (sizeof(V) == 4) {
-      const float4* src = reinterpret_cast<const float4*>(w + kW * (int64_t)trow[e]);
+  auto load_w = [&](int64_t e, double* wi) {
+    const double2* src = reinterpret_cast<const double2*>(w + kW * (int64_t)trow[e]);
 #pragma unroll
-      for (int k = 0; k < 5; ++k) {
-        const float4 x = src[k];
-        wi[4 * k] = x.x; wi[4 * k + 1] = x.y; wi[4 * k + 2] = x.z; wi[4 * k + 3] = x.w;
-      }
-    } else {
-      const double2* src = reinterpret_cast<const double2*>(w + kW * (int64_t)trow[e]);
-#pragma unroll
-      for (int k = 0; k < 9; ++k) {
-        const double2 x = src[k];
-        wi[2 * k] = x.x; wi[2 * k + 1] = x.y;
-      }
+    for (int k = 0; k < 9; ++k) {
+      const double2 x = src[k];
+      wi[2 * k] = x.x; wi[2 * k + 1] = x.y;
     }
   };
-  auto add = [&](int64_t e, const V* wi) {
+  auto add = [&](int64_t e, const double* wi) {
 #pragma unroll
     for (int c = 0; c < 6; ++c) {
-      const V sv = st.v[c][e];
+      const double sv = st.v[c][e];
       f0 += wi[c] * sv;
       f1 += wi[6 + c] * sv;
       f2 += wi[12 + c] * sv;
@@ -337,14 +325,14 @@ __global__ void __launch_bounds__(256) k_nsni_force(int32_t n, const int64_t* __
   int64_t e = colptr[J] + q;
   const int64_t ee = colptr[J + 1];
   for (; e + kNL < ee; e += 2 * kNL) {
-    V wa[kW], wb[kW];
+    double wa[18], wb[18];
     load_w(e, wa);
     load_w(e + kNL, wb);
     add(e, wa);
     add(e + kNL, wb);
   }
   if (e < ee) {
-    V wa[kW];
+    double wa[18];
     load_w(e, wa);
     add(e, wa);
   }
@@ -355,9 +343,9 @@ __global__ void __launch_bounds__(256) k_nsni_force(int32_t n, const int64_t* __
     f2 += __shfl_xor_sync(gm, f2, o);
   }
   if (q == 0) {
-    fstab[3 * J] = (double)f0;
-    fstab[3 * J + 1] = (double)f1;
-    fstab[3 * J + 2] = (double)f2;
+    fstab[3 * J] = f0;
+    fstab[3 * J + 1] = f1;
+    fstab[3 * J + 2] = f2;
   }
 }
 
@@ -389,9 +377,9 @@ int nsni_step(cudaStream_t s, const NsniStepArgs& a, const DevCSR& csr, const Ns
   const unsigned gg = (unsigned)(((int64_t)a.n * kNL + 255) / 256);
   const unsigned gn = (unsigned)((a.n + 127) / 128);
   if (mixed && stage != 1) return MEGA_ERR_UNSUPPORTED;  // the tiled gathers carry those terms
-  if (stage == 0) return launch_overlapped(k_nsni_h<double>, gg, 256, 0, s, a.n, csr.rowptr, csr.col, rows, du, a.hq);
+  if (stage == 0) return launch_overlapped(k_nsni_h, gg, 256, 0, s, a.n, csr.rowptr, csr.col, rows, du, a.hq);
   if (stage == 1) return launch_overlapped(mixed ? k_nsni_stress<float> : k_nsni_stress<double>, gn, 128, 0, s, a);
-  return launch_overlapped(k_nsni_force<double>, gg, 256, 0, s, a.n, csr.colptr, csr.trow, cols, (const double*)a.w,
+  return launch_overlapped(k_nsni_force, gg, 256, 0, s, a.n, csr.colptr, csr.trow, cols, (const double*)a.w,
                            a.fstab);
 }
 

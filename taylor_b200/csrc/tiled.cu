@@ -268,15 +268,14 @@ __global__ void k_pad_f32(int32_t n, int32_t R, int64_t slots, SliceView v, cons
 // the row's remaining entries allow (greedy, lanes in order, each taking its
 // first entry whose class is free or holds the same rank); a row keeps all
 // its entries, only their order changes.
-// pos, when given, is permuted with lidx.  One warp per warp of the gather's
+// pos (the identity on entry) is permuted with lidx.  One warp per warp of the gather's
 // blocks, four warps per block.
 constexpr int kBankCap = 2048;  // entries of one warp's rows that its pass stages in shared memory
 
 template <int KG, int NC, int GL>
 __global__ void __launch_bounds__(128) k_bank_order(int32_t n, int32_t R, int64_t nwarps,
                                                     const uint8_t* __restrict__ ord,
-                                                    const int64_t* __restrict__ ptr, uint16_t* lidx,
-                                                    const int64_t* __restrict__ pos_src, int64_t* pos) {
+                                                    const int64_t* __restrict__ ptr, uint16_t* lidx, int64_t* pos) {
   __shared__ int held_s[4][32];
   __shared__ uint16_t sl_s[4][kBankCap], so_s[4][kBankCap];  // ranks, and offsets in the row before
   const int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
@@ -345,7 +344,7 @@ __global__ void __launch_bounds__(128) k_bank_order(int32_t n, int32_t R, int64_
   if (fast)
     for (int k = q; k < len; k += KG) {
       lidx[b + k] = sl[k];
-      pos[b + k] = pos_src ? pos_src[b + so[k]] : b + so[k];
+      pos[b + k] = b + so[k];
     }
 }
 
@@ -786,11 +785,11 @@ __global__ void __launch_bounds__(kHasStress<SA> && KG == 16 ? 512 : 64 * KG,
         L[3 * k] += d[k] * g[0]; L[3 * k + 1] += d[k] * g[1]; L[3 * k + 2] += d[k] * g[2];
       }
       if constexpr (NS) {
-  double sq[6];
-  sr.get(sq);
-  // FP64: du_J itself
-  const double e0 = F64 ? (double)v[0] : (double)d[0], e1 = F64 ? (double)v[1] : (double)d[1],
-               e2 = F64 ? (double)v[2] : (double)d[2];
+        double sq[6];
+        sr.get(sq);
+        // FP64: du_J itself
+        const double e0 = F64 ? (double)v[0] : (double)d[0], e1 = F64 ? (double)v[1] : (double)d[1],
+                     e2 = F64 ? (double)v[2] : (double)d[2];
 #pragma unroll
         for (int c = 0; c < 6; ++c) { H[c] += sq[c] * e0; H[6 + c] += sq[c] * e1; H[12 + c] += sq[c] * e2; }
       }
@@ -806,7 +805,7 @@ __global__ void __launch_bounds__(kHasStress<SA> && KG == 16 ? 512 : 64 * KG,
     // Each lane sums its entries in list order.  Where the registers allow
     // (kPipe) the next KU records are requested before this KU's sums, so a
     // lane keeps loads in flight while it computes.
-      int it = 0;
+    int it = 0;
     while (have) {
       const bool hn = it + 2 * KU <= nit;
       Rec<F64> nxt[KU];
@@ -835,8 +834,8 @@ __global__ void __launch_bounds__(kHasStress<SA> && KG == 16 ? 512 : 64 * KG,
       Rec<F64> rec;
       load_rec(pk, sv.nrec, walk.at(it), rec);
       SRec<F64> sr;
-    if constexpr (NS) sr.load(ns.srow, sv.nrec, walk.at(it));
-    body(it, rec, sr);
+      if constexpr (NS) sr.load(ns.srow, sv.nrec, walk.at(it));
+      body(it, rec, sr);
     }
 #pragma unroll
     for (int o = 1; o < KG; o <<= 1) {
@@ -863,7 +862,8 @@ __global__ void __launch_bounds__(kHasStress<SA> && KG == 16 ? 512 : 64 * KG,
 #pragma unroll
         for (int k = 0; k < 3; ++k)
 #pragma unroll
-          for (int c = 0; c < 6; ++c) ns.hq[(6 * k + c) * fg_ld(n) + i] = F64 ? H[6 * k + c] : H[6 * k + c] + di[k] * ss[c];
+          for (int c = 0; c < 6; ++c)
+            ns.hq[(6 * k + c) * fg_ld(n) + i] = F64 ? H[6 * k + c] : H[6 * k + c] + di[k] * ss[c];
       }
       const double sd3[3] = {sdphi[3 * i], sdphi[3 * i + 1], sdphi[3 * i + 2]};
       const int64_t ld = fg_ld(n);
@@ -1090,7 +1090,7 @@ constexpr int force_blocks() {  // blocks per SM the register cap asks for (NS: 
 }
 
 // TS = storage of T_i (float / double), A = accumulation, F64 = record width
-// NS (mixed): the NSNI stabilisation force rides along,
+// NS: the NSNI stabilisation force rides along,
 // f_J += sum_i sum_q W_i(k, q) S_q(i, J) (FINT.F90:1127-1208 layout), with the
 // row weights W_i staged beside T_i.
 // BODY: a body force (compiled apart: its sums and branches cost registers the
@@ -1165,7 +1165,7 @@ __global__ void __launch_bounds__(64 * KG, force_blocks<F64, KG, KU, NS>()) k_fo
         }
       }
     };
-      int it = 0;
+    int it = 0;
     while (have) {  // as in the row gather
       const bool hn = it + 2 * KU <= nit;
       Rec<F64> nxt[KU];
@@ -1580,13 +1580,13 @@ int pad_records32(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* p
 }
 
 int bank_order(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* ptr, uint16_t* lidx,
-               const int64_t* pos_src, int64_t* pos, int lanes) {
+               int64_t* pos, int lanes) {
   if (n <= 0) return 0;
   if ((lanes != 4 && lanes != 8) || ts.R * lanes < 32) return MEGA_ERR_UNSUPPORTED;
   const int64_t nwarps = ts.ntiles * (int64_t)(ts.R * lanes / 32);
   const unsigned grid = (unsigned)((nwarps * 32 + 127) / 128);
-  if (lanes == 4) k_bank_order<4, 8, 8><<<grid, 128, 0, s>>>(n, ts.R, nwarps, ts.ord, ptr, lidx, pos_src, pos);
-  else k_bank_order<8, 8, 8><<<grid, 128, 0, s>>>(n, ts.R, nwarps, ts.ord, ptr, lidx, pos_src, pos);
+  if (lanes == 4) k_bank_order<4, 8, 8><<<grid, 128, 0, s>>>(n, ts.R, nwarps, ts.ord, ptr, lidx, pos);
+  else k_bank_order<8, 8, 8><<<grid, 128, 0, s>>>(n, ts.R, nwarps, ts.ord, ptr, lidx, pos);
   MEGA_CHECK_LAUNCH();
   return 0;
 }

@@ -15,7 +15,7 @@ struct SliceView {
 };
 
 struct TileSet {
-  int32_t R = 0;           // rows (columns) per tile; the kernels run R*4 threads per tile
+  int32_t R = 0;           // rows (columns) per tile; the kernels run 4, 8 or 16 threads per row
   int64_t ntiles = 0;
   int32_t jmax = 0;        // stride of jset per tile
   int32_t maxcnt = 0;      // largest neighbour set of any tile
@@ -102,10 +102,9 @@ int pad_records32(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* p
 // lanes of a warp of a gather with `lanes` (4 or 8) lanes per row read
 // distinct shared-memory banks of the staged neighbour data (16-byte vectors
 // by rank) where possible.  lidx is reordered in place;
-// pos[e] receives pos_src (or, when null, the identity) at the entry's
-// position before, and must hold that same array on entry.
+// pos, the identity on entry, receives each entry's position before.
 int bank_order(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* ptr, uint16_t* lidx,
-               const int64_t* pos_src, int64_t* pos, int lanes);
+               int64_t* pos, int lanes);
 // out[e] = e;  entry e takes the record of entry pos[e] of its row
 int iota64(cudaStream_t s, int64_t m, int64_t* out);
 int gather_records(cudaStream_t s, int32_t n, const TileSet& ts, const int64_t* ptr, const int64_t* pos, bool f64,
