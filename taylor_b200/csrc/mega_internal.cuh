@@ -86,7 +86,8 @@ void cached_free(void* p, size_t block_bytes, cudaStream_t s);
 struct DevPool {
   std::vector<void*> ptrs;
   std::vector<size_t> blocks;  // block size of each pointer (bound pools)
-  int64_t bytes = 0;
+  std::vector<int64_t> sizes;  // what was asked for
+  int64_t bytes = 0;           // their sum
   cudaStream_t stream = nullptr;
   bool ordered = false;
   DevPool() = default;
@@ -123,7 +124,8 @@ struct DevPool {
     }
     ptrs.push_back((void*)*p);
     blocks.push_back(blk);
-    bytes += (int64_t)(count * sizeof(T));
+    sizes.push_back((int64_t)(count * sizeof(T)));
+    bytes += sizes.back();
     return 0;
   }
   void drop(void* p, size_t blk) {
@@ -134,8 +136,10 @@ struct DevPool {
     for (size_t k = 0; k < ptrs.size(); ++k)
       if (ptrs[k] == p) {
         drop(p, blocks[k]);
+        bytes -= sizes[k];
         ptrs.erase(ptrs.begin() + k);
         blocks.erase(blocks.begin() + k);
+        sizes.erase(sizes.begin() + k);
         return;
       }
   }
@@ -144,16 +148,19 @@ struct DevPool {
     for (size_t k = 0; k < o.ptrs.size(); ++k) {
       ptrs.push_back(o.ptrs[k]);
       blocks.push_back(o.blocks[k]);
+      sizes.push_back(o.sizes[k]);
     }
     bytes += o.bytes;
     o.ptrs.clear();
     o.blocks.clear();
+    o.sizes.clear();
     o.bytes = 0;
   }
   void free_all() {
     for (size_t k = 0; k < ptrs.size(); ++k) drop(ptrs[k], blocks[k]);
     ptrs.clear();
     blocks.clear();
+    sizes.clear();
     bytes = 0;
   }
   ~DevPool() { free_all(); }

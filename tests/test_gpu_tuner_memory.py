@@ -32,3 +32,16 @@ def test_autotune_without_room_for_reordered_records():
         m.close()
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("mode", ["fp64", "mixed"])
+def test_device_bytes_after_the_tuner(mode):
+    """The reordered records take the place of the ones before: the context holds
+    one array more, the interpolation's shape values in the records' order."""
+    c = cases.taylor_bar(h=0.5e-3)
+    m = mega.Mega(c, _lib.params(**cases.param_kwargs(c)))
+    nnz = m.search_and_shapes()["nnz"]
+    held = m.device_bytes()
+    m.autotune(cases.lattice_dt(c, 0.3), mode=mode, reps=1)
+    assert m.device_bytes() == held + 8 * nnz
+    m.close()
