@@ -649,6 +649,19 @@ __device__ __forceinline__ void stage_disp(const StageIds<KG>& ids, int cnt, con
   });
 }
 
+// The sums of a step, cleared by the first 32 threads of a block: a tile of 8
+// rows has no more (a loop over the slots cost the joined kernels spills).
+template <typename T>
+__device__ __forceinline__ void clear_slots(T* v) {
+  static_assert(kSlots == 64, "two a thread");
+  v[threadIdx.x] = T(0);
+  v[threadIdx.x + 32] = T(0);
+}
+__device__ __forceinline__ void clear_counts(StepAccum* acc) {
+  clear_slots(acc->newton_iters);
+  clear_slots(acc->plastic);
+}
+
 // FULL: F - I is formed besides G0.  Without it the gather stages and reads
 // the increments alone, half the shared-memory traffic and sums: at 130 k nodes
 // FP64 ran at 75 % of the L1 data pipe with both, half of it staged reads.
@@ -718,16 +731,10 @@ __global__ void __launch_bounds__(kHasStress<SA> && KG == 16 ? 512 : 64 * KG,
     }
   }
   grid_wait();
-  if (acc && blockIdx.x == 0) {
-    for (int k = threadIdx.x; k < kSlots; k += blockDim.x) {  // (a tile of 8 rows has 32 threads)
-      if constexpr (kHasStress<SA>) {
-        // (no counts of this step alone: a call's last step is not one of these)
-        acc->ke[k] = 0.0;
-      } else {
-        acc->newton_iters[k] = 0ull;
-        acc->plastic[k] = 0ull;
-      }
-    }
+  if (acc && blockIdx.x == 0 && threadIdx.x < 32) {
+    // (no counts of this step alone where it joins: a call's last step is not one of these)
+    if constexpr (kHasStress<SA>) clear_slots(acc->ke);
+    else clear_counts(acc);
   }
   double ur[3] = {0.0, 0.0, 0.0}, dr[3] = {0.0, 0.0, 0.0};
   if (!F64) {
@@ -1313,12 +1320,7 @@ __global__ void __launch_bounds__(64 * KG)
   const unsigned gmask = group_mask<KG>();
   const bool valid = i < n;
   grid_wait();
-  if (acc && blockIdx.x == 0) {
-    for (int k = threadIdx.x; k < kSlots; k += blockDim.x) {
-      acc->newton_iters[k] = 0ull;
-      acc->plastic[k] = 0ull;
-    }
-  }
+  if (acc && blockIdx.x == 0 && threadIdx.x < 32) clear_counts(acc);
   double dr[3] = {0.0, 0.0, 0.0};
   if (!F64) {
 #pragma unroll
