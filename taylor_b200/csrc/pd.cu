@@ -435,7 +435,8 @@ __global__ void k_pmb_extent(int32_t n, const double* __restrict__ X, unsigned l
   for (int o = 16; o > 0; o >>= 1) b = max(b, __shfl_xor_sync(0xffffffffu, b, o));
   if ((threadIdx.x & 31) == 0 && b) atomicMax(ext, b);
 }
-// warp per row; *shortest starts at infinity
+// (in the maximum norm, at most the length); warp per row; *shortest starts at
+// infinity
 __global__ void k_pmb_shortest(int32_t n, const double* __restrict__ X, const int64_t* __restrict__ rowptr,
                                const int32_t* __restrict__ col, unsigned long long* shortest) {
   const int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
@@ -443,8 +444,8 @@ __global__ void k_pmb_shortest(int32_t n, const double* __restrict__ X, const in
   double least = INFINITY;
   for (int64_t p = rowptr[r] + (threadIdx.x & 31); p < rowptr[r + 1]; p += 32) {
     const int64_t j = col[p];
-    const double x = X[3 * j] - X[3 * r], y = X[3 * j + 1] - X[3 * r + 1], z = X[3 * j + 2] - X[3 * r + 2];
-    const double d = sqrt(x * x + y * y + z * z);
+    const double d = fmax(fabs(X[3 * j] - X[3 * r]),
+                          fmax(fabs(X[3 * j + 1] - X[3 * r + 1]), fabs(X[3 * j + 2] - X[3 * r + 2])));
     if (d > 0.0) least = fmin(least, d);
   }
   unsigned long long b = (unsigned long long)__double_as_longlong(least);
@@ -570,14 +571,16 @@ __global__ void __launch_bounds__(512, WIDE ? 2 : 3) k_pmb_step_f32(PmbArgs a) {
     for (int g = 0; g < 4; ++g) {
       if (g >= ng) break;
       const int lj = (int)(((g < 2 ? rc.x : rc.y) >> (16 * (g & 1))) & 0xFFFFu);
-      const float4 B = sb[lj];
       float x0, x1, x2;
+      float4 B;
       if constexpr (WIDE) {
+        B = sb[lj];
         x0 = (float)(sx[lj] - Xi0);
         x1 = (float)(sx[cnt + lj] - Xi1);
         x2 = (float)(sz[lj] - Xi2);
       } else {
         const float4 A = sa[lj];
+        B = sb[lj];
         const float2 C = sc2[lj];
         x0 = (A.x - hi.x) + (C.x - lo.x);
         x1 = (A.y - hi.y) + (C.y - lo.y);

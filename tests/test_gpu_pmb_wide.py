@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 H = 0.5e-3
 
 
-@pytest.mark.parametrize("far", [None, 120.0, 140.0, 2.0 ** 16 * 3.015])  # in H; pairs are H / 2^13 apart
+@pytest.mark.parametrize("far", [None, 60.0, 140.0, 2.0 ** 16 * 3.015])  # in H; pairs are H / 2^13 apart
 def test_short_bonds_match_fp64(far):
     c = cases.pd_plate(h=H, nx=17, ny=9, nz=3, horizon=3.015, jitter=0.2, s_c=1e9)
     rng = np.random.default_rng(4)
