@@ -267,13 +267,16 @@ void host_parallel(int64_t n, F fn, int64_t grain = 65536) {
 // 4 MiB pieces and each piece moves with its own DMA as soon as it is there
 // (downloads the other way round), instead of the driver staging pageable
 // memory on the calling thread.  One user at a time; a failed pinned
-// allocation falls back to plain pageable copies.
+// allocation falls back to plain pageable copies.  It holds a context's node
+// arrays at set-up; drop-in calls and downloads go in rounds and grow it to
+// kStageMost at most.  mega_release_cached_memory gives it back.
 struct PinnedStage {
   std::mutex mu;
   unsigned char* p = nullptr;
   size_t cap = 0;
 };
 PinnedStage g_stage;
+constexpr size_t kStageMost = (size_t)128 << 20;
 
 // one array to upload: copied from src, or written by fill(staging) when
 // the host array is formed on the way (fill writes `bytes` bytes)
@@ -362,11 +365,12 @@ int download_parts(cudaStream_t s, const void* src, const std::vector<HostPart>&
     }
   };
   std::lock_guard<std::mutex> lk(g_stage.mu);
-  if (g_stage.cap < bytes) {
+  const size_t want = std::min(bytes, kStageMost);
+  if (g_stage.cap < want) {
     if (g_stage.p) cudaFreeHost(g_stage.p);
     g_stage.p = nullptr;
     g_stage.cap = 0;
-    if (cudaHostAlloc((void**)&g_stage.p, bytes, cudaHostAllocDefault) == cudaSuccess) g_stage.cap = bytes;
+    if (cudaHostAlloc((void**)&g_stage.p, want, cudaHostAllocDefault) == cudaSuccess) g_stage.cap = want;
     else { g_stage.p = nullptr; cudaGetLastError(); }
   }
   if (!g_stage.p) {
@@ -378,35 +382,39 @@ int download_parts(cudaStream_t s, const void* src, const std::vector<HostPart>&
     MEGA_TRY(cudaStreamSynchronize(s));
     return 0;
   }
-  // 4 MiB pieces, each copied out by a pool thread as soon as its DMA is done
+  // rounds of what the stage holds, in 4 MiB pieces, each copied out by a pool
+  // thread as soon as its DMA is done
   constexpr size_t kPiece = (size_t)4 << 20;
-  const int64_t np = (int64_t)((bytes + kPiece - 1) / kPiece);
-  std::vector<cudaEvent_t> ev(np, nullptr);
   int r = 0;
-  for (int64_t k = 0; k < np && !r; ++k) {
-    const size_t a = (size_t)k * kPiece, len = std::min(kPiece, bytes - a);
-    if (cudaMemcpyAsync(g_stage.p + a, (const unsigned char*)src + a, len, cudaMemcpyDeviceToHost, s) !=
-            cudaSuccess ||
-        cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventRecord(ev[k], s) != cudaSuccess)
+  for (size_t base = 0; base < bytes && !r; base += g_stage.cap) {
+    const size_t held = std::min(g_stage.cap, bytes - base);
+    const int64_t np = (int64_t)((held + kPiece - 1) / kPiece);
+    std::vector<cudaEvent_t> ev(np, nullptr);
+    for (int64_t k = 0; k < np && !r; ++k) {
+      const size_t a = (size_t)k * kPiece, len = std::min(kPiece, held - a);
+      if (cudaMemcpyAsync(g_stage.p + a, (const unsigned char*)src + base + a, len, cudaMemcpyDeviceToHost, s) !=
+              cudaSuccess ||
+          cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming) != cudaSuccess ||
+          cudaEventRecord(ev[k], s) != cudaSuccess)
+        r = MEGA_ERR_CUDA;
+    }
+    std::atomic<int> bad(0);
+    if (!r)
+      host_parallel(np, [&](int64_t lo, int64_t hi) {
+        for (int64_t k = lo; k < hi; ++k) {
+          const size_t a = (size_t)k * kPiece, len = std::min(kPiece, held - a);
+          if (cudaEventSynchronize(ev[k]) != cudaSuccess) { bad.store(1); continue; }
+          scatter(base + a, len, g_stage.p + a);
+        }
+      }, 1);
+    if (r || bad.load()) {
+      cudaStreamSynchronize(s);  // no DMA may still write the stage
+      record_cuda_error(cudaGetLastError(), "download_parts", __FILE__, __LINE__);
       r = MEGA_ERR_CUDA;
+    }
+    for (auto e : ev)
+      if (e) cudaEventDestroy(e);
   }
-  std::atomic<int> bad(0);
-  if (!r)
-    host_parallel(np, [&](int64_t lo, int64_t hi) {
-      for (int64_t k = lo; k < hi; ++k) {
-        const size_t a = (size_t)k * kPiece, len = std::min(kPiece, bytes - a);
-        if (cudaEventSynchronize(ev[k]) != cudaSuccess) { bad.store(1); continue; }
-        scatter(a, len, g_stage.p + a);
-      }
-    }, 1);
-  if (r || bad.load()) {
-    cudaStreamSynchronize(s);  // no DMA may still write the stage
-    record_cuda_error(cudaGetLastError(), "download_parts", __FILE__, __LINE__);
-    r = MEGA_ERR_CUDA;
-  }
-  for (auto e : ev)
-    if (e) cudaEventDestroy(e);
   return r;
 }
 
@@ -414,16 +422,14 @@ int download_staged(cudaStream_t s, void* dst, const void* src, size_t bytes) {
   return download_parts(s, src, {{dst, bytes}});
 }
 
-// upload_staged in batches of at most 128 MiB of staging (lists of a large
-// model; the staging buffer stays with the process)
+// upload_staged in batches of at most kStageMost (lists of a large model)
 static int upload_batched(cudaStream_t s, const std::vector<HostToDevice>& items) {
-  constexpr size_t kMost = (size_t)128 << 20;
   std::vector<HostToDevice> batch;
   size_t held = 0;
   for (const auto& it : items)
     for (size_t at = 0; at < it.bytes || (at == 0 && it.fill);) {
-      const size_t len = it.fill ? it.bytes : std::min(it.bytes - at, kMost);
-      if (held + len > kMost && !batch.empty()) {
+      const size_t len = it.fill ? it.bytes : std::min(it.bytes - at, kStageMost);
+      if (held + len > kStageMost && !batch.empty()) {
         if (int r = upload_staged(s, batch)) return r;
         batch.clear();
         held = 0;
@@ -2563,6 +2569,12 @@ int mega_release_cached_memory(void) {
     for (const auto& kv : g_blk) devs.insert(kv.second.dev);
   }
   int rc = 0;
+  {
+    std::lock_guard<std::mutex> lk(g_stage.mu);
+    if (g_stage.p && cudaFreeHost(g_stage.p) != cudaSuccess) { cudaGetLastError(); rc = MEGA_ERR_CUDA; }
+    g_stage.p = nullptr;
+    g_stage.cap = 0;
+  }
   for (int dev : devs) {
     cudaStream_t s = nullptr;
     if (cudaSetDevice(dev) != cudaSuccess || make_stream(&s)) { cudaGetLastError(); rc = MEGA_ERR_CUDA; continue; }
