@@ -224,7 +224,11 @@ int mega_constitution(const mega_params* p, int32_t n,
  * (RK1) and written to gstack_shp / gstack_dshp; otherwise they are read.
  * In/out arrays follow FINT.F90: gstress, gstrain (6,n), gstate (20,n).
  * Outputs: fint, fext (3n), gmax_wvel (n), gstrain_eq (n), *gint_work
- * (accumulated, as GINT_WORK is). */
+ * (accumulated, as GINT_WORK is).
+ * The rows of the list may lie anywhere in gstack, in any order and with
+ * places between them: the device holds their entries only.  The call's device
+ * blocks, and up to 128 MiB of pinned host memory, stay with the process for
+ * the next call (mega_release_cached_memory gives both back). */
 int mega_construct_fint(const mega_params* p, int32_t n,
                         const double* gcoo, const double* gwin,
                         const double* gvol, const double* gprop,
@@ -435,10 +439,18 @@ int mega_download(int64_t h, int32_t field, double* dst);
  * layout and the caller's node order (the arrays VTK_OUTPUT.F90 writes at
  * MAIN's output steps, gathered without one round trip per field). */
 int mega_snapshot(int64_t h, int32_t nfields, const int32_t* fields, double* dst);
-/* Replace a field from host memory (DSP_TOT, VEL, ACL, STRESS, STRAIN, EPS). */
+/* Replace a field from host memory (DSP_TOT, VEL, ACL, STRESS, STRAIN, EPS).
+ * A restart from uploaded fields: the steps advance the deformation gradient
+ * by each step's increment and form it from DSP_TOT on every 16th step, and on
+ * the first one after DSP_TOT was uploaded, after a change of precision, and
+ * after a call that failed or reported MEGA_ST_NONFINITE or
+ * MEGA_ST_WAIT_TIMEOUT.  A restarted run repeats the unbroken one bit for bit
+ * where it starts at a multiple of 16 steps of that context; elsewhere the
+ * two differ by the rounding of at most 15 increments (double, or in mixed
+ * precision float). */
 int mega_upload(int64_t h, int32_t field, const double* src);
 int mega_get_scalars(int64_t h, mega_scalars_t* out);
-/* Device bytes held by the context. */
+/* Device bytes held by the context (what was given back left out). */
 int64_t mega_device_bytes(int64_t h);
 /* Number of kernels launched by the context since creation. */
 int64_t mega_kernel_launches(int64_t h);
@@ -501,8 +513,11 @@ int mega_train_surrogate(int64_t h, float* theta, int32_t epochs, int32_t batch,
  * c; critical stretch s_c; density rho; broken0 (nnz) initial broken flags
  * per neighbour-list entry (may be NULL; the list is the SOFT_SEARCH
  * ellipsoidal-support list with window = horizon, as mega_bin_search(...,
- * shsup = 1) returns it).  mode: MEGA_MODE_MIXED = float bond arithmetic,
- * MEGA_MODE_FP64 = double.  *nbonds = list entries (self included). */
+ * shsup = 1) returns it).  mode: MEGA_MODE_MIXED = float bond arithmetic on
+ * bond vectors rounded to float from positions in double, or, where the
+ * extent of coo is at most 2^20 of its shortest bond, in sums of two floats
+ * (to 2^-46 of the extent); MEGA_MODE_FP64 = double.  *nbonds = list entries
+ * (self included). */
 int mega_pmb_init(int32_t n, const double* coo, const double* vol, const double* vinit,
                   const int32_t* fixed, double horizon, double micromodulus, double s_c,
                   double rho, const uint8_t* broken0, int32_t mode, int64_t* handle,
@@ -528,9 +543,11 @@ int mega_gpu_finalize(int64_t h);
  * temporaries and finalised contexts leave their device blocks in a
  * process-wide cache (at most a quarter of each device's memory) and in the
  * device's default memory pool, whose release threshold the library raises
- * to its maximum, so a repeated set-up allocates nothing from the driver.
- * This call hands every cached block to the pool, puts back each device's
- * previous release threshold and trims the pool to what live contexts hold,
+ * to its maximum, so a repeated set-up allocates nothing from the driver; the
+ * stateless calls (mega_construct_fint, mega_bin_search, mega_rk_shapes) leave
+ * theirs there too.  This call hands every cached block to the pool, puts back
+ * each device's previous release threshold and trims the pool to what live
+ * contexts hold, and frees the pinned host buffer the copies go through,
  * for a host program whose own allocator needs the memory.  Contexts stay
  * valid; a later set-up caches again.  Call it with no library call in
  * flight on another thread. */

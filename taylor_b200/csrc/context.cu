@@ -785,10 +785,9 @@ static int step_once(Ctx* c, double dt, int mode, int predict, cudaEvent_t* ev, 
 }
 
 // Rows per tile: 64, or 32 where 64 would leave more than half of the SMs
-// without a tile (one block per tile).  4,455 nodes, 70 -> 140 tiles: FP64
-// step 19.7 -> 18.9 us and 17.4 -> 15.3 tuned, with NSNI 49.2 -> 43.8 and mixed
-// NSNI 35.7 -> 33.3; 7,458 nodes, 117 tiles at 64: FP64 NSNI 53.5 -> 57.2 with
-// 32, the rest within 2 %.  16 rows gained nothing more at 957 to 3,807.
+// without a tile (one block per tile).  4,455 nodes, 70 -> 140 tiles: FP64 NSNI
+// step 49.2 -> 43.8 us, DNI 19.7 -> 18.9; 7,458 nodes, 117 tiles at 64: 53.5 ->
+// 57.2, the rest within 2 %.  16 rows gained nothing more at 957 to 3,807.
 static int32_t tile_rows(int32_t n) { return (int64_t)n <= 32 * (int64_t)device_sm_count() ? 32 : 64; }
 
 static int graph_for(Ctx* c, double dt, int mode, int len) {

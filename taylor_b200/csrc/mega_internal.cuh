@@ -35,16 +35,15 @@ void record_error_text(const char* msg);
 
 // Launches in a row that overlap (programmatic dependent launch): a kernel
 // launched so may start while the last blocks of the kernel before it on the
-// stream drain, which hides its launch and its first loads (1-2 us a kernel:
-// the FP64 step of 4,455 nodes 23.1 -> 21.2 us, the mixed one 18.5 -> 16.3).
+// stream drain, which hides its launch and its first loads (1-2 us a kernel).
 // Such a kernel reads only what the set-up left (records, lists) before
 // grid_wait(), where the kernel before it has completed and its writes are
 // visible, and reads what earlier kernels write with plain loads after it;
 // every thread of every kernel in the row calls grid_wait() once, so the
 // kernels complete in order.  No kernel releases the next one early
 // (griddepcontrol.launch_dependents): waiting blocks beside running ones of
-// another shared-memory size cost more than they hid below 100 k nodes (FP64
-// NSNI of 4,455 nodes 56 -> 89 us) and gained 3 % above.
+// another shared-memory size cost more than they hid (FP64 NSNI of 4,455 nodes 56
+// -> 89 us a step).
 template <typename... KA, typename... A>
 inline int launch_overlapped(void (*k)(KA...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
                              A&&... args) {

@@ -1642,8 +1642,8 @@ constexpr int kFullKU = 2;
 constexpr int kBulkSmemMax = 227 * 1024 - 1024;
 
 // The dynamic shared-memory limit is raised, to the same value by every caller,
-// only for a launch that may pass 48 KB with the kernel's static part (4 KB
-// at most), and a kernel's code is loaded at its first use: raising all of them at set-up loaded all of them (20 ms of a
+// only for a launch that may pass 48 KB with the kernel's static part (4 KB at
+// most): raising it for every kernel at set-up loaded all of them (20 ms of a
 // process's first search).  load_only does both ahead of a stream capture.
 template <typename K>
 static int raise_smem(K k, int lim) {
@@ -1805,14 +1805,12 @@ static int defgrad_stress(cudaStream_t s, const DefgradArgs& d, const StressArgs
 
 // Fetched ahead where a gather's blocks are all resident at once, so that only
 // their own latency counts (steps of 4,455 nodes, FP64 17.3 -> 16.5 us, mixed 13.3
-// -> 12.5; 16,154 nodes 25.4 -> 24.9 and 17.7 -> 17.5; FP64 in the joined row gather
-// alone: the test cost its other gathers 1 %), and mixed where bank-ordered
+// -> 12.5; FP64 in the joined row gather alone), and mixed where the bank-ordered
 // records of both gathers pass the L2 three times, so that they come from HBM
-// (1.04 M nodes: row gather 217 -> 203 us, column gather 288 -> 278, step 601 ->
-// 576; 383 k 243 -> 236; 255 k, four times the L2, 168 -> 164).  In between part of
-// the records is still in L2, and the requests only take its bandwidth: 130 k
-// nodes, twice the L2, step 88 -> 93; FP64 135 -> 148, and at 1.04 M nodes no gain.
-// In list order the gathers wait for bank conflicts instead (383 k 250 -> 253).
+// (1.04 M nodes 601 -> 576; 255 k, four times the L2, 168 -> 164).  In between part
+// of them is still in L2 and the requests only take its bandwidth (130 k nodes,
+// twice the L2, 88 -> 93; FP64 135 -> 148); in list order the gathers wait for bank
+// conflicts instead (383 k 250 -> 253).
 bool records_ahead(const TileSet& ts, bool mixed) {
   static const int64_t l2 = [] {
     int dev = 0, bytes = 0;
@@ -1825,10 +1823,9 @@ bool records_ahead(const TileSet& ts, bool mixed) {
 }
 
 // Joined where every block is resident at once (two of 256 threads an SM, one
-// of 512).  Steps joined and apart: 4,455 nodes FP64 16.6 and 18.3 us, mixed 12.3
-// and 14.5; 16,154 nodes FP64 24.9 and 27.3, mixed 17.5 and 19.9; past the line,
-// where the update's registers cost the gather its warps, 23,782 nodes FP64 38.8
-// and 34.4, mixed 26.8 and 23.1; 129,911 nodes mixed 109 and 90.
+// of 512): joined and apart, 4,455 nodes FP64 16.6 and 18.3 us a step, 16,154 24.9
+// and 27.3; past the line the update's registers cost the gather its warps, 23,782
+// nodes 38.8 and 34.4 (mixed alike).
 bool defgrad_stress_fits(const TileSet& ts, int variant) {
   const int lanes = variant >= 6 ? 16 : (variant == 3 || variant == 5 ? 8 : 4);
   const int threads = ts.R * lanes;
